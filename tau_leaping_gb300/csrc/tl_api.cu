@@ -159,6 +159,37 @@ static size_t slot_bytes(const tl_model* m, bool sens = false) {
     return al16((size_t)m->h.N * w) * 2 + al16((size_t)m->h.M * 4) * (sens ? 2 : 1);
 }
 
+// The slot with its queue of long Poisson draws (pass_fire_queued): a 16-bit
+// channel for each of the four channels that a lane may mark in one turn,
+// times the turns between two drains.  Turns: enough for a whole leap of
+// models up to 32 channels a lane, whose few long draws then fill one pass;
+// four for wide CTA groups, where 128 channels a turn and warp fill a pass
+// sooner and 32 queues take 32 KB.  The queue lies over x', which a leap
+// writes only after it has fired, when x' is large enough; thread groups and
+// the general build have none.
+struct SlotLayout {
+    size_t bytes = 0;    // the slot, with the queue if it is its own
+    size_t q_bytes = 0;  // all of a group's queues
+    int q_off = -1;      // -1: over x'
+    int q_rounds = 0;
+};
+
+static SlotLayout slot_layout(const tl_model* m, bool sens, int mode, int kind, int block) {
+    SlotLayout L;
+    L.bytes = slot_bytes(m, sens);
+    if (mode == kModeGeneral || kind == 1) return L;
+    const size_t w = m->h.pop_bits == 64 ? 8 : 4, xb = al16((size_t)m->h.N * w);
+    const int lanes = kind ? kind : block;
+    const int turns = (m->h.M + 4 * lanes - 1) / (4 * lanes);
+    L.q_rounds = std::min(turns, lanes > 256 ? 4 : 8);
+    L.q_bytes = al16((size_t)L.q_rounds * lanes * 4 * 2);
+    if (xb < L.q_bytes) {
+        L.q_off = (int)L.bytes;
+        L.bytes += L.q_bytes;
+    }
+    return L;
+}
+
 static int max_smem_optin() {
     int dev = 0, v = 0;
     cudaGetDevice(&dev);
@@ -183,6 +214,8 @@ struct Plan {
     int variant = TL_VARIANT_WARP;
     bool row_warp = false;
     bool gslot = false;  // CTA groups: the slot lives in global memory
+    int mode = kModeFast;  // the kernel build
+    SlotLayout slot;
 };
 
 // The kernel a plan launches (CTA groups with global slots are their own build).
@@ -222,7 +255,7 @@ static int heuristic_variant(const tl_model* m, size_t sb, long long total, int 
     return TL_VARIANT_WARP;
 }
 
-static tl_status make_plan(const tl_model* m, int variant, int block_req, int mode, bool compat_stoich,
+static tl_status make_plan(const tl_model* m, int variant, int block_req, int mode, bool sens, bool compat_stoich,
                            bool no_stage, long long total, Plan& pl, bool force_gslot = false) {
     const size_t sb = slot_bytes(m, mode != kModeFast);
     const int smax = max_smem_optin() - 2048;
@@ -267,12 +300,20 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
         return TL_ERR_INVALID_ARGUMENT;
     }
     // shrink the block until the slots fit
-    while ((size_t)groups_per_block * sb > (size_t)smax && pl.kind != 0 && pl.block > 32) {
+    pl.mode = mode;
+    pl.slot = slot_layout(m, sens, mode, pl.kind, pl.block);
+    while ((size_t)groups_per_block * pl.slot.bytes > (size_t)smax && pl.kind != 0 && pl.block > 32) {
         pl.block -= 32;
         groups_per_block = pl.block / pl.kind;
     }
     if (force_gslot && pl.kind == 0) pl.gslot = true;
-    if ((size_t)groups_per_block * sb > (size_t)smax) {
+    if (!pl.gslot && (size_t)groups_per_block * pl.slot.bytes > (size_t)smax && mode != kModeGeneral &&
+        (size_t)groups_per_block * slot_bytes(m, sens) <= (size_t)smax) {
+        // the state fits but not with its queue beside it: the general build
+        pl.mode = kModeGeneral;
+        pl.slot = slot_layout(m, sens, pl.mode, pl.kind, pl.block);
+    }
+    if ((size_t)groups_per_block * pl.slot.bytes > (size_t)smax) {
         if (pl.kind != 0) {
             set_last_error("model too large for the shared-memory slot of this variant");
             return TL_ERR_UNSUPPORTED;
@@ -284,14 +325,18 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
     // chain-sized CTA groups leave the tables in L1/L2 (staging them would
     // cost more shared memory than the realization itself)
     const bool stage_ok = !(autov && pl.kind == 0 && sb <= 64 * 1024);
-    const size_t slot_smem = pl.gslot ? 0 : (size_t)groups_per_block * sb;
+    if (pl.gslot) {  // the queue stays in shared memory
+        pl.slot.bytes = slot_bytes(m, sens);
+        pl.slot.q_off = -1;
+    }
+    const size_t slot_smem = pl.gslot ? pl.slot.q_bytes : (size_t)groups_per_block * pl.slot.bytes;
     pl.stage = (stage_ok && slot_smem + (size_t)stage <= (size_t)smax) ? stage : 0;
     pl.smem = (size_t)pl.stage + slot_smem;
     pl.row_warp = pl.kind == 0 && m->h.max_row > 32;
     int bps = 0;
     const int lk = pl.gslot ? kKindCtaGlobal : pl.kind;
-    cudaError_t e = m->h.pop_bits == 64 ? fused_occupancy<long long>(lk, mode, pl.block, pl.smem, &bps)
-                                        : fused_occupancy<int>(lk, mode, pl.block, pl.smem, &bps);
+    cudaError_t e = m->h.pop_bits == 64 ? fused_occupancy<long long>(lk, pl.mode, pl.block, pl.smem, &bps)
+                                        : fused_occupancy<int>(lk, pl.mode, pl.block, pl.smem, &bps);
     if (e != cudaSuccess) return cuda_fail(e, "occupancy");
     if (bps < 1) {
         set_last_error("the launch does not fit an SM");
@@ -441,7 +486,7 @@ static void job_layout(Job& J, Carver& c) {
     J.o_ps = J.plain ? c.take((size_t)J.total * 64) : 0;
     J.o_pslot = J.plain ? c.take((size_t)J.total * 2 * al16((size_t)N * J.w)) : 0;
     J.o_aall = J.plain ? c.take((size_t)J.total * M * 4) : 0;
-    J.o_gslot = (!J.plain && J.pl.gslot) ? c.take((size_t)J.pl.grid * slot_bytes(J.m, J.mode != kModeFast)) : 0;
+    J.o_gslot = (!J.plain && J.pl.gslot) ? c.take((size_t)J.pl.grid * J.pl.slot.bytes) : 0;
 }
 
 static tl_status job_bind(Job& J, unsigned char* B, cudaStream_t st) {
@@ -510,7 +555,9 @@ static tl_status job_bind(Job& J, unsigned char* B, cudaStream_t st) {
     p.off_vc = m->d.off_vc;
     p.off_cp = m->d.off_cp;
     p.off_rv = m->d.off_rv;
-    p.slot_bytes = (int)slot_bytes(m, J.mode != kModeFast);
+    p.slot_bytes = (int)J.pl.slot.bytes;
+    p.q_off = J.pl.slot.q_off;
+    p.q_rounds = J.pl.slot.q_rounds;
     p.row_warp = J.pl.row_warp ? 1 : 0;
     p.gslots = J.pl.gslot ? B + J.o_gslot : nullptr;
     p.ctr = rb.ctr;
@@ -647,17 +694,20 @@ static tl_status autotune_measure(Job& J, cudaStream_t st) {
         Cand win{0, 0, false};
         for (const Cand& c : cands) {
             Plan pl;
-            if (make_plan(m, c.variant, c.block, J.mode, J.compat_stoich, c.nostage, trial, pl) != TL_OK) continue;
+            if (make_plan(m, c.variant, c.block, J.mode, J.sens, J.compat_stoich, c.nostage, trial, pl) != TL_OK) continue;
             if (c.variant == TL_VARIANT_THREAD && c.block != pl.block) continue;
             // global slots exist for the launch the heuristic planned
             if (pl.gslot && (!planned_gslot || pl.grid > planned_grid)) continue;
             tp.stage_bytes = pl.stage;
             tp.row_warp = pl.row_warp ? 1 : 0;
             tp.gslots = pl.gslot ? planned_gslots : nullptr;
+            tp.slot_bytes = (int)pl.slot.bytes;
+            tp.q_off = pl.slot.q_off;
+            tp.q_rounds = pl.slot.q_rounds;
             if (cudaMemsetAsync(tp.ctr, 0, 64, st) != cudaSuccess) break;
             cudaEventRecord(e0, st);
-            cudaError_t le = J.w == 8 ? launch_fused<long long>(tp, launch_kind(pl), J.mode, pl.block, pl.grid, pl.smem, st)
-                                      : launch_fused<int>(tp, launch_kind(pl), J.mode, pl.block, pl.grid, pl.smem, st);
+            cudaError_t le = J.w == 8 ? launch_fused<long long>(tp, launch_kind(pl), pl.mode, pl.block, pl.grid, pl.smem, st)
+                                      : launch_fused<int>(tp, launch_kind(pl), pl.mode, pl.block, pl.grid, pl.smem, st);
             cudaEventRecord(e1, st);
             if (le != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess) {
                 cudaGetLastError();
@@ -682,19 +732,22 @@ static tl_status autotune_measure(Job& J, cudaStream_t st) {
         m->tuned_block = win.block;
         m->tuned_nostage = win.nostage ? 1 : 0;
     }
-    tl_status ps = make_plan(m, m->tuned_variant, m->tuned_block, J.mode, J.compat_stoich, m->tuned_nostage != 0,
+    tl_status ps = make_plan(m, m->tuned_variant, m->tuned_block, J.mode, J.sens, J.compat_stoich, m->tuned_nostage != 0,
                              J.total, J.pl);
     if (ps != TL_OK) return ps;
     if (J.pl.gslot && (!planned_gslot || J.pl.grid > planned_grid)) {
         // a cached global-slot plan that needs more slots than were laid out:
         // keep the planned launch
-        ps = make_plan(m, TL_VARIANT_AUTO, 0, J.mode, J.compat_stoich, (J.cfg->flags & TL_FLAG_NO_STAGE) != 0,
+        ps = make_plan(m, TL_VARIANT_AUTO, 0, J.mode, J.sens, J.compat_stoich, (J.cfg->flags & TL_FLAG_NO_STAGE) != 0,
                        J.total, J.pl);
         if (ps != TL_OK) return ps;
     }
     J.p.stage_bytes = J.pl.stage;
     J.p.row_warp = J.pl.row_warp ? 1 : 0;
     J.p.gslots = J.pl.gslot ? planned_gslots : nullptr;
+    J.p.slot_bytes = (int)J.pl.slot.bytes;
+    J.p.q_off = J.pl.slot.q_off;
+    J.p.q_rounds = J.pl.slot.q_rounds;
     return TL_OK;
 }
 
@@ -712,7 +765,7 @@ static tl_status run(tl_model* m, const tl_run_cfg* cfg, tl_result* res, tl_grad
     const bool no_stage = (cfg->flags & TL_FLAG_NO_STAGE) != 0;
     const bool measure = !J.plain && cfg->variant == TL_VARIANT_AUTO && (cfg->flags & TL_FLAG_AUTOTUNE_MEASURE);
     if (!J.plain) {
-        ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.compat_stoich, no_stage, J.total, J.pl,
+        ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.sens, J.compat_stoich, no_stage, J.total, J.pl,
                        (cfg->flags & TL_FLAG_GLOBAL_SLOTS) != 0);
         if (ps != TL_OK) return ps;
     } else {
@@ -742,8 +795,8 @@ static tl_status run(tl_model* m, const tl_run_cfg* cfg, tl_result* res, tl_grad
     cudaError_t le = cudaEventRecord(e0, st);
     if (le == cudaSuccess) {
         if (!J.plain) {
-            le = w == 8 ? launch_fused<long long>(p, launch_kind(J.pl), J.mode, J.pl.block, J.pl.grid, J.pl.smem, st)
-                        : launch_fused<int>(p, launch_kind(J.pl), J.mode, J.pl.block, J.pl.grid, J.pl.smem, st);
+            le = w == 8 ? launch_fused<long long>(p, launch_kind(J.pl), J.pl.mode, J.pl.block, J.pl.grid, J.pl.smem, st)
+                        : launch_fused<int>(p, launch_kind(J.pl), J.pl.mode, J.pl.block, J.pl.grid, J.pl.smem, st);
             launches = 1;
         } else {
             le = w == 8 ? launch_plain_init<long long>(p, st) : launch_plain_init<int>(p, st);
@@ -856,17 +909,25 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     // unit kind per item; the warp slot is the largest need
     std::vector<int> lane(n);
     size_t wslot = 0;
-    for (int i = 0; i < n; ++i) {
-        const tl_model* m = jobs[(size_t)i].m;
-        lane[(size_t)i] = (m->h.M <= 16 && m->h.N <= 16) ? 1 : 0;
-        const size_t sbi = slot_bytes(m, jobs[(size_t)i].mode != kModeFast);
-        const size_t need = lane[(size_t)i] ? 32 * sbi : sbi;
-        wslot = std::max(wslot, need);
-        Plan& pl = jobs[(size_t)i].pl;
-        pl.variant = lane[(size_t)i] ? TL_VARIANT_THREAD : TL_VARIANT_WARP;
-    }
-    wslot = al16(wslot);
+    int bmode = kModeFast;  // the build every item can run on
+    for (auto& J : jobs) bmode = std::max(bmode, J.mode);
     const size_t spb = al16(sizeof(SimParams));
+    for (;;) {
+        wslot = 0;
+        for (int i = 0; i < n; ++i) {
+            Job& J = jobs[(size_t)i];
+            const tl_model* m = J.m;
+            lane[(size_t)i] = (m->h.M <= 16 && m->h.N <= 16) ? 1 : 0;
+            Plan& pl = J.pl;
+            pl.variant = lane[(size_t)i] ? TL_VARIANT_THREAD : TL_VARIANT_WARP;
+            pl.slot = slot_layout(m, J.sens, bmode, lane[(size_t)i] ? 1 : 32, 32);
+            wslot = std::max(wslot, lane[(size_t)i] ? 32 * pl.slot.bytes : pl.slot.bytes);
+        }
+        wslot = al16(wslot);
+        // a slot that fits only without its queue takes the general build
+        if (wslot + spb <= (size_t)smax || bmode == kModeGeneral) break;
+        bmode = kModeGeneral;
+    }
     // stage every model's tables when they fit next to 4 warps' slots
     std::vector<tl_model*> uniq;
     for (auto& J : jobs)
@@ -942,8 +1003,6 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     bp.warp_slot_bytes = (int)wslot;
     bp.params_bytes = (int)spb;
     bp.wctr = reinterpret_cast<unsigned long long*>(B + o_wctr);
-    int bmode = kModeFast;  // the build every item can run on
-    for (auto& J : jobs) bmode = std::max(bmode, J.mode);
     const size_t smem = stage + (size_t)warps * (wslot + spb);
     int bps = 0;
     cudaError_t le = pop == 64 ? batch_occupancy<long long>(bmode, 32 * warps, smem, &bps)
@@ -1478,7 +1537,7 @@ extern "C" tl_status tl_simulate_static(tl_model* m, const tl_run_cfg* cfg, tl_r
     if (ps != TL_OK) return ps;
     TLC(cudaSetDevice(m->d.device));
     cudaStream_t st = (cudaStream_t)cfg->stream;
-    ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.compat_stoich,
+    ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.sens, J.compat_stoich,
                    (cfg->flags & TL_FLAG_NO_STAGE) != 0, J.total, J.pl, (cfg->flags & TL_FLAG_GLOBAL_SLOTS) != 0);
     if (ps != TL_OK) return ps;
     Carver c;
@@ -1495,8 +1554,8 @@ extern "C" tl_status tl_simulate_static(tl_model* m, const tl_run_cfg* cfg, tl_r
     ps = job_bind(J, reinterpret_cast<unsigned char*>(base), st);  // clears the counters
     if (ps != TL_OK) return ps;
     const auto tk = std::chrono::steady_clock::now();
-    cudaError_t le = J.w == 8 ? launch_fused<long long>(J.p, launch_kind(J.pl), J.mode, J.pl.block, J.pl.grid, J.pl.smem, st)
-                              : launch_fused<int>(J.p, launch_kind(J.pl), J.mode, J.pl.block, J.pl.grid, J.pl.smem, st);
+    cudaError_t le = J.w == 8 ? launch_fused<long long>(J.p, launch_kind(J.pl), J.pl.mode, J.pl.block, J.pl.grid, J.pl.smem, st)
+                              : launch_fused<int>(J.p, launch_kind(J.pl), J.pl.mode, J.pl.block, J.pl.grid, J.pl.smem, st);
     if (le != cudaSuccess) return cuda_fail(le, "simulation launch");
     ps = job_reduce(J, st);
     if (ps != TL_OK) return ps;

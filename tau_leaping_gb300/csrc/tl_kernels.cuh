@@ -111,6 +111,7 @@ TL_D Slot<Pop> carve_slot(unsigned char* base, const SimParams& p) {
     // scored runs keep the counts apart (their slots hold M more ints)
     s.k = p.scores ? reinterpret_cast<int*>(base + 2 * xb + (((size_t)p.M * 4 + 15) & ~(size_t)15))
                    : reinterpret_cast<int*>(s.a);
+    s.q = p.q_off >= 0 ? reinterpret_cast<unsigned short*>(base + p.q_off) : nullptr;
     return s;
 }
 
@@ -161,6 +162,8 @@ TL_D void run_realization(const Grp& g, const SimParams& p, const MView& mv, Slo
     float* score = (SENS && p.scores) ? p.scores + (size_t)w * p.M : nullptr;
     const Pop* x0 = reinterpret_cast<const Pop*>(p.x0);
     for (int i = g.rank(); i < p.N; i += g.size()) s.x[i] = x0[i];
+    // the padding of the last block of four channels (pass_fire_queued)
+    if (Grp::kWidth != 1 && g.rank() < ((4 - (p.M & 3)) & 3)) s.a[p.M + g.rank()] = 0.f;
     if (SENS && score)
         for (int j = g.rank(); j < p.M; j += g.size()) score[j] = 0.f;
     g.sync();
@@ -235,6 +238,7 @@ __global__ void __launch_bounds__(KIND == 0 ? 1024 : 256, KIND == 0 ? 1 : KIND =
     const Grp g = GroupOf<KIND>::make(red);
     if constexpr (GSLOT) slots = p.gslots + (size_t)blockIdx.x * (size_t)p.slot_bytes;
     Slot<Pop> s = carve_slot<Pop>(slots + (size_t)GroupOf<KIND>::index() * p.slot_bytes, p);
+    if constexpr (GSLOT) s.q = reinterpret_cast<unsigned short*>(smem + p.stage_bytes);
     const long long total = p.R * (long long)p.S;
 
     for (;;) {
