@@ -93,7 +93,7 @@ def _build_lib() -> Path:
         units.append((o, [CXX, *CXXFLAGS, "-c", str(cpp), "-o", str(o)]))
     todo = [(o, c) for o, c in units if _stale(o, deps)]
     if todo:
-        with ThreadPoolExecutor(max_workers=min(8, len(todo))) as ex:
+        with ThreadPoolExecutor(max_workers=min(16, len(todo))) as ex:
             list(ex.map(lambda oc: _run(oc[1]), todo))
     objs = [str(o) for o, _ in units]
     if todo or _stale(LIB, [Path(o) for o in objs]):

@@ -57,6 +57,112 @@ struct Carver {
     }
 };
 
+// Tables of the fast and scores builds, in the layout tl_step.cuh reads:
+//  chan  per channel the byte offsets in X of its two factors: 16 bits each,
+//        or 32 where X is past 64 KB
+//  row   per reacting species, longest row first: {first chunk | chunks << 20,
+//        species | g kind << 28}, a chunk being four entries
+//  ent   row entries: byte offset in a[] << 12 | the stoichiometry's FP32 bits
+//        >> 20, from 2^18 channels on (col << 3) | ((v + 2) & 7); padding
+//        reads the zero block behind the last channel
+//  col   per channel, chunks of four net entries: byte offset of the species
+//        in an int array << 12 | stoichiometry & 0xfff, 0 stoichiometry = none
+//  cp    first chunk of each channel, where a channel needs more than one
+//  sp    per species the index in X of its |x - 1|, 0 if it has none
+static void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned char>& out) {
+    const int N = h.N, M = h.M;
+    std::vector<int> x2((size_t)N, 0);
+    d.n_2s = 0;
+    for (int j = 0; j < M; ++j)
+        if (h.order[(size_t)j] == 3 && !x2[(size_t)h.s0[(size_t)j]]) {
+            x2[(size_t)h.s0[(size_t)j]] = 1;
+            ++d.n_2s;
+        }
+    int next = N;
+    for (int i = 0; i < N; ++i)
+        if (x2[(size_t)i]) x2[(size_t)i] = next++;
+    const int one = N + d.n_2s;
+    const int pad = (M + 3) & ~3;  // the zero block behind a[]
+    d.chan8 = (size_t)one * 4 > 0xffff;
+    d.ent_wide = M + 8 > (1 << 18);
+    d.fast_ok = false;
+    if (N >= (1 << 18) || next > 0xffff || M >= (1 << 28) - 8) return;
+    size_t ent_chunks = 0, col_chunks = 0;
+    int max_chunks = 0, max_col = 0;
+    for (int i = 0; i < N; ++i) {
+        const int n = (h.net_rp[(size_t)i + 1] - h.net_rp[(size_t)i] + 3) / 4;
+        if (h.gkind[(size_t)i]) ent_chunks += (size_t)n;
+        max_chunks = std::max(max_chunks, n);
+    }
+    for (int j = 0; j < M; ++j) max_col = std::max(max_col, h.net_cp[(size_t)j + 1] - h.net_cp[(size_t)j]);
+    if (ent_chunks >= (1u << 20) || max_chunks >= (1 << 12)) return;
+    for (int j = 0; j < M; ++j)
+        col_chunks += max_col <= 4 ? 1 : (size_t)(h.net_cp[(size_t)j + 1] - h.net_cp[(size_t)j] + 3) / 4;
+    d.n_rows = 0;
+    for (int i = 0; i < N; ++i) d.n_rows += h.gkind[(size_t)i] != 0;
+    size_t off = 0;
+    const auto sect = [&](size_t bytes) {
+        const size_t o = off;
+        off += al16(bytes);
+        return (int)o;
+    };
+    d.t_chan = sect((size_t)M * (d.chan8 ? 8 : 4));
+    d.t_row = sect((size_t)d.n_rows * 8);
+    d.t_ent = sect(ent_chunks * 16);
+    d.t_col = sect(col_chunks * 16);
+    d.t_cp = max_col > 4 ? sect((size_t)(M + 1) * 4) : -1;
+    d.t_sp = sect((size_t)N * 2);
+    if (off >= (1u << 31)) return;
+    d.f_stage_bytes = (int)std::max<size_t>(off, 16);
+    out.assign((size_t)d.f_stage_bytes, 0);
+    uint32_t* chan = reinterpret_cast<uint32_t*>(out.data() + d.t_chan);
+    for (int j = 0; j < M; ++j) {
+        const int o = h.order[(size_t)j], s0 = h.s0[(size_t)j], s1 = h.s1[(size_t)j];
+        const uint32_t f0 = 4u * (uint32_t)(o == 0 ? one : s0);
+        const uint32_t f1 = 4u * (uint32_t)(o == 2 ? s1 : o == 3 ? x2[(size_t)s0] : one);
+        if (d.chan8) {
+            chan[2 * (size_t)j] = f0;
+            chan[2 * (size_t)j + 1] = f1;
+        } else {
+            chan[j] = f0 | f1 << 16;
+        }
+    }
+    uint32_t* row = reinterpret_cast<uint32_t*>(out.data() + d.t_row);
+    uint32_t* ent = reinterpret_cast<uint32_t*>(out.data() + d.t_ent);
+    size_t e = 0;
+    int nr = 0;
+    for (int ii = 0; ii < N; ++ii) {
+        const int i = h.rowperm[(size_t)ii];
+        if (!h.gkind[(size_t)i]) continue;
+        const int q0 = h.net_rp[(size_t)i], q1 = h.net_rp[(size_t)i + 1], n = (q1 - q0 + 3) / 4;
+        row[2 * nr] = (uint32_t)(e / 4) | (uint32_t)n << 20;
+        row[2 * nr + 1] = (uint32_t)i | (uint32_t)h.gkind[(size_t)i] << 28;
+        ++nr;
+        for (int q = q0; q < q0 + 4 * n; ++q) {
+            const int c = q < q1 ? unpack_idx(h.net_vc[(size_t)q]) : pad, v = q < q1 ? unpack_v(h.net_vc[(size_t)q]) : 0;
+            const float vf = (float)v;
+            uint32_t vb;
+            memcpy(&vb, &vf, 4);
+            ent[e++] = d.ent_wide ? (uint32_t)c << 3 | (uint32_t)((v + 2) & 7) : (uint32_t)c << 14 | vb >> 20;
+        }
+    }
+    uint32_t* col = reinterpret_cast<uint32_t*>(out.data() + d.t_col);
+    uint32_t* cp = d.t_cp >= 0 ? reinterpret_cast<uint32_t*>(out.data() + d.t_cp) : nullptr;
+    size_t c4 = 0;
+    for (int j = 0; j < M; ++j) {
+        const int q0 = h.net_cp[(size_t)j], q1 = h.net_cp[(size_t)j + 1];
+        if (cp) cp[j] = (uint32_t)c4;
+        for (int q = q0; q < q1; ++q)
+            col[4 * c4 + (size_t)(q - q0)] = (uint32_t)unpack_idx(h.net_rv[(size_t)q]) << 14 |
+                                            ((uint32_t)unpack_v(h.net_rv[(size_t)q]) & 0xfffu);
+        c4 += cp ? (size_t)(q1 - q0 + 3) / 4 : 1;
+    }
+    if (cp) cp[M] = (uint32_t)c4;
+    unsigned short* sp = reinterpret_cast<unsigned short*>(out.data() + d.t_sp);
+    for (int i = 0; i < N; ++i) sp[i] = (unsigned short)x2[(size_t)i];
+    d.fast_ok = true;
+}
+
 static tl_status upload(tl_model* m) {
     HostModel& h = m->h;
     DevModel& d = m->d;
@@ -96,8 +202,15 @@ static tl_status upload(tl_model* m) {
     if (d.nnz_net) memcpy(hb.data() + d.off_rv, h.net_rv.data(), (size_t)d.nnz_net * 4);
     memcpy(hb.data() + d.off_raw_rp, h.raw_rp.data(), (size_t)(N + 1) * 4);
     if (d.nnz_raw) memcpy(hb.data() + d.off_raw_vc, h.raw_vc.data(), (size_t)d.nnz_raw * 4);
-    TLC(cudaMalloc(&d.blob, off));
-    TLC(cudaMemcpy(d.blob, hb.data(), off, cudaMemcpyHostToDevice));
+    // both table sets in one allocation and one copy
+    std::vector<unsigned char> fb;
+    fast_tables(h, d, fb);
+    const size_t f_off = off;
+    hb.resize(off + fb.size());
+    if (!fb.empty()) memcpy(hb.data() + f_off, fb.data(), fb.size());
+    TLC(cudaMalloc(&d.blob, hb.size()));
+    d.fblob = d.blob + f_off;
+    TLC(cudaMemcpy(d.blob, hb.data(), hb.size(), cudaMemcpyHostToDevice));
     const size_t w = h.pop_bits == 64 ? 8 : 4;
     TLC(cudaMalloc(&d.x0, (size_t)N * w));
     if (w == 8) {
@@ -159,34 +272,41 @@ static size_t slot_bytes(const tl_model* m, bool sens = false) {
     return al16((size_t)m->h.N * w) * 2 + al16((size_t)m->h.M * 4) * (sens ? 2 : 1);
 }
 
-// The slot with its queue of long Poisson draws (pass_fire_queued): a 16-bit
-// channel for each of the four channels that a lane may mark in one turn,
-// times the turns between two drains.  Turns: enough for a whole leap of
-// models up to 32 channels a lane, whose few long draws then fill one pass;
-// four for wide CTA groups, where 128 channels a turn and warp fill a pass
-// sooner and 32 queues take 32 KB.  The queue lies over x', which a leap
-// writes only after it has fired, when x' is large enough; thread groups and
-// the general build have none.
+// The slot of the fast and scores builds (tl_step.cuh): the state x, D and X,
+// with the queue of long draws over X, then a[] and in scored runs the counts
+// and, where they fit, the scores.  The queue takes a 16-bit channel for each
+// of the four channels that a lane may mark in one turn, times the turns
+// between two drains: enough for a whole leap of models up to 28 channels a
+// lane, whose few long draws then fill one pass; four for wide CTA groups,
+// where 128 channels a turn and warp fill a pass sooner.
 struct SlotLayout {
-    size_t bytes = 0;    // the slot, with the queue if it is its own
-    size_t q_bytes = 0;  // all of a group's queues
-    int q_off = -1;      // -1: over x'
+    size_t bytes = 0;  // the whole slot
+    size_t state = 0;  // its state part
+    int f_D = 0, f_X = 0, f_a = 0;
     int q_rounds = 0;
+    bool score_global = false;
 };
 
-static SlotLayout slot_layout(const tl_model* m, bool sens, int mode, int kind, int block) {
+static SlotLayout slot_layout(const tl_model* m, int mode, int kind, int block) {
     SlotLayout L;
-    L.bytes = slot_bytes(m, sens);
-    if (mode == kModeGeneral || kind == 1) return L;
-    const size_t w = m->h.pop_bits == 64 ? 8 : 4, xb = al16((size_t)m->h.N * w);
-    const int lanes = kind ? kind : block;
-    const int turns = (m->h.M + 4 * lanes - 1) / (4 * lanes);
-    L.q_rounds = std::min(turns, lanes > 256 ? 4 : 8);
-    L.q_bytes = al16((size_t)L.q_rounds * lanes * 4 * 2);
-    if (xb < L.q_bytes) {
-        L.q_off = (int)L.bytes;
-        L.bytes += L.q_bytes;
+    const int N = m->h.N, M = m->h.M;
+    if (mode == kModeGeneral) {
+        L.bytes = slot_bytes(m, true);
+        return L;
     }
+    const size_t w = m->h.pop_bits == 64 ? 8 : 4;
+    size_t q_bytes = 0;
+    if (kind != 1) {
+        const int lanes = kind ? kind : block;
+        const int turns = (M + 4 * lanes - 1) / (4 * lanes);
+        L.q_rounds = std::min(turns, lanes > 256 ? 4 : 7);
+        q_bytes = (size_t)L.q_rounds * lanes * 4 * 2 + 4 * (size_t)(kind ? 1 : block / 32);  // and a counter each
+    }
+    L.f_D = (int)al16((size_t)N * w);
+    L.f_X = L.f_D + (int)al16((size_t)N * 4);
+    L.state = (size_t)L.f_X + al16(std::max((size_t)(N + m->d.n_2s + 1) * 4, q_bytes));
+    L.f_a = ((M + 3) / 4 * 4 + 4) * 4;
+    L.bytes = L.state + (size_t)L.f_a * (mode == kModeScores ? 3 : 1);
     return L;
 }
 
@@ -215,11 +335,18 @@ struct Plan {
     bool row_warp = false;
     bool gslot = false;  // CTA groups: the slot lives in global memory
     int mode = kModeFast;  // the kernel build
+    int lanes = 32;        // thread groups: lanes of a warp that take realizations
+    int thin = 1;          // and lanes of one realization
+    bool state_global = false;  // global slots: the state as well as a[]
     SlotLayout slot;
 };
 
 // The kernel a plan launches (CTA groups with global slots are their own build).
-static int launch_kind(const Plan& pl) { return pl.gslot ? kKindCtaGlobal : pl.kind; }
+static int launch_kind(const Plan& pl) {
+    if (pl.gslot) return kKindCtaGlobal;
+    if (pl.kind == 1 && pl.mode != kModeGeneral) return pl.thin == 4 ? kKindThin4 : kKindThin1;
+    return pl.kind;
+}
 
 // Autotuner, heuristic part: the group width follows the model size.
 //  * a handful of channels: one realization per thread (all lanes busy on
@@ -255,11 +382,32 @@ static int heuristic_variant(const tl_model* m, size_t sb, long long total, int 
     return TL_VARIANT_WARP;
 }
 
-static tl_status make_plan(const tl_model* m, int variant, int block_req, int mode, bool sens, bool compat_stoich,
+// Thin groups: lanes per realization (W), and lanes of each warp that take
+// realizations.  One realization's chain of dependent steps sets the time of
+// small and mid-sized ensembles, so four lanes share its channels' draws until
+// about 16 such warps per SM are busy; past that the lanes do more as four
+// realizations.  And the realizations of a warp lengthen one another's chains
+// (they sit in different steps, branches and draws), so small ensembles leave
+// lanes idle while that keeps the warps of an SM below about ten.  Measured on
+// GB300, dimer decay to t = 10 (ms):
+//   realizations        32    1000   3000   10000  30000  100000
+//   W = 1, 32 lanes    5.11   5.19   5.20   5.21   5.62    8.95
+//   W = 4, 32 lanes    3.08   3.11   3.12   3.45   6.94   15.85
+//   W = 4, 8 lanes     2.43   2.47   2.78   6.10  15.16   47.86
+//   W = 4, 4 lanes     2.20   2.35   3.02   9.38  25.90   84.12
+// and a 12 x 16 network in direct-method steps 4.67 against 5.91 at 10000 and
+// 10.3 against 6.5 at 50000 (W = 4 against 1).
+static void thin_plan(long long total, int nsm, int& thin, int& lanes) {
+    thin = total <= (long long)nsm * 16 * 8 ? 4 : 1;
+    lanes = 32;
+    if (thin == 4)
+        while (lanes > 4 && total * 8 / lanes <= 10LL * nsm) lanes /= 2;
+}
+
+static tl_status make_plan(const tl_model* m, int variant, int block_req, int mode, bool compat_stoich,
                            bool no_stage, long long total, Plan& pl, bool force_gslot = false) {
     const size_t sb = slot_bytes(m, mode != kModeFast);
     const int smax = max_smem_optin() - 2048;
-    const int stage = (compat_stoich || no_stage) ? 0 : m->d.stage_bytes;
     const bool autov = variant == TL_VARIANT_AUTO;
     const int nsm = sm_count();
     if (autov) variant = heuristic_variant(m, sb, total, mode, nsm);
@@ -267,14 +415,16 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
     int groups_per_block = 1;
     if (variant == TL_VARIANT_THREAD) {
         pl.kind = 1;
+        if (mode != kModeGeneral) thin_plan(total, nsm, pl.thin, pl.lanes);
         int b = block_req;
         if (b <= 0) {
             // spread small ensembles over every SM
-            const long long per_sm = (total + nsm - 1) / nsm;
-            b = (int)std::min<long long>(128, std::max<long long>(32, (per_sm + 31) / 32 * 32));
+            const int per_warp = pl.lanes / pl.thin;
+            const long long per_sm = ((total + per_warp - 1) / per_warp + nsm - 1) / nsm;  // warps
+            b = 32 * (int)std::min<long long>(4, std::max<long long>(1, per_sm));
         }
         pl.block = b;
-        groups_per_block = pl.block;
+        groups_per_block = pl.block;  // the fit below is that of whole warps
     } else if (variant == TL_VARIANT_WARP) {
         pl.kind = 32;
         pl.block = block_req > 0 ? block_req : 256;
@@ -300,43 +450,65 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
         return TL_ERR_INVALID_ARGUMENT;
     }
     // shrink the block until the slots fit
-    pl.mode = mode;
-    pl.slot = slot_layout(m, sens, mode, pl.kind, pl.block);
-    while ((size_t)groups_per_block * pl.slot.bytes > (size_t)smax && pl.kind != 0 && pl.block > 32) {
-        pl.block -= 32;
-        groups_per_block = pl.block / pl.kind;
-    }
-    if (force_gslot && pl.kind == 0) pl.gslot = true;
-    if (!pl.gslot && (size_t)groups_per_block * pl.slot.bytes > (size_t)smax && mode != kModeGeneral &&
-        (size_t)groups_per_block * slot_bytes(m, sens) <= (size_t)smax) {
-        // the state fits but not with its queue beside it: the general build
-        pl.mode = kModeGeneral;
-        pl.slot = slot_layout(m, sens, pl.mode, pl.kind, pl.block);
-    }
-    if ((size_t)groups_per_block * pl.slot.bytes > (size_t)smax) {
-        if (pl.kind != 0) {
-            set_last_error("model too large for the shared-memory slot of this variant");
-            return TL_ERR_UNSUPPORTED;
+    const int asked = pl.block;
+    const auto fit = [&](int mode_) {
+        pl.mode = mode_;
+        pl.block = asked;
+        pl.slot = slot_layout(m, mode_, pl.kind, pl.block);
+        groups_per_block = pl.kind ? pl.block / pl.kind : 1;
+        while ((size_t)groups_per_block * pl.slot.bytes > (size_t)smax && pl.kind != 0 && pl.block > 32) {
+            pl.block -= 32;
+            groups_per_block = pl.block / pl.kind;
         }
-        // one realization's state exceeds shared memory: CTA groups keep it
-        // in global memory (one slot per CTA, served from L2)
-        pl.gslot = true;
+        return (size_t)groups_per_block * pl.slot.bytes <= (size_t)smax;
+    };
+    pl.gslot = force_gslot && pl.kind == 0;
+    // the packed tables hold the model (CTA groups: wide forms too)?
+    const bool packed = m->d.fast_ok && (pl.kind == 0 || (!m->d.chan8 && !m->d.ent_wide));
+    // the sub-warp and global-slot kinds have no scores build
+    if (!packed || (mode == kModeScores && (pl.gslot || (pl.kind > 1 && pl.kind < 32)))) mode = kModeGeneral;
+    if (!fit(mode) && !pl.gslot) {
+        // the general build's slot is smaller for wide models
+        if (mode == kModeGeneral || !fit(kModeGeneral)) {
+            if (pl.kind != 0) {
+                set_last_error("model too large for the shared-memory slot of this variant");
+                return TL_ERR_UNSUPPORTED;
+            }
+            // one realization's state exceeds shared memory: CTA groups keep it
+            // in global memory (one slot per CTA, served from L2)
+            pl.gslot = true;
+            fit(mode == kModeScores ? kModeGeneral : mode);
+        }
     }
+    if (pl.kind == 1) groups_per_block = pl.mode == kModeGeneral ? pl.block : pl.block / 32 * (pl.lanes / pl.thin);
+    size_t slot_smem = (size_t)groups_per_block * pl.slot.bytes;
+    if (pl.gslot) {
+        // fast build: a[] in global memory, the state beside it only if it
+        // does not fit either
+        slot_smem = pl.mode == kModeGeneral ? 0 : pl.slot.state;
+        pl.state_global = slot_smem > (size_t)smax;
+        if (pl.state_global) slot_smem = 0;
+    }
+    const int stage = (compat_stoich || no_stage || pl.gslot) ? 0
+                      : pl.mode == kModeGeneral               ? m->d.stage_bytes
+                                                              : m->d.f_stage_bytes;
     // chain-sized CTA groups leave the tables in L1/L2 (staging them would
     // cost more shared memory than the realization itself)
     const bool stage_ok = !(autov && pl.kind == 0 && sb <= 64 * 1024);
-    if (pl.gslot) {  // the queue stays in shared memory
-        pl.slot.bytes = slot_bytes(m, sens);
-        pl.slot.q_off = -1;
-    }
-    const size_t slot_smem = pl.gslot ? pl.slot.q_bytes : (size_t)groups_per_block * pl.slot.bytes;
     pl.stage = (stage_ok && slot_smem + (size_t)stage <= (size_t)smax) ? stage : 0;
     pl.smem = (size_t)pl.stage + slot_smem;
+    // scores beside the counts while four such CTAs fit an SM, else in global memory
+    if (pl.mode == kModeScores && pl.smem > (size_t)smax / 4) {
+        pl.slot.score_global = true;
+        pl.slot.bytes -= (size_t)pl.slot.f_a;
+        pl.smem -= (size_t)groups_per_block * (size_t)pl.slot.f_a;
+    }
     pl.row_warp = pl.kind == 0 && m->h.max_row > 32;
     int bps = 0;
-    const int lk = pl.gslot ? kKindCtaGlobal : pl.kind;
-    cudaError_t e = m->h.pop_bits == 64 ? fused_occupancy<long long>(lk, pl.mode, pl.block, pl.smem, &bps)
-                                        : fused_occupancy<int>(lk, pl.mode, pl.block, pl.smem, &bps);
+    const int lk = launch_kind(pl);
+    const bool staged = pl.stage > 0;
+    cudaError_t e = m->h.pop_bits == 64 ? fused_occupancy<long long>(lk, pl.mode, staged, pl.block, pl.smem, &bps)
+                                        : fused_occupancy<int>(lk, pl.mode, staged, pl.block, pl.smem, &bps);
     if (e != cudaSuccess) return cuda_fail(e, "occupancy");
     if (bps < 1) {
         set_last_error("the launch does not fit an SM");
@@ -440,8 +612,9 @@ static tl_status job_prepare(Job& J) {
         set_last_error("sensitivity needs at least one tracked species");
         return TL_ERR_INVALID_ARGUMENT;
     }
-    J.hrates.assign((size_t)J.S * M, 0.f);
+    J.hrates.assign((size_t)2 * J.S * M, 0.f);  // as given, then halved for 2S channels
     J.htf.assign((size_t)J.S, cfg->t_final);
+    bool halvable = true;
     for (int s = 0; s < J.S; ++s)
         for (int j = 0; j < M; ++j) {
             const double c = cfg->n_rate_sets > 0 ? cfg->rate_sets[(size_t)s * M + j] : h.rate[(size_t)j];
@@ -449,8 +622,14 @@ static tl_status job_prepare(Job& J) {
                 set_last_error("rate constants must be finite and >= 0");
                 return TL_ERR_NUMERIC;
             }
-            J.hrates[(size_t)s * M + j] = (float)c;
+            const float cf = (float)c;
+            J.hrates[(size_t)s * M + j] = cf;
+            const bool twice = h.order[(size_t)j] == 3;
+            J.hrates[(size_t)(J.S + s) * M + j] = twice ? 0.5f * cf : cf;
+            // the fast builds halve 2S rates, which is exact far from FP32's ends
+            if (twice && cf != 0.f && !(cf >= 7.8886e-31f && cf <= 1.1529e18f)) halvable = false;
         }
+    if (!halvable) J.mode = kModeGeneral;
     if (cfg->n_rate_sets > 0 && cfg->t_final_sets)
         for (int s = 0; s < J.S; ++s) {
             J.htf[(size_t)s] = cfg->t_final_sets[s];
@@ -469,9 +648,25 @@ static tl_status job_prepare(Job& J) {
     return ensure_device(m);
 }
 
+// The plan's part of the launch parameters.
+static void bind_plan(const tl_model* m, const Plan& pl, SimParams& p) {
+    p.blob = pl.mode == kModeGeneral ? m->d.blob : m->d.fblob;
+    p.stage_bytes = pl.stage;
+    p.slot_bytes = (int)pl.slot.bytes;
+    p.f_D = pl.slot.f_D;
+    p.f_X = pl.slot.f_X;
+    p.f_a = pl.slot.f_a;
+    p.f_big = pl.gslot && !pl.state_global ? 0 : (int)pl.slot.state;
+    p.score_global = pl.slot.score_global ? 1 : 0;
+    p.state_global = pl.state_global ? 1 : 0;
+    p.q_rounds = pl.slot.q_rounds;
+    p.lanes = pl.lanes;
+    p.row_warp = pl.row_warp ? 1 : 0;
+}
+
 static void job_layout(Job& J, Carver& c) {
     const int M = J.m->h.M, N = J.m->h.N, K1 = std::max(J.K, 1);
-    J.o_rates = c.take((size_t)J.S * M * 4);
+    J.o_rates = c.take((size_t)2 * J.S * M * 4);
     J.o_tf = c.take((size_t)J.S * 8);
     J.o_grid = c.take((size_t)J.S * J.P * 8);
     J.o_tr = c.take((size_t)K1 * 4);
@@ -545,8 +740,7 @@ static tl_status job_bind(Job& J, unsigned char* B, cudaStream_t st) {
     p.flags = cfg->flags;
     p.max_halv = cfg->max_halvings > 0 ? cfg->max_halvings : 64;
     p.wait_polls = cfg->stage_wait_polls == 0 ? (1 << 22) : std::max(cfg->stage_wait_polls, 0);
-    p.blob = m->d.blob;
-    p.stage_bytes = J.pl.stage;
+    p.frates = rb.rates + (size_t)J.S * m->h.M;
     p.off_chan = m->d.off_chan;
     p.off_rord = m->d.off_rord;
     p.off_gkind = m->d.off_gkind;
@@ -555,10 +749,17 @@ static tl_status job_bind(Job& J, unsigned char* B, cudaStream_t st) {
     p.off_vc = m->d.off_vc;
     p.off_cp = m->d.off_cp;
     p.off_rv = m->d.off_rv;
-    p.slot_bytes = (int)J.pl.slot.bytes;
-    p.q_off = J.pl.slot.q_off;
-    p.q_rounds = J.pl.slot.q_rounds;
-    p.row_warp = J.pl.row_warp ? 1 : 0;
+    p.n_rows = m->d.n_rows;
+    p.x_one = m->h.N + m->d.n_2s;
+    p.chan8 = m->d.chan8 ? 1 : 0;
+    p.ent_wide = m->d.ent_wide ? 1 : 0;
+    p.t_chan = m->d.t_chan;
+    p.t_row = m->d.t_row;
+    p.t_ent = m->d.t_ent;
+    p.t_col = m->d.t_col;
+    p.t_cp = m->d.t_cp;
+    p.t_sp = m->d.t_sp;
+    bind_plan(m, J.pl, p);
     p.gslots = J.pl.gslot ? B + J.o_gslot : nullptr;
     p.ctr = rb.ctr;
     p.pstate = rb.pstate;
@@ -694,20 +895,16 @@ static tl_status autotune_measure(Job& J, cudaStream_t st) {
         Cand win{0, 0, false};
         for (const Cand& c : cands) {
             Plan pl;
-            if (make_plan(m, c.variant, c.block, J.mode, J.sens, J.compat_stoich, c.nostage, trial, pl) != TL_OK) continue;
+            if (make_plan(m, c.variant, c.block, J.mode, J.compat_stoich, c.nostage, trial, pl) != TL_OK) continue;
             if (c.variant == TL_VARIANT_THREAD && c.block != pl.block) continue;
             // global slots exist for the launch the heuristic planned
             if (pl.gslot && (!planned_gslot || pl.grid > planned_grid)) continue;
-            tp.stage_bytes = pl.stage;
-            tp.row_warp = pl.row_warp ? 1 : 0;
+            bind_plan(m, pl, tp);
             tp.gslots = pl.gslot ? planned_gslots : nullptr;
-            tp.slot_bytes = (int)pl.slot.bytes;
-            tp.q_off = pl.slot.q_off;
-            tp.q_rounds = pl.slot.q_rounds;
             if (cudaMemsetAsync(tp.ctr, 0, 64, st) != cudaSuccess) break;
             cudaEventRecord(e0, st);
-            cudaError_t le = J.w == 8 ? launch_fused<long long>(tp, launch_kind(pl), pl.mode, pl.block, pl.grid, pl.smem, st)
-                                      : launch_fused<int>(tp, launch_kind(pl), pl.mode, pl.block, pl.grid, pl.smem, st);
+            cudaError_t le = J.w == 8 ? launch_fused<long long>(tp, launch_kind(pl), pl.mode, pl.stage > 0, pl.block, pl.grid, pl.smem, st)
+                                      : launch_fused<int>(tp, launch_kind(pl), pl.mode, pl.stage > 0, pl.block, pl.grid, pl.smem, st);
             cudaEventRecord(e1, st);
             if (le != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess) {
                 cudaGetLastError();
@@ -732,22 +929,18 @@ static tl_status autotune_measure(Job& J, cudaStream_t st) {
         m->tuned_block = win.block;
         m->tuned_nostage = win.nostage ? 1 : 0;
     }
-    tl_status ps = make_plan(m, m->tuned_variant, m->tuned_block, J.mode, J.sens, J.compat_stoich, m->tuned_nostage != 0,
+    tl_status ps = make_plan(m, m->tuned_variant, m->tuned_block, J.mode, J.compat_stoich, m->tuned_nostage != 0,
                              J.total, J.pl);
     if (ps != TL_OK) return ps;
     if (J.pl.gslot && (!planned_gslot || J.pl.grid > planned_grid)) {
         // a cached global-slot plan that needs more slots than were laid out:
         // keep the planned launch
-        ps = make_plan(m, TL_VARIANT_AUTO, 0, J.mode, J.sens, J.compat_stoich, (J.cfg->flags & TL_FLAG_NO_STAGE) != 0,
+        ps = make_plan(m, TL_VARIANT_AUTO, 0, J.mode, J.compat_stoich, (J.cfg->flags & TL_FLAG_NO_STAGE) != 0,
                        J.total, J.pl);
         if (ps != TL_OK) return ps;
     }
-    J.p.stage_bytes = J.pl.stage;
-    J.p.row_warp = J.pl.row_warp ? 1 : 0;
+    bind_plan(m, J.pl, J.p);
     J.p.gslots = J.pl.gslot ? planned_gslots : nullptr;
-    J.p.slot_bytes = (int)J.pl.slot.bytes;
-    J.p.q_off = J.pl.slot.q_off;
-    J.p.q_rounds = J.pl.slot.q_rounds;
     return TL_OK;
 }
 
@@ -765,7 +958,7 @@ static tl_status run(tl_model* m, const tl_run_cfg* cfg, tl_result* res, tl_grad
     const bool no_stage = (cfg->flags & TL_FLAG_NO_STAGE) != 0;
     const bool measure = !J.plain && cfg->variant == TL_VARIANT_AUTO && (cfg->flags & TL_FLAG_AUTOTUNE_MEASURE);
     if (!J.plain) {
-        ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.sens, J.compat_stoich, no_stage, J.total, J.pl,
+        ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.compat_stoich, no_stage, J.total, J.pl,
                        (cfg->flags & TL_FLAG_GLOBAL_SLOTS) != 0);
         if (ps != TL_OK) return ps;
     } else {
@@ -795,8 +988,8 @@ static tl_status run(tl_model* m, const tl_run_cfg* cfg, tl_result* res, tl_grad
     cudaError_t le = cudaEventRecord(e0, st);
     if (le == cudaSuccess) {
         if (!J.plain) {
-            le = w == 8 ? launch_fused<long long>(p, launch_kind(J.pl), J.pl.mode, J.pl.block, J.pl.grid, J.pl.smem, st)
-                        : launch_fused<int>(p, launch_kind(J.pl), J.pl.mode, J.pl.block, J.pl.grid, J.pl.smem, st);
+            le = w == 8 ? launch_fused<long long>(p, launch_kind(J.pl), J.pl.mode, J.pl.stage > 0, J.pl.block, J.pl.grid, J.pl.smem, st)
+                        : launch_fused<int>(p, launch_kind(J.pl), J.pl.mode, J.pl.stage > 0, J.pl.block, J.pl.grid, J.pl.smem, st);
             launches = 1;
         } else {
             le = w == 8 ? launch_plain_init<long long>(p, st) : launch_plain_init<int>(p, st);
@@ -910,24 +1103,41 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     std::vector<int> lane(n);
     size_t wslot = 0;
     int bmode = kModeFast;  // the build every item can run on
-    for (auto& J : jobs) bmode = std::max(bmode, J.mode);
+    long long lane_total = 0;
+    for (int i = 0; i < n; ++i) {
+        Job& J = jobs[(size_t)i];
+        const tl_model* m = J.m;
+        bmode = std::max(bmode, J.mode);
+        if (!m->d.fast_ok || m->d.chan8 || m->d.ent_wide) bmode = kModeGeneral;
+        lane[(size_t)i] = (m->h.M <= 16 && m->h.N <= 16) ? 1 : 0;
+        if (lane[(size_t)i]) lane_total += J.total;
+    }
     const size_t spb = al16(sizeof(SimParams));
+    int thin = 1, unit_lanes = 32;
     for (;;) {
+        thin = 1;
+        unit_lanes = 32;
+        if (bmode != kModeGeneral) thin_plan(lane_total, sm_count(), thin, unit_lanes);
         wslot = 0;
         for (int i = 0; i < n; ++i) {
             Job& J = jobs[(size_t)i];
-            const tl_model* m = J.m;
-            lane[(size_t)i] = (m->h.M <= 16 && m->h.N <= 16) ? 1 : 0;
             Plan& pl = J.pl;
             pl.variant = lane[(size_t)i] ? TL_VARIANT_THREAD : TL_VARIANT_WARP;
-            pl.slot = slot_layout(m, J.sens, bmode, lane[(size_t)i] ? 1 : 32, 32);
-            wslot = std::max(wslot, lane[(size_t)i] ? 32 * pl.slot.bytes : pl.slot.bytes);
+            pl.mode = bmode;
+            pl.lanes = unit_lanes;
+            pl.thin = thin;
+            pl.slot = slot_layout(J.m, bmode, lane[(size_t)i] ? 1 : 32, 32);
+            wslot = std::max(wslot, lane[(size_t)i] ? (size_t)(unit_lanes / thin) * pl.slot.bytes : pl.slot.bytes);
         }
         wslot = al16(wslot);
-        // a slot that fits only without its queue takes the general build
+        // the general build's slot is smaller for wide models
         if (wslot + spb <= (size_t)smax || bmode == kModeGeneral) break;
         bmode = kModeGeneral;
     }
+    const auto tables = [&](const tl_model* m) { return bmode == kModeGeneral ? m->d.blob : m->d.fblob; };
+    const auto table_bytes = [&](const tl_model* m) {
+        return bmode == kModeGeneral ? m->d.stage_bytes : m->d.f_stage_bytes;
+    };
     // stage every model's tables when they fit next to 4 warps' slots
     std::vector<tl_model*> uniq;
     for (auto& J : jobs)
@@ -936,7 +1146,7 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     std::vector<size_t> stage_off(uniq.size());
     for (size_t u = 0; u < uniq.size(); ++u) {
         stage_off[u] = stage;
-        stage += (size_t)uniq[u]->d.stage_bytes;
+        stage += (size_t)table_bytes(uniq[u]);
     }
     bool staged = true;
     for (auto& J : jobs) staged &= !J.compat_stoich;
@@ -965,7 +1175,7 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     }
     if (staged)
         for (size_t u = 0; u < uniq.size(); ++u)
-            TLC(cudaMemcpyAsync(B + o_stage + stage_off[u], uniq[u]->d.blob, (size_t)uniq[u]->d.stage_bytes,
+            TLC(cudaMemcpyAsync(B + o_stage + stage_off[u], tables(uniq[u]), (size_t)table_bytes(uniq[u]),
                                 cudaMemcpyDeviceToDevice, st));
     // unit table: warp-unit items first (longer realizations), then lane units
     std::vector<int> order;
@@ -974,6 +1184,7 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     for (int i = 0; i < n; ++i)
         if (lane[(size_t)i]) order.push_back(i);
     std::vector<BatchItem> hb((size_t)n);
+    const int per_unit = unit_lanes / thin;
     long long units = 0;
     for (int k = 0; k < n; ++k) {
         const int i = order[(size_t)k];
@@ -983,7 +1194,7 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
         b.p.stage_bytes = 0;
         b.lane_mode = lane[(size_t)i];
         b.unit_begin = units;
-        b.units = lane[(size_t)i] ? (J.total + 31) / 32 : J.total;
+        b.units = lane[(size_t)i] ? (J.total + per_unit - 1) / per_unit : J.total;
         units += b.units;
         b.stage_off = -1;
         if (staged) {
@@ -1005,8 +1216,8 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     bp.wctr = reinterpret_cast<unsigned long long*>(B + o_wctr);
     const size_t smem = stage + (size_t)warps * (wslot + spb);
     int bps = 0;
-    cudaError_t le = pop == 64 ? batch_occupancy<long long>(bmode, 32 * warps, smem, &bps)
-                               : batch_occupancy<int>(bmode, 32 * warps, smem, &bps);
+    cudaError_t le = pop == 64 ? batch_occupancy<long long>(bmode, staged, thin, 32 * warps, smem, &bps)
+                               : batch_occupancy<int>(bmode, staged, thin, 32 * warps, smem, &bps);
     if (le != cudaSuccess) return cuda_fail(le, "batch occupancy");
     const int grid = (int)std::min<long long>((long long)sm_count() * std::max(bps, 1),
                                               (units + warps - 1) / warps);
@@ -1016,8 +1227,8 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     TLC(cudaEventCreate(&e1));
     le = cudaEventRecord(e0, st);
     if (le == cudaSuccess)
-        le = pop == 64 ? launch_batch<long long>(bp, bmode, 32 * warps, grid, smem, st)
-                       : launch_batch<int>(bp, bmode, 32 * warps, grid, smem, st);
+        le = pop == 64 ? launch_batch<long long>(bp, bmode, thin, 32 * warps, grid, smem, st)
+                       : launch_batch<int>(bp, bmode, thin, 32 * warps, grid, smem, st);
     if (le == cudaSuccess) le = cudaEventRecord(e1, st);
     if (le != cudaSuccess) {
         cudaEventDestroy(e0);
@@ -1537,7 +1748,7 @@ extern "C" tl_status tl_simulate_static(tl_model* m, const tl_run_cfg* cfg, tl_r
     if (ps != TL_OK) return ps;
     TLC(cudaSetDevice(m->d.device));
     cudaStream_t st = (cudaStream_t)cfg->stream;
-    ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.sens, J.compat_stoich,
+    ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.compat_stoich,
                    (cfg->flags & TL_FLAG_NO_STAGE) != 0, J.total, J.pl, (cfg->flags & TL_FLAG_GLOBAL_SLOTS) != 0);
     if (ps != TL_OK) return ps;
     Carver c;
@@ -1554,8 +1765,8 @@ extern "C" tl_status tl_simulate_static(tl_model* m, const tl_run_cfg* cfg, tl_r
     ps = job_bind(J, reinterpret_cast<unsigned char*>(base), st);  // clears the counters
     if (ps != TL_OK) return ps;
     const auto tk = std::chrono::steady_clock::now();
-    cudaError_t le = J.w == 8 ? launch_fused<long long>(J.p, launch_kind(J.pl), J.pl.mode, J.pl.block, J.pl.grid, J.pl.smem, st)
-                              : launch_fused<int>(J.p, launch_kind(J.pl), J.pl.mode, J.pl.block, J.pl.grid, J.pl.smem, st);
+    cudaError_t le = J.w == 8 ? launch_fused<long long>(J.p, launch_kind(J.pl), J.pl.mode, J.pl.stage > 0, J.pl.block, J.pl.grid, J.pl.smem, st)
+                              : launch_fused<int>(J.p, launch_kind(J.pl), J.pl.mode, J.pl.stage > 0, J.pl.block, J.pl.grid, J.pl.smem, st);
     if (le != cudaSuccess) return cuda_fail(le, "simulation launch");
     ps = job_reduce(J, st);
     if (ps != TL_OK) return ps;

@@ -135,6 +135,15 @@ struct ChanRng {
     }
 };
 
+// a / b as a times the approximate reciprocal of b: the same FP32 value as
+// __fdividef(a, b), without its range handling, for normal b below 2^126
+// (compared on GB300 over 2.7e8 pairs); b = 0 gives infinity.
+TL_D float fast_rcp(float b) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    return r;
+}
+
 // ---------------------------------------------------------------------------
 // Poisson samplers (FP32).
 // ---------------------------------------------------------------------------
@@ -170,25 +179,43 @@ TL_D float log_poisson_pmf(float kf, float mu, float lmu) {
 // boundaries move by ~1e-7 relative, the size of FP32 rounding, and the
 // sampler runs 8-14 % faster on the chain and dimer models.
 struct Ptrs {
-    float mu, lmu, b, a, inv_alpha, vr;
+    float mu, b, a, vr;
     TL_D explicit Ptrs(float mu_) : mu(mu_) {
         const float smu = sqrtf(mu);
-        lmu = logf(mu);
         b = 0.931f + 2.53f * smu;
         a = -0.059f + 0.02483f * b;
-        inv_alpha = 1.1239f + __fdividef(1.1328f, b - 3.4f);
-        vr = 0.9277f - __fdividef(3.6224f, b - 2.f);
+        vr = 0.9277f - 3.6224f * fast_rcp(b - 2.f);
+    }
+    // The acceptance test proper.
+    TL_D bool accept(float V, float us, float kf) const {
+        const float inv_alpha = 1.1239f + __fdividef(1.1328f, b - 3.4f);
+        const float lhs = logf(__fdividef(V * inv_alpha, __fdividef(a, us * us) + b));
+        return lhs <= log_poisson_pmf(kf, mu, logf(mu));
+    }
+    // The same test with fast logarithms: lhs - log p(k) as
+    //   log(V inv_alpha sqrt(2 pi k) / (a / us^2 + b)) + k log(k / mu) - (k - mu) + 1/(12k) - 1/(360k^3).
+    // Its error is below 5e-7 k + 4e-6 (__logf: 3.6e-7 absolute near 1), that
+    // of the test proper below 2e-7 k + 3e-6; within the margin of zero, and
+    // for small k, the test proper decides.  About 30 instructions for 150,
+    // on a path that some lane of a warp takes at nearly every attempt.
+    TL_D float excess(float V, float rus, float kf) const {
+        const float inv_alpha = 1.1239f + 1.1328f * fast_rcp(b - 3.4f);
+        const float ik = fast_rcp(kf);
+        const float q = V * inv_alpha * (2.5066283f * kf * rsqrtf(kf)) * fast_rcp(a * rus * rus + b);
+        return __logf(q) + kf * __logf(kf * fast_rcp(mu)) - (kf - mu) + ik * (1.f / 12.f - ik * ik * (1.f / 360.f));
     }
     // one attempt on the uniforms (u, v); true: accepted, k drawn
     TL_D bool attempt(float u, float V, int& k) const {
         const float U = u - 0.5f;
         const float us = 0.5f - fabsf(U);
-        const float kf = floorf((__fdividef(2.f * a, us) + b) * U + mu + 0.43f);
+        const float rus = fast_rcp(us);
+        const float kf = floorf((2.f * a * rus + b) * U + mu + 0.43f);
         k = (int)kf;
         if (us >= 0.07f && V <= vr) return true;
         if (kf < 0.f || (us < 0.013f && V > us)) return false;
-        const float lhs = logf(__fdividef(V * inv_alpha, __fdividef(a, us * us) + b));
-        return lhs <= log_poisson_pmf(kf, mu, lmu);
+        const float d = excess(V, rus, kf), m = 3e-6f * kf + 3e-5f;
+        if (kf >= 4.f && fabsf(d) > m) return d < 0.f;
+        return accept(V, us, kf);
     }
 };
 constexpr int kPtrsTries = 512;  // never reached in practice (acceptance > 0.89)
@@ -458,6 +485,8 @@ struct GWarp {
         }
         return v;
     }
+    TL_D int max_int(int v) const { return __reduce_max_sync(0xffffffffu, v); }
+    TL_D unsigned long long shfl_up(unsigned long long v, int o) const { return __shfl_up_sync(0xffffffffu, v, o); }
     TL_D double excl_scan(double v) const {
         double s = v;
 #pragma unroll
@@ -528,6 +557,12 @@ struct GSub {
         }
         return v;
     }
+    TL_D int max_int(int v) const {
+#pragma unroll
+        for (int o = W / 2; o; o >>= 1) v = max(v, __shfl_xor_sync(mask, v, o, W));
+        return v;
+    }
+    TL_D unsigned long long shfl_up(unsigned long long v, int o) const { return __shfl_up_sync(mask, v, o, W); }
     TL_D double excl_scan(double v) const {
         double s = v;
 #pragma unroll
@@ -666,7 +701,7 @@ struct GCta {
     }
 };
 
-// The lanes that share one queue of long Poisson draws (pass_fire_queued):
+// The lanes that share one queue of long Poisson draws (fast_fire):
 // the group itself, or each warp of a CTA group.
 template <class Grp>
 TL_D Grp queue_group(const Grp& g) {
@@ -726,8 +761,20 @@ struct SimParams {
     int stage_bytes;    // 0 = no staging
     int off_chan, off_rord, off_gkind, off_perm, off_rp, off_vc, off_cp, off_rv;  // byte offsets (net)
     int slot_bytes;     // per group
-    int q_off;          // queue of long draws in the slot, -1: over x' (free while a leap fires)
-    int q_rounds;       // turns of a queue group before its queue is drained
+    // fast and scores builds (tl_step.cuh)
+    const float* frates;  // [S][M] rates, halved for 2S channels
+    int n_rows;           // species rows that bound a step
+    int x_one;            // index of the constant 1 in X
+    int chan8;            // channel records of two 32-bit offsets (wide CTA models)
+    int ent_wide;         // row entries packed as (col<<3)|((v+2)&7)
+    int t_chan, t_row, t_ent, t_col, t_cp, t_sp;  // byte offsets of the tables, t_cp -1: none
+    int f_D, f_X;         // byte offsets in the state
+    int f_big;            // offset of a[] in the slot (or in a global slot)
+    int f_a;              // bytes of a[]
+    int score_global;     // scores accumulate in global memory
+    int state_global;     // global-slot builds: the state too
+    int q_rounds;         // turns of a queue group before its queue is drained
+    int lanes;            // thin groups: lanes of a warp that take realizations
     int row_warp;       // CTA groups: one warp per species row (long rows)
     unsigned char* gslots;  // CTA groups whose slot exceeds shared memory:
                             // one slot per CTA in global memory (else null)
@@ -764,7 +811,6 @@ struct Slot {
     float* a;  // propensity (sign bit = critical)
     int* k;    // firing counts of the leap: over a[] unless the run keeps
                // likelihood-ratio scores, which read a[] after the leap
-    unsigned short* q;  // queue of the leap's long draws (null: over xn)
 };
 
 // Per-realization progress.  Every leap attempt and every direct-method
@@ -983,6 +1029,7 @@ __device__ __noinline__ int select_channel_impl(const Grp g, const int M, const 
         // -inf, so that for a float acc  rd(t) < acc  <=>  t < acc exactly.
         const AccT trem = target - excl;
         const float tf = sizeof(AccT) == 8 ? __double2float_rd((double)trem) : (float)trem;
+#pragma unroll 1
         for (int j = g.rank(); j < M; j += g.size()) {
             const float aj = a[j];
             const bool c = is_crit(aj);
@@ -1142,140 +1189,6 @@ TL_D void pass_fire(const Grp& g, const SimParams& p, const float* a, int* kk, f
     }
 }
 
-// The same counts for groups of lanes (fast and scores builds).  What bounds
-// this pass is instruction issue, and most of it went into lanes that waited
-// for a neighbour's long draw: a lane took its channels' long draws one at a
-// time, and a warp ran each as often as its unluckiest lane needed it.
-//  * A channel whose mean lies in [0, 10) compares the shared word's
-//    u = 1 - q with F0 = exp(-mu) and F1 = F0 (1 + mu), both from one fast
-//    exponential and without a branch.  kFireMargin bounds what the fast forms
-//    and poisson_first's own tests together can be off (under 2.3e-6: the
-//    truncated word 1.8e-7, __expf 3.5e-7, poisson_p1 / p2 1.3e-6 and the
-//    sums), so outside the margin both give the same count.
-//  * Every other draw (k >= 2, within the margin, means >= 10) is marked in
-//    the lane's masks.  After at most q_rounds turns the lanes list their
-//    marked channels in a queue and take them in turn: inversions from the
-//    front, transformed-rejection draws (PTRS) from the back, so that a pass
-//    runs one kind on all lanes.  A PTRS lane moves on to its next draw after
-//    an accepted attempt instead of waiting for the warp's last one.
-// Measured on GB300 against in-place draws: toy network, 60 000 realizations
-// to 5e-4 (58 long draws a leap) 109.0 -> 76.3 ms, 4665 -> 3160 warp
-// instructions a realization-step; 4000 realizations to 2e-3 48.0 -> 41.2 ms;
-// 1024-species chain (all PTRS) 4.59 -> 4.13 ms; colloid-250 5.14 -> 4.75 ms.
-// Listing the channels turn by turn with ballots instead of one scan a leap
-// gave only 102.7 ms on the first.
-// A marked channel keeps its propensity in place until its count is drawn.
-// a[] and the counts are padded to whole blocks of four; the padding holds 0.
-constexpr float kFireMargin = 5e-6f;
-
-template <class Grp>
-TL_D void pass_fire_queued(const Grp& g, const SimParams& p, const float* a, int* kk, unsigned short* q, float tauf,
-                           int jc, uint32_t step, uint32_t r, uint32_t set) {
-    const auto qg = queue_group(g);
-    constexpr int kTurn = 4 * decltype(queue_group(g))::kWidth;  // channels of a queue group's turn
-    const int cap = p.q_rounds * kTurn;
-    if constexpr (Grp::kWidth == 0) q += g.warp * cap;
-    const int G4 = (p.M + 3) >> 2;
-    for (int b0 = g.rank() - qg.rank(); b0 < G4;) {
-        const int j_first = 4 * b0;
-        unsigned inv = 0, big = 0;  // this lane's marked channels, four bits a turn
-        int sh = 0;
-        for (int m = 0; m < p.q_rounds && b0 < G4; ++m, b0 += g.size(), sh += 4) {
-            const int g4 = b0 + qg.rank();
-            if (g4 >= G4) continue;
-            const float4 v4 = *reinterpret_cast<const float4*>(a + 4 * g4);
-            const float av[4] = {v4.x, v4.y, v4.z, v4.w};
-            float mu[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) mu[e] = fmaxf(av[e], 0.f) * tauf;  // critical channels: 0
-            U4 gw{0u, 0u, 0u, 0u};
-            if (fminf(fminf(mu[0], mu[1]), fminf(mu[2], mu[3])) < 10.f)
-                gw = group_words(p.rk, (uint32_t)g4, step, r, set);
-            int kv[4];
-            unsigned all = 0, far = 0;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float ex = __expf(-mu[e]);
-                // 2 - (1 - q) from the word's top 23 bits
-                const float v = __uint_as_float((word_of(gw, e) >> 9) | 0x3f800000u);
-                const float d0 = v + (ex - 2.f);          // F0 - u
-                const float d1 = fmaf(ex, mu[e], d0);     // F1 - u >= F0 - u
-                const bool is_far = mu[e] >= 10.f;
-                const bool mark = d1 < kFireMargin || fabsf(d0) < kFireMargin || is_far;
-                if (mark) all |= 1u << e;
-                if (is_far) far |= 1u << e;
-                kv[e] = mark ? __float_as_int(av[e]) : (int)(__float_as_uint(d0) >> 31);
-            }
-            inv |= (all & ~far) << sh;
-            big |= far << sh;
-            *reinterpret_cast<int4*>(kk + 4 * g4) = make_int4(kv[0], kv[1], kv[2], kv[3]);
-        }
-        if (!qg.any((inv | big) != 0u)) continue;
-        // list the marked channels: positions from one scan of both counts
-        const unsigned mine = (unsigned)__popc(inv) | (unsigned)__popc(big) << 16;
-        const unsigned upto = qg.incl_scan(mine);
-        const unsigned total = qg.bcast(upto, qg.size() - 1);
-        {
-            int at = (int)((upto - mine) & 0xffffu);
-            while (inv) {
-                const int bit = __ffs(inv) - 1;
-                inv &= inv - 1;
-                q[at++] = (unsigned short)((bit >> 2) * kTurn + qg.rank() * 4 + (bit & 3));
-            }
-            at = cap - 1 - (int)((upto - mine) >> 16);
-            while (big) {
-                const int bit = __ffs(big) - 1;
-                big &= big - 1;
-                q[at--] = (unsigned short)((bit >> 2) * kTurn + qg.rank() * 4 + (bit & 3));
-            }
-        }
-        qg.sync();
-        const int n_inv = (int)(total & 0xffffu), n_big = (int)(total >> 16);
-        const auto channel = [&](int id) {
-            if constexpr (Grp::kWidth == 0) return j_first + (id / kTurn) * 4 * g.size() + id % kTurn;
-            else return j_first + id;
-        };
-        for (int i = qg.rank(); i < n_inv; i += qg.size()) {
-            const int j = channel(q[i]);
-            const float mu = fmaxf(a[j], 0.f) * tauf;
-            const U4 gw = group_words(p.rk, (uint32_t)j >> 2, step, r, set);
-            const float qf = ((float)word_of(gw, j & 3) + 0.5f) * 2.3283064365386963e-10f;
-            const float ex = __expf(-mu);
-            int k = 2;
-            if (fmaf(ex, mu, ex) - (1.f - qf) > -kFireMargin)  // k >= 2 not settled
-                k = qf >= poisson_p1(mu) ? 0 : qf >= poisson_p2(mu) ? 1 : 2;
-            if (k == 2) {
-                ChanRng rng;
-                rng.init((uint32_t)j, step, r, set, p.rk);
-                k = poisson_search2(mu, qf, rng);
-            }
-            kk[j] = k;
-        }
-        int it = 0;  // attempts so far on draw i
-        for (int i = qg.rank(); i < n_big;) {
-            const int j = channel(q[cap - 1 - i]);
-            const float mu = a[j] * tauf;
-            const U4 w = philox10rk(U4{(uint32_t)j, step, r, (set << 8) + (uint32_t)(it >> 1)}, p.rk);
-            const bool odd = it & 1;
-            const Ptrs d(mu);
-            int k;
-            bool ok = d.attempt(u01f(odd ? w.z : w.x), u01f(odd ? w.w : w.y), k);
-            if (++it == kPtrsTries && !ok) {
-                k = (int)(mu + 0.5f);
-                ok = true;
-            }
-            if (ok) {
-                kk[j] = k;
-                it = 0;
-                i += qg.size();
-            }
-        }
-        qg.sync();
-    }
-    // the critical channel that fires, by the lane that wrote its block
-    if (jc >= 0 && (jc >> 2) % g.size() == g.rank()) kk[jc] = 1;
-}
-
 // ---------------------------------------------------------------------------
 // One step of one realization: a tau-leap (with rejection + halving) or a
 // block of direct-method steps (model.cu:301-413).
@@ -1400,11 +1313,7 @@ TL_D void do_step(const Grp& g, const SimParams& p, const MView& mv, Slot<Pop>& 
             jc = select_channel<Grp, TimeT>(g, p, s.a, pac, (TimeT)u01d(w.z, w.w) * a0c, 1);
         }
         if (!fire) jc = -1;
-        if constexpr (Grp::kWidth == 1 || COMPAT)
-            pass_fire<Grp, COMPAT>(g, p, s.a, s.k, tauf, jc, st.step, r, (uint32_t)set);
-        else
-            pass_fire_queued<Grp>(g, p, s.a, s.k, s.q ? s.q : reinterpret_cast<unsigned short*>(s.xn), tauf, jc, st.step, r,
-                                  (uint32_t)set);
+        pass_fire<Grp, COMPAT>(g, p, s.a, s.k, tauf, jc, st.step, r, (uint32_t)set);
         g.sync();
         bool ovf = false;
         const bool bad = pass_update<Grp, Pop>(g, p, mv, s.x, s.k, s.xn, ovf);

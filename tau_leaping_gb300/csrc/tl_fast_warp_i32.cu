@@ -1,0 +1,6 @@
+// Fast and scores builds, 32-bit populations: thin and warp groups.
+#include "tl_kernels.cuh"
+#include "tl_call.cuh"
+#define TL_POP int
+#define TL_FAST_PART 1
+#include "tl_fast.inc"

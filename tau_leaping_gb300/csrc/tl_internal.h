@@ -68,6 +68,14 @@ struct DevModel {
     int stage_bytes = 0;            // bytes of the net part (what a CTA stages)
     int off_chan = 0, off_rord = 0, off_gkind = 0, off_perm = 0, off_rp = 0, off_vc = 0, off_cp = 0, off_rv = 0;
     int off_raw_rp = 0, off_raw_vc = 0;
+    // tables of the fast and scores builds (tl_step.cuh), staged as one piece
+    unsigned char* fblob = nullptr;
+    int f_stage_bytes = 0;
+    int t_chan = 0, t_row = 0, t_ent = 0, t_col = 0, t_cp = -1, t_sp = 0;
+    int n_rows = 0;                 // species that react: rows of the step bound
+    int n_2s = 0;                   // species of 2S channels
+    bool chan8 = false, ent_wide = false;
+    bool fast_ok = false;           // the model fits the packed fields
     void* x0 = nullptr;             // Pop[N]
     float* rate = nullptr;          // [M]
     int nnz_net = 0, nnz_raw = 0;

@@ -13,6 +13,7 @@
 #pragma once
 
 #include "tl_device.cuh"
+#include "tl_step.cuh"
 #include "tl_launch.h"
 
 namespace tl {
@@ -111,7 +112,6 @@ TL_D Slot<Pop> carve_slot(unsigned char* base, const SimParams& p) {
     // scored runs keep the counts apart (their slots hold M more ints)
     s.k = p.scores ? reinterpret_cast<int*>(base + 2 * xb + (((size_t)p.M * 4 + 15) & ~(size_t)15))
                    : reinterpret_cast<int*>(s.a);
-    s.q = p.q_off >= 0 ? reinterpret_cast<unsigned short*>(base + p.q_off) : nullptr;
     return s;
 }
 
@@ -162,8 +162,6 @@ TL_D void run_realization(const Grp& g, const SimParams& p, const MView& mv, Slo
     float* score = (SENS && p.scores) ? p.scores + (size_t)w * p.M : nullptr;
     const Pop* x0 = reinterpret_cast<const Pop*>(p.x0);
     for (int i = g.rank(); i < p.N; i += g.size()) s.x[i] = x0[i];
-    // the padding of the last block of four channels (pass_fire_queued)
-    if (Grp::kWidth != 1 && g.rank() < ((4 - (p.M & 3)) & 3)) s.a[p.M + g.rank()] = 0.f;
     if (SENS && score)
         for (int j = g.rank(); j < p.M; j += g.size()) score[j] = 0.f;
     g.sync();
@@ -191,34 +189,13 @@ TL_D void run_realization(const Grp& g, const SimParams& p, const MView& mv, Slo
 // ---------------------------------------------------------------------------
 // Fused persistent kernel.
 // ---------------------------------------------------------------------------
-// Thread, sub-warp and warp groups launch at most 256 threads per CTA and
-// ask the compiler for a number of resident CTAs per SM, which sets the
-// register budget 65536 / (256 * n) per thread: TL_THREAD_MINB for thread
-// groups, TL_WARP_MINB for the others.  CTA groups use up to 1024 threads.
-// Defaults from sweeps on GB300: warp groups run best at 5 CTAs (51
-// registers; 4 and 6 were 9 % slower on the toy network), thread groups
-// at 3 (85 registers; 8 % faster than 4 on the dimer).
-#ifndef TL_WARP_MINB
-#define TL_WARP_MINB 5
-#endif
-#ifndef TL_THREAD_MINB
-#define TL_THREAD_MINB 3
-#endif
-// The batch kernel (thread and warp units, scores on) at 2 CTAs per SM
-// (128 registers): 1 gives 160 registers and one CTA per SM (-37 %), 4 and
-// 5 spill (-24 %, -22 %).
-#ifndef TL_BATCH_MINB
-#define TL_BATCH_MINB 2
-#endif
-// MODE: kModeFast has neither likelihood-ratio scores nor the
-// reference-compatibility switches; kModeScores has the scores;
-// kModeGeneral has both.  Smaller builds spill fewer registers: the fast
-// one is ~6 % faster than the general one, and the scores-only batch 15 %.
-// GSLOT (CTA groups only): each CTA's slot lives in global memory, for
-// realizations whose state exceeds shared memory.  A separate build, so
-// that the shared-memory kernels keep shared-memory addressing.
-template <int KIND, class Pop, int MODE, bool GSLOT = false>
-__global__ void __launch_bounds__(KIND == 0 ? 1024 : 256, KIND == 0 ? 1 : KIND == 1 ? TL_THREAD_MINB : TL_WARP_MINB)
+// The general build: likelihood-ratio scores and the reference-compatibility
+// switches at run time, on do_step().  GSLOT (CTA groups only): each CTA's
+// slot lives in global memory, for realizations whose state exceeds shared
+// memory.  A separate build, so that the shared-memory kernels keep
+// shared-memory addressing.
+template <int KIND, class Pop, bool GSLOT = false>
+__global__ void __launch_bounds__(KIND == 0 ? 1024 : 256, KIND == 0 ? 1 : KIND == 1 ? TL_THREAD_MINB : TL_GENERAL_MINB)
     k_fused(const __grid_constant__ SimParams p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ __align__(8) unsigned long long mbar;
@@ -238,7 +215,6 @@ __global__ void __launch_bounds__(KIND == 0 ? 1024 : 256, KIND == 0 ? 1 : KIND =
     const Grp g = GroupOf<KIND>::make(red);
     if constexpr (GSLOT) slots = p.gslots + (size_t)blockIdx.x * (size_t)p.slot_bytes;
     Slot<Pop> s = carve_slot<Pop>(slots + (size_t)GroupOf<KIND>::index() * p.slot_bytes, p);
-    if constexpr (GSLOT) s.q = reinterpret_cast<unsigned short*>(smem + p.stage_bytes);
     const long long total = p.R * (long long)p.S;
 
     for (;;) {
@@ -246,16 +222,85 @@ __global__ void __launch_bounds__(KIND == 0 ? 1024 : 256, KIND == 0 ? 1 : KIND =
         if (g.leader()) w = (long long)atomicAdd(p.ctr + 0, 1ull);
         w = g.bcast(w, 0);
         if (w >= total) break;
-        run_realization<Grp, Pop, (MODE >= kModeScores), (MODE == kModeGeneral)>(g, p, mv, s, w);
+        run_realization<Grp, Pop, true, true>(g, p, mv, s, w);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Fast and scores builds (tl_step.cuh).  STAGED: the tables in shared memory
+// (and every access to them a shared-memory access); GSLOT: a[] in global
+// memory, and the whole state where even that is too large.
+// ---------------------------------------------------------------------------
+template <int KIND>
+struct FastGroupOf {
+    using type = typename GroupOf<KIND>::type;
+    static constexpr int kPerWarp = KIND == 0 ? 0 : 32 / KIND;
+    static TL_D type make(double* red) { return GroupOf<KIND>::make(red); }
+    static TL_D int index(const SimParams&) { return GroupOf<KIND>::index(); }
+    static TL_D bool idle(const SimParams&) { return false; }
+};
+template <int W>
+struct ThinGroupOf {
+    using type = GThin<W>;
+    static TL_D type make(double*) { return type::make(); }
+    static TL_D int index(const SimParams& p) {
+        return (int)(threadIdx.x >> 5) * (p.lanes / W) + (int)(threadIdx.x & 31) / W;
+    }
+    static TL_D bool idle(const SimParams& p) { return (int)(threadIdx.x & 31) >= p.lanes; }
+};
+template <>
+struct FastGroupOf<kKindThin1> : ThinGroupOf<1> {};
+template <>
+struct FastGroupOf<kKindThin4> : ThinGroupOf<4> {};
+
+constexpr bool is_thin_kind(int kind) { return kind == kKindThin1 || kind == kKindThin4; }
+
+template <int KIND, class Pop, bool SENS, bool STAGED, bool GSLOT = false>
+__global__ void __launch_bounds__(KIND == 0 ? 1024 : 256,
+                                  KIND == 0 ? 1 : is_thin_kind(KIND) ? TL_THREAD_MINB : TL_WARP_MINB)
+    k_fast(const __grid_constant__ SimParams p) {
+    __shared__ __align__(8) unsigned long long mbar;
+    __shared__ double red[34];
+    using Of = FastGroupOf<KIND>;
+    using Lay = tl::Lay<Pop, STAGED, GSLOT>;
+
+    uint32_t slots = 0;
+    if constexpr (STAGED) {
+        if (!stage_blob(tl_smem, p.blob, p.stage_bytes, p.wait_polls, &mbar)) {
+            if (threadIdx.x == 0) atomicOr((unsigned*)(p.ctr + 5), kErrWaitTimeout | kErrStage);
+            return;
+        }
+        slots = (uint32_t)p.stage_bytes;
+    }
+    if (Of::idle(p)) return;
+    const auto g = Of::make(red);
+    unsigned char* g_state = nullptr;
+    unsigned char* g_big = nullptr;
+    if constexpr (GSLOT) {
+        unsigned char* mine = p.gslots + (size_t)blockIdx.x * (size_t)p.slot_bytes;
+        g_state = p.state_global ? mine : tl_smem;
+        g_big = mine + p.f_big;
+    }
+    const Lay L{p, slots + (uint32_t)(Of::index(p) * p.slot_bytes), 0u, g_state, g_big};
+    const long long total = p.R * (long long)p.S;
+    for (;;) {
+        long long w = 0;
+        if (g.leader()) w = (long long)atomicAdd(p.ctr + 0, 1ull);
+        w = g.bcast(w, 0);
+        if (w >= total) break;
+        fast_realization<typename Of::type, Lay, SENS>(g, p, L, w);
     }
 }
 
 // ---------------------------------------------------------------------------
 // Batched persistent kernel: items of several models / configurations.
 // ---------------------------------------------------------------------------
-template <class Pop, int MODE>
+// FAST: the fast build, or with SENS the scores build, of every item;
+// otherwise the general one.  STAGED: every item's tables in shared memory.
+// W: lanes of a thin item's realization.
+template <class Pop, bool FAST, bool SENS, bool STAGED, int W>
 __global__ void __launch_bounds__(256, TL_BATCH_MINB) k_batch(BatchParams bp) {
-    extern __shared__ __align__(16) unsigned char smem[];
+    unsigned char* const smem = tl_smem;
     __shared__ __align__(8) unsigned long long mbar;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     if (bp.stage_bytes > 0) {
@@ -285,18 +330,34 @@ __global__ void __launch_bounds__(256, TL_BATCH_MINB) k_batch(BatchParams bp) {
         }
         const SimParams& p = *sp;
         const int soff = bp.items[it].stage_off;
-        const MView mv = soff >= 0 ? staged_view(smem + soff, p) : p.g;
         const long long local = u - bp.items[it].unit_begin;
-        if (!bp.items[it].lane_mode) {
-            const GWarp g{lane};
-            Slot<Pop> s = carve_slot<Pop>(wslot, p);
-            run_realization<GWarp, Pop, (MODE >= kModeScores), (MODE == kModeGeneral)>(g, p, mv, s, local);
+        const long long total = p.R * (long long)p.S;
+        if constexpr (FAST) {
+            using Lay = tl::Lay<Pop, STAGED, false>;
+            const uint32_t my_slot = (uint32_t)(bp.stage_bytes + warp * bp.warp_slot_bytes);
+            if (!bp.items[it].lane_mode) {
+                const Lay L{p, my_slot, (uint32_t)soff, nullptr, nullptr};
+                fast_realization<GWarp, Lay, SENS>(GWarp{lane}, p, L, local);
+            } else if (lane < p.lanes) {
+                const GThin<W> g = GThin<W>::make();
+                const long long wi = local * (p.lanes / W) + lane / W;
+                if (wi < total) {
+                    const Lay L{p, my_slot + (uint32_t)(lane / W * p.slot_bytes), (uint32_t)soff, nullptr, nullptr};
+                    fast_realization<GThin<W>, Lay, SENS>(g, p, L, wi);
+                }
+            }
         } else {
-            const long long wi = local * 32 + lane;
-            if (wi < p.R * (long long)p.S) {
-                const G1 g{};
-                Slot<Pop> s = carve_slot<Pop>(wslot + (size_t)lane * p.slot_bytes, p);
-                run_realization<G1, Pop, (MODE >= kModeScores), (MODE == kModeGeneral)>(g, p, mv, s, wi);
+            const MView mv = soff >= 0 ? staged_view(smem + soff, p) : p.g;
+            if (!bp.items[it].lane_mode) {
+                const GWarp g{lane};
+                Slot<Pop> s = carve_slot<Pop>(wslot, p);
+                run_realization<GWarp, Pop, true, true>(g, p, mv, s, local);
+            } else {
+                const long long wi = local * 32 + lane;
+                if (wi < total) {
+                    Slot<Pop> s = carve_slot<Pop>(wslot + (size_t)lane * p.slot_bytes, p);
+                    run_realization<G1, Pop, true, true>(G1{}, p, mv, s, wi);
+                }
             }
         }
         __syncwarp();

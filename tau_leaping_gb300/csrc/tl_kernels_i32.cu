@@ -1,6 +1,7 @@
 // Kernels and launchers for 32-bit populations.
 #define TL_COMMON_KERNELS
 #include "tl_kernels.cuh"
+#include "tl_call.cuh"
 #define TL_POP int
 #include "tl_kernels_pop.inc"
 #undef TL_POP

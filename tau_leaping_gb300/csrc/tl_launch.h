@@ -9,28 +9,68 @@ namespace tl {
 struct SimParams;
 
 // kind: 1 = thread, 32 = warp, 0 = CTA, 2/4/8/16 = lanes per realization,
-// kKindCtaGlobal = CTA with its slot in global memory.
+// kKindCtaGlobal = CTA with its propensities (or whole slot) in global memory;
+// in the fast and scores builds thread groups are thin groups of 1 or 4 lanes.
 constexpr int kKindCtaGlobal = 64;
+constexpr int kKindThin1 = 101, kKindThin4 = 104;
 // mode: the kernel build a run needs.  Fast: no likelihood-ratio scores and
 // no reference-compatibility switches; Scores: with scores; General: both.
 // The sub-warp and global-slot kinds come in Fast and General only.
 constexpr int kModeFast = 0, kModeScores = 1, kModeGeneral = 2;
+// Thread, sub-warp and warp groups launch at most 256 threads per CTA and
+// ask the compiler for a number of resident CTAs per SM, which sets the
+// register budget 65536 / (256 * n) per thread: TL_THREAD_MINB for thread
+// groups, TL_WARP_MINB for the others.  CTA groups use up to 1024 threads.
+// Sweeps on GB300: warp and sub-warp groups of the fast builds run best at 4
+// (64 registers, no spills to speak of: toy network 67.6 ms against 75.7 at 5
+// and 74.4 at 3, the 45 x 83 network 90.9 against 102.2 and 98.1), thread
+// groups at 3 (dimer 3.49 ms against 3.67 at 4).
+#ifndef TL_WARP_MINB
+#define TL_WARP_MINB 4
+#endif
+#ifndef TL_THREAD_MINB
+#define TL_THREAD_MINB 3
+#endif
+// the general build's warp and sub-warp groups
+#ifndef TL_GENERAL_MINB
+#define TL_GENERAL_MINB 5
+#endif
+// The batch kernel (thread and warp units, scores on) at 2 CTAs per SM
+// (128 registers): 1 gives 160 registers and one CTA per SM (-37 %), 4 and
+// 5 spill (-24 %, -22 %).
+#ifndef TL_BATCH_MINB
+#define TL_BATCH_MINB 2
+#endif
+// staged: the tables are staged in shared memory.
 template <class Pop>
-cudaError_t launch_fused(const SimParams& p, int kind, int mode, int block, int grid, size_t smem,
+cudaError_t launch_fused(const SimParams& p, int kind, int mode, bool staged, int block, int grid, size_t smem,
                          cudaStream_t st);
 template <class Pop>
-cudaError_t fused_occupancy(int kind, int mode, int block, size_t smem, int* blocks_per_sm);
-// sub-warp kinds (2, 4, 8, 16 lanes per realization), compiled in their own units
+cudaError_t fused_occupancy(int kind, int mode, bool staged, int block, size_t smem, int* blocks_per_sm);
+// parts of the two above, compiled in units of their own: a launch, or the
+// occupancy where bps is not null
+struct FusedCall {
+    const SimParams* p;
+    int kind, mode;
+    bool staged;
+    int block, grid;
+    size_t smem;
+    cudaStream_t st;
+    int* bps;
+};
 template <class Pop>
-cudaError_t launch_fused_sub(const SimParams& p, int kind, int mode, int block, int grid, size_t smem,
-                             cudaStream_t st);
+cudaError_t call_general_sub(const FusedCall& c);
 template <class Pop>
-cudaError_t fused_occupancy_sub(int kind, int mode, int block, size_t smem, int* blocks_per_sm);
+cudaError_t call_fast(const FusedCall& c);  // thin and warp groups
+template <class Pop>
+cudaError_t call_fast_cta(const FusedCall& c);
+template <class Pop>
+cudaError_t call_fast_sub(const FusedCall& c);
 struct BatchParams;
 template <class Pop>
-cudaError_t launch_batch(const BatchParams& bp, int mode, int block, int grid, size_t smem, cudaStream_t st);
+cudaError_t launch_batch(const BatchParams& bp, int mode, int thin, int block, int grid, size_t smem, cudaStream_t st);
 template <class Pop>
-cudaError_t batch_occupancy(int mode, int block, size_t smem, int* blocks_per_sm);
+cudaError_t batch_occupancy(int mode, bool staged, int thin, int block, size_t smem, int* blocks_per_sm);
 template <class Pop>
 cudaError_t launch_plain_init(const SimParams& p, cudaStream_t st);
 template <class Pop>

@@ -1,0 +1,995 @@
+// tl_step.cuh - one step of one realization for the fast and scores builds.
+//
+// The same method, streams and sums as do_step() (tl_device.cuh), which the
+// general build, the plain form and the parity kernels keep: for one group
+// kind the trajectories are bit-identical.  What differs is how the state and
+// the tables lie in memory, because the path is bound by instruction issue:
+//
+//  * X[]: every population as FP32 with its criticality (x < n_c) in the sign
+//    bit, then |x - 1| with the 2S criticality (x < 2 n_c) for the species of
+//    2S channels, then the constant 1.  A propensity is the product
+//    c |X_p| |X_q| for every order, with c halved for 2S (an exact scaling),
+//    and its channel is critical when either sign is set: two loads and two
+//    multiplies, no conversion, no case per order.
+//  * Table entries hold byte offsets and the stoichiometry's FP32 bits, so an
+//    entry costs two integer instructions to take apart.  Rows are padded to
+//    four entries (the padding reads a zero propensity), and a row of a
+//    species that reacts nowhere is left out.
+//  * A leap adds its firings to D[] (int32) by shared-memory atomics, channel
+//    by channel as they are drawn, instead of every row gathering over all its
+//    channels: most channels of a leap do not fire.  The propensities stay in
+//    place, so a rejected leap needs no second pass over the channels.
+//  * Long Poisson draws go through a queue (fast_fire), which lies over X[]:
+//    a leap does not read X between its step bound and its commit.
+//  * Direct-method steps draw their channel on exact integers (lane groups) or
+//    on FP32 with a margin (thin groups); the FP64 form decides the cases
+//    neither can (ssa_select).
+// Measured on GB300 against do_step() with in-place draws (4000 to 60 000
+// realizations, ms): toy network 109.7 -> 63.3 on 16 lanes and 47.3 -> 29.8 on
+// warps, 45 x 83 network with int64 populations 127.0 -> 83.3, 12 x 20 network
+// in direct-method steps 9.55 -> 3.15, 1024-species chain 4.60 -> 3.36, colloid
+// of 250 species 5.14 -> 3.44, of 400 species (global propensities) 2.74 -> 1.78.
+#pragma once
+
+#include "tl_device.cuh"
+
+namespace tl {
+
+// W lanes of a warp for one realization of a small model (up to 16 species
+// and channels), W = 1, 2, 4, 8.  Every sum runs over the channels in order,
+// as one thread would form it, so the results do not depend on W: a thread
+// group's trajectories, with the channels' draws side by side.
+template <int W>
+struct GThin {
+    static constexpr int kWidth = W;
+    static constexpr bool kThin = true;
+    int lane;
+    int base;
+    unsigned mask;
+    static TL_D GThin make() {
+        GThin g;
+        const int l = (int)(threadIdx.x & 31);
+        g.lane = l & (W - 1);
+        g.base = l & ~(W - 1);
+        g.mask = ((1u << W) - 1u) << g.base;
+        return g;
+    }
+    TL_D int rank() const { return W == 1 ? 0 : lane; }
+    TL_D int size() const { return W; }
+    TL_D void sync() const {
+        if (W > 1) __syncwarp(mask);
+    }
+    TL_D bool leader() const { return W == 1 || lane == 0; }
+    TL_D float minf(float v) const {
+#pragma unroll
+        for (int o = W / 2; o; o >>= 1) v = fminf(v, __shfl_xor_sync(mask, v, o, W));
+        return v;
+    }
+    TL_D bool any(bool p) const { return W == 1 ? p : (__ballot_sync(mask, p) & mask) != 0u; }
+    template <class T>
+    TL_D T bcast(T v, int src) const {
+        if (W == 1) return v;
+        return __shfl_sync(mask, v, src, W);
+    }
+};
+
+template <class G>
+struct is_thin {
+    static constexpr bool value = false;
+};
+template <int W>
+struct is_thin<GThin<W>> {
+    static constexpr bool value = true;
+};
+
+// Where one realization's state and the tables lie.  Only offsets are kept:
+// an array's address is formed from them and the launch parameters where it is
+// used, which costs an operand of the constant bank and no register.
+// STAGED: the tables at the start of (or `tab` bytes into) shared memory, else
+// in global memory.  GLOBAL: the slot's propensities, and where `state` is set
+// the whole slot, in global memory.
+extern __shared__ __align__(16) unsigned char tl_smem[];
+
+template <class P, bool STAGED, bool GLOBAL>
+struct Lay {
+    using Pop = P;
+    const SimParams& p;
+    uint32_t slot;             // byte offset of the slot in shared memory
+    uint32_t tab;              // byte offset of the tables in shared memory
+    unsigned char* g_state;    // GLOBAL: the state, in either memory
+    unsigned char* g_big;      // GLOBAL: a[]
+
+    TL_D unsigned char* state(int off) const { return GLOBAL ? g_state + off : tl_smem + (slot + (uint32_t)off); }
+    TL_D unsigned char* big(int off) const {
+        return GLOBAL ? g_big + off : tl_smem + (slot + (uint32_t)(p.f_big + off));
+    }
+    template <class T>
+    TL_D const T* table(int off) const {
+        if constexpr (STAGED) return reinterpret_cast<const T*>(tl_smem + (tab + (uint32_t)off));
+        else return reinterpret_cast<const T*>(p.blob + off);
+    }
+    TL_D P* x() const { return reinterpret_cast<P*>(state(0)); }
+    TL_D int* D() const { return reinterpret_cast<int*>(state(p.f_D)); }
+    TL_D float* X() const { return reinterpret_cast<float*>(state(p.f_X)); }
+    TL_D unsigned short* q() const { return reinterpret_cast<unsigned short*>(state(p.f_X)); }
+    TL_D float* a() const { return reinterpret_cast<float*>(big(0)); }
+    TL_D int* k() const { return reinterpret_cast<int*>(big(p.f_a)); }  // counts of the leap, scored runs only
+    TL_D const uint32_t* chan() const { return table<uint32_t>(p.t_chan); }
+    TL_D const uint2* row() const { return table<uint2>(p.t_row); }
+    TL_D const uint4* ent() const { return table<uint4>(p.t_ent); }
+    TL_D const uint4* col() const { return table<uint4>(p.t_col); }
+    TL_D const uint32_t* cp() const { return table<uint32_t>(p.t_cp); }  // p.t_cp < 0: one chunk per channel
+    TL_D const unsigned short* sp() const { return table<unsigned short>(p.t_sp); }
+    // scores of realization w, scored runs only
+    TL_D float* score(long long w) const {
+        return p.score_global ? p.scores + (size_t)w * p.M : reinterpret_cast<float*>(big(2 * p.f_a));
+    }
+};
+
+template <class T>
+TL_D T& at_byte(T* p, uint32_t off) {
+    return *reinterpret_cast<T*>(reinterpret_cast<char*>(p) + off);
+}
+template <class T>
+TL_D const T& at_byte(const T* p, uint32_t off) {
+    return *reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + off);
+}
+
+// |f| with the sign bit of s
+TL_D float with_sign(float f, int s) {
+    return __uint_as_float((__float_as_uint(f) & 0x7fffffffu) | ((uint32_t)s & 0x80000000u));
+}
+// Species i holds x: its entries of X.  Populations and thresholds are >= 0,
+// so the sign of x - n_c is the criticality.
+template <class Lay>
+TL_D void set_species32(const Lay& L, int i, int x) {
+    const int nc = L.p.nc;
+    L.X()[i] = with_sign((float)x, x - nc);
+    const unsigned s3 = L.sp()[i];
+    if (s3) L.X()[s3] = with_sign((float)(x - 1), x - 2 * nc);
+}
+template <class Lay>
+__device__ __noinline__ void set_species64(const Lay L, int i, long long x) {
+    const int nc = L.p.nc;
+    L.X()[i] = with_sign((float)x, x < (long long)nc ? (int)0x80000000 : 0);
+    const unsigned s3 = L.sp()[i];
+    if (s3) L.X()[s3] = with_sign((float)(x - 1), x < (long long)(2 * nc) ? (int)0x80000000 : 0);
+}
+template <class Lay>
+TL_D void set_species(const Lay& L, int i, int x) {
+    set_species32(L, i, x);
+}
+// int64 -> FP32 runs at the reduced FP64 rate; a population that fits int32
+// (the usual case) rounds to the same float from there
+template <class Lay>
+TL_D void set_species(const Lay& L, int i, long long x) {
+    if ((long long)(int)x == x) set_species32(L, i, (int)x);
+    else set_species64(L, i, x);
+}
+
+// Propensities into a[] (sign = critical) and the lane's partial sums; thin
+// groups form the sums over all channels in order.
+template <class Grp, class Lay>
+TL_D void fast_props(const Grp& g, const SimParams& p, const Lay& L, const float* rate, float& pa, float& pac) {
+    float s = 0.f, sc = 0.f;
+#pragma unroll 2
+    for (int j = g.rank(); j < p.M; j += g.size()) {
+        uint32_t o0, o1;
+        if (Grp::kWidth == 0 && p.chan8) {
+            const uint2 r = reinterpret_cast<const uint2*>(L.chan())[j];
+            o0 = r.x;
+            o1 = r.y;
+        } else {
+            const uint32_t r = L.chan()[j];
+            o0 = r & 0xffffu;
+            o1 = r >> 16;
+        }
+        const float f0 = at_byte(L.X(), o0), f1 = at_byte(L.X(), o1);
+        const float v = __ldg(rate + j) * fabsf(f0) * fabsf(f1);
+        const uint32_t cr = (__float_as_uint(f0) | __float_as_uint(f1)) & 0x80000000u;
+        L.a()[j] = __uint_as_float(__float_as_uint(v) | cr);
+        if constexpr (!is_thin<Grp>::value) {
+            s += v;
+            sc += cr ? v : 0.f;
+        }
+    }
+    g.sync();
+    if constexpr (is_thin<Grp>::value) {
+        // a[] is padded with zeros to whole blocks of four
+        for (int j = 0; j < p.M; j += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(L.a() + j);
+            s += fabsf(v.x);
+            sc += fmaxf(-v.x, 0.f);
+            s += fabsf(v.y);
+            sc += fmaxf(-v.y, 0.f);
+            s += fabsf(v.z);
+            sc += fmaxf(-v.z, 0.f);
+            s += fabsf(v.w);
+            sc += fmaxf(-v.w, 0.f);
+        }
+    }
+    pa = s;
+    pac = sc;
+}
+
+// One entry's term of mu and sigma^2.
+TL_D void add_moments(float v, float aj, float& mu, float& s2) {
+    const float t = v * aj;
+    mu += t;
+    s2 += v * t;
+}
+template <bool WIDE>
+TL_D void add_entry(const float* a, uint32_t e, float& mu, float& s2) {
+    // critical channels are stored negative: max(a, 0) drops them
+    // WIDE: models of 2^18 channels and more, beyond the 20-bit offsets
+    if constexpr (WIDE) add_moments(unpack_vf((int)e), fmaxf(a[e >> 3], 0.f), mu, s2);
+    else add_moments(__uint_as_float(e << 20), fmaxf(at_byte(a, e >> 12), 0.f), mu, s2);
+}
+
+// The CGP bound of a species (species_bound's values, without its branches:
+// g is 1, 2 or 2 + 1/(x - 1), with 3 below x = 2; a moment of 0, or below
+// FP32's normal range, bounds nothing).
+TL_D float row_bound(const SimParams& p, float xi, int kind, float mu, float s2) {
+    float gi = kind == 1 ? 1.f : 2.f;
+    if (kind == 3) gi = 2.f + __frcp_rn(fmaxf(xi - 1.f, 1.f));
+    const float num = fmaxf(p.eps * (xi * fast_rcp(gi)), 1.f);
+    return fminf(num * fast_rcp(fabsf(mu)), num * num * fast_rcp(s2));
+}
+
+// The CGP step bound (CSRMatrixPacked.cu:311-358).
+template <bool kWide, class Grp, class Lay>
+TL_D float fast_tau_rows(const Grp& g, const SimParams& p, const Lay& L) {
+    float tmin = kInfF;
+    if constexpr (Grp::kWidth == 0) {
+        if (p.row_warp) {
+            // long rows: one warp per row, lanes stride the entries
+#pragma unroll 1
+            for (int ii = g.warp; ii < p.n_rows; ii += g.nwarps) {
+                const uint2 rec = L.row()[ii];
+                const uint32_t* e = reinterpret_cast<const uint32_t*>(L.ent() + (rec.x & 0xfffffu));
+                const int n = 4 * (int)(rec.x >> 20);
+                float mu = 0.f, s2 = 0.f;
+                for (int q = g.lane; q < n; q += 32) add_entry<kWide>(L.a(), e[q], mu, s2);
+#pragma unroll
+                for (int o = 16; o; o >>= 1) {
+                    mu += __shfl_xor_sync(0xffffffffu, mu, o);
+                    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+                }
+                const float xi = fabsf(L.X()[rec.y & 0x0fffffffu]);
+                tmin = fminf(tmin, row_bound(p, xi, (int)(rec.y >> 28), mu, s2));
+            }
+            return g.minf(tmin);
+        }
+    }
+#pragma unroll 1
+    for (int ii = g.rank(); ii < p.n_rows; ii += g.size()) {
+        const uint2 rec = L.row()[ii];
+        const uint4* e = L.ent() + (rec.x & 0xfffffu);
+        const int n = (int)(rec.x >> 20);
+        float mu = 0.f, s2 = 0.f;
+#pragma unroll 1
+        for (int q = 0; q < n; ++q) {
+            const uint4 w = e[q];
+            add_entry<kWide>(L.a(), w.x, mu, s2);
+            add_entry<kWide>(L.a(), w.y, mu, s2);
+            add_entry<kWide>(L.a(), w.z, mu, s2);
+            add_entry<kWide>(L.a(), w.w, mu, s2);
+        }
+        const float xi = fabsf(L.X()[rec.y & 0x0fffffffu]);
+        tmin = fminf(tmin, row_bound(p, xi, (int)(rec.y >> 28), mu, s2));
+    }
+    return g.minf(tmin);
+}
+
+template <class Grp, class Lay>
+TL_D float fast_tau(const Grp& g, const SimParams& p, const Lay& L) {
+    if constexpr (Grp::kWidth == 0)
+        if (p.ent_wide) return fast_tau_rows<true>(g, p, L);
+    return fast_tau_rows<false>(g, p, L);
+}
+
+// Calls f(byte offset of the species in an int array, stoichiometry) for channel j's net entries.
+template <class Lay, class F>
+TL_D void for_column(const Lay& L, int j, F f) {
+    const SimParams& p = L.p;
+    int c0 = j, n = 1;
+    if (p.t_cp >= 0) {
+        c0 = (int)L.cp()[j];
+        n = (int)L.cp()[j + 1] - c0;
+    }
+#pragma unroll 1
+    for (int q = 0; q < n; ++q) {
+        const uint4 w = L.col()[c0 + q];
+        const uint32_t e[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (e[i] & 0xfffu) f(e[i] >> 12, (int)(e[i] << 20) >> 20);
+    }
+}
+
+// k firings of channel j.
+template <class Grp, class Lay>
+TL_D void fire_channel(const Lay& L, int j, int k) {
+    for_column(L, j, [&](uint32_t off, int v) {
+        if constexpr (Grp::kWidth == 1) at_byte(L.D(), off) += v * k;
+        else atomicAdd(&at_byte(L.D(), off), v * k);
+    });
+}
+
+
+// All of X from x.  D is zero.
+template <class Grp, class Lay>
+TL_D void fast_refresh(const Grp& g, const SimParams& p, const Lay& L) {
+#pragma unroll 1
+    for (int i = g.rank(); i < p.N; i += g.size()) set_species(L, i, L.x()[i]);
+    if (g.leader()) L.X()[p.x_one] = 1.f;
+}
+
+// The firing counts of one leap into D (and k[] in scored runs), for groups
+// of lanes.  Instruction issue bounds this pass, and most of it would go into
+// lanes that wait for a neighbour's long draw, were each lane to make its
+// channels' draws one at a time.
+//  * A channel whose mean lies in [0, 10) compares the shared word's
+//    u = 1 - q with F0 = exp(-mu) and F1 = F0 (1 + mu), both from one fast
+//    exponential and without a branch.  kFireMargin bounds what the fast forms
+//    and poisson_first's own tests together can be off (under 2.3e-6: the
+//    truncated word 1.8e-7, __expf 3.5e-7, poisson_p1 / p2 1.3e-6 and the
+//    sums), so outside the margin both give the same count.
+//  * Every other draw (k >= 2, within the margin, means >= 10) and every
+//    channel with k = 1 is marked in the lane's masks.  After at most
+//    q_rounds turns the lanes list their marked channels in a queue and take
+//    them in turn: inversions and single firings from the front,
+//    transformed-rejection draws (PTRS) from the back, so that a pass runs one
+//    kind on all lanes and a channel's firing is spread over the lanes with
+//    its draw.  A PTRS lane moves on to its next draw after an accepted
+//    attempt instead of waiting for the warp's last one.
+// a[] is padded to whole blocks of four; the padding holds 0.
+constexpr float kFireMargin = 5e-6f;
+constexpr int kMaxRounds = 7;  // marked channels of a queue group fit ten bits
+
+// One attempt of a queued draw of mean < 10 (poisson_first).  Attempt 0 is on
+// the shared word w: k <= 1 by the exact tests unless k >= 2 is settled, else
+// the sequential search.  Where the FP32 sums stop growing below u, attempts
+// 1 to 16 search on fresh uniforms w (poisson_inversion).  False: try again.
+TL_D bool queued_inversion(float mu, uint32_t w, int attempt, int& k) {
+    float u, pk, F;
+    const float e = expf(-mu);
+    if (attempt == 0) {
+        const float qf = ((float)w + 0.5f) * 2.3283064365386963e-10f;
+        u = 1.f - qf;
+        if (fmaf(e, mu, e) - u > -kFireMargin) {
+            k = 0;
+            if (qf >= poisson_p1(mu)) return true;
+            k = 1;
+            if (qf >= poisson_p2(mu)) return true;
+        }
+        pk = e * mu;
+        F = e + pk;
+        k = 1;
+    } else {
+        u = u01f(w);
+        pk = F = e;
+        k = 0;
+        if (u <= F) return true;
+    }
+    float kf = (float)k, last;
+#pragma unroll 1
+    do {
+        last = F;
+        kf += 1.f;
+        pk = pk * (mu * fast_rcp(kf));
+        F = last + pk;
+    } while (u > F && F != last);
+    if (u <= F) {
+        k = (int)kf;
+        return true;
+    }
+    k = (int)mu;  // u above the representable mass
+    return attempt == 16;
+}
+
+template <class Grp, class Lay, bool SENS>
+TL_D void fast_fire(const Grp& g, const SimParams& p, const Lay& L, float tauf, int jc, uint32_t step,
+                    uint32_t r, uint32_t set) {
+    const auto qg = queue_group(g);
+    constexpr int kTurn = 4 * decltype(queue_group(g))::kWidth;  // channels of a queue group's turn
+    const int cap = p.q_rounds * kTurn;
+    unsigned short* q = L.q();
+    if constexpr (Grp::kWidth == 0) q += g.warp * (cap + 2);
+    const float* a = L.a();
+    const int G4 = (p.M + 3) >> 2;
+    for (int b0 = g.rank() - qg.rank(); b0 < G4;) {
+        const int j_first = 4 * b0;
+        unsigned inv = 0, big = 0, one = 0;  // this lane's marked channels, four bits a turn
+        int sh = 0;
+#pragma unroll 1
+        for (int m = 0; m < p.q_rounds && b0 < G4; ++m, b0 += g.size(), sh += 4) {
+            const int g4 = b0 + qg.rank();
+            if (g4 >= G4) continue;
+            const float4 v4 = *reinterpret_cast<const float4*>(a + 4 * g4);
+            const float av[4] = {v4.x, v4.y, v4.z, v4.w};
+            float mu[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) mu[e] = fmaxf(av[e], 0.f) * tauf;  // critical channels: 0
+            U4 gw{0u, 0u, 0u, 0u};
+            if (fminf(fminf(mu[0], mu[1]), fminf(mu[2], mu[3])) < 10.f)
+                gw = group_words(p.rk, (uint32_t)g4, step, r, set);
+            unsigned all = 0, far = 0, fired = 0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float ex = __expf(-mu[e]);
+                // 2 - (1 - q) from the word's top 23 bits
+                const float v = __uint_as_float((word_of(gw, e) >> 9) | 0x3f800000u);
+                const float d0 = v + (ex - 2.f);          // F0 - u
+                const float d1 = fmaf(ex, mu[e], d0);     // F1 - u >= F0 - u
+                const bool is_far = mu[e] >= 10.f;
+                if (d1 < kFireMargin || fabsf(d0) < kFireMargin || is_far) all |= 1u << e;
+                if (is_far) far |= 1u << e;
+                if (d0 < 0.f) fired |= 1u << e;
+            }
+            inv |= (all & ~far) << sh;
+            big |= far << sh;
+            fired &= ~all;
+            one |= fired << sh;
+            if constexpr (SENS)
+                *reinterpret_cast<int4*>(L.k() + 4 * g4) =
+                    make_int4(fired & 1, fired >> 1 & 1, fired >> 2 & 1, fired >> 3);
+        }
+        if (!qg.any((inv | big | one) != 0u)) continue;
+        // list the marked channels: positions from one scan of the counts
+        const unsigned mine =
+            (unsigned)__popc(inv) | (unsigned)__popc(one) << 10 | (unsigned)__popc(big) << 20;
+        const unsigned upto = qg.incl_scan(mine);
+        const unsigned total = qg.bcast(upto, qg.size() - 1), before = upto - mine;
+        const int n_inv = (int)(total & 1023u), n_front = n_inv + (int)(total >> 10 & 1023u), n_big = (int)(total >> 20);
+        const auto list = [&](unsigned marks, int at, int by) {
+            while (marks) {
+                const int bit = __ffs(marks) - 1;
+                marks &= marks - 1;
+                q[at] = (unsigned short)((bit >> 2) * kTurn + qg.rank() * 4 + (bit & 3));
+                at += by;
+            }
+        };
+        list(inv, (int)(before & 1023u), 1);
+        list(one, n_inv + (int)(before >> 10 & 1023u), 1);
+        list(big, cap - 1 - (int)(before >> 20), -1);
+        int* next = reinterpret_cast<int*>(q + cap);
+        if (qg.rank() == 0) *next = 0;
+        qg.sync();
+        const auto channel = [&](int id) {
+            if constexpr (Grp::kWidth == 0) return j_first + (id / kTurn) * 4 * g.size() + id % kTurn;
+            else return j_first + id;
+        };
+        for (int i = qg.rank(); i < n_front; i += qg.size()) {
+            const int j = channel(q[i]);
+            int k = 1;
+            if (i < n_inv) {
+                const float mu = fmaxf(a[j], 0.f) * tauf;
+                U4 w = group_words(p.rk, (uint32_t)j >> 2, step, r, set);
+                uint32_t word = word_of(w, j & 3);
+                for (int it = 0; !queued_inversion(mu, word, it, k); ++it) {
+                    w = philox10(U4{(uint32_t)j, step, r, (set << 8) + (uint32_t)(it >> 2)}, p.k0, p.k1);
+                    word = word_of(w, it & 3);
+                }
+                if constexpr (SENS) L.k()[j] = k;
+            }
+            fire_channel<Grp>(L, j, k);
+        }
+        // PTRS draws need one to several attempts: a lane that is done with
+        // one takes the next that no lane has.  (A counter for the others too
+        // cost the colloid model 14 %.)
+        if (n_big) {
+            int it = 0;  // attempts so far on this draw
+            for (int i = atomicAdd(next, 1); i < n_big;) {
+                const int j = channel(q[cap - 1 - i]);
+                const float mu = a[j] * tauf;
+                const U4 w = philox10rk(U4{(uint32_t)j, step, r, (set << 8) + (uint32_t)(it >> 1)}, p.rk);
+                const bool odd = it & 1;
+                int k;
+                bool ok = Ptrs(mu).attempt(u01f(odd ? w.z : w.x), u01f(odd ? w.w : w.y), k);
+                if (++it == kPtrsTries && !ok) {
+                    k = (int)(mu + 0.5f);
+                    ok = true;
+                }
+                if (ok) {
+                    if constexpr (SENS) L.k()[j] = k;
+                    fire_channel<Grp>(L, j, k);
+                    it = 0;
+                    i = atomicAdd(next, 1);
+                }
+            }
+        }
+        qg.sync();
+    }
+    // the critical channel that fires, by the lane that owns its block
+    if (jc >= 0 && (jc >> 2) % g.size() == g.rank()) {
+        if constexpr (SENS) L.k()[jc] = 1;
+        fire_channel<Grp>(L, jc, 1);
+    }
+}
+
+// The same for thin groups: each lane draws its channels in place.
+template <int W, class Lay, bool SENS>
+TL_D void thin_fire(const GThin<W>& g, const SimParams& p, const Lay& L, float tauf, int jc, uint32_t step,
+                    uint32_t r, uint32_t set) {
+    for (int j = g.rank(); j < p.M; j += W) {
+        const float aj = L.a()[j];
+        int k = 0;
+        if (is_crit(aj)) {
+            k = j == jc ? 1 : 0;
+        } else {
+            const float mu = aj * tauf;
+            if (mu > 0.f) {
+                ChanRng rng;
+                rng.init((uint32_t)j, step, r, set, p.rk);
+                if (mu >= 10.f) {
+                    k = poisson_ptrs(mu, rng);
+                } else {
+                    const U4 gw = group_words(p.rk, (uint32_t)j >> 2, step, r, set);
+                    const uint32_t w = word_of(gw, j & 3);
+                    // P(K >= 1) as computed never exceeds mu
+                    if (((float)w + 0.5f) * 2.3283064365386963e-10f < mu) k = poisson_first(mu, w, rng);
+                }
+            }
+        }
+        if constexpr (SENS) L.k()[j] = k;
+        if (k) fire_channel<GThin<W>>(L, j, k);
+    }
+}
+
+// x + D: any population negative?  (or past the population type, in *over)
+template <class Grp, class Lay>
+TL_D bool fast_check(const Grp& g, const SimParams& p, const Lay& L, bool& over) {
+    using Pop = typename Lay::Pop;
+    bool bad = false, of = false;
+#pragma unroll 2
+    for (int i = g.rank(); i < p.N; i += g.size()) {
+        const int d = L.D()[i];
+        if constexpr (sizeof(Pop) == 4) {
+            const int nx = (int)((unsigned)L.x()[i] + (unsigned)d);
+            bad |= nx < 0;
+            of |= nx < 0 && d > 0;  // wrapped: |D| < 2^31
+        } else {
+            bad |= L.x()[i] + (Pop)d < 0;
+        }
+    }
+    const bool b = g.any(bad);
+    over = false;
+    if (sizeof(Pop) == 4 && b) over = g.any(of);
+    return b;
+}
+
+template <class Grp, class Lay>
+TL_D void fast_commit(const Grp& g, const SimParams& p, const Lay& L) {
+    using Pop = typename Lay::Pop;
+#pragma unroll 2
+    for (int i = g.rank(); i < p.N; i += g.size()) {
+        const Pop nx = L.x()[i] + (Pop)L.D()[i];
+        L.x()[i] = nx;
+        L.D()[i] = 0;
+        set_species(L, i, nx);
+    }
+    if (g.leader()) L.X()[p.x_one] = 1.f;
+}
+
+// A leap that may hold more than 10^8 firings, whose sums could leave int32:
+// the counts are drawn in place and added in 64 bits, over D and X together.
+// Returns as fast_check and commits where that allows it.
+constexpr float kWideLeap = 1e8f;
+
+template <class Grp, class Lay, bool SENS>
+TL_D bool wide_leap(const Grp& g, const SimParams& p, const Lay& L, float tauf, int jc, uint32_t step, uint32_t r,
+                    uint32_t set, bool& over) {
+    using Pop = typename Lay::Pop;
+    unsigned long long* D64 = reinterpret_cast<unsigned long long*>(L.D());
+#pragma unroll 1
+    for (int i = g.rank(); i < p.N; i += g.size()) D64[i] = 0ull;
+    g.sync();
+#pragma unroll 1
+    for (int j = g.rank(); j < p.M; j += g.size()) {
+        const float aj = L.a()[j];
+        int k = 0;
+        if (is_crit(aj)) {
+            k = j == jc ? 1 : 0;
+        } else {
+            const U4 gw = group_words(p.rk, (uint32_t)j >> 2, step, r, set);
+            ChanRng rng;
+            rng.init((uint32_t)j, step, r, set, p.rk);
+            k = poisson_first(aj * tauf, word_of(gw, j & 3), rng);
+        }
+        if constexpr (SENS) L.k()[j] = k;
+        for_column(L, j, [&](uint32_t off, int v) { atomicAdd(&D64[off >> 2], (unsigned long long)((long long)v * k)); });
+    }
+    g.sync();
+    bool bad = false, of = false;
+#pragma unroll 1
+    for (int i = g.rank(); i < p.N; i += g.size()) {
+        const long long nx = (long long)L.x()[i] + (long long)D64[i];
+        of |= sizeof(Pop) == 4 && nx > 2147483647LL;
+        bad |= nx < 0 || of;
+    }
+    over = g.any(of);
+    bad = g.any(bad);
+    if (!bad)
+#pragma unroll 1
+        for (int i = g.rank(); i < p.N; i += g.size()) L.x()[i] = (Pop)((long long)L.x()[i] + (long long)D64[i]);
+    g.sync();
+#pragma unroll 1
+    for (int i = g.rank(); i < p.N; i += g.size()) L.D()[i] = 0;
+    if (!bad) fast_refresh(g, p, L);
+    g.sync();
+    return bad;
+}
+
+// ---------------------------------------------------------------------------
+// Direct-method steps: the channel with probability a_j / a0 and a0 in FP32.
+// ---------------------------------------------------------------------------
+// Thin groups: one running sum in channel order, target u * a0 with u of 52
+// bits.  FP32 decides every channel whose running sum is further from the
+// target than the products' rounding (2^-23 a0, margin 4e-7 a0); the FP64
+// target decides the others.
+template <int W, class Lay>
+TL_D int thin_select(const GThin<W>& g, const SimParams& p, const Lay& L, float part, uint32_t w_hi,
+                     uint32_t w_lo) {
+    const float t = ((float)(w_hi >> 6) * 1.4901161193847656e-08f) * part;  // 2^-26
+    const float m = 4e-7f * part;
+    float acc = 0.f;
+    int last = -1;
+    for (int j = 0; j < p.M; ++j) {
+        const float v = fabsf(L.a()[j]);
+        if (!(v > 0.f)) continue;
+        acc += v;
+        last = j;
+        if (acc > t + m) break;
+        if (acc >= t - m && __double2float_rd(u01d(w_hi, w_lo) * (double)part) < acc) break;
+    }
+    return last;
+}
+
+// Lane groups.  The lanes' partial sums are put on one integer grid, the lsb
+// of the largest one's exponent - 24; when every partial lies on it, the FP64
+// sums of the general form are exact too, and 64-bit integers give a0, the
+// cumulative sums and the target.  Where a partial falls off the grid, the
+// target lies within the FP64 product's rounding of a lane's boundary, or the
+// search inside a lane of several channels comes within FP32 rounding, the
+// FP64 form decides (select_channel_impl).  GB300's FP64 rate is 1/64 of FP32:
+// the FP64 butterfly and scan took 82 % of that pipe on a 12 x 20 network.
+template <class Grp, class Lay>
+__device__ __noinline__ int ssa_select_fp64(const Grp g, const SimParams& p, const Lay& L, float part, uint32_t w_hi,
+                                            uint32_t w_lo, float& a0f) {
+    const double a0 = g.sumd((double)part);
+    a0f = (float)a0;
+    return select_channel_impl<Grp, double>(g, p.M, L.a(), part, u01d(w_hi, w_lo) * a0, 0);
+}
+
+template <class Grp, class Lay>
+TL_D int ssa_select(const Grp& g, const SimParams& p, const Lay& L, float part, uint32_t w_hi, uint32_t w_lo,
+                    float& a0f) {
+    const uint32_t bits = __float_as_uint(part);
+    const int e = (int)(bits >> 23);
+    const int emax = (int)g.max_int(e);
+    const int eb = emax - 24;
+    const bool off = bits != 0u && e < eb;
+    if (emax < 60 || emax > 250 || g.any(off)) return ssa_select_fp64(g, p, L, part, w_hi, w_lo, a0f);
+    unsigned long long F = 0ull;
+    if (bits) F = (unsigned long long)((bits & 0x7fffffu) | 0x800000u) << (e - eb);
+    // inclusive scan; the last lane holds the total
+    unsigned long long P = F;
+#pragma unroll
+    for (int o = 1; o < Grp::kWidth; o <<= 1) {
+        const unsigned long long n = g.shfl_up(P, o);
+        if (g.rank() >= o) P += n;
+    }
+    const unsigned long long S = g.bcast(P, g.size() - 1);
+    const float unit = __uint_as_float((uint32_t)(eb - 23) << 23);  // value of the grid's lsb; eb >= 36
+    a0f = __ull2float_rn(S) * unit;
+    // floor of u * S, u = (2k + 1) 2^-53 with k of 52 bits
+    const unsigned long long k2 = (((unsigned long long)(w_hi >> 6) << 26 | (w_lo >> 6)) << 1) | 1ull;
+    const unsigned long long T = __umul64hi(k2 << 11, S);
+    // general form: target < excl + part = P with target = u * S rounded to FP64
+    bool close = F != 0ull && T + 1ull == P;
+    const int first = g.first(F != 0ull && T < P);
+    const int Ls = first >= 0 ? first : g.last(F != 0ull);
+    int sel = -1;
+    if (g.rank() == Ls && !close) {
+        const float tf = __ull2float_rn(T + F - P) * unit;  // target - excl
+        float acc = 0.f;
+        for (int j = g.rank(); j < p.M; j += g.size()) {
+            const float v = fabsf(L.a()[j]);
+            if (!(v > 0.f)) continue;
+            acc += v;
+            sel = j;
+            if (j + g.size() < p.M) {  // not the lane's last channel
+                if (fabsf(acc - tf) <= 4e-7f * part) {
+                    close = true;
+                    break;
+                }
+                if (tf < acc) break;
+            }
+        }
+    }
+    if (g.any(close)) return ssa_select_fp64(g, p, L, part, w_hi, w_lo, a0f);
+    return g.bcast(sel, Ls);
+}
+
+
+// ---------------------------------------------------------------------------
+// One step (model.cu:301-413): a tau-leap with rejection and halving, or one
+// direct-method step.
+// ---------------------------------------------------------------------------
+// Every leap attempt and every direct-method step advances the Philox step
+// counter once: accepted steps = step - rej, leaps = accepted - ssa.
+struct FastState {
+    double t;
+    double t_next;  // grid time kpt; done may be set before the last point: the state holds
+    int kpt;        // next grid point to record
+    uint32_t step;
+    uint32_t rej, ssa;
+    int ssa_left;  // direct-method steps left in the block
+    bool wide;     // the next step is a wide leap
+    bool done;
+};
+
+// Index of realization r of a set in this call's samples and scores.
+TL_D size_t realization_index(const SimParams& p, int set, uint32_t r) {
+    return (size_t)((long long)set * p.R + ((long long)r - p.r_off));
+}
+
+template <class Grp, class Lay>
+TL_D void fast_record(const Grp& g, const SimParams& p, const Lay& L, int set, uint32_t r, int kpt) {
+    using Pop = typename Lay::Pop;
+    Pop* samp = reinterpret_cast<Pop*>(p.samples) + realization_index(p, set, r) * (p.n_int + 1) * p.K;
+    samp += (size_t)kpt * p.K;
+#pragma unroll 1
+    for (int q = g.rank(); q < p.K; q += g.size()) samp[q] = L.x()[p.tracked[q]];
+}
+
+// Records the state at the next grid point.
+template <class Grp, class Lay>
+TL_D void record_next(const Grp& g, const SimParams& p, const Lay& L, int set, uint32_t r, FastState& st) {
+    fast_record(g, p, L, set, r, st.kpt++);
+    if (st.kpt <= p.n_int) st.t_next = grid_time<double>(p, set, st.kpt);
+}
+
+// score_m += term(m) / c_m over the group's channels.
+template <class Grp, class Lay, class F>
+TL_D void add_scores(const Grp& g, const SimParams& p, const Lay& L, int set, uint32_t r, F term) {
+    float* score = L.score((long long)realization_index(p, set, r));
+    const float* c0 = p.rates + (size_t)set * p.M;
+#pragma unroll 1
+    for (int m = g.rank(); m < p.M; m += g.size()) {
+        const float c = __ldg(c0 + m);
+        if (c > 0.f) score[m] += term(m) / c;
+    }
+}
+
+template <class Grp, class Lay, bool SENS, bool WIDE>
+TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uint32_t r, FastState& st) {
+    using Pop = typename Lay::Pop;
+    constexpr bool kThin = is_thin<Grp>::value;
+    const float* rate = p.frates + (size_t)set * p.M;  // halved for 2S
+    float pa, pac;
+    fast_props(g, p, L, rate, pa, pac);
+    float tau1 = 0.f, a0f = 0.f;
+    if (st.ssa_left == 0) {
+        if constexpr (kThin) a0f = pa;
+        else a0f = g.sumf(pa);
+        if (a0f > 0.f) {
+            tau1 = fast_tau(g, p, L);
+            if (tau1 * a0f < p.ssa_factor) st.ssa_left = p.ssa_block;
+        } else {
+            st.done = true;
+        }
+    } else if (!g.any(pa > 0.f)) {
+        st.done = true;
+    }
+    if (st.done) return;  // nothing can fire: the state holds to t_final
+
+    if (!WIDE && st.ssa_left > 0) {
+        // ---- direct method, a block of ssa_block steps (CGP 2006 step 2; model.cu:334-345) ----
+        const U4 w = step_words(p.rk, st.step, r, (uint32_t)set);
+        int j;
+        float a0;  // total for the waiting time
+        if constexpr (kThin) {
+            a0 = pa;
+            j = thin_select(g, p, L, pa, w.z, w.w);
+        } else if constexpr (Grp::kWidth == 0) {
+            const double total = g.sumd((double)pa);
+            a0 = (float)total;
+            j = select_channel<Grp, double>(g, p, L.a(), pa, u01d(w.z, w.w) * total, 0);
+        } else {
+            j = ssa_select(g, p, L, pa, w.z, w.w, a0);
+        }
+        // the waiting time in FP32 (FP64 keeps only the time sum)
+        const double dt = (double)(-logf(u01f(w.x)) / a0);
+        const double t_new = st.t + dt;
+        while (st.kpt <= p.n_int && t_new >= st.t_next) record_next(g, p, L, set, r, st);
+        if (st.kpt > p.n_int) {
+            if (SENS && p.scores) {
+                const float rem = (float)(p.t_final[set] - st.t);
+                add_scores(g, p, L, set, r, [&](int m) { return -(fabsf(L.a()[m]) * rem); });
+            }
+            st.done = true;
+            g.sync();
+            return;
+        }
+        if (SENS && p.scores) {
+            const float dtf = (float)dt;
+            add_scores(g, p, L, set, r,
+                       [&](int m) { return (m == j ? 1.f : 0.f) - fabsf(L.a()[m]) * dtf; });
+        }
+        g.sync();
+        if (j >= 0) {
+            // the channel's entries, one lane each (the first lane of thin groups takes all)
+            int c0 = j, n = 1;
+            if (p.t_cp >= 0) {
+                c0 = (int)L.cp()[j];
+                n = (int)L.cp()[j + 1] - c0;
+            }
+            constexpr int kBy = Grp::kWidth == 1 || Grp::kWidth == 2 ? Grp::kWidth : 4;
+            if (g.rank() < kBy)
+                for (int e = 4 * c0 + g.rank(); e < 4 * (c0 + n); e += kBy) {
+                    const uint32_t en = reinterpret_cast<const uint32_t*>(L.col())[e];
+                    if (!(en & 0xfffu)) continue;
+                    const int i = (int)(en >> 14);
+                    const Pop nx = L.x()[i] + (Pop)((int)(en << 20) >> 20);
+                    L.x()[i] = nx;
+                    set_species(L, i, nx);
+                }
+        }
+        g.sync();
+        st.t = t_new;
+        st.step++;
+        st.ssa++;
+        st.ssa_left--;
+        return;
+    }
+
+    if (!WIDE && tau1 * a0f >= kWideLeap && a0f * (float)(st.t_next - st.t) >= kWideLeap) {
+        st.wide = true;  // nothing has changed: wide_step starts over
+        return;
+    }
+
+    // ---- tau-leap with negative-population rejection (CGP 2006 steps 3-5) ----
+    double t_new;    // time after the leap (unless clamped to the next grid time)
+    float tau_used;  // the leap's tau
+    bool clamp;
+    float a0cf;
+    if constexpr (kThin) a0cf = pac;
+    else a0cf = g.sumf(pac);
+    for (int attempt = 0;; ++attempt) {
+        // the step's scalar words are needed only when a channel is critical
+        float tau2 = kInfF;
+        U4 w{0u, 0u, 0u, 0u};
+        if (a0cf > 0.f) {
+            w = step_words(p.rk, st.step, r, (uint32_t)set);
+            tau2 = -logf(u01f(w.x)) / a0cf;
+        }
+        float tauf = fminf(tau1, tau2);
+        bool fire = tau2 < tau1;
+        t_new = st.t + (double)tauf;
+        clamp = t_new >= st.t_next;
+        if (clamp) {
+            tauf = (float)(st.t_next - st.t);
+            fire = false;
+        }
+        tau_used = tauf;
+        int jc = -1;
+        if (fire) {
+            if constexpr (kThin) {
+                const double a0c = (double)pac;
+                jc = select_channel<G1, double>(G1{}, p, L.a(), pac, u01d(w.z, w.w) * a0c, 1);
+            } else {
+                const double a0c = g.sumd((double)pac);
+                jc = select_channel<Grp, double>(g, p, L.a(), pac, u01d(w.z, w.w) * a0c, 1);
+            }
+        }
+        bool over = false, bad;
+        if constexpr (WIDE) {
+            bad = wide_leap<Grp, Lay, SENS>(g, p, L, tauf, jc, st.step, r, (uint32_t)set, over);
+        } else {
+            if constexpr (kThin) thin_fire<Grp::kWidth, Lay, SENS>(g, p, L, tauf, jc, st.step, r, (uint32_t)set);
+            else fast_fire<Grp, Lay, SENS>(g, p, L, tauf, jc, st.step, r, (uint32_t)set);
+            g.sync();
+            bad = fast_check(g, p, L, over);
+            if (!bad) {
+                fast_commit(g, p, L);
+            } else {
+#pragma unroll 1
+                for (int i = g.rank(); i < p.N; i += g.size()) L.D()[i] = 0;
+                g.sync();
+            }
+        }
+        if (over) {
+            if (g.leader()) atomicOr((unsigned*)(p.ctr + 5), kErrOverflow);
+            st.done = true;
+            return;
+        }
+        if (!bad) break;
+        // reject: halve tau1, fresh counters, same state and propensities
+        st.step++;
+        st.rej++;
+        tau1 *= 0.5f;
+        if (attempt + 1 > p.max_halv) {
+            if (g.leader()) atomicOr((unsigned*)(p.ctr + 5), kErrHalving);
+            st.done = true;
+            return;
+        }
+    }
+    if (SENS && p.scores) {
+        // score_j += (k_j - a_j*tau)/c_j with a_j of the pre-leap state
+        add_scores(g, p, L, set, r, [&](int m) { return (float)L.k()[m] - fabsf(L.a()[m]) * tau_used; });
+    }
+    g.sync();
+    st.step++;
+    if (clamp) {
+        st.t = st.t_next;
+        record_next(g, p, L, set, r, st);
+        if (st.kpt > p.n_int) st.done = true;
+    } else {
+        st.t = t_new;
+    }
+}
+
+// The same step as a wide leap, out of line.
+template <class Grp, class Lay, bool SENS>
+__device__ __noinline__ void wide_step(const Grp g, const SimParams& p, const Lay L, int set, uint32_t r,
+                                       FastState* st) {
+    st->wide = false;
+    fast_step<Grp, Lay, SENS, true>(g, p, L, set, r, *st);
+}
+
+// One realization from x0 to t_final.  The step counts go straight to the
+// run's counters (one atomic each), so no totals stay live across the loop.
+template <class Grp, class Lay, bool SENS>
+TL_D void fast_realization(const Grp& g, const SimParams& p, const Lay& L, long long w) {
+    using Pop = typename Lay::Pop;
+    const int set = p.S == 1 ? 0 : (int)(w / p.R);
+    const uint32_t r = (uint32_t)(p.r_off + w - (long long)set * p.R);
+    const Pop* x0 = reinterpret_cast<const Pop*>(p.x0);
+    for (int i = g.rank(); i < p.N; i += g.size()) {
+        L.x()[i] = x0[i];
+        L.D()[i] = 0;
+    }
+    // the padding of a[]: the rest of the last block of four, and the block
+    // that the padding of the rows reads
+    for (int j = p.M + g.rank(); j < ((p.M + 3) & ~3) + 4; j += g.size()) L.a()[j] = 0.f;
+    if (SENS && p.scores)
+        for (int j = g.rank(); j < p.M; j += g.size()) L.score(w)[j] = 0.f;
+    g.sync();
+    fast_refresh(g, p, L);
+    fast_record(g, p, L, set, r, 0);
+    g.sync();
+    FastState st{0.0, grid_time<double>(p, set, 1), 1, 0u, 0u, 0u, 0, false, false};
+    bool trunc = false;
+    while (!st.done) {
+        fast_step<Grp, Lay, SENS, false>(g, p, L, set, r, st);
+        if (st.wide) {
+            FastState tmp = st;
+            wide_step<Grp, Lay, SENS>(g, p, L, set, r, &tmp);
+            st = tmp;
+        }
+        if (!st.done && p.max_steps > 0 && (long long)(st.step - st.rej) >= p.max_steps) {
+            st.done = true;
+            trunc = true;
+        }
+    }
+    // a realization that ends early holds its state on the rest of the grid
+#pragma unroll 1
+    while (st.kpt <= p.n_int) fast_record(g, p, L, set, r, st.kpt++);
+    g.sync();
+    if (SENS && p.scores && !p.score_global) {
+        float* to = p.scores + realization_index(p, set, r) * p.M;
+        for (int j = g.rank(); j < p.M; j += g.size()) to[j] = L.score(0)[j];
+    }
+    if (g.leader()) {
+        const uint32_t leaps = st.step - st.rej - st.ssa;
+        if (leaps) atomicAdd(p.ctr + 1, (unsigned long long)leaps);
+        if (st.ssa) atomicAdd(p.ctr + 2, (unsigned long long)st.ssa);
+        if (st.rej) atomicAdd(p.ctr + 3, (unsigned long long)st.rej);
+        if (trunc) atomicAdd(p.ctr + 4, 1ull);
+    }
+    g.sync();
+}
+
+}  // namespace tl
