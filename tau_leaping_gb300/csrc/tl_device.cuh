@@ -486,6 +486,7 @@ struct GWarp {
         return v;
     }
     TL_D int max_int(int v) const { return __reduce_max_sync(0xffffffffu, v); }
+    TL_D unsigned sum_uint(unsigned v) const { return __reduce_add_sync(0xffffffffu, v); }
     TL_D unsigned long long shfl_up(unsigned long long v, int o) const { return __shfl_up_sync(0xffffffffu, v, o); }
     TL_D double excl_scan(double v) const {
         double s = v;
@@ -560,6 +561,11 @@ struct GSub {
     TL_D int max_int(int v) const {
 #pragma unroll
         for (int o = W / 2; o; o >>= 1) v = max(v, __shfl_xor_sync(mask, v, o, W));
+        return v;
+    }
+    TL_D unsigned sum_uint(unsigned v) const {
+#pragma unroll
+        for (int o = W / 2; o; o >>= 1) v += __shfl_xor_sync(mask, v, o, W);
         return v;
     }
     TL_D unsigned long long shfl_up(unsigned long long v, int o) const { return __shfl_up_sync(mask, v, o, W); }

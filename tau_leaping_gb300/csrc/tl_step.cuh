@@ -139,6 +139,18 @@ TL_D const T& at_byte(const T* p, uint32_t off) {
 TL_D float with_sign(float f, int s) {
     return __uint_as_float((__float_as_uint(f) & 0x7fffffffu) | ((uint32_t)s & 0x80000000u));
 }
+// FP32 -> FP64 and FP64 >= on integers: GB300 runs FP64 at 1/64 of the FP32
+// rate, and a step needs one addition of it.
+TL_D double widen(float f) {
+    const uint32_t b = __float_as_uint(f);
+    if (b - 0x00800000u < 0x7f000000u)  // normal and positive
+        return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+    return (double)f;
+}
+TL_D bool reached(double t, double limit) {  // both >= 0
+    return __double_as_longlong(t) >= __double_as_longlong(limit);
+}
+
 // Species i holds x: its entries of X.  Populations and thresholds are >= 0,
 // so the sign of x - n_c is the criticality.
 template <class Lay>
@@ -172,7 +184,8 @@ TL_D void set_species(const Lay& L, int i, long long x) {
 template <class Grp, class Lay>
 TL_D void fast_props(const Grp& g, const SimParams& p, const Lay& L, const float* rate, float& pa, float& pac) {
     float s = 0.f, sc = 0.f;
-#pragma unroll 2
+    constexpr int kUnroll = is_thin<Grp>::value ? 4 : 2;
+#pragma unroll kUnroll
     for (int j = g.rank(); j < p.M; j += g.size()) {
         uint32_t o0, o1;
         if (Grp::kWidth == 0 && p.chan8) {
@@ -632,18 +645,36 @@ template <int W, class Lay>
 TL_D int thin_select(const GThin<W>& g, const SimParams& p, const Lay& L, float part, uint32_t w_hi,
                      uint32_t w_lo) {
     const float t = ((float)(w_hi >> 6) * 1.4901161193847656e-08f) * part;  // 2^-26
-    const float m = 4e-7f * part;
+    const float m = 4e-7f * part, above = t + m, below = t - m;
     float acc = 0.f;
-    int last = -1;
-    for (int j = 0; j < p.M; ++j) {
-        const float v = fabsf(L.a()[j]);
-        if (!(v > 0.f)) continue;
-        acc += v;
-        last = j;
-        if (acc > t + m) break;
-        if (acc >= t - m && __double2float_rd(u01d(w_hi, w_lo) * (double)part) < acc) break;
+    int sel = -1, last = -1;
+    bool close = false;
+    // four channels a turn without a branch; the padding is 0
+#pragma unroll 1
+    for (int j = 0; j < p.M && sel < 0; j += 4) {
+        const float4 v4 = *reinterpret_cast<const float4*>(L.a() + j);
+        const float v[4] = {fabsf(v4.x), fabsf(v4.y), fabsf(v4.z), fabsf(v4.w)};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            acc += v[e];
+            const bool some = v[e] > 0.f;
+            close |= some && acc >= below && acc <= above;
+            if (some && sel < 0 && acc > above) sel = j + e;
+            if (some) last = j + e;
+        }
     }
-    return last;
+    if (close) {
+        const float tf = __double2float_rd(u01d(w_hi, w_lo) * (double)part);
+        acc = 0.f;
+        sel = -1;
+#pragma unroll 1
+        for (int j = 0; j < p.M && sel < 0; ++j) {
+            const float v = fabsf(L.a()[j]);
+            acc += v;
+            if (v > 0.f && tf < acc) sel = j;
+        }
+    }
+    return sel >= 0 ? sel : last;
 }
 
 // Lane groups.  The lanes' partial sums are put on one integer grid, the lsb
@@ -654,6 +685,17 @@ TL_D int thin_select(const GThin<W>& g, const SimParams& p, const Lay& L, float 
 // search inside a lane of several channels comes within FP32 rounding, the
 // FP64 form decides (select_channel_impl).  GB300's FP64 rate is 1/64 of FP32:
 // the FP64 butterfly and scan took 82 % of that pipe on a 12 x 20 network.
+// S to FP32, to nearest even, for 2^32 <= S < 2^53 (the largest partial alone
+// is 2^47): the conversion instruction runs at the FP64 rate.
+TL_D float round53(unsigned long long S) {
+    const int lz = __clz((int)(S >> 32));
+    const unsigned long long X = S << lz;  // top bit at 63
+    uint32_t m = (uint32_t)(X >> 40);
+    const unsigned long long rest = X & ((1ull << 40) - 1), half = 1ull << 39;
+    m += rest > half || (rest == half && (m & 1u)) ? 1u : 0u;
+    return (float)m * __uint_as_float((uint32_t)(127 + 40 - lz) << 23);
+}
+
 template <class Grp, class Lay>
 __device__ __noinline__ int ssa_select_fp64(const Grp g, const SimParams& p, const Lay& L, float part, uint32_t w_hi,
                                             uint32_t w_lo, float& a0f) {
@@ -673,6 +715,22 @@ TL_D int ssa_select(const Grp& g, const SimParams& p, const Lay& L, float part, 
     if (emax < 60 || emax > 250 || g.any(off)) return ssa_select_fp64(g, p, L, part, w_hi, w_lo, a0f);
     unsigned long long F = 0ull;
     if (bits) F = (unsigned long long)((bits & 0x7fffffu) | 0x800000u) << (e - eb);
+    // u = k2 2^-53 and, below, T = floor(u S)
+    const unsigned long long k2 = (((unsigned long long)(w_hi >> 6) << 26 | (w_lo >> 6)) << 1) | 1ull;
+    const float unit = __uint_as_float((uint32_t)(eb - 23) << 23);  // value of the grid's lsb; eb >= 36
+    if (p.M <= g.size()) {
+        // one channel a lane: the sums of the halves, and the cumulative sums
+        // of the top 27 bits, which place the target up to 33 units
+        const uint32_t hi = (uint32_t)(F >> 24), lo = (uint32_t)F & 0xffffffu;
+        const unsigned long long S = ((unsigned long long)g.sum_uint(hi) << 24) + g.sum_uint(lo);
+        a0f = round53(S) * unit;
+        const uint32_t T = (uint32_t)(__umul64hi(k2 << 11, S) >> 21);
+        const uint32_t P = g.incl_scan(hi << 3 | lo >> 21);
+        const bool some = F != 0ull;
+        if (g.any(some && T >= P && T - P < 33u)) return ssa_select_fp64(g, p, L, part, w_hi, w_lo, a0f);
+        const int first = g.first(some && T < P);
+        return first >= 0 ? first : g.last(some);
+    }
     // inclusive scan; the last lane holds the total
     unsigned long long P = F;
 #pragma unroll
@@ -681,10 +739,7 @@ TL_D int ssa_select(const Grp& g, const SimParams& p, const Lay& L, float part, 
         if (g.rank() >= o) P += n;
     }
     const unsigned long long S = g.bcast(P, g.size() - 1);
-    const float unit = __uint_as_float((uint32_t)(eb - 23) << 23);  // value of the grid's lsb; eb >= 36
-    a0f = __ull2float_rn(S) * unit;
-    // floor of u * S, u = (2k + 1) 2^-53 with k of 52 bits
-    const unsigned long long k2 = (((unsigned long long)(w_hi >> 6) << 26 | (w_lo >> 6)) << 1) | 1ull;
+    a0f = round53(S) * unit;
     const unsigned long long T = __umul64hi(k2 << 11, S);
     // general form: target < excl + part = P with target = u * S rounded to FP64
     bool close = F != 0ull && T + 1ull == P;
@@ -714,8 +769,8 @@ TL_D int ssa_select(const Grp& g, const SimParams& p, const Lay& L, float part, 
 
 
 // ---------------------------------------------------------------------------
-// One step (model.cu:301-413): a tau-leap with rejection and halving, or one
-// direct-method step.
+// One step (model.cu:301-413): a tau-leap with rejection and halving, or a
+// block of direct-method steps.
 // ---------------------------------------------------------------------------
 // Every leap attempt and every direct-method step advances the Philox step
 // counter once: accepted steps = step - rej, leaps = accepted - ssa.
@@ -725,7 +780,6 @@ struct FastState {
     int kpt;        // next grid point to record
     uint32_t step;
     uint32_t rej, ssa;
-    int ssa_left;  // direct-method steps left in the block
     bool wide;     // the next step is a wide leap
     bool done;
 };
@@ -763,47 +817,42 @@ TL_D void add_scores(const Grp& g, const SimParams& p, const Lay& L, int set, ui
     }
 }
 
-template <class Grp, class Lay, bool SENS, bool WIDE>
-TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uint32_t r, FastState& st) {
+// A block of direct-method steps (CGP 2006 step 2; model.cu:334-345) from the
+// propensities in a[] (pa: the lane's partial sum).  The lanes draw the words
+// of a run of steps at once, each its own step's, and hand them out: every
+// lane drawing every step's took 20 % of the instructions.
+template <class Grp, class Lay, bool SENS>
+TL_D void direct_steps(const Grp& g, const SimParams& p, const Lay& L, int set, uint32_t r, float pa,
+                       FastState& st) {
     using Pop = typename Lay::Pop;
     constexpr bool kThin = is_thin<Grp>::value;
-    const float* rate = p.frates + (size_t)set * p.M;  // halved for 2S
-    float pa, pac;
-    fast_props(g, p, L, rate, pa, pac);
-    float tau1 = 0.f, a0f = 0.f;
-    if (st.ssa_left == 0) {
-        if constexpr (kThin) a0f = pa;
-        else a0f = g.sumf(pa);
-        if (a0f > 0.f) {
-            tau1 = fast_tau(g, p, L);
-            if (tau1 * a0f < p.ssa_factor) st.ssa_left = p.ssa_block;
-        } else {
-            st.done = true;
+    const auto qg = queue_group(g);
+    const float* rate = p.frates + (size_t)set * p.M;
+    U4 w{0u, 0u, 0u, 0u};
+    float ex = 0.f;
+    for (int q = 0;;) {
+        if ((q & (qg.size() - 1)) == 0) {
+            w = step_words(p.rk, st.step + (uint32_t)qg.rank(), r, (uint32_t)set);
+            ex = -logf(u01f(w.x));
         }
-    } else if (!g.any(pa > 0.f)) {
-        st.done = true;
-    }
-    if (st.done) return;  // nothing can fire: the state holds to t_final
-
-    if (!WIDE && st.ssa_left > 0) {
-        // ---- direct method, a block of ssa_block steps (CGP 2006 step 2; model.cu:334-345) ----
-        const U4 w = step_words(p.rk, st.step, r, (uint32_t)set);
+        const int from = q & (qg.size() - 1);
+        const uint32_t w_hi = qg.bcast(w.z, from), w_lo = qg.bcast(w.w, from);
         int j;
         float a0;  // total for the waiting time
         if constexpr (kThin) {
             a0 = pa;
-            j = thin_select(g, p, L, pa, w.z, w.w);
+            j = thin_select(g, p, L, pa, w_hi, w_lo);
         } else if constexpr (Grp::kWidth == 0) {
             const double total = g.sumd((double)pa);
             a0 = (float)total;
-            j = select_channel<Grp, double>(g, p, L.a(), pa, u01d(w.z, w.w) * total, 0);
+            j = select_channel<Grp, double>(g, p, L.a(), pa, u01d(w_hi, w_lo) * total, 0);
         } else {
-            j = ssa_select(g, p, L, pa, w.z, w.w, a0);
+            j = ssa_select(g, p, L, pa, w_hi, w_lo, a0);
         }
         // the waiting time in FP32 (FP64 keeps only the time sum)
-        const double dt = (double)(-logf(u01f(w.x)) / a0);
-        const double t_new = st.t + dt;
-        while (st.kpt <= p.n_int && t_new >= st.t_next) record_next(g, p, L, set, r, st);
+        const float dtf = qg.bcast(ex, from) / a0;
+        const double t_new = st.t + widen(dtf);
+        while (st.kpt <= p.n_int && reached(t_new, st.t_next)) record_next(g, p, L, set, r, st);
         if (st.kpt > p.n_int) {
             if (SENS && p.scores) {
                 const float rem = (float)(p.t_final[set] - st.t);
@@ -813,14 +862,12 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
             g.sync();
             return;
         }
-        if (SENS && p.scores) {
-            const float dtf = (float)dt;
+        if (SENS && p.scores)
             add_scores(g, p, L, set, r,
                        [&](int m) { return (m == j ? 1.f : 0.f) - fabsf(L.a()[m]) * dtf; });
-        }
         g.sync();
         if (j >= 0) {
-            // the channel's entries, one lane each (the first lane of thin groups takes all)
+            // the channel's entries, one lane each
             int c0 = j, n = 1;
             if (p.t_cp >= 0) {
                 c0 = (int)L.cp()[j];
@@ -828,6 +875,7 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
             }
             constexpr int kBy = Grp::kWidth == 1 || Grp::kWidth == 2 ? Grp::kWidth : 4;
             if (g.rank() < kBy)
+#pragma unroll 1
                 for (int e = 4 * c0 + g.rank(); e < 4 * (c0 + n); e += kBy) {
                     const uint32_t en = reinterpret_cast<const uint32_t*>(L.col())[e];
                     if (!(en & 0xfffu)) continue;
@@ -841,7 +889,34 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
         st.t = t_new;
         st.step++;
         st.ssa++;
-        st.ssa_left--;
+        if (++q == p.ssa_block || (p.max_steps > 0 && (long long)(st.step - st.rej) >= p.max_steps)) return;
+        float pac;
+        fast_props(g, p, L, rate, pa, pac);
+        if (!g.any(pa > 0.f)) {
+            st.done = true;
+            return;
+        }
+    }
+}
+
+template <class Grp, class Lay, bool SENS, bool WIDE>
+TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uint32_t r, FastState& st) {
+    using Pop = typename Lay::Pop;
+    constexpr bool kThin = is_thin<Grp>::value;
+    const float* rate = p.frates + (size_t)set * p.M;  // halved for 2S
+    float pa, pac;
+    fast_props(g, p, L, rate, pa, pac);
+    float a0f;
+    if constexpr (kThin) a0f = pa;
+    else a0f = g.sumf(pa);
+    if (!(a0f > 0.f)) {
+        st.done = true;  // nothing can fire: the state holds to t_final
+        return;
+    }
+    float tau1 = fast_tau(g, p, L);
+
+    if (!WIDE && tau1 * a0f < p.ssa_factor) {
+        direct_steps<Grp, Lay, SENS>(g, p, L, set, r, pa, st);
         return;
     }
 
@@ -867,8 +942,8 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
         }
         float tauf = fminf(tau1, tau2);
         bool fire = tau2 < tau1;
-        t_new = st.t + (double)tauf;
-        clamp = t_new >= st.t_next;
+        t_new = st.t + widen(tauf);
+        clamp = reached(t_new, st.t_next);
         if (clamp) {
             tauf = (float)(st.t_next - st.t);
             fire = false;
@@ -960,7 +1035,7 @@ TL_D void fast_realization(const Grp& g, const SimParams& p, const Lay& L, long 
     fast_refresh(g, p, L);
     fast_record(g, p, L, set, r, 0);
     g.sync();
-    FastState st{0.0, grid_time<double>(p, set, 1), 1, 0u, 0u, 0u, 0, false, false};
+    FastState st{0.0, grid_time<double>(p, set, 1), 1, 0u, 0u, 0u, false, false};
     bool trunc = false;
     while (!st.done) {
         fast_step<Grp, Lay, SENS, false>(g, p, L, set, r, st);
