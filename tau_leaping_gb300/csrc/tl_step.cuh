@@ -385,17 +385,25 @@ TL_D bool queued_inversion(float mu, uint32_t w, int attempt, int& k) {
         k = 0;
         if (u <= F) return true;
     }
-    float kf = (float)k, last;
+    // Four terms a turn: the sums grow until they stay at one value, so the
+    // last two tell whether they stopped below u (once the terms fall, k > mu,
+    // a sum that repeats repeats for good).  One term a turn leaves a warp with
+    // the latency of a reciprocal and a branch for each.
+    float kf = (float)k;
 #pragma unroll 1
-    do {
-        last = F;
-        kf += 1.f;
-        pk = pk * (mu * fast_rcp(kf));
-        F = last + pk;
-    } while (u > F && F != last);
-    if (u <= F) {
-        k = (int)kf;
-        return true;
+    for (;;) {
+        const float q1 = mu * fast_rcp(kf + 1.f), q2 = mu * fast_rcp(kf + 2.f), q3 = mu * fast_rcp(kf + 3.f),
+                    q4 = mu * fast_rcp(kf + 4.f);
+        const float p1 = pk * q1, p2 = p1 * q2, p3 = p2 * q3, p4 = p3 * q4;
+        const float F1 = F + p1, F2 = F1 + p2, F3 = F2 + p3, F4 = F3 + p4;
+        if (u <= F4) {
+            k = (int)kf + 1 + (u > F1 ? 1 : 0) + (u > F2 ? 1 : 0) + (u > F3 ? 1 : 0);
+            return true;
+        }
+        if (F4 == F3) break;
+        kf += 4.f;
+        pk = p4;
+        F = F4;
     }
     k = (int)mu;  // u above the representable mass
     return attempt == 16;
@@ -527,21 +535,31 @@ TL_D void thin_fire(const GThin<W>& g, const SimParams& p, const Lay& L, float t
                     uint32_t r, uint32_t set) {
     for (int j = g.rank(); j < p.M; j += W) {
         const float aj = L.a()[j];
-        int k = 0;
-        if (is_crit(aj)) {
-            k = j == jc ? 1 : 0;
-        } else {
-            const float mu = aj * tauf;
-            if (mu > 0.f) {
-                ChanRng rng;
-                rng.init((uint32_t)j, step, r, set, p.rk);
-                if (mu >= 10.f) {
-                    k = poisson_ptrs(mu, rng);
+        const float mu = fmaxf(aj, 0.f) * tauf;
+        int k = is_crit(aj) && j == jc ? 1 : 0;
+        if (mu > 0.f) {
+            const bool ptrs = mu >= 10.f;
+            bool ok = false;
+            for (int it = 0; !ok; ++it) {
+                // the shared block of first words, or the private stream: two
+                // uniforms for a PTRS attempt, one for an inversion's
+                const bool shared = !ptrs && it == 0;
+                const int at = ptrs ? 2 * it : it - 1;
+                const U4 w = philox10rk(shared ? U4{(uint32_t)j >> 2, step, r, (set << 8) | 0xFFu}
+                                               : U4{(uint32_t)j, step, r, (set << 8) + (uint32_t)(at >> 2)},
+                                        p.rk);
+                if (ptrs) {
+                    const bool odd = it & 1;
+                    ok = Ptrs(mu).attempt(u01f(odd ? w.z : w.x), u01f(odd ? w.w : w.y), k);
+                    if (it == kPtrsTries - 1 && !ok) {
+                        k = (int)(mu + 0.5f);
+                        ok = true;
+                    }
                 } else {
-                    const U4 gw = group_words(p.rk, (uint32_t)j >> 2, step, r, set);
-                    const uint32_t w = word_of(gw, j & 3);
+                    const uint32_t word = word_of(w, shared ? j & 3 : at & 3);
                     // P(K >= 1) as computed never exceeds mu
-                    if (((float)w + 0.5f) * 2.3283064365386963e-10f < mu) k = poisson_first(mu, w, rng);
+                    ok = shared && ((float)word + 0.5f) * 2.3283064365386963e-10f >= mu;
+                    if (!ok) ok = queued_inversion(mu, word, it, k);
                 }
             }
         }
