@@ -78,10 +78,11 @@ static void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned ch
             x2[(size_t)h.s0[(size_t)j]] = 1;
             ++d.n_2s;
         }
-    int next = N;
+    const int Np = (N + 3) & ~3;  // X pads the species to whole blocks of four
+    int next = Np;
     for (int i = 0; i < N; ++i)
         if (x2[(size_t)i]) x2[(size_t)i] = next++;
-    const int one = N + d.n_2s;
+    const int one = Np + d.n_2s;
     const int pad = (M + 3) & ~3;  // the zero block behind a[]
     d.chan8 = (size_t)one * 4 > 0xffff;
     d.ent_wide = M + 8 > (1 << 18);
@@ -111,7 +112,7 @@ static void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned ch
     d.t_ent = sect(ent_chunks * 16);
     d.t_col = sect(col_chunks * 16);
     d.t_cp = max_col > 4 ? sect((size_t)(M + 1) * 4) : -1;
-    d.t_sp = sect((size_t)N * 2);
+    d.t_sp = sect((size_t)Np * 2);
     if (off >= (1u << 31)) return;
     d.f_stage_bytes = (int)std::max<size_t>(off, 16);
     out.assign((size_t)d.f_stage_bytes, 0);
@@ -302,9 +303,10 @@ static SlotLayout slot_layout(const tl_model* m, int mode, int kind, int block) 
         L.q_rounds = std::min(turns, lanes > 256 ? 4 : 7);
         q_bytes = (size_t)L.q_rounds * lanes * 4 * 2 + 4 * (size_t)(kind ? 1 : block / 32);  // and a counter each
     }
-    L.f_D = (int)al16((size_t)N * w);
-    L.f_X = L.f_D + (int)al16((size_t)N * 4);
-    L.state = (size_t)L.f_X + al16(std::max((size_t)(N + m->d.n_2s + 1) * 4, q_bytes));
+    const size_t Np = ((size_t)N + 3) & ~(size_t)3;  // whole blocks of four species
+    L.f_D = (int)(Np * w);
+    L.f_X = L.f_D + (int)(Np * 4);
+    L.state = (size_t)L.f_X + al16(std::max((Np + (size_t)m->d.n_2s + 1) * 4, q_bytes));
     L.f_a = ((M + 3) / 4 * 4 + 4) * 4;
     L.bytes = L.state + (size_t)L.f_a * (mode == kModeScores ? 3 : 1);
     return L;
@@ -750,7 +752,7 @@ static tl_status job_bind(Job& J, unsigned char* B, cudaStream_t st) {
     p.off_cp = m->d.off_cp;
     p.off_rv = m->d.off_rv;
     p.n_rows = m->d.n_rows;
-    p.x_one = m->h.N + m->d.n_2s;
+    p.x_one = ((m->h.N + 3) & ~3) + m->d.n_2s;
     p.chan8 = m->d.chan8 ? 1 : 0;
     p.ent_wide = m->d.ent_wide ? 1 : 0;
     p.t_chan = m->d.t_chan;

@@ -330,6 +330,54 @@ TL_D void fire_channel(const Lay& L, int j, int k) {
 }
 
 
+// Four species at a time: x, D and X are padded to whole blocks of four (the
+// padding holds 0 and no channel reads it).
+template <class Pop>
+struct Four {
+    Pop v[4];
+};
+TL_D Four<int> load_four(const int* p, int i4) {
+    const int4 t = reinterpret_cast<const int4*>(p)[i4];
+    return {{t.x, t.y, t.z, t.w}};
+}
+TL_D Four<long long> load_four(const long long* p, int i4) {
+    const longlong2 t = reinterpret_cast<const longlong2*>(p)[2 * i4], u = reinterpret_cast<const longlong2*>(p)[2 * i4 + 1];
+    return {{t.x, t.y, u.x, u.y}};
+}
+TL_D void store_four(int* p, int i4, const Four<int>& f) {
+    reinterpret_cast<int4*>(p)[i4] = make_int4(f.v[0], f.v[1], f.v[2], f.v[3]);
+}
+TL_D void store_four(long long* p, int i4, const Four<long long>& f) {
+    reinterpret_cast<longlong2*>(p)[2 * i4] = make_longlong2(f.v[0], f.v[1]);
+    reinterpret_cast<longlong2*>(p)[2 * i4 + 1] = make_longlong2(f.v[2], f.v[3]);
+}
+TL_D int add_pop(int x, int d) { return (int)((unsigned)x + (unsigned)d); }
+TL_D long long add_pop(long long x, int d) { return x + d; }
+
+template <class Lay>
+TL_D void set_four(const Lay& L, int i4, const Four<int>& x) {
+    const int nc = L.p.nc;
+    reinterpret_cast<float4*>(L.X())[i4] =
+        make_float4(with_sign((float)x.v[0], x.v[0] - nc), with_sign((float)x.v[1], x.v[1] - nc),
+                    with_sign((float)x.v[2], x.v[2] - nc), with_sign((float)x.v[3], x.v[3] - nc));
+    const uint2 s3 = reinterpret_cast<const uint2*>(L.sp())[i4];
+    const unsigned at[4] = {s3.x & 0xffffu, s3.x >> 16, s3.y & 0xffffu, s3.y >> 16};
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        if (at[e]) L.X()[at[e]] = with_sign((float)(x.v[e] - 1), x.v[e] - 2 * nc);
+}
+template <class Lay>
+TL_D void set_four(const Lay& L, int i4, const Four<long long>& x) {
+    // all four within int32, as they nearly always are
+    const auto fits = [](long long v) { return (long long)(int)v == v; };
+    if (fits(x.v[0]) && fits(x.v[1]) && fits(x.v[2]) && fits(x.v[3])) {
+        set_four(L, i4, Four<int>{{(int)x.v[0], (int)x.v[1], (int)x.v[2], (int)x.v[3]}});
+    } else {
+#pragma unroll 1
+        for (int e = 0; e < 4; ++e) set_species64(L, 4 * i4 + e, x.v[e]);
+    }
+}
+
 // All of X from x.  D is zero.
 template <class Grp, class Lay>
 TL_D void fast_refresh(const Grp& g, const SimParams& p, const Lay& L) {
@@ -436,6 +484,7 @@ TL_D void fast_fire(const Grp& g, const SimParams& p, const Lay& L, float tauf, 
             if (fminf(fminf(mu[0], mu[1]), fminf(mu[2], mu[3])) < 10.f)
                 gw = group_words(p.rk, (uint32_t)g4, step, r, set);
             unsigned all = 0, far = 0, fired = 0;
+            const bool any_far = fmaxf(fmaxf(mu[0], mu[1]), fmaxf(mu[2], mu[3])) >= 10.f;
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const float ex = __expf(-mu[e]);
@@ -443,10 +492,14 @@ TL_D void fast_fire(const Grp& g, const SimParams& p, const Lay& L, float tauf, 
                 const float v = __uint_as_float((word_of(gw, e) >> 9) | 0x3f800000u);
                 const float d0 = v + (ex - 2.f);          // F0 - u
                 const float d1 = fmaf(ex, mu[e], d0);     // F1 - u >= F0 - u
-                const bool is_far = mu[e] >= 10.f;
-                if (d1 < kFireMargin || fabsf(d0) < kFireMargin || is_far) all |= 1u << e;
-                if (is_far) far |= 1u << e;
-                if (d0 < 0.f) fired |= 1u << e;
+                if (fminf(d1, fabsf(d0)) < kFireMargin) all |= 1u << e;
+                fired |= __float_as_uint(d0) >> 31 << e;
+            }
+            if (any_far) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (mu[e] >= 10.f) far |= 1u << e;
+                all |= far;
             }
             inv |= (all & ~far) << sh;
             big |= far << sh;
@@ -572,35 +625,67 @@ TL_D void thin_fire(const GThin<W>& g, const SimParams& p, const Lay& L, float t
 template <class Grp, class Lay>
 TL_D bool fast_check(const Grp& g, const SimParams& p, const Lay& L, bool& over) {
     using Pop = typename Lay::Pop;
-    bool bad = false, of = false;
-#pragma unroll 2
-    for (int i = g.rank(); i < p.N; i += g.size()) {
-        const int d = L.D()[i];
-        if constexpr (sizeof(Pop) == 4) {
-            const int nx = (int)((unsigned)L.x()[i] + (unsigned)d);
-            bad |= nx < 0;
-            of |= nx < 0 && d > 0;  // wrapped: |D| < 2^31
-        } else {
-            bad |= L.x()[i] + (Pop)d < 0;
-        }
+    const int n4 = (p.N + 3) >> 2;
+    Pop sign = 0;
+#pragma unroll 1
+    for (int i = g.rank(); i < n4; i += g.size()) {
+        const Four<Pop> x = load_four(L.x(), i);
+        const Four<int> d = load_four(L.D(), i);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sign |= add_pop(x.v[e], d.v[e]);
     }
-    const bool b = g.any(bad);
+    const bool bad = g.any(sign < 0);
     over = false;
-    if (sizeof(Pop) == 4 && b) over = g.any(of);
-    return b;
+    if (sizeof(Pop) == 4 && bad) {
+        bool of = false;  // a sum that wrapped: |D| < 2^31
+#pragma unroll 1
+        for (int i = g.rank(); i < p.N; i += g.size()) of |= L.D()[i] > 0 && add_pop(L.x()[i], L.D()[i]) < 0;
+        over = g.any(of);
+    }
+    return bad;
 }
 
 template <class Grp, class Lay>
 TL_D void fast_commit(const Grp& g, const SimParams& p, const Lay& L) {
     using Pop = typename Lay::Pop;
-#pragma unroll 2
-    for (int i = g.rank(); i < p.N; i += g.size()) {
-        const Pop nx = L.x()[i] + (Pop)L.D()[i];
+    const int n4 = (p.N + 3) >> 2;
+#pragma unroll 1
+    for (int i = g.rank(); i < n4; i += g.size()) {
+        Four<Pop> x = load_four(L.x(), i);
+        const Four<int> d = load_four(L.D(), i);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x.v[e] = add_pop(x.v[e], d.v[e]);
+        store_four(L.x(), i, x);
+        store_four(L.D(), i, Four<int>{{0, 0, 0, 0}});
+        set_four(L, i, x);
+    }
+    if (g.leader()) L.X()[p.x_one] = 1.f;
+}
+
+// The same for thin groups, whose lanes each take a species.
+template <int W, class Lay>
+TL_D bool thin_commit(const GThin<W>& g, const SimParams& p, const Lay& L, bool& over) {
+    using Pop = typename Lay::Pop;
+    bool bad = false, of = false;
+    for (int i = g.rank(); i < p.N; i += W) {
+        const int d = L.D()[i];
+        const bool b = add_pop(L.x()[i], d) < 0;
+        bad |= b;
+        of |= sizeof(Pop) == 4 && b && d > 0;
+    }
+    over = false;
+    if (g.any(bad)) {
+        if (sizeof(Pop) == 4) over = g.any(of);
+        return true;
+    }
+    for (int i = g.rank(); i < p.N; i += W) {
+        const Pop nx = add_pop(L.x()[i], L.D()[i]);
         L.x()[i] = nx;
         L.D()[i] = 0;
         set_species(L, i, nx);
     }
     if (g.leader()) L.X()[p.x_one] = 1.f;
+    return false;
 }
 
 // A leap that may hold more than 10^8 firings, whose sums could leave int32:
@@ -645,8 +730,9 @@ TL_D bool wide_leap(const Grp& g, const SimParams& p, const Lay& L, float tauf, 
 #pragma unroll 1
         for (int i = g.rank(); i < p.N; i += g.size()) L.x()[i] = (Pop)((long long)L.x()[i] + (long long)D64[i]);
     g.sync();
+    // the padding of D too: the 64-bit sums lay over it
 #pragma unroll 1
-    for (int i = g.rank(); i < p.N; i += g.size()) L.D()[i] = 0;
+    for (int i = g.rank(); i < ((p.N + 3) & ~3); i += g.size()) L.D()[i] = 0;
     if (!bad) fast_refresh(g, p, L);
     g.sync();
     return bad;
@@ -798,6 +884,8 @@ struct FastState {
     int kpt;        // next grid point to record
     uint32_t step;
     uint32_t rej, ssa;
+    uint32_t ex_from;  // the lanes hold the critical waiting times (unit rate) of the steps from here
+    float ex;
     bool wide;     // the next step is a wide leap
     bool done;
 };
@@ -952,11 +1040,15 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
     else a0cf = g.sumf(pac);
     for (int attempt = 0;; ++attempt) {
         // the step's scalar words are needed only when a channel is critical
+        // and each lane draws another step's
         float tau2 = kInfF;
-        U4 w{0u, 0u, 0u, 0u};
         if (a0cf > 0.f) {
-            w = step_words(p.rk, st.step, r, (uint32_t)set);
-            tau2 = -logf(u01f(w.x)) / a0cf;
+            const auto qg = queue_group(g);
+            if (st.step - st.ex_from >= (uint32_t)qg.size()) {
+                st.ex_from = st.step;
+                st.ex = -logf(u01f(step_words(p.rk, st.step + (uint32_t)qg.rank(), r, (uint32_t)set).x));
+            }
+            tau2 = qg.bcast(st.ex, (int)(st.step - st.ex_from)) / a0cf;
         }
         float tauf = fminf(tau1, tau2);
         bool fire = tau2 < tau1;
@@ -969,6 +1061,7 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
         tau_used = tauf;
         int jc = -1;
         if (fire) {
+            const U4 w = step_words(p.rk, st.step, r, (uint32_t)set);
             if constexpr (kThin) {
                 const double a0c = (double)pac;
                 jc = select_channel<G1, double>(G1{}, p, L.a(), pac, u01d(w.z, w.w) * a0c, 1);
@@ -981,13 +1074,17 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
         if constexpr (WIDE) {
             bad = wide_leap<Grp, Lay, SENS>(g, p, L, tauf, jc, st.step, r, (uint32_t)set, over);
         } else {
-            if constexpr (kThin) thin_fire<Grp::kWidth, Lay, SENS>(g, p, L, tauf, jc, st.step, r, (uint32_t)set);
-            else fast_fire<Grp, Lay, SENS>(g, p, L, tauf, jc, st.step, r, (uint32_t)set);
-            g.sync();
-            bad = fast_check(g, p, L, over);
-            if (!bad) {
-                fast_commit(g, p, L);
+            if constexpr (kThin) {
+                thin_fire<Grp::kWidth, Lay, SENS>(g, p, L, tauf, jc, st.step, r, (uint32_t)set);
+                g.sync();
+                bad = thin_commit(g, p, L, over);
             } else {
+                fast_fire<Grp, Lay, SENS>(g, p, L, tauf, jc, st.step, r, (uint32_t)set);
+                g.sync();
+                bad = fast_check(g, p, L, over);
+                if (!bad) fast_commit(g, p, L);
+            }
+            if (bad) {
 #pragma unroll 1
                 for (int i = g.rank(); i < p.N; i += g.size()) L.D()[i] = 0;
                 g.sync();
@@ -1040,8 +1137,9 @@ TL_D void fast_realization(const Grp& g, const SimParams& p, const Lay& L, long 
     const int set = p.S == 1 ? 0 : (int)(w / p.R);
     const uint32_t r = (uint32_t)(p.r_off + w - (long long)set * p.R);
     const Pop* x0 = reinterpret_cast<const Pop*>(p.x0);
-    for (int i = g.rank(); i < p.N; i += g.size()) {
-        L.x()[i] = x0[i];
+#pragma unroll 1
+    for (int i = g.rank(); i < ((p.N + 3) & ~3); i += g.size()) {
+        L.x()[i] = i < p.N ? x0[i] : (Pop)0;
         L.D()[i] = 0;
     }
     // the padding of a[]: the rest of the last block of four, and the block
@@ -1053,7 +1151,7 @@ TL_D void fast_realization(const Grp& g, const SimParams& p, const Lay& L, long 
     fast_refresh(g, p, L);
     fast_record(g, p, L, set, r, 0);
     g.sync();
-    FastState st{0.0, grid_time<double>(p, set, 1), 1, 0u, 0u, 0u, false, false};
+    FastState st{0.0, grid_time<double>(p, set, 1), 1, 0u, 0u, 0u, 0u - 32u, 0.f, false, false};  // ex: not drawn yet
     bool trunc = false;
     while (!st.done) {
         fast_step<Grp, Lay, SENS, false>(g, p, L, set, r, st);
