@@ -144,6 +144,24 @@ TL_D float fast_rcp(float b) {
     return r;
 }
 
+// 2^x, log2 x and x^-1/2 as the hardware approximates them, without the
+// scaling of subnormals: for tests whose margin covers the error.
+TL_D float fast_ex2(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+TL_D float fast_lg2(float x) {
+    float r;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+TL_D float fast_rsqrt(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // ---------------------------------------------------------------------------
 // Poisson samplers (FP32).
 // ---------------------------------------------------------------------------
@@ -194,15 +212,16 @@ struct Ptrs {
     }
     // The same test with fast logarithms: lhs - log p(k) as
     //   log(V inv_alpha sqrt(2 pi k) / (a / us^2 + b)) + k log(k / mu) - (k - mu) + 1/(12k) - 1/(360k^3).
-    // Its error is below 5e-7 k + 4e-6 (__logf: 3.6e-7 absolute near 1), that
+    // Its error is below 5e-7 k + 4e-6 (lg2: 3e-7 absolute near 1), that
     // of the test proper below 2e-7 k + 3e-6; within the margin of zero, and
     // for small k, the test proper decides.  About 30 instructions for 150,
     // on a path that some lane of a warp takes at nearly every attempt.
     TL_D float excess(float V, float rus, float kf) const {
         const float inv_alpha = 1.1239f + 1.1328f * fast_rcp(b - 3.4f);
         const float ik = fast_rcp(kf);
-        const float q = V * inv_alpha * (2.5066283f * kf * rsqrtf(kf)) * fast_rcp(a * rus * rus + b);
-        return __logf(q) + kf * __logf(kf * fast_rcp(mu)) - (kf - mu) + ik * (1.f / 12.f - ik * ik * (1.f / 360.f));
+        const float q = V * inv_alpha * (2.5066283f * kf * fast_rsqrt(kf)) * fast_rcp(a * rus * rus + b);
+        return 0.69314718f * (fast_lg2(q) + kf * fast_lg2(kf * fast_rcp(mu))) - (kf - mu) +
+               ik * (1.f / 12.f - ik * ik * (1.f / 360.f));
     }
     // one attempt on the uniforms (u, v); true: accepted, k drawn
     TL_D bool attempt(float u, float V, int& k) const {

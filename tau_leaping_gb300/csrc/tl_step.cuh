@@ -394,7 +394,7 @@ TL_D void fast_refresh(const Grp& g, const SimParams& p, const Lay& L) {
 //    u = 1 - q with F0 = exp(-mu) and F1 = F0 (1 + mu), both from one fast
 //    exponential and without a branch.  kFireMargin bounds what the fast forms
 //    and poisson_first's own tests together can be off (under 2.3e-6: the
-//    truncated word 1.8e-7, __expf 3.5e-7, poisson_p1 / p2 1.3e-6 and the
+//    truncated word 1.8e-7, the exponential 3.5e-7, poisson_p1 / p2 1.3e-6 and the
 //    sums), so outside the margin both give the same count.
 //  * Every other draw (k >= 2, within the margin, means >= 10) and every
 //    channel with k = 1 is marked in the lane's masks.  After at most
@@ -487,9 +487,9 @@ TL_D void fast_fire(const Grp& g, const SimParams& p, const Lay& L, float tauf, 
             const bool any_far = fmaxf(fmaxf(mu[0], mu[1]), fmaxf(mu[2], mu[3])) >= 10.f;
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const float ex = __expf(-mu[e]);
+                const float ex = fast_ex2(mu[e] * -1.44269504f);
                 // 2 - (1 - q) from the word's top 23 bits
-                const float v = __uint_as_float((word_of(gw, e) >> 9) | 0x3f800000u);
+                const float v = __uint_as_float((word_of(gw, e) >> 9) + 0x3f800000u);
                 const float d0 = v + (ex - 2.f);          // F0 - u
                 const float d1 = fmaf(ex, mu[e], d0);     // F1 - u >= F0 - u
                 if (fminf(d1, fabsf(d0)) < kFireMargin) all |= 1u << e;
