@@ -69,6 +69,7 @@ struct Carver {
 //        in an int array << 12 | stoichiometry & 0xfff, 0 stoichiometry = none
 //  cp    first chunk of each channel, where a channel needs more than one
 //  sp    per species the index in X of its |x - 1|, 0 if it has none
+//  tiny  a TinyTable, for models of up to 16 channels and species
 static void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned char>& out) {
     const int N = h.N, M = h.M;
     std::vector<int> x2((size_t)N, 0);
@@ -113,6 +114,8 @@ static void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned ch
     d.t_col = sect(col_chunks * 16);
     d.t_cp = max_col > 4 ? sect((size_t)(M + 1) * 4) : -1;
     d.t_sp = sect((size_t)Np * 2);
+    const bool tiny = N <= 16 && M <= 16;
+    d.t_tiny = tiny ? sect(sizeof(TinyTable)) : 0;
     if (off >= (1u << 31)) return;
     d.f_stage_bytes = (int)std::max<size_t>(off, 16);
     out.assign((size_t)d.f_stage_bytes, 0);
@@ -161,6 +164,15 @@ static void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned ch
     if (cp) cp[M] = (uint32_t)c4;
     unsigned short* sp = reinterpret_cast<unsigned short*>(out.data() + d.t_sp);
     for (int i = 0; i < N; ++i) sp[i] = (unsigned short)x2[(size_t)i];
+    if (tiny) {
+        TinyTable* tt = reinterpret_cast<TinyTable*>(out.data() + d.t_tiny);
+        for (int j = 0; j < M; ++j) {
+            tt->chan[j] = (uint32_t)h.s0[(size_t)j] | (uint32_t)h.s1[(size_t)j] << 8 | (uint32_t)h.order[(size_t)j] << 16;
+            for (int q = h.net_cp[(size_t)j]; q < h.net_cp[(size_t)j + 1]; ++q)
+                tt->v[unpack_idx(h.net_rv[(size_t)q])][j] = (int8_t)unpack_v(h.net_rv[(size_t)q]);
+        }
+        for (int i = 0; i < N; ++i) tt->gkind[i] = (uint8_t)h.gkind[(size_t)i];
+    }
     d.fast_ok = true;
 }
 
@@ -340,13 +352,14 @@ struct Plan {
     int lanes = 32;        // thread groups: lanes of a warp that take realizations
     int thin = 1;          // and lanes of one realization
     bool state_global = false;  // global slots: the state as well as a[]
+    bool batch = false;
     SlotLayout slot;
 };
 
 // The kernel a plan launches (CTA groups with global slots are their own build).
 static int launch_kind(const Plan& pl) {
     if (pl.gslot) return kKindCtaGlobal;
-    if (pl.kind == 1 && pl.mode != kModeGeneral) return pl.thin == 4 ? kKindThin4 : kKindThin1;
+    if (pl.kind == 1 && pl.mode != kModeGeneral) return 100 + pl.thin;
     return pl.kind;
 }
 
@@ -384,26 +397,29 @@ static int heuristic_variant(const tl_model* m, size_t sb, long long total, int 
     return TL_VARIANT_WARP;
 }
 
-// Thin groups: lanes per realization (W), and lanes of each warp that take
-// realizations.  One realization's chain of dependent steps sets the time of
-// small and mid-sized ensembles, so four lanes share its channels' draws until
-// about 16 such warps per SM are busy; past that the lanes do more as four
-// realizations.  And the realizations of a warp lengthen one another's chains
-// (they sit in different steps, branches and draws), so small ensembles leave
-// lanes idle while that keeps the warps of an SM below about ten.  Measured on
-// GB300, dimer decay to t = 10 (ms):
-//   realizations        32    1000   3000   10000  30000  100000
-//   W = 1, 32 lanes    5.11   5.19   5.20   5.21   5.62    8.95
-//   W = 4, 32 lanes    3.08   3.11   3.12   3.45   6.94   15.85
-//   W = 4, 8 lanes     2.43   2.47   2.78   6.10  15.16   47.86
-//   W = 4, 4 lanes     2.20   2.35   3.02   9.38  25.90   84.12
-// and a 12 x 16 network in direct-method steps 4.67 against 5.91 at 10000 and
-// 10.3 against 6.5 at 50000 (W = 4 against 1).
-static void thin_plan(long long total, int nsm, int& thin, int& lanes) {
-    thin = total <= (long long)nsm * 16 * 8 ? 4 : 1;
+// Thread-group plans of a model of `size` channels or species at most: lanes
+// per realization (W; 1: thread groups on shared memory, else tl_tiny.cuh), and
+// lanes of each warp that take realizations.  One realization's chain of
+// dependent steps sets the time of small and mid-sized ensembles, so W lanes
+// share its draws until the ensemble is some 56 warps per SM, more than twice
+// what is resident; past that the lanes do more as W realizations.  And the
+// realizations of a warp lengthen one another's chains (they sit in different
+// steps, branches and draws), so small ensembles leave lanes idle.  Measured on
+// GB300 (ms; the last row: shared memory, four lanes, before tl_tiny.cuh):
+//   dimer decay, t = 10   32    1000   3000   10000  30000  100000
+//   W = 4, 32 lanes      1.96   1.97   1.98    2.23   3.28    9.91
+//   W = 4, 8 lanes       1.36   1.38   1.59    3.38   8.49   26.3
+//   W = 4, 4 lanes       1.16   1.24   1.72    5.09  14.1    45.4
+//   W = 1, 32 lanes      4.39   4.44   4.45    4.45   4.89    8.12
+//   shared, 32 lanes     3.08   3.11   3.12    3.45   6.94   15.9
+// and a 12 x 16 network in direct-method steps, W = 16 against 1: 1.29 against
+// 5.38 at 32, 4.67 against 6.91 at 10000, 20.0 against 8.03 at 50000.
+static void thin_plan(int size, long long total, int nsm, int& thin, int& lanes) {
+    thin = size <= 4 ? 4 : size <= 8 ? 8 : size <= 16 ? 16 : 1;
+    if (total * thin > 56LL * 32 * nsm) thin = 1;
     lanes = 32;
-    if (thin == 4)
-        while (lanes > 4 && total * 8 / lanes <= 10LL * nsm) lanes /= 2;
+    if (thin > 1)
+        while (lanes > thin && total * 2 * thin <= (thin == 4 ? 10LL : 3LL) * nsm * lanes) lanes /= 2;
 }
 
 static tl_status make_plan(const tl_model* m, int variant, int block_req, int mode, bool compat_stoich,
@@ -417,7 +433,7 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
     int groups_per_block = 1;
     if (variant == TL_VARIANT_THREAD) {
         pl.kind = 1;
-        if (mode != kModeGeneral) thin_plan(total, nsm, pl.thin, pl.lanes);
+        if (mode != kModeGeneral) thin_plan(std::max(m->h.N, m->h.M), total, nsm, pl.thin, pl.lanes);
         int b = block_req;
         if (b <= 0) {
             // spread small ensembles over every SM
@@ -483,7 +499,8 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
         }
     }
     if (pl.kind == 1) groups_per_block = pl.mode == kModeGeneral ? pl.block : pl.block / 32 * (pl.lanes / pl.thin);
-    size_t slot_smem = (size_t)groups_per_block * pl.slot.bytes;
+    const bool tiny = pl.kind == 1 && pl.mode != kModeGeneral && pl.thin > 1;  // no slots: registers
+    size_t slot_smem = tiny ? 0 : (size_t)groups_per_block * pl.slot.bytes;
     if (pl.gslot) {
         // fast build: a[] in global memory, the state beside it only if it
         // does not fit either
@@ -493,6 +510,7 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
     }
     const int stage = (compat_stoich || no_stage || pl.gslot) ? 0
                       : pl.mode == kModeGeneral               ? m->d.stage_bytes
+                      : tiny                                  ? (int)sizeof(TinyTable)
                                                               : m->d.f_stage_bytes;
     // chain-sized CTA groups leave the tables in L1/L2 (staging them would
     // cost more shared memory than the realization itself)
@@ -500,7 +518,7 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
     pl.stage = (stage_ok && slot_smem + (size_t)stage <= (size_t)smax) ? stage : 0;
     pl.smem = (size_t)pl.stage + slot_smem;
     // scores beside the counts while four such CTAs fit an SM, else in global memory
-    if (pl.mode == kModeScores && pl.smem > (size_t)smax / 4) {
+    if (pl.mode == kModeScores && !tiny && pl.smem > (size_t)smax / 4) {
         pl.slot.score_global = true;
         pl.slot.bytes -= (size_t)pl.slot.f_a;
         pl.smem -= (size_t)groups_per_block * (size_t)pl.slot.f_a;
@@ -653,6 +671,8 @@ static tl_status job_prepare(Job& J) {
 // The plan's part of the launch parameters.
 static void bind_plan(const tl_model* m, const Plan& pl, SimParams& p) {
     p.blob = pl.mode == kModeGeneral ? m->d.blob : m->d.fblob;
+    // (a batch keeps the tables' start: its items differ)
+    if (pl.kind == 1 && pl.mode != kModeGeneral && pl.thin > 1 && !pl.batch) p.blob += m->d.t_tiny;
     p.stage_bytes = pl.stage;
     p.slot_bytes = (int)pl.slot.bytes;
     p.f_D = pl.slot.f_D;
@@ -761,6 +781,7 @@ static tl_status job_bind(Job& J, unsigned char* B, cudaStream_t st) {
     p.t_col = m->d.t_col;
     p.t_cp = m->d.t_cp;
     p.t_sp = m->d.t_sp;
+    p.t_tiny = m->d.t_tiny;
     bind_plan(m, J.pl, p);
     p.gslots = J.pl.gslot ? B + J.o_gslot : nullptr;
     p.ctr = rb.ctr;
@@ -1106,30 +1127,36 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     size_t wslot = 0;
     int bmode = kModeFast;  // the build every item can run on
     long long lane_total = 0;
+    int lane_size = 1;  // channels or species of the largest thread-group item
     for (int i = 0; i < n; ++i) {
         Job& J = jobs[(size_t)i];
         const tl_model* m = J.m;
         bmode = std::max(bmode, J.mode);
         if (!m->d.fast_ok || m->d.chan8 || m->d.ent_wide) bmode = kModeGeneral;
         lane[(size_t)i] = (m->h.M <= 16 && m->h.N <= 16) ? 1 : 0;
-        if (lane[(size_t)i]) lane_total += J.total;
+        if (lane[(size_t)i]) {
+            lane_total += J.total;
+            lane_size = std::max(lane_size, std::max(m->h.M, m->h.N));
+        }
     }
     const size_t spb = al16(sizeof(SimParams));
     int thin = 1, unit_lanes = 32;
     for (;;) {
         thin = 1;
         unit_lanes = 32;
-        if (bmode != kModeGeneral) thin_plan(lane_total, sm_count(), thin, unit_lanes);
+        if (bmode != kModeGeneral) thin_plan(lane_size <= 4 ? 4 : 16, lane_total, sm_count(), thin, unit_lanes);
         wslot = 0;
         for (int i = 0; i < n; ++i) {
             Job& J = jobs[(size_t)i];
             Plan& pl = J.pl;
             pl.variant = lane[(size_t)i] ? TL_VARIANT_THREAD : TL_VARIANT_WARP;
             pl.mode = bmode;
+            pl.batch = true;
             pl.lanes = unit_lanes;
             pl.thin = thin;
             pl.slot = slot_layout(J.m, bmode, lane[(size_t)i] ? 1 : 32, 32);
-            wslot = std::max(wslot, lane[(size_t)i] ? (size_t)(unit_lanes / thin) * pl.slot.bytes : pl.slot.bytes);
+            const size_t unit = !lane[(size_t)i] ? pl.slot.bytes : thin == 1 ? (size_t)unit_lanes * pl.slot.bytes : 0;
+            wslot = std::max(wslot, unit);
         }
         wslot = al16(wslot);
         // the general build's slot is smaller for wide models

@@ -792,7 +792,7 @@ struct SimParams {
     int x_one;            // index of the constant 1 in X
     int chan8;            // channel records of two 32-bit offsets (wide CTA models)
     int ent_wide;         // row entries packed as (col<<3)|((v+2)&7)
-    int t_chan, t_row, t_ent, t_col, t_cp, t_sp;  // byte offsets of the tables, t_cp -1: none
+    int t_chan, t_row, t_ent, t_col, t_cp, t_sp, t_tiny;  // byte offsets of the tables, t_cp -1: none
     int f_D, f_X;         // byte offsets in the state
     int f_big;            // offset of a[] in the slot (or in a global slot)
     int f_a;              // bytes of a[]

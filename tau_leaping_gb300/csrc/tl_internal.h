@@ -71,7 +71,7 @@ struct DevModel {
     // tables of the fast and scores builds (tl_step.cuh), staged as one piece
     unsigned char* fblob = nullptr;
     int f_stage_bytes = 0;
-    int t_chan = 0, t_row = 0, t_ent = 0, t_col = 0, t_cp = -1, t_sp = 0;
+    int t_chan = 0, t_row = 0, t_ent = 0, t_col = 0, t_cp = -1, t_sp = 0, t_tiny = 0;
     int n_rows = 0;                 // species that react: rows of the step bound
     int n_2s = 0;                   // species of 2S channels
     bool chan8 = false, ent_wide = false;

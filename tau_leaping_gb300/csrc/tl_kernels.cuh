@@ -14,6 +14,7 @@
 
 #include "tl_device.cuh"
 #include "tl_step.cuh"
+#include "tl_tiny.cuh"
 #include "tl_launch.h"
 
 namespace tl {
@@ -250,14 +251,10 @@ struct ThinGroupOf {
 };
 template <>
 struct FastGroupOf<kKindThin1> : ThinGroupOf<1> {};
-template <>
-struct FastGroupOf<kKindThin4> : ThinGroupOf<4> {};
-
-constexpr bool is_thin_kind(int kind) { return kind == kKindThin1 || kind == kKindThin4; }
 
 template <int KIND, class Pop, bool SENS, bool STAGED, bool GSLOT = false>
 __global__ void __launch_bounds__(KIND == 0 ? 1024 : 256,
-                                  KIND == 0 ? 1 : is_thin_kind(KIND) ? TL_THREAD_MINB : TL_WARP_MINB)
+                                  KIND == 0 ? 1 : KIND == kKindThin1 ? TL_THREAD_MINB : TL_WARP_MINB)
     k_fast(const __grid_constant__ SimParams p) {
     __shared__ __align__(8) unsigned long long mbar;
     __shared__ double red[34];
@@ -292,12 +289,38 @@ __global__ void __launch_bounds__(KIND == 0 ? 1024 : 256,
     }
 }
 
+// Small models on W lanes each (tl_tiny.cuh); p.blob is the model's TinyTable.
+template <int W, class Pop, bool SENS>
+__global__ void __launch_bounds__(256, TL_THREAD_MINB) k_tiny(const __grid_constant__ SimParams p) {
+    __shared__ __align__(8) unsigned long long mbar;
+    const TinyTable* tab = reinterpret_cast<const TinyTable*>(p.blob);
+    if (p.stage_bytes > 0) {
+        if (!stage_blob(tl_smem, p.blob, p.stage_bytes, p.wait_polls, &mbar)) {
+            if (threadIdx.x == 0) atomicOr((unsigned*)(p.ctr + 5), kErrWaitTimeout | kErrStage);
+            return;
+        }
+        tab = reinterpret_cast<const TinyTable*>(tl_smem);
+    }
+    if ((int)(threadIdx.x & 31) >= p.lanes) return;
+    const auto g = TinyGroup<W>::make();
+    TinyLane<W, Pop> L;
+    L.load(tab, g.lane);
+    const long long total = p.R * (long long)p.S;
+    for (;;) {
+        long long w = 0;
+        if (g.lane == 0) w = (long long)atomicAdd(p.ctr + 0, 1ull);
+        w = g.from(w, 0);
+        if (w >= total) break;
+        tiny_realization<W, Pop, SENS>(g, p, L, w);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Batched persistent kernel: items of several models / configurations.
 // ---------------------------------------------------------------------------
 // FAST: the fast build, or with SENS the scores build, of every item;
 // otherwise the general one.  STAGED: every item's tables in shared memory.
-// W: lanes of a thin item's realization.
+// W: lanes of a small item's realization (1: thread groups).
 template <class Pop, bool FAST, bool SENS, bool STAGED, int W>
 __global__ void __launch_bounds__(256, TL_BATCH_MINB) k_batch(BatchParams bp) {
     unsigned char* const smem = tl_smem;
@@ -339,11 +362,17 @@ __global__ void __launch_bounds__(256, TL_BATCH_MINB) k_batch(BatchParams bp) {
                 const Lay L{p, my_slot, (uint32_t)soff, nullptr, nullptr};
                 fast_realization<GWarp, Lay, SENS>(GWarp{lane}, p, L, local);
             } else if (lane < p.lanes) {
-                const GThin<W> g = GThin<W>::make();
                 const long long wi = local * (p.lanes / W) + lane / W;
                 if (wi < total) {
-                    const Lay L{p, my_slot + (uint32_t)(lane / W * p.slot_bytes), (uint32_t)soff, nullptr, nullptr};
-                    fast_realization<GThin<W>, Lay, SENS>(g, p, L, wi);
+                    if constexpr (W == 1) {
+                        const Lay L{p, my_slot + (uint32_t)(lane * p.slot_bytes), (uint32_t)soff, nullptr, nullptr};
+                        fast_realization<GThin<1>, Lay, SENS>(GThin<1>::make(), p, L, wi);
+                    } else {
+                        const auto g = TinyGroup<W>::make();
+                        TinyLane<W, Pop> L;
+                        L.load(reinterpret_cast<const TinyTable*>((STAGED ? smem + soff : p.blob) + p.t_tiny), g.lane);
+                        tiny_realization<W, Pop, SENS>(g, p, L, wi);
+                    }
                 }
             }
         } else {

@@ -2,6 +2,8 @@
 // (Pop = int for 32-bit, long long for 64-bit populations).
 #pragma once
 
+#include <cstdint>
+
 #include <cuda_runtime.h>
 
 namespace tl {
@@ -10,9 +12,18 @@ struct SimParams;
 
 // kind: 1 = thread, 32 = warp, 0 = CTA, 2/4/8/16 = lanes per realization,
 // kKindCtaGlobal = CTA with its propensities (or whole slot) in global memory;
-// in the fast and scores builds thread groups are thin groups of 1 or 4 lanes.
+// in the fast and scores builds thread groups are thin groups of one lane or,
+// for small models, 4, 8 or 16 lanes (tl_tiny.cuh).
 constexpr int kKindCtaGlobal = 64;
-constexpr int kKindThin1 = 101, kKindThin4 = 104;
+constexpr int kKindThin1 = 101, kKindTiny4 = 104, kKindTiny8 = 108, kKindTiny16 = 116;
+
+// Table of a small model (N, M <= 16): per channel {s0, s1, order, 0}, then per
+// species its 16 stoichiometries, then per species the g kind.
+struct TinyTable {
+    uint32_t chan[16];
+    int8_t v[16][16];
+    uint8_t gkind[16];
+};
 // mode: the kernel build a run needs.  Fast: no likelihood-ratio scores and
 // no reference-compatibility switches; Scores: with scores; General: both.
 // The sub-warp and global-slot kinds come in Fast and General only.

@@ -582,40 +582,46 @@ TL_D void fast_fire(const Grp& g, const SimParams& p, const Lay& L, float tauf, 
     }
 }
 
-// The same for thin groups: each lane draws its channels in place.
+// The count of channel j in a leap, drawn in place: thread groups and the
+// lanes of small models.
+TL_D int poisson_channel(float aj, float tauf, int j, int jc, uint32_t step, uint32_t r, uint32_t set,
+                         const uint32_t* rk) {
+    const float mu = fmaxf(aj, 0.f) * tauf;
+    int k = is_crit(aj) && j == jc ? 1 : 0;
+    if (mu > 0.f) {
+        const bool ptrs = mu >= 10.f;
+        bool ok = false;
+        for (int it = 0; !ok; ++it) {
+            // the shared block of first words, or the private stream: two
+            // uniforms for a PTRS attempt, one for an inversion's
+            const bool shared = !ptrs && it == 0;
+            const int at = ptrs ? 2 * it : it - 1;
+            const U4 w = philox10rk(shared ? U4{(uint32_t)j >> 2, step, r, (set << 8) | 0xFFu}
+                                           : U4{(uint32_t)j, step, r, (set << 8) + (uint32_t)(at >> 2)},
+                                    rk);
+            if (ptrs) {
+                const bool odd = it & 1;
+                ok = Ptrs(mu).attempt(u01f(odd ? w.z : w.x), u01f(odd ? w.w : w.y), k);
+                if (it == kPtrsTries - 1 && !ok) {
+                    k = (int)(mu + 0.5f);
+                    ok = true;
+                }
+            } else {
+                const uint32_t word = word_of(w, shared ? j & 3 : at & 3);
+                // P(K >= 1) as computed never exceeds mu
+                ok = shared && ((float)word + 0.5f) * 2.3283064365386963e-10f >= mu;
+                if (!ok) ok = queued_inversion(mu, word, it, k);
+            }
+        }
+    }
+    return k;
+}
+
 template <int W, class Lay, bool SENS>
 TL_D void thin_fire(const GThin<W>& g, const SimParams& p, const Lay& L, float tauf, int jc, uint32_t step,
                     uint32_t r, uint32_t set) {
     for (int j = g.rank(); j < p.M; j += W) {
-        const float aj = L.a()[j];
-        const float mu = fmaxf(aj, 0.f) * tauf;
-        int k = is_crit(aj) && j == jc ? 1 : 0;
-        if (mu > 0.f) {
-            const bool ptrs = mu >= 10.f;
-            bool ok = false;
-            for (int it = 0; !ok; ++it) {
-                // the shared block of first words, or the private stream: two
-                // uniforms for a PTRS attempt, one for an inversion's
-                const bool shared = !ptrs && it == 0;
-                const int at = ptrs ? 2 * it : it - 1;
-                const U4 w = philox10rk(shared ? U4{(uint32_t)j >> 2, step, r, (set << 8) | 0xFFu}
-                                               : U4{(uint32_t)j, step, r, (set << 8) + (uint32_t)(at >> 2)},
-                                        p.rk);
-                if (ptrs) {
-                    const bool odd = it & 1;
-                    ok = Ptrs(mu).attempt(u01f(odd ? w.z : w.x), u01f(odd ? w.w : w.y), k);
-                    if (it == kPtrsTries - 1 && !ok) {
-                        k = (int)(mu + 0.5f);
-                        ok = true;
-                    }
-                } else {
-                    const uint32_t word = word_of(w, shared ? j & 3 : at & 3);
-                    // P(K >= 1) as computed never exceeds mu
-                    ok = shared && ((float)word + 0.5f) * 2.3283064365386963e-10f >= mu;
-                    if (!ok) ok = queued_inversion(mu, word, it, k);
-                }
-            }
-        }
+        const int k = poisson_channel(L.a()[j], tauf, j, jc, step, r, set, p.rk);
         if constexpr (SENS) L.k()[j] = k;
         if (k) fire_channel<GThin<W>>(L, j, k);
     }
