@@ -4,6 +4,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -56,6 +57,20 @@ struct Carver {
         return o;
     }
 };
+
+// One set's rates in FP32, as given and halved for 2S channels (the fast
+// builds).  False where halving might not be exact: near FP32's ends.
+static bool fill_rates(const HostModel& h, const double* c, float* plain, float* halved) {
+    bool exact = true;
+    for (int j = 0; j < h.M; ++j) {
+        const float cf = (float)c[j];
+        const bool twice = h.order[(size_t)j] == 3;
+        if (plain) plain[j] = cf;
+        if (halved) halved[j] = twice ? 0.5f * cf : cf;
+        if (twice && cf != 0.f && !(cf >= 7.8886e-31f && cf <= 1.1529e18f)) exact = false;
+    }
+    return exact;
+}
 
 // Tables of the fast and scores builds, in the layout tl_step.cuh reads:
 //  chan  per channel the byte offsets in X of its two factors: 16 bits each,
@@ -233,9 +248,10 @@ static tl_status upload(tl_model* m) {
         std::vector<int> x(h.x0.begin(), h.x0.end());
         TLC(cudaMemcpy(d.x0, x.data(), (size_t)N * 4, cudaMemcpyHostToDevice));
     }
-    std::vector<float> r(h.rate.begin(), h.rate.end());
-    TLC(cudaMalloc(&d.rate, (size_t)M * 4));
-    TLC(cudaMemcpy(d.rate, r.data(), (size_t)M * 4, cudaMemcpyHostToDevice));
+    std::vector<float> r(2 * (size_t)M);
+    d.halvable = fill_rates(h, h.rate.data(), r.data(), r.data() + M);
+    TLC(cudaMalloc(&d.rate, r.size() * 4));
+    TLC(cudaMemcpy(d.rate, r.data(), r.size() * 4, cudaMemcpyHostToDevice));
     return TL_OK;
 }
 
@@ -300,11 +316,11 @@ struct SlotLayout {
     bool score_global = false;
 };
 
-static SlotLayout slot_layout(const tl_model* m, int mode, int kind, int block) {
+static SlotLayout slot_layout(const tl_model* m, bool sens, int mode, int kind, int block) {
     SlotLayout L;
     const int N = m->h.N, M = m->h.M;
     if (mode == kModeGeneral) {
-        L.bytes = slot_bytes(m, true);
+        L.bytes = slot_bytes(m, sens);
         return L;
     }
     const size_t w = m->h.pop_bits == 64 ? 8 : 4;
@@ -422,7 +438,7 @@ static void thin_plan(int size, long long total, int nsm, int& thin, int& lanes)
         while (lanes > thin && total * 2 * thin <= (thin == 4 ? 10LL : 3LL) * nsm * lanes) lanes /= 2;
 }
 
-static tl_status make_plan(const tl_model* m, int variant, int block_req, int mode, bool compat_stoich,
+static tl_status make_plan(const tl_model* m, int variant, int block_req, int mode, bool sens, bool compat_stoich,
                            bool no_stage, long long total, Plan& pl, bool force_gslot = false) {
     const size_t sb = slot_bytes(m, mode != kModeFast);
     const int smax = max_smem_optin() - 2048;
@@ -472,7 +488,7 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
     const auto fit = [&](int mode_) {
         pl.mode = mode_;
         pl.block = asked;
-        pl.slot = slot_layout(m, mode_, pl.kind, pl.block);
+        pl.slot = slot_layout(m, sens, mode_, pl.kind, pl.block);
         groups_per_block = pl.kind ? pl.block / pl.kind : 1;
         while ((size_t)groups_per_block * pl.slot.bytes > (size_t)smax && pl.kind != 0 && pl.block > 32) {
             pl.block -= 32;
@@ -569,7 +585,11 @@ struct Job {
     bool sens = false, keep = false, plain = false, compat_stoich = false;
     int mode = kModeFast;  // the kernel build: scores and / or compatibility switches
     size_t w = 4;
-    std::vector<float> hrates;
+    std::vector<float> hrates;  // the call's rate sets; empty: the model's own
+    int rates_first = 0, rates_sets = 0;  // the sets of hrates that go to the device
+    bool measure = false;
+    std::vector<unsigned char> hin;  // what goes to the device
+    size_t o_in = 0;
     std::vector<double> htf;
     std::vector<double> hgrid;  // [S][P] grid times
     Plan pl;
@@ -577,7 +597,8 @@ struct Job {
            o_gse = 0, o_gm = 0, o_ps = 0, o_pslot = 0, o_aall = 0, o_gslot = 0;
     RunBuffers rb;
     SimParams p{};
-    std::vector<unsigned char> hs;
+    std::unique_ptr<int[]> hs;  // 32-bit samples on their way to the result
+    std::vector<unsigned char> hout;
     unsigned long long hc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 };
 
@@ -632,23 +653,23 @@ static tl_status job_prepare(Job& J) {
         set_last_error("sensitivity needs at least one tracked species");
         return TL_ERR_INVALID_ARGUMENT;
     }
-    J.hrates.assign((size_t)2 * J.S * M, 0.f);  // as given, then halved for 2S channels
     J.htf.assign((size_t)J.S, cfg->t_final);
     bool halvable = true;
-    for (int s = 0; s < J.S; ++s)
-        for (int j = 0; j < M; ++j) {
-            const double c = cfg->n_rate_sets > 0 ? cfg->rate_sets[(size_t)s * M + j] : h.rate[(size_t)j];
-            if (!std::isfinite(c) || c < 0.0) {
-                set_last_error("rate constants must be finite and >= 0");
-                return TL_ERR_NUMERIC;
-            }
-            const float cf = (float)c;
-            J.hrates[(size_t)s * M + j] = cf;
-            const bool twice = h.order[(size_t)j] == 3;
-            J.hrates[(size_t)(J.S + s) * M + j] = twice ? 0.5f * cf : cf;
-            // the fast builds halve 2S rates, which is exact far from FP32's ends
-            if (twice && cf != 0.f && !(cf >= 7.8886e-31f && cf <= 1.1529e18f)) halvable = false;
+    for (size_t q = 0; q < (size_t)cfg->n_rate_sets * (size_t)M; ++q)
+        if (!std::isfinite(cfg->rate_sets[q]) || cfg->rate_sets[q] < 0.0) {
+            set_last_error("rate constants must be finite and >= 0");
+            return TL_ERR_NUMERIC;
         }
+    if (cfg->n_rate_sets > 0) {
+        J.hrates.resize((size_t)2 * J.S * M);  // all sets as given, then halved for 2S channels
+        float* to = J.hrates.data();
+        for (int s = 0; s < J.S; ++s)
+            halvable &= fill_rates(h, cfg->rate_sets + (size_t)s * M, to + (size_t)s * M, to + (size_t)(J.S + s) * M);
+    } else {
+        const tl_status ds = ensure_device(m);  // the model's own rates are resident
+        if (ds != TL_OK) return ds;
+        halvable = m->d.halvable;
+    }
     if (!halvable) J.mode = kModeGeneral;
     if (cfg->n_rate_sets > 0 && cfg->t_final_sets)
         for (int s = 0; s < J.S; ++s) {
@@ -668,13 +689,18 @@ static tl_status job_prepare(Job& J) {
     return ensure_device(m);
 }
 
+// A CTA's slot in global memory: without the state where that is in shared memory.
+static size_t global_slot_bytes(const Plan& pl) {
+    return pl.mode == kModeGeneral || pl.state_global ? pl.slot.bytes : pl.slot.bytes - pl.slot.state;
+}
+
 // The plan's part of the launch parameters.
 static void bind_plan(const tl_model* m, const Plan& pl, SimParams& p) {
     p.blob = pl.mode == kModeGeneral ? m->d.blob : m->d.fblob;
     // (a batch keeps the tables' start: its items differ)
     if (pl.kind == 1 && pl.mode != kModeGeneral && pl.thin > 1 && !pl.batch) p.blob += m->d.t_tiny;
     p.stage_bytes = pl.stage;
-    p.slot_bytes = (int)pl.slot.bytes;
+    p.slot_bytes = (int)(pl.gslot ? global_slot_bytes(pl) : pl.slot.bytes);
     p.f_D = pl.slot.f_D;
     p.f_X = pl.slot.f_X;
     p.f_a = pl.slot.f_a;
@@ -688,22 +714,37 @@ static void bind_plan(const tl_model* m, const Plan& pl, SimParams& p) {
 
 static void job_layout(Job& J, Carver& c) {
     const int M = J.m->h.M, N = J.m->h.N, K1 = std::max(J.K, 1);
-    J.o_rates = c.take((size_t)2 * J.S * M * 4);
-    J.o_tf = c.take((size_t)J.S * 8);
-    J.o_grid = c.take((size_t)J.S * J.P * 8);
-    J.o_tr = c.take((size_t)K1 * 4);
+    // what goes to the device in one copy: rate sets, end times, grid, tracked
+    // species and zeroed counters, which come back with the statistics.  The
+    // fast build reads only the halved rates, the general one the others.
+    J.rates_first = J.pl.mode == kModeFast && !J.plain && !J.measure ? J.S : 0;
+    J.rates_sets = J.hrates.empty() ? 0 : J.pl.mode == kModeScores || J.measure ? 2 * J.S : J.S;
+    size_t o = 0;
+    const auto put = [&](size_t& at, size_t bytes) {
+        at = o;
+        o += al16(bytes);
+    };
+    put(J.o_rates, (size_t)J.rates_sets * M * 4);
+    put(J.o_tf, (size_t)J.S * 8);
+    put(J.o_grid, (size_t)J.S * J.P * 8);
+    put(J.o_tr, (size_t)K1 * 4);
+    put(J.o_ctr, 8 * 8);
+    const size_t in = o;
+    put(J.o_mean, (size_t)J.S * J.P * K1 * 8);
+    put(J.o_sd, (size_t)J.S * J.P * K1 * 8);
+    const size_t at = c.take(o);
+    J.hin.resize(in);
+    for (size_t* q : {&J.o_rates, &J.o_tf, &J.o_grid, &J.o_tr, &J.o_ctr, &J.o_mean, &J.o_sd}) *q += at;
+    J.o_in = at;
     J.o_samp = c.take((size_t)J.total * J.P * K1 * J.w);
     J.o_sc = J.sens ? c.take((size_t)J.total * M * 4) : 0;
-    J.o_ctr = c.take(8 * 8);
-    J.o_mean = c.take((size_t)J.S * J.P * K1 * 8);
-    J.o_sd = c.take((size_t)J.S * J.P * K1 * 8);
     J.o_grad = J.sens ? c.take((size_t)J.S * J.K * M * 8) : 0;
     J.o_gse = J.sens ? c.take((size_t)J.S * J.K * M * 8) : 0;
     J.o_gm = J.sens ? c.take((size_t)J.S * J.K * 8) : 0;
     J.o_ps = J.plain ? c.take((size_t)J.total * 64) : 0;
     J.o_pslot = J.plain ? c.take((size_t)J.total * 2 * al16((size_t)N * J.w)) : 0;
     J.o_aall = J.plain ? c.take((size_t)J.total * M * 4) : 0;
-    J.o_gslot = (!J.plain && J.pl.gslot) ? c.take((size_t)J.pl.grid * J.pl.slot.bytes) : 0;
+    J.o_gslot = (!J.plain && J.pl.gslot) ? c.take((size_t)J.pl.grid * global_slot_bytes(J.pl)) : 0;
 }
 
 static tl_status job_bind(Job& J, unsigned char* B, cudaStream_t st) {
@@ -729,18 +770,25 @@ static tl_status job_bind(Job& J, unsigned char* B, cudaStream_t st) {
         rb.pslots = B + J.o_pslot;
         rb.a_all = reinterpret_cast<float*>(B + J.o_aall);
     }
-    TLC(cudaMemcpyAsync(rb.rates, J.hrates.data(), J.hrates.size() * 4, cudaMemcpyHostToDevice, st));
-    TLC(cudaMemcpyAsync(rb.tfin, J.htf.data(), J.htf.size() * 8, cudaMemcpyHostToDevice, st));
-    TLC(cudaMemcpyAsync(rb.grid, J.hgrid.data(), J.hgrid.size() * 8, cudaMemcpyHostToDevice, st));
-    if (J.K > 0) TLC(cudaMemcpyAsync(rb.tracked, cfg->tracked, (size_t)J.K * 4, cudaMemcpyHostToDevice, st));
-    TLC(cudaMemsetAsync(rb.ctr, 0, 64, st));
+    const auto fill = [&](size_t at, const void* from, size_t bytes) {
+        if (bytes) memcpy(J.hin.data() + (at - J.o_in), from, bytes);
+    };
+    std::fill(J.hin.begin(), J.hin.end(), (unsigned char)0);
+    const size_t M = (size_t)m->h.M;
+    fill(J.o_rates, J.hrates.data() + (size_t)J.rates_first * M * (J.rates_sets ? 1 : 0), (size_t)J.rates_sets * M * 4);
+    fill(J.o_tf, J.htf.data(), J.htf.size() * 8);
+    fill(J.o_grid, J.hgrid.data(), J.hgrid.size() * 8);
+    fill(J.o_tr, cfg->tracked, (size_t)J.K * 4);
+    TLC(cudaMemcpyAsync(B + J.o_in, J.hin.data(), J.hin.size(), cudaMemcpyHostToDevice, st));
+    const float* const plain = J.rates_sets ? rb.rates : m->d.rate;
+    const float* const halved = !J.rates_sets ? m->d.rate + M : J.rates_sets == J.S ? rb.rates : rb.rates + (size_t)J.S * M;
     SimParams& p = J.p;
     p = SimParams{};
     p.N = m->h.N;
     p.M = m->h.M;
     p.g = global_view(m, J.compat_stoich, false);
     p.x0 = m->d.x0;
-    p.rates = rb.rates;
+    p.rates = plain;
     p.t_final = rb.tfin;
     p.grid = rb.grid;
     p.R = J.R;
@@ -762,7 +810,7 @@ static tl_status job_bind(Job& J, unsigned char* B, cudaStream_t st) {
     p.flags = cfg->flags;
     p.max_halv = cfg->max_halvings > 0 ? cfg->max_halvings : 64;
     p.wait_polls = cfg->stage_wait_polls == 0 ? (1 << 22) : std::max(cfg->stage_wait_polls, 0);
-    p.frates = rb.rates + (size_t)J.S * m->h.M;
+    p.frates = halved;
     p.off_chan = m->d.off_chan;
     p.off_rord = m->d.off_rord;
     p.off_gkind = m->d.off_gkind;
@@ -805,15 +853,19 @@ static tl_status job_reduce(Job& J, cudaStream_t st) {
                       : launch_grad<int>(rb.samples, rb.scores, J.R, J.P, J.K, M, J.S, rb.grad, rb.gse, rb.gmean, st);
         if (le != cudaSuccess) return cuda_fail(le, "gradient launch");
     }
-    TLC(cudaMemcpyAsync(J.hc, rb.ctr, 64, cudaMemcpyDeviceToHost, st));
+    // counters, means and deviations in one copy
+    const bool stats = J.res && J.K > 0 && (J.res->mean || J.res->stddev);
     const size_t SPK = (size_t)J.S * J.P * J.K;
-    if (J.res) {
-        if (J.res->mean && J.K > 0) TLC(cudaMemcpyAsync(J.res->mean, rb.mean, SPK * 8, cudaMemcpyDeviceToHost, st));
-        if (J.res->stddev && J.K > 0) TLC(cudaMemcpyAsync(J.res->stddev, rb.sd, SPK * 8, cudaMemcpyDeviceToHost, st));
-        if (J.res->samples && J.keep && J.K > 0) {
-            J.hs.resize((size_t)J.total * J.P * J.K * J.w);
-            TLC(cudaMemcpyAsync(J.hs.data(), rb.samples, J.hs.size(), cudaMemcpyDeviceToHost, st));
+    J.hout.resize(stats ? J.o_sd - J.o_ctr + SPK * 8 : 64);
+    TLC(cudaMemcpyAsync(J.hout.data(), rb.ctr, J.hout.size(), cudaMemcpyDeviceToHost, st));
+    if (J.res && J.res->samples && J.keep && J.K > 0) {
+        const size_t n = (size_t)J.total * J.P * J.K;
+        void* to = J.res->samples;
+        if (J.w == 4) {
+            J.hs.reset(new int[n]);
+            to = J.hs.get();
         }
+        TLC(cudaMemcpyAsync(to, rb.samples, n * J.w, cudaMemcpyDeviceToHost, st));
     }
     if (J.sens) {
         tl_grad_result* g = J.grad;
@@ -829,13 +881,16 @@ static tl_status job_reduce(Job& J, cudaStream_t st) {
 // After the stream is synchronised: fill the result, map error bits.
 static tl_status job_finish(Job& J, double kernel_ms, int launches, double total_ms) {
     tl_result* res = J.res;
-    if (!J.hs.empty()) {
+    if (J.hs) {
         const size_t n = (size_t)J.total * J.P * J.K;
-        if (J.w == 8) memcpy(res->samples, J.hs.data(), n * 8);
-        else {
-            const int* src = reinterpret_cast<const int*>(J.hs.data());
-            for (size_t q = 0; q < n; ++q) res->samples[q] = src[q];
-        }
+        const int* src = J.hs.get();
+        for (size_t q = 0; q < n; ++q) res->samples[q] = src[q];
+    }
+    memcpy(J.hc, J.hout.data(), 64);
+    if (res && J.hout.size() > 64) {
+        const size_t n = (size_t)J.S * J.P * J.K * 8;
+        if (res->mean) memcpy(res->mean, J.hout.data() + (J.o_mean - J.o_ctr), n);
+        if (res->stddev) memcpy(res->stddev, J.hout.data() + (J.o_sd - J.o_ctr), n);
     }
     if (res) {
         if (res->times) std::copy(J.hgrid.begin(), J.hgrid.end(), res->times);
@@ -868,6 +923,19 @@ static tl_status job_finish(Job& J, double kernel_ms, int launches, double total
         set_last_error("max_steps reached; truncated realizations hold their last state");
         return TL_ERR_STEP_CAP;
     }
+    return TL_OK;
+}
+
+// The model's pair of timing events.
+static tl_status timing_events(tl_model* m, cudaEvent_t* e0, cudaEvent_t* e1) {
+    for (void*& e : m->ev)
+        if (!e) {
+            cudaEvent_t made = nullptr;
+            TLC(cudaEventCreate(&made));
+            e = made;
+        }
+    *e0 = (cudaEvent_t)m->ev[0];
+    *e1 = (cudaEvent_t)m->ev[1];
     return TL_OK;
 }
 
@@ -918,7 +986,7 @@ static tl_status autotune_measure(Job& J, cudaStream_t st) {
         Cand win{0, 0, false};
         for (const Cand& c : cands) {
             Plan pl;
-            if (make_plan(m, c.variant, c.block, J.mode, J.compat_stoich, c.nostage, trial, pl) != TL_OK) continue;
+            if (make_plan(m, c.variant, c.block, J.mode, J.sens, J.compat_stoich, c.nostage, trial, pl) != TL_OK) continue;
             if (c.variant == TL_VARIANT_THREAD && c.block != pl.block) continue;
             // global slots exist for the launch the heuristic planned
             if (pl.gslot && (!planned_gslot || pl.grid > planned_grid)) continue;
@@ -952,13 +1020,13 @@ static tl_status autotune_measure(Job& J, cudaStream_t st) {
         m->tuned_block = win.block;
         m->tuned_nostage = win.nostage ? 1 : 0;
     }
-    tl_status ps = make_plan(m, m->tuned_variant, m->tuned_block, J.mode, J.compat_stoich, m->tuned_nostage != 0,
+    tl_status ps = make_plan(m, m->tuned_variant, m->tuned_block, J.mode, J.sens, J.compat_stoich, m->tuned_nostage != 0,
                              J.total, J.pl);
     if (ps != TL_OK) return ps;
     if (J.pl.gslot && (!planned_gslot || J.pl.grid > planned_grid)) {
         // a cached global-slot plan that needs more slots than were laid out:
         // keep the planned launch
-        ps = make_plan(m, TL_VARIANT_AUTO, 0, J.mode, J.compat_stoich, (J.cfg->flags & TL_FLAG_NO_STAGE) != 0,
+        ps = make_plan(m, TL_VARIANT_AUTO, 0, J.mode, J.sens, J.compat_stoich, (J.cfg->flags & TL_FLAG_NO_STAGE) != 0,
                        J.total, J.pl);
         if (ps != TL_OK) return ps;
     }
@@ -979,9 +1047,9 @@ static tl_status run(tl_model* m, const tl_run_cfg* cfg, tl_result* res, tl_grad
     TLC(cudaSetDevice(m->d.device));
     cudaStream_t st = (cudaStream_t)cfg->stream;
     const bool no_stage = (cfg->flags & TL_FLAG_NO_STAGE) != 0;
-    const bool measure = !J.plain && cfg->variant == TL_VARIANT_AUTO && (cfg->flags & TL_FLAG_AUTOTUNE_MEASURE);
+    J.measure = !J.plain && cfg->variant == TL_VARIANT_AUTO && (cfg->flags & TL_FLAG_AUTOTUNE_MEASURE);
     if (!J.plain) {
-        ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.compat_stoich, no_stage, J.total, J.pl,
+        ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.sens, J.compat_stoich, no_stage, J.total, J.pl,
                        (cfg->flags & TL_FLAG_GLOBAL_SLOTS) != 0);
         if (ps != TL_OK) return ps;
     } else {
@@ -997,7 +1065,7 @@ static tl_status run(tl_model* m, const tl_run_cfg* cfg, tl_result* res, tl_grad
     if (ps != TL_OK) return ps;
     ps = job_bind(J, reinterpret_cast<unsigned char*>(base), st);
     if (ps != TL_OK) return ps;
-    if (measure) {
+    if (J.measure) {
         ps = autotune_measure(J, st);
         if (ps != TL_OK) return ps;
     }
@@ -1005,8 +1073,8 @@ static tl_status run(tl_model* m, const tl_run_cfg* cfg, tl_result* res, tl_grad
     const size_t w = J.w;
 
     cudaEvent_t e0, e1;
-    TLC(cudaEventCreate(&e0));
-    TLC(cudaEventCreate(&e1));
+    ps = timing_events(m, &e0, &e1);
+    if (ps != TL_OK) return ps;
     int launches = 0;
     cudaError_t le = cudaEventRecord(e0, st);
     if (le == cudaSuccess) {
@@ -1056,8 +1124,6 @@ static tl_status run(tl_model* m, const tl_run_cfg* cfg, tl_result* res, tl_grad
                 if (launches > (1 << 26)) {  // a realization that never ends
                     if (gexec) cudaGraphExecDestroy(gexec);
                     cudaFreeHost(hdone);
-                    cudaEventDestroy(e0);
-                    cudaEventDestroy(e1);
                     set_last_error("plain form exceeded 2^26 launches; set max_steps");
                     return TL_ERR_STEP_CAP;
                 }
@@ -1069,22 +1135,12 @@ static tl_status run(tl_model* m, const tl_run_cfg* cfg, tl_result* res, tl_grad
         }
     }
     if (le == cudaSuccess) le = cudaEventRecord(e1, st);
-    if (le != cudaSuccess) {
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        return cuda_fail(le, "simulation launch");
-    }
+    if (le != cudaSuccess) return cuda_fail(le, "simulation launch");
     ps = job_reduce(J, st);
-    if (ps != TL_OK) {
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        return ps;
-    }
+    if (ps != TL_OK) return ps;
     TLC(cudaStreamSynchronize(st));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     return job_finish(J, ms, launches, ms_since(t0));
 }
 
@@ -1154,7 +1210,7 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
             pl.batch = true;
             pl.lanes = unit_lanes;
             pl.thin = thin;
-            pl.slot = slot_layout(J.m, bmode, lane[(size_t)i] ? 1 : 32, 32);
+            pl.slot = slot_layout(J.m, J.sens, bmode, lane[(size_t)i] ? 1 : 32, 32);
             const size_t unit = !lane[(size_t)i] ? pl.slot.bytes : thin == 1 ? (size_t)unit_lanes * pl.slot.bytes : 0;
             wslot = std::max(wslot, unit);
         }
@@ -1252,31 +1308,21 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
                                               (units + warps - 1) / warps);
     for (auto& J : jobs) J.pl.grid = grid;
     cudaEvent_t e0, e1;
-    TLC(cudaEventCreate(&e0));
-    TLC(cudaEventCreate(&e1));
+    ps = timing_events(owner, &e0, &e1);
+    if (ps != TL_OK) return ps;
     le = cudaEventRecord(e0, st);
     if (le == cudaSuccess)
         le = pop == 64 ? launch_batch<long long>(bp, bmode, thin, 32 * warps, grid, smem, st)
                        : launch_batch<int>(bp, bmode, thin, 32 * warps, grid, smem, st);
     if (le == cudaSuccess) le = cudaEventRecord(e1, st);
-    if (le != cudaSuccess) {
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        return cuda_fail(le, "batch launch");
-    }
+    if (le != cudaSuccess) return cuda_fail(le, "batch launch");
     for (auto& J : jobs) {
         ps = job_reduce(J, st);
-        if (ps != TL_OK) {
-            cudaEventDestroy(e0);
-            cudaEventDestroy(e1);
-            return ps;
-        }
+        if (ps != TL_OK) return ps;
     }
     TLC(cudaStreamSynchronize(st));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     tl_status worst = TL_OK;
     for (auto& J : jobs) {
         const tl_status s2 = job_finish(J, ms, 1, ms_since(t0));
@@ -1439,6 +1485,8 @@ void tl_model_destroy(tl_model* m) {
         if (m->d.x0) cudaFree(m->d.x0);
         if (m->d.rate) cudaFree(m->d.rate);
         if (m->scratch) cudaFree(m->scratch);
+        for (void* e : m->ev)
+            if (e) cudaEventDestroy((cudaEvent_t)e);
         cudaSetDevice(cur);
     }
     delete m;
@@ -1582,7 +1630,6 @@ tl_status tl_eval_leap(tl_model* m, const int64_t* x, int32_t n, double eps, uin
                                            B + oc, reinterpret_cast<float*>(B + om), reinterpret_cast<float*>(B + os),
                                            reinterpret_cast<float*>(B + ot), reinterpret_cast<double*>(B + o0), smem, 0);
     if (e != cudaSuccess) return cuda_fail(e, "eval launch");
-    TLC(cudaDeviceSynchronize());
     if (a) TLC(cudaMemcpy(a, B + oa, (size_t)n * M * 4, cudaMemcpyDeviceToHost));
     if (crit) TLC(cudaMemcpy(crit, B + oc, (size_t)n * M, cudaMemcpyDeviceToHost));
     if (mu) TLC(cudaMemcpy(mu, B + om, (size_t)n * N * 4, cudaMemcpyDeviceToHost));
@@ -1777,11 +1824,19 @@ extern "C" tl_status tl_simulate_static(tl_model* m, const tl_run_cfg* cfg, tl_r
     if (ps != TL_OK) return ps;
     TLC(cudaSetDevice(m->d.device));
     cudaStream_t st = (cudaStream_t)cfg->stream;
-    ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.compat_stoich,
+    ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.sens, J.compat_stoich,
                    (cfg->flags & TL_FLAG_NO_STAGE) != 0, J.total, J.pl, (cfg->flags & TL_FLAG_GLOBAL_SLOTS) != 0);
     if (ps != TL_OK) return ps;
     Carver c;
     job_layout(J, c);
+    if (c.off > (size_t)TL_STATIC_SCRATCH_BYTES && J.pl.state_global) {
+        // the general build's global slots are smaller
+        ps = make_plan(m, cfg->variant, cfg->block_threads, kModeGeneral, J.sens, J.compat_stoich,
+                       (cfg->flags & TL_FLAG_NO_STAGE) != 0, J.total, J.pl, (cfg->flags & TL_FLAG_GLOBAL_SLOTS) != 0);
+        if (ps != TL_OK) return ps;
+        c = Carver{};
+        job_layout(J, c);
+    }
     if (c.off > (size_t)TL_STATIC_SCRATCH_BYTES) {
         set_last_error("this run needs " + std::to_string(c.off) + " bytes of device scratch; tl_simulate_static has " +
                        std::to_string((size_t)TL_STATIC_SCRATCH_BYTES) +

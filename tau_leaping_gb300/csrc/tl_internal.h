@@ -77,7 +77,8 @@ struct DevModel {
     bool chan8 = false, ent_wide = false;
     bool fast_ok = false;           // the model fits the packed fields
     void* x0 = nullptr;             // Pop[N]
-    float* rate = nullptr;          // [M]
+    float* rate = nullptr;          // [2][M]: as given, and halved for 2S channels
+    bool halvable = true;           // the halving is exact
     int nnz_net = 0, nnz_raw = 0;
 };
 
@@ -90,6 +91,7 @@ struct tl_model {
     // scratch (grow-only)
     void* scratch = nullptr;
     size_t scratch_bytes = 0;
+    void* ev[2] = {nullptr, nullptr};  // kernel timing (cudaEvent_t)
     // measured autotuner cache (TL_FLAG_AUTOTUNE_MEASURE)
     int tuned_variant = 0, tuned_block = 0, tuned_nostage = 0;
     unsigned tuned_key = 0;
