@@ -536,6 +536,69 @@ __global__ void k_stats(const Pop* samp, long long R, int P, int K, double* mean
     }
 }
 
+#ifdef TL_COMMON_KERNELS
+// The same statistics where many columns lie side by side (32-bit
+// populations): k_stats reads one 4-byte value per 32-byte sector there, twice,
+// and spends five FP64 operations a value.  Here a warp reads 32 columns of a
+// row at once, and the sums of d = x - x_first and d^2 (in halves) are exact
+// integers, so that any number of CTAs may add to them in any order.  Memory
+// bounds it.  1024 species on two grid points, 8192 realizations (67 MB):
+// 187 us -> 25 us (and 5 us for the results).
+__global__ void k_stats_wide(const int* samp, long long R, int PK, unsigned long long* acc) {
+    __shared__ unsigned long long sh[3][8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int col = blockIdx.x * 32 + lane, set = blockIdx.z;
+    const int* base = samp + (size_t)set * R * PK;
+    unsigned long long s1 = 0, lo = 0, hi = 0;
+    if (col < PK) {
+        const int first = base[col];
+        const long long by = 8LL * gridDim.y;
+        long long r = 8LL * blockIdx.y + warp;
+        const auto add = [&](int x) {
+            const long long d = (long long)x - (long long)first;
+            const unsigned long long a = (unsigned long long)(d < 0 ? -d : d), q = a * a;  // |d| < 2^32
+            s1 += (unsigned long long)d;
+            lo += q & 0xffffffffull;
+            hi += q >> 32;
+        };
+        for (; r + 3 * by < R; r += 4 * by) {
+            int x[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) x[t] = __ldcs(base + (size_t)(r + t * by) * PK + col);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) add(x[t]);
+        }
+        for (; r < R; r += by) add(__ldcs(base + (size_t)r * PK + col));
+    }
+    sh[0][warp][lane] = s1;
+    sh[1][warp][lane] = lo;
+    sh[2][warp][lane] = hi;
+    __syncthreads();
+    if (warp < 3 && col < PK) {
+        unsigned long long t = 0;
+        for (int w = 0; w < 8; ++w) t += sh[warp][w][lane];
+        atomicAdd(acc + 3 * ((size_t)set * PK + col) + warp, t);
+    }
+}
+
+// mean = first + S1/n; the variance's numerator n S2 - S1^2 is exact in 128 bits.
+__global__ void k_stats_wide_finish(const int* samp, long long R, int PK, int cols, const unsigned long long* acc,
+                                    double* mean, double* sd) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= cols) return;
+    const int set = c / PK;
+    const int first = samp[(size_t)set * R * PK + (c - set * PK)];
+    const long long s1 = (long long)acc[3 * (size_t)c];
+    const unsigned __int128 s2 = ((unsigned __int128)acc[3 * (size_t)c + 2] << 32) + acc[3 * (size_t)c + 1];
+    const unsigned long long a1 = (unsigned long long)(s1 < 0 ? -s1 : s1);
+    const unsigned __int128 num = s2 * (unsigned long long)R - (unsigned __int128)a1 * a1;
+    const double n = (double)R;
+    mean[c] = (double)first + (double)s1 / n;
+    const double numd = (double)(unsigned long long)(num >> 64) * 18446744073709551616.0 + (double)(unsigned long long)num;
+    sd[c] = R > 1 ? sqrt(numd / (n * (n - 1.0))) : 0.0;
+}
+#endif
+
 // Likelihood-ratio estimator: grad[s][k][j] = Cov_r(X_k(T), score_j),
 // stderr from the spread of the per-realization products.
 template <class Pop>

@@ -1,4 +1,5 @@
 // Kernels and launchers for 32-bit populations.
+#include <algorithm>
 #define TL_COMMON_KERNELS
 #include "tl_kernels.cuh"
 #include "tl_call.cuh"
@@ -10,6 +11,23 @@ namespace tl {
 
 cudaError_t launch_plain_tally(const SimParams& p, cudaStream_t st) {
     k_plain_tally<<<152, 256, 0, st>>>(p);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_stats_wide(const void* samp, long long R, int PK, int S, void* acc, double* mean, double* sd,
+                              cudaStream_t st) {
+    const size_t cols = (size_t)S * PK;
+    cudaError_t e = cudaMemsetAsync(acc, 0, cols * 24, st);
+    if (e != cudaSuccess) return e;
+    // about eight CTAs an SM over the rows, 32 rows a CTA at least
+    const int tiles = (PK + 31) / 32;
+    const long long want = (152LL * 8 + (long long)tiles * S - 1) / ((long long)tiles * S);
+    const int split = (int)std::max<long long>(1, std::min<long long>(std::min<long long>(want, (R + 31) / 32), 65535));
+    k_stats_wide<<<dim3((unsigned)tiles, (unsigned)split, (unsigned)S), 256, 0, st>>>(
+        reinterpret_cast<const int*>(samp), R, PK, reinterpret_cast<unsigned long long*>(acc));
+    k_stats_wide_finish<<<(unsigned)((cols + 127) / 128), 128, 0, st>>>(reinterpret_cast<const int*>(samp), R, PK,
+                                                                       (int)cols,
+                                                                       reinterpret_cast<unsigned long long*>(acc), mean, sd);
     return cudaGetLastError();
 }
 

@@ -117,3 +117,16 @@ def test_global_propensities_and_batches_are_bit_identical():
     slow = simulate_batch([dict(it, flags=general) for it in items])
     for x, y in zip(fast, slow):
         assert np.array_equal(x["samples"], y["samples"]) and x["leaps"] == y["leaps"]
+
+
+@pytest.mark.parametrize("n,K,intervals,sets", [(64, 64, 1, 1), (1001, 33, 2, 3), (257, 130, 1, 2)])
+def test_statistics_of_many_columns(n, K, intervals, sets):
+    """Means and deviations of 64 columns and more: exact integer sums, so
+    within FP64 rounding of numpy's on the same samples."""
+    m, _ = network(K, 2 * K, 7)
+    rates = np.tile(m.desc()["rate"], (sets, 1))
+    r = m.simulate(0.01, n, seed=5, intervals=intervals, keep_samples=True, rate_sets=rates, max_steps=50,
+                   allow_truncation=True)
+    x = r.samples.astype(np.float64)
+    assert np.allclose(r.mean, x.mean(axis=1), rtol=1e-13, atol=1e-13)
+    assert np.allclose(r.stddev, x.std(axis=1, ddof=1), rtol=1e-11, atol=1e-11)
