@@ -369,12 +369,14 @@ struct Plan {
     int thin = 1;          // and lanes of one realization
     bool state_global = false;  // global slots: the state as well as a[]
     bool batch = false;
+    bool team = false;     // warp groups: four warps per realization
     SlotLayout slot;
 };
 
 // The kernel a plan launches (CTA groups with global slots are their own build).
 static int launch_kind(const Plan& pl) {
     if (pl.gslot) return kKindCtaGlobal;
+    if (pl.team) return kKindTeam;
     if (pl.kind == 1 && pl.mode != kModeGeneral) return 100 + pl.thin;
     return pl.kind;
 }
@@ -436,6 +438,13 @@ static void thin_plan(int size, long long total, int nsm, int& thin, int& lanes)
     lanes = 32;
     if (thin > 1)
         while (lanes > thin && total * 2 * thin <= (thin == 4 ? 10LL : 3LL) * nsm * lanes) lanes /= 2;
+}
+
+// Four-warp teams for a warp-group ensemble of up to eight realizations an SM:
+// enough channels for 128 threads, and a chain of steps that sets the time.
+// %%TEAM%%
+static bool team_pays(const tl_model* m, long long total, int nsm) {
+    return m->h.M >= 128 && total <= 8LL * nsm;
 }
 
 static tl_status make_plan(const tl_model* m, int variant, int block_req, int mode, bool sens, bool compat_stoich,
@@ -549,6 +558,25 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
     if (bps < 1) {
         set_last_error("the launch does not fit an SM");
         return TL_ERR_UNSUPPORTED;
+    }
+    if (pl.kind == 32 && pl.mode != kModeGeneral && block_req <= 0 && staged && !pl.slot.score_global &&
+        team_pays(m, total, nsm)) {
+        Plan t = pl;
+        t.team = true;
+        t.block = 128;
+        t.slot = slot_layout(m, sens, pl.mode, 0, 128);
+        t.smem = (size_t)t.stage + t.slot.bytes;
+        int tb = 0;
+        if (t.smem <= (size_t)smax) {
+            e = m->h.pop_bits == 64 ? fused_occupancy<long long>(kKindTeam, t.mode, true, 128, t.smem, &tb)
+                                    : fused_occupancy<int>(kKindTeam, t.mode, true, 128, t.smem, &tb);
+            if (e != cudaSuccess) return cuda_fail(e, "occupancy");
+        }
+        if (total <= (long long)nsm * tb) {  // all realizations at once
+            pl = t;
+            groups_per_block = 1;
+            bps = tb;
+        }
     }
     const long long need = (total + groups_per_block - 1) / groups_per_block;
     pl.grid = (int)std::min<long long>((long long)nsm * bps, std::max<long long>(need, 1));
@@ -1254,6 +1282,34 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
         set_last_error("a batched model is too large for a warp unit; run it with tl_simulate");
         return TL_ERR_UNSUPPORTED;
     }
+    // four-warp teams where all larger items' realizations run at once on them
+    bool team = bmode != kModeGeneral && staged && thin > 1;
+    long long big_total = 0;
+    bool wide_item = false;
+    size_t tslot = 0;
+    for (int i = 0; i < n; ++i)
+        if (!lane[(size_t)i]) {
+            const Job& J = jobs[(size_t)i];
+            big_total += J.total;
+            wide_item |= team_pays(J.m, J.total, sm_count());
+            tslot = std::max(tslot, slot_layout(J.m, J.sens, bmode, 0, 128).bytes);
+        }
+    tslot = al16(tslot);
+    const size_t team_smem = stage + 2 * (tslot + spb);
+    int team_bps = 0;
+    if (team && wide_item && team_smem <= (size_t)smax) {
+        const BatchParams none{};
+        const cudaError_t oe = pop == 64 ? launch_batch_team<long long>(none, bmode, thin, 0, team_smem, st, &team_bps)
+                                         : launch_batch_team<int>(none, bmode, thin, 0, team_smem, st, &team_bps);
+        if (oe != cudaSuccess) return cuda_fail(oe, "batch occupancy");
+    }
+    team = big_total > 0 && big_total <= 2LL * team_bps * sm_count();
+    if (team) {
+        warps = 8;
+        wslot = tslot;
+        for (int i = 0; i < n; ++i)
+            if (!lane[(size_t)i]) jobs[(size_t)i].pl.slot = slot_layout(jobs[(size_t)i].m, jobs[(size_t)i].sens, bmode, 0, 128);
+    }
     // scratch: every job's buffers, the item table, the staged tables, a counter
     Carver c;
     for (auto& J : jobs) job_layout(J, c);
@@ -1280,7 +1336,7 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     for (int i = 0; i < n; ++i)
         if (lane[(size_t)i]) order.push_back(i);
     std::vector<BatchItem> hb((size_t)n);
-    const int per_unit = unit_lanes / thin;
+    const int per_unit = unit_lanes / thin * (team ? 4 : 1);
     long long units = 0;
     for (int k = 0; k < n; ++k) {
         const int i = order[(size_t)k];
@@ -1310,20 +1366,22 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     bp.warp_slot_bytes = (int)wslot;
     bp.params_bytes = (int)spb;
     bp.wctr = reinterpret_cast<unsigned long long*>(B + o_wctr);
-    const size_t smem = stage + (size_t)warps * (wslot + spb);
-    int bps = 0;
-    cudaError_t le = pop == 64 ? batch_occupancy<long long>(bmode, staged, thin, 32 * warps, smem, &bps)
+    const size_t smem = team ? team_smem : stage + (size_t)warps * (wslot + spb);
+    int bps = team_bps;
+    cudaError_t le = team ? cudaSuccess : pop == 64 ? batch_occupancy<long long>(bmode, staged, thin, 32 * warps, smem, &bps)
                                : batch_occupancy<int>(bmode, staged, thin, 32 * warps, smem, &bps);
     if (le != cudaSuccess) return cuda_fail(le, "batch occupancy");
     const int grid = (int)std::min<long long>((long long)sm_count() * std::max(bps, 1),
-                                              (units + warps - 1) / warps);
+                                              team ? (units + 1) / 2 : (units + warps - 1) / warps);
     for (auto& J : jobs) J.pl.grid = grid;
     cudaEvent_t e0, e1;
     ps = timing_events(owner, &e0, &e1);
     if (ps != TL_OK) return ps;
     le = cudaEventRecord(e0, st);
     if (le == cudaSuccess)
-        le = pop == 64 ? launch_batch<long long>(bp, bmode, thin, 32 * warps, grid, smem, st)
+        le = team ? (pop == 64 ? launch_batch_team<long long>(bp, bmode, thin, grid, smem, st, nullptr)
+                               : launch_batch_team<int>(bp, bmode, thin, grid, smem, st, nullptr))
+             : pop == 64 ? launch_batch<long long>(bp, bmode, thin, 32 * warps, grid, smem, st)
                        : launch_batch<int>(bp, bmode, thin, 32 * warps, grid, smem, st);
     if (le == cudaSuccess) le = cudaEventRecord(e1, st);
     if (le != cudaSuccess) return cuda_fail(le, "batch launch");

@@ -250,12 +250,23 @@ struct ThinGroupOf {
     static TL_D bool idle(const SimParams& p) { return (int)(threadIdx.x & 31) >= p.lanes; }
 };
 template <>
+struct FastGroupOf<kKindTeam> {
+    using type = GTeam;
+    static TL_D GTeam make(double* red) {
+        return GTeam::make(0, reinterpret_cast<float*>(red), reinterpret_cast<long long*>(red + 4));
+    }
+    static TL_D int index(const SimParams&) { return 0; }
+    static TL_D bool idle(const SimParams&) { return false; }
+};
+template <>
 struct FastGroupOf<kKindThin1> : ThinGroupOf<1> {};
 
 template <int KIND, class Pop, bool SENS, bool STAGED, bool GSLOT = false>
-__global__ void __launch_bounds__(KIND == 0 ? 1024 : 256,
-                                  KIND == 0 ? 1 : KIND == kKindThin1 ? TL_THREAD_MINB : TL_WARP_MINB)
-    k_fast(const __grid_constant__ SimParams p) {
+__global__ void __launch_bounds__(KIND == 0 ? 1024 : KIND == kKindTeam ? 128 : 256,
+                                  KIND == 0           ? 1
+                                  : KIND == kKindTeam ? 8
+                                  : KIND == kKindThin1 ? TL_THREAD_MINB
+                                                       : TL_WARP_MINB) k_fast(const __grid_constant__ SimParams p) {
     __shared__ __align__(8) unsigned long long mbar;
     __shared__ double red[34];
     using Of = FastGroupOf<KIND>;
@@ -390,6 +401,56 @@ __global__ void __launch_bounds__(256, TL_BATCH_MINB) k_batch(BatchParams bp) {
             }
         }
         __syncwarp();
+    }
+}
+
+// The batched kernel on teams: two four-warp teams per CTA, each taking units
+// from the counter.  A small item's unit is four warps of realizations.
+template <class Pop, bool SENS, int W>
+__global__ void __launch_bounds__(256, 4) k_batch_team(BatchParams bp) {
+    __shared__ __align__(8) unsigned long long mbar;
+    __shared__ float red[2][4];
+    __shared__ long long box[2];
+    if (!stage_blob(tl_smem, bp.stage_src, bp.stage_bytes, bp.items[0].p.wait_polls, &mbar)) {
+        if (threadIdx.x == 0) atomicOr((unsigned*)(bp.items[0].p.ctr + 5), kErrWaitTimeout | kErrStage);
+        return;
+    }
+    using Lay = tl::Lay<Pop, true, false>;
+    const int team = threadIdx.x >> 7;
+    const GTeam g = GTeam::make(1 + team, red[team], &box[team]);
+    const uint32_t my_slot = (uint32_t)(bp.stage_bytes + team * bp.warp_slot_bytes);
+    SimParams* sp = reinterpret_cast<SimParams*>(tl_smem + bp.stage_bytes + 2 * bp.warp_slot_bytes + team * bp.params_bytes);
+    int cur = -1;
+    for (;;) {
+        long long u = 0;
+        if (g.leader()) u = (long long)atomicAdd(bp.wctr, 1ull);
+        u = g.bcast(u, 0);
+        if (u >= bp.total_units) break;
+        int it = 0;
+        while (it + 1 < bp.n_items && u >= bp.items[it + 1].unit_begin) ++it;
+        if (it != cur) {
+            const int* src = reinterpret_cast<const int*>(&bp.items[it].p);
+            int* dst = reinterpret_cast<int*>(sp);
+            for (int k = g.tid; k < (int)(sizeof(SimParams) / 4); k += 128) dst[k] = src[k];
+            g.sync();
+            cur = it;
+        }
+        const SimParams& p = *sp;
+        const uint32_t tab = (uint32_t)bp.items[it].stage_off;
+        const long long local = u - bp.items[it].unit_begin;
+        if (!bp.items[it].lane_mode) {
+            const Lay L{p, my_slot, tab, nullptr, nullptr};
+            fast_realization<GTeam, Lay, SENS>(g, p, L, local);
+        } else if (g.lane < p.lanes) {
+            const long long wi = (local * 4 + g.warp) * (p.lanes / W) + g.lane / W;
+            if (wi < p.R * (long long)p.S) {
+                const auto tg = TinyGroup<W>::make();
+                TinyLane<W, Pop> L;
+                L.load(reinterpret_cast<const TinyTable*>(tl_smem + tab + p.t_tiny), tg.lane);
+                tiny_realization<W, Pop, SENS>(tg, p, L, wi);
+            }
+        }
+        g.sync();
     }
 }
 

@@ -15,6 +15,7 @@ struct SimParams;
 // in the fast and scores builds thread groups are thin groups of one lane or,
 // for small models, 4, 8 or 16 lanes (tl_tiny.cuh).
 constexpr int kKindCtaGlobal = 64;
+constexpr int kKindTeam = 132;  // four warps for one realization of a warp group
 constexpr int kKindThin1 = 101, kKindTiny4 = 104, kKindTiny8 = 108, kKindTiny16 = 116;
 
 // Table of a small model (N, M <= 16): per channel {s0, s1, order, 0}, then per
@@ -82,6 +83,10 @@ template <class Pop>
 cudaError_t launch_batch(const BatchParams& bp, int mode, int thin, int block, int grid, size_t smem, cudaStream_t st);
 template <class Pop>
 cudaError_t batch_occupancy(int mode, bool staged, int thin, int block, size_t smem, int* blocks_per_sm);
+// the same with four-warp teams in place of the warp units (staged tables only)
+template <class Pop>
+cudaError_t launch_batch_team(const BatchParams& bp, int mode, int thin, int grid, size_t smem, cudaStream_t st,
+                              int* blocks_per_sm);
 template <class Pop>
 cudaError_t launch_plain_init(const SimParams& p, cudaStream_t st);
 template <class Pop>

@@ -31,6 +31,8 @@
 // of 250 species 5.14 -> 3.44, of 400 species (global propensities) 2.74 -> 1.78.
 #pragma once
 
+#include <type_traits>
+
 #include "tl_device.cuh"
 
 namespace tl {
@@ -80,6 +82,66 @@ struct is_thin {
 template <int W>
 struct is_thin<GThin<W>> {
     static constexpr bool value = true;
+};
+
+// Four warps for one realization of a warp-group model in a small ensemble,
+// where the latency of one realization's steps sets the time.  Passes are
+// spread over 128 threads; every sum runs as a warp group forms it (each warp
+// forms all of them: sum_group), so the results are the warp group's.  One
+// named barrier per team.
+struct GTeam {
+    static constexpr int kWidth = 128;
+    int tid, lane, warp, bar;
+    float* red;      // one value per warp
+    long long* box;  // a broadcast value
+    static TL_D GTeam make(int bar, float* red, long long* box) {
+        const int t = (int)threadIdx.x & 127;
+        return GTeam{t, t & 31, t >> 5, bar, red, box};
+    }
+    TL_D int rank() const { return tid; }
+    TL_D int size() const { return 128; }
+    TL_D void sync() const { asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory"); }
+    TL_D bool leader() const { return tid == 0; }
+    TL_D bool any(bool p) const {
+        unsigned r;
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\t"
+            "setp.ne.u32 p, %1, 0;\n\t"
+            "bar.red.or.pred q, %2, 128, p;\n\t"
+            "selp.u32 %0, 1, 0, q;\n\t}"
+            : "=r"(r)
+            : "r"(p ? 1u : 0u), "r"(bar)
+            : "memory");
+        return r != 0u;
+    }
+    // (other barriers lie between two calls)
+    TL_D float minf(float v) const {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
+        if (lane == 0) red[warp] = v;
+        sync();
+        return fminf(fminf(red[0], red[1]), fminf(red[2], red[3]));
+    }
+    TL_D long long bcast(long long v, int) const {
+        if (tid == 0) *box = v;
+        sync();
+        const long long r = *box;
+        sync();
+        return r;
+    }
+};
+TL_D GWarp queue_group(const GTeam& g) { return GWarp{g.lane}; }
+
+// The lanes over which a group's sums run.
+template <class Grp>
+TL_D const Grp& sum_group(const Grp& g) {
+    return g;
+}
+TL_D GWarp sum_group(const GTeam& g) { return GWarp{g.lane}; }
+
+template <class Grp>
+struct many_warps {
+    static constexpr bool value = Grp::kWidth == 0 || Grp::kWidth == 128;
 };
 
 // Where one realization's state and the tables lie.  Only offsets are kept:
@@ -201,12 +263,21 @@ TL_D void fast_props(const Grp& g, const SimParams& p, const Lay& L, const float
         const float v = __ldg(rate + j) * fabsf(f0) * fabsf(f1);
         const uint32_t cr = (__float_as_uint(f0) | __float_as_uint(f1)) & 0x80000000u;
         L.a()[j] = __uint_as_float(__float_as_uint(v) | cr);
-        if constexpr (!is_thin<Grp>::value) {
+        if constexpr (!is_thin<Grp>::value && Grp::kWidth != 128) {
             s += v;
             sc += cr ? v : 0.f;
         }
     }
     g.sync();
+    if constexpr (Grp::kWidth == 128) {
+        // the partial sums of a warp group's lane
+#pragma unroll 4
+        for (int j = sum_group(g).rank(); j < p.M; j += 32) {
+            const float v = L.a()[j];
+            s += fabsf(v);
+            sc += fmaxf(-v, 0.f);
+        }
+    }
     if constexpr (is_thin<Grp>::value) {
         // a[] is padded with zeros to whole blocks of four
         for (int j = 0; j < p.M; j += 4) {
@@ -464,7 +535,7 @@ TL_D void fast_fire(const Grp& g, const SimParams& p, const Lay& L, float tauf, 
     constexpr int kTurn = 4 * decltype(queue_group(g))::kWidth;  // channels of a queue group's turn
     const int cap = p.q_rounds * kTurn;
     unsigned short* q = L.q();
-    if constexpr (Grp::kWidth == 0) q += g.warp * (cap + 2);
+    if constexpr (many_warps<Grp>::value) q += g.warp * (cap + 2);
     const float* a = L.a();
     const int G4 = (p.M + 3) >> 2;
     for (int b0 = g.rank() - qg.rank(); b0 < G4;) {
@@ -531,7 +602,7 @@ TL_D void fast_fire(const Grp& g, const SimParams& p, const Lay& L, float tauf, 
         if (qg.rank() == 0) *next = 0;
         qg.sync();
         const auto channel = [&](int id) {
-            if constexpr (Grp::kWidth == 0) return j_first + (id / kTurn) * 4 * g.size() + id % kTurn;
+            if constexpr (many_warps<Grp>::value) return j_first + (id / kTurn) * 4 * g.size() + id % kTurn;
             else return j_first + id;
         };
         for (int i = qg.rank(); i < n_front; i += qg.size()) {
@@ -976,7 +1047,7 @@ TL_D void direct_steps(const Grp& g, const SimParams& p, const Lay& L, int set, 
             a0 = (float)total;
             j = select_channel<Grp, double>(g, p, L.a(), pa, u01d(w_hi, w_lo) * total, 0);
         } else {
-            j = ssa_select(g, p, L, pa, w_hi, w_lo, a0);
+            j = ssa_select(sum_group(g), p, L, pa, w_hi, w_lo, a0);
         }
         // the waiting time in FP32 (FP64 keeps only the time sum)
         const float dtf = qg.bcast(ex, from) / a0;
@@ -1037,7 +1108,7 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
     fast_props(g, p, L, rate, pa, pac);
     float a0f;
     if constexpr (kThin) a0f = pa;
-    else a0f = g.sumf(pa);
+    else a0f = sum_group(g).sumf(pa);
     if (!(a0f > 0.f)) {
         st.done = true;  // nothing can fire: the state holds to t_final
         return;
@@ -1060,7 +1131,7 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
     bool clamp;
     float a0cf;
     if constexpr (kThin) a0cf = pac;
-    else a0cf = g.sumf(pac);
+    else a0cf = sum_group(g).sumf(pac);
     for (int attempt = 0;; ++attempt) {
         // the step's scalar words are needed only when a channel is critical
         // and each lane draws another step's
@@ -1089,8 +1160,9 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
                 const double a0c = (double)pac;
                 jc = select_channel<G1, double>(G1{}, p, L.a(), pac, u01d(w.z, w.w) * a0c, 1);
             } else {
-                const double a0c = g.sumd((double)pac);
-                jc = select_channel<Grp, double>(g, p, L.a(), pac, u01d(w.z, w.w) * a0c, 1);
+                const auto sg = sum_group(g);
+                const double a0c = sg.sumd((double)pac);
+                jc = select_channel<std::decay_t<decltype(sum_group(g))>, double>(sg, p, L.a(), pac, u01d(w.z, w.w) * a0c, 1);
             }
         }
         bool over = false, bad;
