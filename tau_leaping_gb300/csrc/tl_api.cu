@@ -1284,6 +1284,7 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     }
     // four-warp teams where all larger items' realizations run at once on them
     bool team = bmode != kModeGeneral && staged && thin > 1;
+    for (auto& J : jobs) team &= J.cfg->seed == jobs[0].cfg->seed;
     long long big_total = 0;
     bool wide_item = false;
     size_t tslot = 0;
@@ -1366,6 +1367,7 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     bp.warp_slot_bytes = (int)wslot;
     bp.params_bytes = (int)spb;
     bp.wctr = reinterpret_cast<unsigned long long*>(B + o_wctr);
+    round_keys(jobs[0].p.k0, jobs[0].p.k1, bp.rk);
     const size_t smem = team ? team_smem : stage + (size_t)warps * (wslot + spb);
     int bps = team_bps;
     cudaError_t le = team ? cudaSuccess : pop == 64 ? batch_occupancy<long long>(bmode, staged, thin, 32 * warps, smem, &bps)

@@ -827,6 +827,7 @@ struct BatchParams {
     int warp_slot_bytes;
     int params_bytes;
     unsigned long long* wctr;
+    uint32_t rk[20];  // round keys, where all items share one seed
 };
 
 template <class Pop>

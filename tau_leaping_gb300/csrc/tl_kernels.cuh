@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(KIND == 0 ? 1024 : KIND == kKindTeam ? 128 : 2
         g_state = p.state_global ? mine : tl_smem;
         g_big = mine + p.f_big;
     }
-    const Lay L{p, slots + (uint32_t)(Of::index(p) * p.slot_bytes), 0u, g_state, g_big};
+    const Lay L{p, slots + (uint32_t)(Of::index(p) * p.slot_bytes), 0u, g_state, g_big, p.rk};
     const long long total = p.R * (long long)p.S;
     for (;;) {
         long long w = 0;
@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(256, TL_THREAD_MINB) k_tiny(const __grid_const
         if (g.lane == 0) w = (long long)atomicAdd(p.ctr + 0, 1ull);
         w = g.from(w, 0);
         if (w >= total) break;
-        tiny_realization<W, Pop, SENS>(g, p, L, w);
+        tiny_realization<W, Pop, SENS>(g, p, p.rk, L, w);
     }
 }
 
@@ -370,19 +370,19 @@ __global__ void __launch_bounds__(256, TL_BATCH_MINB) k_batch(BatchParams bp) {
             using Lay = tl::Lay<Pop, STAGED, false>;
             const uint32_t my_slot = (uint32_t)(bp.stage_bytes + warp * bp.warp_slot_bytes);
             if (!bp.items[it].lane_mode) {
-                const Lay L{p, my_slot, (uint32_t)soff, nullptr, nullptr};
+                const Lay L{p, my_slot, (uint32_t)soff, nullptr, nullptr, p.rk};
                 fast_realization<GWarp, Lay, SENS>(GWarp{lane}, p, L, local);
             } else if (lane < p.lanes) {
                 const long long wi = local * (p.lanes / W) + lane / W;
                 if (wi < total) {
                     if constexpr (W == 1) {
-                        const Lay L{p, my_slot + (uint32_t)(lane * p.slot_bytes), (uint32_t)soff, nullptr, nullptr};
+                        const Lay L{p, my_slot + (uint32_t)(lane * p.slot_bytes), (uint32_t)soff, nullptr, nullptr, p.rk};
                         fast_realization<GThin<1>, Lay, SENS>(GThin<1>::make(), p, L, wi);
                     } else {
                         const auto g = TinyGroup<W>::make();
                         TinyLane<W, Pop> L;
                         L.load(reinterpret_cast<const TinyTable*>((STAGED ? smem + soff : p.blob) + p.t_tiny), g.lane);
-                        tiny_realization<W, Pop, SENS>(g, p, L, wi);
+                        tiny_realization<W, Pop, SENS>(g, p, p.rk, L, wi);
                     }
                 }
             }
@@ -405,9 +405,10 @@ __global__ void __launch_bounds__(256, TL_BATCH_MINB) k_batch(BatchParams bp) {
 }
 
 // The batched kernel on teams: two four-warp teams per CTA, each taking units
-// from the counter.  A small item's unit is four warps of realizations.
+// from the counter.  A small item's unit is four warps of realizations.  All
+// items share one seed: its round keys are launch parameters.
 template <class Pop, bool SENS, int W>
-__global__ void __launch_bounds__(256, 4) k_batch_team(BatchParams bp) {
+__global__ void __launch_bounds__(256, 4) k_batch_team(const __grid_constant__ BatchParams bp) {
     __shared__ __align__(8) unsigned long long mbar;
     __shared__ float red[2][4];
     __shared__ long long box[2];
@@ -439,7 +440,7 @@ __global__ void __launch_bounds__(256, 4) k_batch_team(BatchParams bp) {
         const uint32_t tab = (uint32_t)bp.items[it].stage_off;
         const long long local = u - bp.items[it].unit_begin;
         if (!bp.items[it].lane_mode) {
-            const Lay L{p, my_slot, tab, nullptr, nullptr};
+            const Lay L{p, my_slot, tab, nullptr, nullptr, bp.rk};
             fast_realization<GTeam, Lay, SENS>(g, p, L, local);
         } else if (g.lane < p.lanes) {
             const long long wi = (local * 4 + g.warp) * (p.lanes / W) + g.lane / W;
@@ -447,7 +448,7 @@ __global__ void __launch_bounds__(256, 4) k_batch_team(BatchParams bp) {
                 const auto tg = TinyGroup<W>::make();
                 TinyLane<W, Pop> L;
                 L.load(reinterpret_cast<const TinyTable*>(tl_smem + tab + p.t_tiny), tg.lane);
-                tiny_realization<W, Pop, SENS>(tg, p, L, wi);
+                tiny_realization<W, Pop, SENS>(tg, p, bp.rk, L, wi);
             }
         }
         g.sync();

@@ -160,6 +160,7 @@ struct Lay {
     uint32_t tab;              // byte offset of the tables in shared memory
     unsigned char* g_state;    // GLOBAL: the state, in either memory
     unsigned char* g_big;      // GLOBAL: a[]
+    const uint32_t* rk;        // Philox round keys, in the launch parameters where one key serves the launch
 
     TL_D unsigned char* state(int off) const { return GLOBAL ? g_state + off : tl_smem + (slot + (uint32_t)off); }
     TL_D unsigned char* big(int off) const {
@@ -553,7 +554,7 @@ TL_D void fast_fire(const Grp& g, const SimParams& p, const Lay& L, float tauf, 
             for (int e = 0; e < 4; ++e) mu[e] = fmaxf(av[e], 0.f) * tauf;  // critical channels: 0
             U4 gw{0u, 0u, 0u, 0u};
             if (fminf(fminf(mu[0], mu[1]), fminf(mu[2], mu[3])) < 10.f)
-                gw = group_words(p.rk, (uint32_t)g4, step, r, set);
+                gw = group_words(L.rk, (uint32_t)g4, step, r, set);
             unsigned all = 0, far = 0, fired = 0;
             const bool any_far = fmaxf(fmaxf(mu[0], mu[1]), fmaxf(mu[2], mu[3])) >= 10.f;
 #pragma unroll
@@ -610,7 +611,7 @@ TL_D void fast_fire(const Grp& g, const SimParams& p, const Lay& L, float tauf, 
             int k = 1;
             if (i < n_inv) {
                 const float mu = fmaxf(a[j], 0.f) * tauf;
-                U4 w = group_words(p.rk, (uint32_t)j >> 2, step, r, set);
+                U4 w = group_words(L.rk, (uint32_t)j >> 2, step, r, set);
                 uint32_t word = word_of(w, j & 3);
                 for (int it = 0; !queued_inversion(mu, word, it, k); ++it) {
                     w = philox10(U4{(uint32_t)j, step, r, (set << 8) + (uint32_t)(it >> 2)}, p.k0, p.k1);
@@ -628,7 +629,7 @@ TL_D void fast_fire(const Grp& g, const SimParams& p, const Lay& L, float tauf, 
             for (int i = atomicAdd(next, 1); i < n_big;) {
                 const int j = channel(q[cap - 1 - i]);
                 const float mu = a[j] * tauf;
-                const U4 w = philox10rk(U4{(uint32_t)j, step, r, (set << 8) + (uint32_t)(it >> 1)}, p.rk);
+                const U4 w = philox10rk(U4{(uint32_t)j, step, r, (set << 8) + (uint32_t)(it >> 1)}, L.rk);
                 const bool odd = it & 1;
                 int k;
                 bool ok = Ptrs(mu).attempt(u01f(odd ? w.z : w.x), u01f(odd ? w.w : w.y), k);
@@ -692,7 +693,7 @@ template <int W, class Lay, bool SENS>
 TL_D void thin_fire(const GThin<W>& g, const SimParams& p, const Lay& L, float tauf, int jc, uint32_t step,
                     uint32_t r, uint32_t set) {
     for (int j = g.rank(); j < p.M; j += W) {
-        const int k = poisson_channel(L.a()[j], tauf, j, jc, step, r, set, p.rk);
+        const int k = poisson_channel(L.a()[j], tauf, j, jc, step, r, set, L.rk);
         if constexpr (SENS) L.k()[j] = k;
         if (k) fire_channel<GThin<W>>(L, j, k);
     }
@@ -785,9 +786,9 @@ TL_D bool wide_leap(const Grp& g, const SimParams& p, const Lay& L, float tauf, 
         if (is_crit(aj)) {
             k = j == jc ? 1 : 0;
         } else {
-            const U4 gw = group_words(p.rk, (uint32_t)j >> 2, step, r, set);
+            const U4 gw = group_words(L.rk, (uint32_t)j >> 2, step, r, set);
             ChanRng rng;
-            rng.init((uint32_t)j, step, r, set, p.rk);
+            rng.init((uint32_t)j, step, r, set, L.rk);
             k = poisson_first(aj * tauf, word_of(gw, j & 3), rng);
         }
         if constexpr (SENS) L.k()[j] = k;
@@ -1032,7 +1033,7 @@ TL_D void direct_steps(const Grp& g, const SimParams& p, const Lay& L, int set, 
     float ex = 0.f;
     for (int q = 0;;) {
         if ((q & (qg.size() - 1)) == 0) {
-            w = step_words(p.rk, st.step + (uint32_t)qg.rank(), r, (uint32_t)set);
+            w = step_words(L.rk, st.step + (uint32_t)qg.rank(), r, (uint32_t)set);
             ex = -logf(u01f(w.x));
         }
         const int from = q & (qg.size() - 1);
@@ -1140,7 +1141,7 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
             const auto qg = queue_group(g);
             if (st.step - st.ex_from >= (uint32_t)qg.size()) {
                 st.ex_from = st.step;
-                st.ex = -logf(u01f(step_words(p.rk, st.step + (uint32_t)qg.rank(), r, (uint32_t)set).x));
+                st.ex = -logf(u01f(step_words(L.rk, st.step + (uint32_t)qg.rank(), r, (uint32_t)set).x));
             }
             tau2 = qg.bcast(st.ex, (int)(st.step - st.ex_from)) / a0cf;
         }
@@ -1155,7 +1156,7 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
         tau_used = tauf;
         int jc = -1;
         if (fire) {
-            const U4 w = step_words(p.rk, st.step, r, (uint32_t)set);
+            const U4 w = step_words(L.rk, st.step, r, (uint32_t)set);
             if constexpr (kThin) {
                 const double a0c = (double)pac;
                 jc = select_channel<G1, double>(G1{}, p, L.a(), pac, u01d(w.z, w.w) * a0c, 1);

@@ -120,7 +120,8 @@ TL_D int tiny_select(const float* av, float part, uint32_t w_hi, uint32_t w_lo, 
 }
 
 template <int W, class Pop, bool SENS>
-TL_D void tiny_realization(const TinyGroup<W>& g, const SimParams& p, TinyLane<W, Pop>& L, long long w_index) {
+TL_D void tiny_realization(const TinyGroup<W>& g, const SimParams& p, const uint32_t* rk, TinyLane<W, Pop>& L,
+                           long long w_index) {
     const int set = p.S == 1 ? 0 : (int)(w_index / p.R);
     const uint32_t r = (uint32_t)(p.r_off + w_index - (long long)set * p.R);
     const bool channel = g.lane < p.M, species = g.lane < p.N;
@@ -141,7 +142,7 @@ TL_D void tiny_realization(const TinyGroup<W>& g, const SimParams& p, TinyLane<W
     const auto words = [&]() {
         if (step - w_from >= (uint32_t)W) {
             w_from = step;
-            w = step_words(p.rk, step + (uint32_t)g.lane, r, (uint32_t)set);
+            w = step_words(rk, step + (uint32_t)g.lane, r, (uint32_t)set);
             ex = -logf(u01f(w.x));
         }
     };
@@ -231,7 +232,7 @@ TL_D void tiny_realization(const TinyGroup<W>& g, const SimParams& p, TinyLane<W
                 const int from = (int)(step - w_from);
                 jc = tiny_select<W>(av, pac, g.from(w.z, from), g.from(w.w, from), true);
             }
-            k = channel ? poisson_channel(aj, tauf, g.lane, jc, step, r, (uint32_t)set, p.rk) : 0;
+            k = channel ? poisson_channel(aj, tauf, g.lane, jc, step, r, (uint32_t)set, rk) : 0;
             long long d = 0;
 #pragma unroll
             for (int j = 0; j < W; ++j) d += (long long)L.v(j) * (long long)g.from(k, j);
