@@ -895,24 +895,27 @@ TL_D int ssa_select(const Grp& g, const SimParams& p, const Lay& L, float part, 
     const int eb = emax - 24;
     const bool off = bits != 0u && e < eb;
     if (emax < 60 || emax > 250 || g.any(off)) return ssa_select_fp64(g, p, L, part, w_hi, w_lo, a0f);
-    unsigned long long F = 0ull;
-    if (bits) F = (unsigned long long)((bits & 0x7fffffu) | 0x800000u) << (e - eb);
-    // u = k2 2^-53 and, below, T = floor(u S)
-    const unsigned long long k2 = (((unsigned long long)(w_hi >> 6) << 26 | (w_lo >> 6)) << 1) | 1ull;
+    const uint32_t mant = bits ? (bits & 0x7fffffu) | 0x800000u : 0u;
+    const int up = e - eb;  // 0..24 where mant != 0
     const float unit = __uint_as_float((uint32_t)(eb - 23) << 23);  // value of the grid's lsb; eb >= 36
     if (p.M <= g.size()) {
-        // one channel a lane: the sums of the halves, and the cumulative sums
-        // of the top 27 bits, which place the target up to 33 units
-        const uint32_t hi = (uint32_t)(F >> 24), lo = (uint32_t)F & 0xffffffu;
+        // One channel a lane.  The total from the sums of the halves; the
+        // target and the cumulative sums from their top 27 bits: P is short of
+        // the true sum by less than 32 units (2^22 of the grid), T of the
+        // target by less than 4, so outside that window both place the target.
+        const uint32_t hi = mant ? mant >> (24 - up) : 0u, lo = mant ? mant << up & 0xffffffu : 0u;
         const unsigned long long S = ((unsigned long long)g.sum_uint(hi) << 24) + g.sum_uint(lo);
         a0f = round53(S) * unit;
-        const uint32_t T = (uint32_t)(__umul64hi(k2 << 11, S) >> 21);
-        const uint32_t P = g.incl_scan(hi << 3 | lo >> 21);
-        const bool some = F != 0ull;
-        if (g.any(some && T >= P && T - P < 33u)) return ssa_select_fp64(g, p, L, part, w_hi, w_lo, a0f);
-        const int first = g.first(some && T < P);
+        const int T = (int)__umulhi((w_hi & ~63u) | w_lo >> 26, (uint32_t)(S >> 22) << 1) >> 1;
+        const int P = (int)g.incl_scan(hi << 2 | lo >> 22);
+        const bool some = mant != 0u;
+        if (g.any(some && P - T > -32 && P - T < 4)) return ssa_select_fp64(g, p, L, part, w_hi, w_lo, a0f);
+        const int first = g.first(some && P > T);
         return first >= 0 ? first : g.last(some);
     }
+    const unsigned long long F = (unsigned long long)mant << (mant ? up : 0);
+    // u = k2 2^-53 and, below, T = floor(u S)
+    const unsigned long long k2 = (((unsigned long long)(w_hi >> 6) << 26 | (w_lo >> 6)) << 1) | 1ull;
     // inclusive scan; the last lane holds the total
     unsigned long long P = F;
 #pragma unroll
