@@ -94,7 +94,15 @@ TL_HD void round_keys(uint32_t k0, uint32_t k1, uint32_t* rk) {
 }
 
 // Uniform in (0,1): 23 random bits at odd multiples of 2^-24 (exact in FP32).
-TL_HD float u01f(uint32_t w) { return ((float)(w >> 9) + 0.5f) * 1.1920928955078125e-07f; }
+// On the device by placing the bits behind the point of [1, 2) and subtracting
+// 1 - 2^-24, both exact: no integer conversion.
+TL_HD float u01f(uint32_t w) {
+#ifdef __CUDA_ARCH__
+    return __uint_as_float((w >> 9) + 0x3f800000u) - 0.99999994f;
+#else
+    return ((float)(w >> 9) + 0.5f) * 1.1920928955078125e-07f;
+#endif
+}
 // Uniform in (0,1) with 52 random bits, exact in FP64.
 TL_HD double u01d(uint32_t hi, uint32_t lo) {
     const uint64_t k = ((uint64_t)(hi >> 6) << 26) | (uint64_t)(lo >> 6);
