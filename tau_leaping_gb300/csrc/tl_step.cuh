@@ -242,28 +242,39 @@ TL_D void set_species(const Lay& L, int i, long long x) {
     else set_species64(L, i, x);
 }
 
-// Propensities into a[] (sign = critical) and the lane's partial sums; thin
-// groups form the sums over all channels in order.
+// Channel j's propensity, and in the sign bit whether it is critical.
 template <class Grp, class Lay>
+TL_D float signed_prop(const SimParams& p, const Lay& L, const float* rate, int j) {
+    uint32_t o0, o1;
+    if (Grp::kWidth == 0 && p.chan8) {
+        const uint2 r = reinterpret_cast<const uint2*>(L.chan())[j];
+        o0 = r.x;
+        o1 = r.y;
+    } else {
+        const uint32_t r = L.chan()[j];
+        o0 = r & 0xffffu;
+        o1 = r >> 16;
+    }
+    const float f0 = at_byte(L.X(), o0), f1 = at_byte(L.X(), o1);
+    const float v = __ldg(rate + j) * fabsf(f0) * fabsf(f1);
+    const uint32_t cr = (__float_as_uint(f0) | __float_as_uint(f1)) & 0x80000000u;
+    return __uint_as_float(__float_as_uint(v) | cr);
+}
+
+// Propensities into a[] and the lane's partial sums; thin groups form the sums
+// over all channels in order.  Critical channels are stored negative, or with
+// ZERO as 0, which spares every net entry of the step bound a max: what reads
+// their propensities forms them again (select_critical, direct steps).
+template <bool ZERO, class Grp, class Lay>
 TL_D void fast_props(const Grp& g, const SimParams& p, const Lay& L, const float* rate, float& pa, float& pac) {
     float s = 0.f, sc = 0.f;
     constexpr int kUnroll = is_thin<Grp>::value ? 4 : 2;
 #pragma unroll kUnroll
     for (int j = g.rank(); j < p.M; j += g.size()) {
-        uint32_t o0, o1;
-        if (Grp::kWidth == 0 && p.chan8) {
-            const uint2 r = reinterpret_cast<const uint2*>(L.chan())[j];
-            o0 = r.x;
-            o1 = r.y;
-        } else {
-            const uint32_t r = L.chan()[j];
-            o0 = r & 0xffffu;
-            o1 = r >> 16;
-        }
-        const float f0 = at_byte(L.X(), o0), f1 = at_byte(L.X(), o1);
-        const float v = __ldg(rate + j) * fabsf(f0) * fabsf(f1);
-        const uint32_t cr = (__float_as_uint(f0) | __float_as_uint(f1)) & 0x80000000u;
-        L.a()[j] = __uint_as_float(__float_as_uint(v) | cr);
+        const float sv = signed_prop<Grp>(p, L, rate, j);
+        const float v = fabsf(sv);
+        const bool cr = is_crit(sv);
+        L.a()[j] = ZERO && cr ? 0.f : sv;
         if constexpr (!is_thin<Grp>::value && Grp::kWidth != 128) {
             s += v;
             sc += cr ? v : 0.f;
@@ -297,18 +308,49 @@ TL_D void fast_props(const Grp& g, const SimParams& p, const Lay& L, const float
     pac = sc;
 }
 
+// select_channel among the critical channels where a[] holds 0 for them: the
+// lane that owns the target forms its channels' propensities again.
+template <class Grp, class Lay>
+__device__ __noinline__ int select_critical(const Grp g, const SimParams& p, const Lay L, const float* rate, float pac,
+                                            double target) {
+    const double part = (double)pac, excl = g.excl_scan(part);
+    int owner = g.first(part > 0.0 && target < excl + part);
+    if (owner < 0) owner = g.last(part > 0.0);
+    int sel = -1;
+    if (g.rank() == owner) {
+        const float limit = __double2float_rd(target - excl);
+        float acc = 0.f;
+#pragma unroll 1
+        for (int j = g.rank(); j < p.M; j += g.size()) {
+            const float v = signed_prop<Grp>(p, L, rate, j);
+            if (!(v < 0.f)) continue;
+            acc -= v;
+            sel = j;
+            if (limit < acc) break;
+        }
+    }
+    return g.bcast(sel, owner < 0 ? 0 : owner);
+}
+
 // One entry's term of mu and sigma^2.
 TL_D void add_moments(float v, float aj, float& mu, float& s2) {
     const float t = v * aj;
     mu += t;
     s2 += v * t;
 }
-template <bool WIDE>
+// WIDE: models of 2^18 channels and more, beyond the 20-bit offsets.  ZERO:
+// critical channels are stored as 0, else negative and max(a, 0) drops them.
+template <bool WIDE, bool ZERO>
 TL_D void add_entry(const float* a, uint32_t e, float& mu, float& s2) {
-    // critical channels are stored negative: max(a, 0) drops them
-    // WIDE: models of 2^18 channels and more, beyond the 20-bit offsets
-    if constexpr (WIDE) add_moments(unpack_vf((int)e), fmaxf(a[e >> 3], 0.f), mu, s2);
-    else add_moments(__uint_as_float(e << 20), fmaxf(at_byte(a, e >> 12), 0.f), mu, s2);
+    float v, aj;
+    if constexpr (WIDE) {
+        v = unpack_vf((int)e);
+        aj = a[e >> 3];
+    } else {
+        v = __uint_as_float(e << 20);
+        aj = at_byte(a, e >> 12);
+    }
+    add_moments(v, ZERO ? aj : fmaxf(aj, 0.f), mu, s2);
 }
 
 // The CGP bound of a species (species_bound's values, without its branches:
@@ -322,7 +364,7 @@ TL_D float row_bound(const SimParams& p, float xi, int kind, float mu, float s2)
 }
 
 // The CGP step bound (CSRMatrixPacked.cu:311-358).
-template <bool kWide, class Grp, class Lay>
+template <bool kWide, bool ZERO, class Grp, class Lay>
 TL_D float fast_tau_rows(const Grp& g, const SimParams& p, const Lay& L) {
     float tmin = kInfF;
     if constexpr (Grp::kWidth == 0) {
@@ -334,7 +376,7 @@ TL_D float fast_tau_rows(const Grp& g, const SimParams& p, const Lay& L) {
                 const uint32_t* e = reinterpret_cast<const uint32_t*>(L.ent() + (rec.x & 0xfffffu));
                 const int n = 4 * (int)(rec.x >> 20);
                 float mu = 0.f, s2 = 0.f;
-                for (int q = g.lane; q < n; q += 32) add_entry<kWide>(L.a(), e[q], mu, s2);
+                for (int q = g.lane; q < n; q += 32) add_entry<kWide, ZERO>(L.a(), e[q], mu, s2);
 #pragma unroll
                 for (int o = 16; o; o >>= 1) {
                     mu += __shfl_xor_sync(0xffffffffu, mu, o);
@@ -355,10 +397,10 @@ TL_D float fast_tau_rows(const Grp& g, const SimParams& p, const Lay& L) {
 #pragma unroll 1
         for (int q = 0; q < n; ++q) {
             const uint4 w = e[q];
-            add_entry<kWide>(L.a(), w.x, mu, s2);
-            add_entry<kWide>(L.a(), w.y, mu, s2);
-            add_entry<kWide>(L.a(), w.z, mu, s2);
-            add_entry<kWide>(L.a(), w.w, mu, s2);
+            add_entry<kWide, ZERO>(L.a(), w.x, mu, s2);
+            add_entry<kWide, ZERO>(L.a(), w.y, mu, s2);
+            add_entry<kWide, ZERO>(L.a(), w.z, mu, s2);
+            add_entry<kWide, ZERO>(L.a(), w.w, mu, s2);
         }
         const float xi = fabsf(L.X()[rec.y & 0x0fffffffu]);
         tmin = fminf(tmin, row_bound(p, xi, (int)(rec.y >> 28), mu, s2));
@@ -366,11 +408,11 @@ TL_D float fast_tau_rows(const Grp& g, const SimParams& p, const Lay& L) {
     return g.minf(tmin);
 }
 
-template <class Grp, class Lay>
+template <bool ZERO, class Grp, class Lay>
 TL_D float fast_tau(const Grp& g, const SimParams& p, const Lay& L) {
     if constexpr (Grp::kWidth == 0)
-        if (p.ent_wide) return fast_tau_rows<true>(g, p, L);
-    return fast_tau_rows<false>(g, p, L);
+        if (p.ent_wide) return fast_tau_rows<true, ZERO>(g, p, L);
+    return fast_tau_rows<false, ZERO>(g, p, L);
 }
 
 // Calls f(byte offset of the species in an int array, stoichiometry) for channel j's net entries.
@@ -456,6 +498,16 @@ TL_D void fast_refresh(const Grp& g, const SimParams& p, const Lay& L) {
 #pragma unroll 1
     for (int i = g.rank(); i < p.N; i += g.size()) set_species(L, i, L.x()[i]);
     if (g.leader()) L.X()[p.x_one] = 1.f;
+}
+
+// After a rejected leap: D to zero, and where select_critical reads X, which
+// the queue lay over, X again.  Out of line: rejections are rare.
+template <bool ZERO, class Grp, class Lay>
+__device__ __noinline__ void undo_leap(const Grp g, const SimParams& p, const Lay L) {
+#pragma unroll 1
+    for (int i = g.rank(); i < p.N; i += g.size()) L.D()[i] = 0;
+    if constexpr (ZERO) fast_refresh(g, p, L);
+    g.sync();
 }
 
 // The firing counts of one leap into D (and k[] in scored runs), for groups
@@ -1180,7 +1232,7 @@ TL_D void direct_steps(const Grp& g, const SimParams& p, const Lay& L, int set, 
         st.ssa++;
         if (++q == p.ssa_block || (p.max_steps > 0 && (long long)(st.step - st.rej) >= p.max_steps)) return;
         float pac;
-        fast_props(g, p, L, rate, pa, pac);
+        fast_props<false>(g, p, L, rate, pa, pac);
         if (!g.any(pa > 0.f)) {
             st.done = true;
             return;
@@ -1194,7 +1246,12 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
     constexpr bool kThin = is_thin<Grp>::value;
     const float* rate = p.frates + (size_t)set * p.M;  // halved for 2S
     float pa, pac;
-    fast_props(g, p, L, rate, pa, pac);
+    // Scores read a critical channel's propensity, and teams form their sums
+    // from a[].  Warps and CTAs gain (500 realizations of the 64 x 1024 network
+    // 27.7 -> 27.15 ms, 250 species of the colloid 3.39 -> 3.34 ms), 16 lanes do
+    // not (81.9 -> 82.3 ms: two realizations share the warp that selects).
+    constexpr bool kZero = !SENS && !WIDE && (Grp::kWidth == 32 || Grp::kWidth == 0);
+    fast_props<kZero>(g, p, L, rate, pa, pac);
     float a0f;
     if constexpr (kThin) a0f = pa;
     else a0f = sum_group(g).sumf(pa);
@@ -1202,9 +1259,10 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
         st.done = true;  // nothing can fire: the state holds to t_final
         return;
     }
-    float tau1 = fast_tau(g, p, L);
+    float tau1 = fast_tau<kZero>(g, p, L);
 
     if (!WIDE && tau1 * a0f < p.ssa_factor) {
+        if constexpr (kZero) fast_props<false>(g, p, L, rate, pa, pac);
         direct_steps<Grp, Lay, SENS>(g, p, L, set, r, pa, st);
         return;
     }
@@ -1251,7 +1309,9 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
             } else {
                 const auto sg = sum_group(g);
                 const double a0c = sg.sumd((double)pac);
-                jc = select_channel<std::decay_t<decltype(sum_group(g))>, double>(sg, p, L.a(), pac, u01d(w.z, w.w) * a0c, 1);
+                const double target = u01d(w.z, w.w) * a0c;
+                if constexpr (kZero) jc = select_critical(g, p, L, rate, pac, target);
+                else jc = select_channel<std::decay_t<decltype(sum_group(g))>, double>(sg, p, L.a(), pac, target, 1);
             }
         }
         bool over = false, bad;
@@ -1268,11 +1328,7 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
                 bad = fast_check(g, p, L, over);
                 if (!bad) fast_commit(g, p, L);
             }
-            if (bad) {
-#pragma unroll 1
-                for (int i = g.rank(); i < p.N; i += g.size()) L.D()[i] = 0;
-                g.sync();
-            }
+            if (bad) undo_leap<kZero>(g, p, L);
         }
         if (over) {
             if (g.leader()) atomicOr((unsigned*)(p.ctr + 5), kErrOverflow);

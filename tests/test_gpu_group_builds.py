@@ -90,6 +90,34 @@ def test_direct_method_steps_are_bit_identical(kind):
         assert r.ssa_steps > 0
 
 
+@pytest.mark.parametrize("kind", ["lanes8", "warp", "cta"])
+@pytest.mark.parametrize("pairs", [1, 16, 37, 300])
+def test_leaps_that_fire_a_critical_channel(kind, pairs):
+    """Pairs A <-> B of 10^5 molecules, which set the leap, and species of
+    about five molecules each, which are born and decay: one critical channel
+    fires in most leaps, from any lane."""
+    cols = []
+    for q in range(pairs):
+        a, b, s = 3 * q, 3 * q + 1, 3 * q + 2
+        cols += [[(a, -1), (b, 1)], [(a, 1), (b, -1)], [(s, 1)], [(s, -1)]]
+    x0 = np.tile([100000, 100000, 5], pairs)
+    rate = np.tile([1.0, 1.0, 1.0 + 200.0 / pairs, 40.0 / pairs], pairs)
+    cp = np.cumsum([0] + [len(c) for c in cols])
+    m = Model.from_arrays(x0, rate, cp, [i for c in cols for i, _ in c], [v for c in cols for _, v in c])
+    r = assert_same(m, _ffi.FLAG_COMPAT_CRIT, variant=KINDS[kind], n=40, t_final=0.2)
+    assert r is not None and r.leaps > 0
+
+
+@pytest.mark.parametrize("kind", ["lanes8", "warp", "cta"])
+def test_rejected_leaps_that_fire_a_critical_channel(kind):
+    """eps = 3 on few molecules: a retry selects among the critical channels
+    of the state before the rejected leap."""
+    for N, M in ((16, 32), (20, 70)):
+        m, general = network(N, M, N + M, x_max=60)
+        r = assert_same(m, general, variant=KINDS[kind], n=1000, t_final=0.5, eps=3.0)
+        assert r is not None and r.rejections > 0
+
+
 @pytest.mark.parametrize("n", [3, 1500, 9000, 21000])
 def test_thread_groups_of_every_ensemble_size(n):
     """Lanes per realization and realizations per warp follow the ensemble."""
