@@ -390,31 +390,15 @@ TL_D int poisson_reference(float mu, Rng& rng) {
 // >= 10, or the reference's sampler is asked for).  Warp and CTA groups run
 // it from one call site after the unrolled channel loop (pass_fire), so one
 // copy of it sits in the loop.
-// REFS: the reference's sampler can be asked for (compatibility builds).
-template <bool REFS>
-TL_D int poisson_rare_inline(float mu, float q, uint32_t j, uint32_t step, uint32_t r, uint32_t set,
-                             const uint32_t* rk, int refs) {
+// Inline: a call would save the registers live across it, and those saves were
+// most of the warp kernel's spills.  Measured on GB300 against the call: toy
+// network +3 %, chain +4 %, colloid +1 %, batch +2 %.
+TL_D int poisson_rare(float mu, float q, uint32_t j, uint32_t step, uint32_t r, uint32_t set, const uint32_t* rk,
+                      int refs) {
     ChanRng rng;
     rng.init(j, step, r, set, rk);
-    if (REFS && refs) return poisson_reference(mu, rng);
+    if (refs) return poisson_reference(mu, rng);
     return poisson_tail2(mu, q, rng);
-}
-// Inlined there by default (TL_RARE_INLINE 1): a call would save the
-// registers live across it, and those saves were most of the warp kernel's
-// spills.  Measured on GB300 against the out-of-line call: toy network +3 %,
-// chain +4 %, colloid +1 %, batch +2 %.
-#ifndef TL_RARE_INLINE
-#define TL_RARE_INLINE 1
-#endif
-#if TL_RARE_INLINE
-#define TL_RARE_ATTR __forceinline__
-#else
-#define TL_RARE_ATTR __noinline__
-#endif
-template <bool REFS>
-static __device__ TL_RARE_ATTR int poisson_rare(float mu, float q, uint32_t j, uint32_t step, uint32_t r,
-                                                uint32_t set, const uint32_t* rk, int refs) {
-    return poisson_rare_inline<REFS>(mu, q, j, step, r, set, rk, refs);
 }
 
 // ---------------------------------------------------------------------------
@@ -862,12 +846,6 @@ struct RState {
 };
 
 TL_HD bool flag(unsigned f, unsigned b) { return (f & b) != 0; }
-// A reference-compatibility switch: compiled out of the kernels built
-// without them (COMPAT = false), read at run time otherwise.
-template <bool COMPAT>
-TL_D bool cflag(unsigned f, unsigned b) {
-    return COMPAT && (f & b) != 0;
-}
 
 // Grid time k of rate set `set`: T*k/n_int (T itself for k = n_int), from
 // the table the host fills with exactly that FP64 expression, so that a leap
@@ -882,10 +860,10 @@ TL_D TimeT grid_time(const SimParams& p, int set, int k) {
 // ---------------------------------------------------------------------------
 
 // Propensities of all channels into a[] (sign = critical); lane partial sums.
-template <class Grp, class Pop, bool COMPAT = true>
+template <class Grp, class Pop>
 TL_D void pass_props(const Grp& g, const SimParams& p, const MView& mv, const float* rate,
                      const Pop* x, float* a, float& pa, float& pac) {
-    const bool cc = cflag<COMPAT>(p.flags, TL_FLAG_COMPAT_CRIT);
+    const bool cc = flag(p.flags, TL_FLAG_COMPAT_CRIT);
     float s = 0.f, sc = 0.f;
     for (int j = g.rank(); j < p.M; j += g.size()) {
         float aj;
@@ -901,10 +879,10 @@ TL_D void pass_props(const Grp& g, const SimParams& p, const MView& mv, const fl
 }
 
 // CGP bound of species i from its CSR row; optional moments out.
-template <class Pop, bool COMPAT = true>
+template <class Pop>
 TL_D float species_bound(const SimParams& p, const MView& mv, const Pop* x, const float* a, int i,
                          float mu, float s2) {
-    const bool cg = cflag<COMPAT>(p.flags, TL_FLAG_COMPAT_G);
+    const bool cg = flag(p.flags, TL_FLAG_COMPAT_G);
     const float xi = popf(x[i]);
     float gi;
     if (cg) {
@@ -920,10 +898,10 @@ TL_D float species_bound(const SimParams& p, const MView& mv, const Pop* x, cons
     return fminf(b1, b2);
 }
 
-template <bool OUT, class Grp, class Pop, bool COMPAT = true>
+template <bool OUT, class Grp, class Pop>
 TL_D float pass_tau(const Grp& g, const SimParams& p, const MView& mv, const Pop* x, const float* a,
                     float* mu_out, float* s2_out) {
-    const bool all_rows = cflag<COMPAT>(p.flags, TL_FLAG_COMPAT_STOICH);
+    const bool all_rows = flag(p.flags, TL_FLAG_COMPAT_STOICH);
     float tmin = kInfF;
     bool done = false;
     if constexpr (Grp::kWidth == 0) {
@@ -953,7 +931,7 @@ TL_D float pass_tau(const Grp& g, const SimParams& p, const MView& mv, const Pop
                     mu_out[i] = mu;
                     s2_out[i] = s2;
                 }
-                if (all_rows || mv.gkind[i] != 0) tmin = fminf(tmin, species_bound<Pop, COMPAT>(p, mv, x, a, i, mu, s2));
+                if (all_rows || mv.gkind[i] != 0) tmin = fminf(tmin, species_bound<Pop>(p, mv, x, a, i, mu, s2));
             }
         }
       }
@@ -978,7 +956,7 @@ TL_D float pass_tau(const Grp& g, const SimParams& p, const MView& mv, const Pop
                 mu_out[i] = mu;
                 s2_out[i] = s2;
             }
-            if (all_rows || mv.gkind[i] != 0) tmin = fminf(tmin, species_bound<Pop, COMPAT>(p, mv, x, a, i, mu, s2));
+            if (all_rows || mv.gkind[i] != 0) tmin = fminf(tmin, species_bound<Pop>(p, mv, x, a, i, mu, s2));
         }
     }
     return g.minf(tmin);
@@ -1104,10 +1082,10 @@ TL_D void record_point(const Grp& g, const SimParams& p, const Pop* x, Pop* samp
 // Poisson firing counts of one leap (model.cu:458-549), written over a[] as
 // ints.  A thread takes four consecutive channels at a time so that they
 // share one Philox block for their first uniforms.
-template <class Grp, bool COMPAT = true>
+template <class Grp>
 TL_D void pass_fire(const Grp& g, const SimParams& p, const float* a, int* kk, float tauf, int jc, uint32_t step,
                     uint32_t r, uint32_t set) {
-    const bool refs = cflag<COMPAT>(p.flags, TL_FLAG_COMPAT_POISSON);
+    const bool refs = flag(p.flags, TL_FLAG_COMPAT_POISSON);
     const bool vec = (reinterpret_cast<uintptr_t>(a) & 15) == 0 && (reinterpret_cast<uintptr_t>(kk) & 15) == 0;
     for (int g4 = g.rank(); 4 * g4 < p.M; g4 += g.size()) {
         const int j0 = 4 * g4;
@@ -1172,7 +1150,7 @@ TL_D void pass_fire(const Grp& g, const SimParams& p, const float* a, int* kk, f
                     }
                     if (more) {
                         if constexpr (Grp::kWidth == 1)
-                            k = poisson_rare_inline<COMPAT>(mu, q, (uint32_t)(j0 + e), step, r, set, p.rk,
+                            k = poisson_rare(mu, q, (uint32_t)(j0 + e), step, r, set, p.rk,
                                                             refs ? 1 : 0);
                         else
                             rare |= 1u << e;
@@ -1206,8 +1184,7 @@ TL_D void pass_fire(const Grp& g, const SimParams& p, const float* a, int* kk, f
             const float mu = (e == 0 ? av[0] : e == 1 ? av[1] : e == 2 ? av[2] : av[3]) * tauf;
             const float q = refs ? 0.f : ((float)word_of(gw, e) + 0.5f) * 2.3283064365386963e-10f;
             const uint32_t j = (uint32_t)(j0 + e);
-            // out of line unless TL_RARE_INLINE
-            const int k = poisson_rare<COMPAT>(mu, q, j, step, r, set, p.rk, refs ? 1 : 0);
+            const int k = poisson_rare(mu, q, j, step, r, set, p.rk, refs ? 1 : 0);
             kv[0] = e == 0 ? k : kv[0];
             kv[1] = e == 1 ? k : kv[1];
             kv[2] = e == 2 ? k : kv[2];
@@ -1227,7 +1204,7 @@ TL_D void pass_fire(const Grp& g, const SimParams& p, const float* a, int* kk, f
 // One step of one realization: a tau-leap (with rejection + halving) or a
 // block of direct-method steps (model.cu:301-413).
 // ---------------------------------------------------------------------------
-template <class Grp, class Pop, class TimeT, bool SENS, bool COMPAT = true>
+template <class Grp, class Pop, class TimeT, bool SENS>
 TL_D void do_step(const Grp& g, const SimParams& p, const MView& mv, Slot<Pop>& s, int set, uint32_t r,
                   Pop* samp, float* score, RState<TimeT>& st) {
     const float* rate = p.rates + (size_t)set * p.M;
@@ -1235,7 +1212,7 @@ TL_D void do_step(const Grp& g, const SimParams& p, const MView& mv, Slot<Pop>& 
     const unsigned f = p.flags;
 
     float pa, pac;
-    pass_props<Grp, Pop, COMPAT>(g, p, mv, rate, s.x, s.a, pa, pac);
+    pass_props<Grp, Pop>(g, p, mv, rate, s.x, s.a, pa, pac);
     g.sync();
     const float a0f = g.sumf(pa);  // FP32: only the branch test and tau2 use it
     if (!(a0f > 0.f)) {
@@ -1245,13 +1222,13 @@ TL_D void do_step(const Grp& g, const SimParams& p, const MView& mv, Slot<Pop>& 
         st.done = 1;
         return;
     }
-    float tau1 = pass_tau<false, Grp, Pop, COMPAT>(g, p, mv, s.x, s.a, nullptr, nullptr);
+    float tau1 = pass_tau<false, Grp, Pop>(g, p, mv, s.x, s.a, nullptr, nullptr);
 
     if (tau1 * a0f < p.ssa_factor) {
         // ---- direct-method block (CGP 2006 step 2; model.cu:334-345) ----
         for (int q = 0; q < p.ssa_block; ++q) {
             if (q > 0) {
-                pass_props<Grp, Pop, COMPAT>(g, p, mv, rate, s.x, s.a, pa, pac);
+                pass_props<Grp, Pop>(g, p, mv, rate, s.x, s.a, pa, pac);
                 g.sync();
             }
             // total for the cumulative search: FP64 over the lane partials
@@ -1272,7 +1249,7 @@ TL_D void do_step(const Grp& g, const SimParams& p, const MView& mv, Slot<Pop>& 
             const int j = select_channel<Grp, TimeT>(g, p, s.a, pa, target, 0);
             // the waiting time in FP32 (FP64 keeps only the time sum)
             const float ex = -logf(u01f(w.x));
-            const TimeT dt = (TimeT)(cflag<COMPAT>(f, TL_FLAG_COMPAT_TAU2) ? ex / fabsf(s.a[j]) : ex / (float)a0);
+            const TimeT dt = (TimeT)(flag(f, TL_FLAG_COMPAT_TAU2) ? ex / fabsf(s.a[j]) : ex / (float)a0);
             while (st.kpt <= p.n_int && st.t + dt >= grid_time<TimeT>(p, set, st.kpt))
                 record_point<Grp, Pop>(g, p, s.x, samp, st.kpt++);
             if (st.kpt > p.n_int) {
@@ -1296,7 +1273,7 @@ TL_D void do_step(const Grp& g, const SimParams& p, const MView& mv, Slot<Pop>& 
                 }
             }
             g.sync();
-            if (!cflag<COMPAT>(f, TL_FLAG_COMPAT_SSA) && j >= 0) {
+            if (!flag(f, TL_FLAG_COMPAT_SSA) && j >= 0) {
                 const int e = mv.cp[j + 1];
                 for (int q2 = mv.cp[j] + g.rank(); q2 < e; q2 += g.size()) {
                     const int pk = mv.rv[q2];
@@ -1325,7 +1302,7 @@ TL_D void do_step(const Grp& g, const SimParams& p, const MView& mv, Slot<Pop>& 
         int jc = -1;
         float tau2 = kInfF;
         if (a0cf > 0.f) {
-            if (cflag<COMPAT>(f, TL_FLAG_COMPAT_TAU2)) {
+            if (flag(f, TL_FLAG_COMPAT_TAU2)) {
                 const TimeT a0c = (TimeT)g.sumd((double)pac);
                 jc = select_channel<Grp, TimeT>(g, p, s.a, pac, (TimeT)u01d(w.z, w.w) * a0c, 1);
                 tau2 = -logf(u01f(w.x)) / fabsf(s.a[jc]);
@@ -1347,7 +1324,7 @@ TL_D void do_step(const Grp& g, const SimParams& p, const MView& mv, Slot<Pop>& 
             jc = select_channel<Grp, TimeT>(g, p, s.a, pac, (TimeT)u01d(w.z, w.w) * a0c, 1);
         }
         if (!fire) jc = -1;
-        pass_fire<Grp, COMPAT>(g, p, s.a, s.k, tauf, jc, st.step, r, (uint32_t)set);
+        pass_fire<Grp>(g, p, s.a, s.k, tauf, jc, st.step, r, (uint32_t)set);
         g.sync();
         bool ovf = false;
         const bool bad = pass_update<Grp, Pop>(g, p, mv, s.x, s.k, s.xn, ovf);
@@ -1362,7 +1339,7 @@ TL_D void do_step(const Grp& g, const SimParams& p, const MView& mv, Slot<Pop>& 
         st.step++;
         tau1 *= 0.5f;
         g.sync();
-        pass_props<Grp, Pop, COMPAT>(g, p, mv, rate, s.x, s.a, pa, pac);
+        pass_props<Grp, Pop>(g, p, mv, rate, s.x, s.a, pa, pac);
         g.sync();
         if (attempt + 1 > p.max_halv) {
             if (g.leader()) atomicOr((unsigned*)(p.ctr + 5), kErrHalving);

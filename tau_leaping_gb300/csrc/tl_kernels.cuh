@@ -154,23 +154,23 @@ struct GroupOf<0> {
 // One realization from x0 to t_final (the body of the persistent loop).
 // The realization's step counts go straight to the run's counters (one
 // atomic each per realization), so no totals stay live across the loop.
-template <class Grp, class Pop, bool SENS, bool COMPAT = true>
+template <class Grp, class Pop>
 TL_D void run_realization(const Grp& g, const SimParams& p, const MView& mv, Slot<Pop>& s, long long w) {
     const int P = p.n_int + 1;
     const int set = (int)(w / p.R);
     const uint32_t r = (uint32_t)(p.r_off + w - (long long)set * p.R);
     Pop* samp = reinterpret_cast<Pop*>(p.samples) + (size_t)w * P * p.K;
-    float* score = (SENS && p.scores) ? p.scores + (size_t)w * p.M : nullptr;
+    float* score = p.scores ? p.scores + (size_t)w * p.M : nullptr;
     const Pop* x0 = reinterpret_cast<const Pop*>(p.x0);
     for (int i = g.rank(); i < p.N; i += g.size()) s.x[i] = x0[i];
-    if (SENS && score)
+    if (score)
         for (int j = g.rank(); j < p.M; j += g.size()) score[j] = 0.f;
     g.sync();
     RState<double> st{0.0, 1, 0u, 0, 0, 0u};
     record_point<Grp, Pop>(g, p, s.x, samp, 0);
     bool trunc = false;
     while (!st.done) {
-        do_step<Grp, Pop, double, SENS, COMPAT>(g, p, mv, s, set, r, samp, score, st);
+        do_step<Grp, Pop, double, true>(g, p, mv, s, set, r, samp, score, st);
         if (!st.done && p.max_steps > 0 && st.nsteps >= p.max_steps) {
             while (st.kpt <= p.n_int) record_point<Grp, Pop>(g, p, s.x, samp, st.kpt++);
             st.done = 1;
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(KIND == 0 ? 1024 : 256, KIND == 0 ? 1 : KIND =
         if (g.leader()) w = (long long)atomicAdd(p.ctr + 0, 1ull);
         w = g.bcast(w, 0);
         if (w >= total) break;
-        run_realization<Grp, Pop, true, true>(g, p, mv, s, w);
+        run_realization<Grp, Pop>(g, p, mv, s, w);
     }
 }
 
@@ -240,12 +240,12 @@ struct FastGroupOf {
     static TL_D int index(const SimParams&) { return GroupOf<KIND>::index(); }
     static TL_D bool idle(const SimParams&) { return false; }
 };
-template <int W>
-struct ThinGroupOf {
-    using type = GThin<W>;
-    static TL_D type make(double*) { return type::make(); }
+template <>
+struct FastGroupOf<kKindThin1> {
+    using type = GThin;
+    static TL_D GThin make(double*) { return GThin{}; }
     static TL_D int index(const SimParams& p) {
-        return (int)(threadIdx.x >> 5) * (p.lanes / W) + (int)(threadIdx.x & 31) / W;
+        return (int)(threadIdx.x >> 5) * p.lanes + (int)(threadIdx.x & 31);
     }
     static TL_D bool idle(const SimParams& p) { return (int)(threadIdx.x & 31) >= p.lanes; }
 };
@@ -258,8 +258,6 @@ struct FastGroupOf<kKindTeam> {
     static TL_D int index(const SimParams&) { return 0; }
     static TL_D bool idle(const SimParams&) { return false; }
 };
-template <>
-struct FastGroupOf<kKindThin1> : ThinGroupOf<1> {};
 
 template <int KIND, class Pop, bool SENS, bool STAGED, bool GSLOT = false>
 __global__ void __launch_bounds__(KIND == 0 ? 1024 : KIND == kKindTeam ? 128 : 256,
@@ -377,7 +375,7 @@ __global__ void __launch_bounds__(256, TL_BATCH_MINB) k_batch(BatchParams bp) {
                 if (wi < total) {
                     if constexpr (W == 1) {
                         const Lay L{p, my_slot + (uint32_t)(lane * p.slot_bytes), (uint32_t)soff, nullptr, nullptr, p.rk};
-                        fast_realization<GThin<1>, Lay, SENS>(GThin<1>::make(), p, L, wi);
+                        fast_realization<GThin, Lay, SENS>(GThin{}, p, L, wi);
                     } else {
                         const auto g = TinyGroup<W>::make();
                         TinyLane<W, Pop> L;
@@ -391,12 +389,12 @@ __global__ void __launch_bounds__(256, TL_BATCH_MINB) k_batch(BatchParams bp) {
             if (!bp.items[it].lane_mode) {
                 const GWarp g{lane};
                 Slot<Pop> s = carve_slot<Pop>(wslot, p);
-                run_realization<GWarp, Pop, true, true>(g, p, mv, s, local);
+                run_realization<GWarp, Pop>(g, p, mv, s, local);
             } else {
                 const long long wi = local * 32 + lane;
                 if (wi < total) {
                     Slot<Pop> s = carve_slot<Pop>(wslot + (size_t)lane * p.slot_bytes, p);
-                    run_realization<G1, Pop, true, true>(G1{}, p, mv, s, wi);
+                    run_realization<G1, Pop>(G1{}, p, mv, s, wi);
                 }
             }
         }

@@ -37,41 +37,20 @@
 
 namespace tl {
 
-// W lanes of a warp for one realization of a small model (up to 16 species
-// and channels), W = 1, 2, 4, 8.  Every sum runs over the channels in order,
-// as one thread would form it, so the results do not depend on W: a thread
-// group's trajectories, with the channels' draws side by side.
-template <int W>
+// One thread for one realization of a model that the registers of a few lanes
+// do not hold (tl_tiny.cuh).  Every sum runs over the channels in order, as
+// there, so a realization's trajectory is the same on either.
 struct GThin {
-    static constexpr int kWidth = W;
-    static constexpr bool kThin = true;
-    int lane;
-    int base;
-    unsigned mask;
-    static TL_D GThin make() {
-        GThin g;
-        const int l = (int)(threadIdx.x & 31);
-        g.lane = l & (W - 1);
-        g.base = l & ~(W - 1);
-        g.mask = ((1u << W) - 1u) << g.base;
-        return g;
-    }
-    TL_D int rank() const { return W == 1 ? 0 : lane; }
-    TL_D int size() const { return W; }
-    TL_D void sync() const {
-        if (W > 1) __syncwarp(mask);
-    }
-    TL_D bool leader() const { return W == 1 || lane == 0; }
-    TL_D float minf(float v) const {
-#pragma unroll
-        for (int o = W / 2; o; o >>= 1) v = fminf(v, __shfl_xor_sync(mask, v, o, W));
-        return v;
-    }
-    TL_D bool any(bool p) const { return W == 1 ? p : (__ballot_sync(mask, p) & mask) != 0u; }
+    static constexpr int kWidth = 1;
+    TL_D int rank() const { return 0; }
+    TL_D int size() const { return 1; }
+    TL_D void sync() const {}
+    TL_D bool leader() const { return true; }
+    TL_D float minf(float v) const { return v; }
+    TL_D bool any(bool p) const { return p; }
     template <class T>
-    TL_D T bcast(T v, int src) const {
-        if (W == 1) return v;
-        return __shfl_sync(mask, v, src, W);
+    TL_D T bcast(T v, int) const {
+        return v;
     }
 };
 
@@ -79,8 +58,8 @@ template <class G>
 struct is_thin {
     static constexpr bool value = false;
 };
-template <int W>
-struct is_thin<GThin<W>> {
+template <>
+struct is_thin<GThin> {
     static constexpr bool value = true;
 };
 
@@ -741,13 +720,12 @@ TL_D int poisson_channel(float aj, float tauf, int j, int jc, uint32_t step, uin
     return k;
 }
 
-template <int W, class Lay, bool SENS>
-TL_D void thin_fire(const GThin<W>& g, const SimParams& p, const Lay& L, float tauf, int jc, uint32_t step,
-                    uint32_t r, uint32_t set) {
-    for (int j = g.rank(); j < p.M; j += W) {
+template <class Lay, bool SENS>
+TL_D void thin_fire(const SimParams& p, const Lay& L, float tauf, int jc, uint32_t step, uint32_t r, uint32_t set) {
+    for (int j = 0; j < p.M; ++j) {
         const int k = poisson_channel(L.a()[j], tauf, j, jc, step, r, set, L.rk);
         if constexpr (SENS) L.k()[j] = k;
-        if (k) fire_channel<GThin<W>>(L, j, k);
+        if (k) fire_channel<GThin>(L, j, k);
     }
 }
 
@@ -792,29 +770,26 @@ TL_D void fast_commit(const Grp& g, const SimParams& p, const Lay& L) {
     if (g.leader()) L.X()[p.x_one] = 1.f;
 }
 
-// The same for thin groups, whose lanes each take a species.
-template <int W, class Lay>
-TL_D bool thin_commit(const GThin<W>& g, const SimParams& p, const Lay& L, bool& over) {
+// The same for one thread.
+template <class Lay>
+TL_D bool thin_commit(const SimParams& p, const Lay& L, bool& over) {
     using Pop = typename Lay::Pop;
-    bool bad = false, of = false;
-    for (int i = g.rank(); i < p.N; i += W) {
+    bool bad = false;
+    over = false;
+    for (int i = 0; i < p.N; ++i) {
         const int d = L.D()[i];
         const bool b = add_pop(L.x()[i], d) < 0;
         bad |= b;
-        of |= sizeof(Pop) == 4 && b && d > 0;
+        over |= sizeof(Pop) == 4 && b && d > 0;
     }
-    over = false;
-    if (g.any(bad)) {
-        if (sizeof(Pop) == 4) over = g.any(of);
-        return true;
-    }
-    for (int i = g.rank(); i < p.N; i += W) {
+    if (bad) return true;
+    for (int i = 0; i < p.N; ++i) {
         const Pop nx = add_pop(L.x()[i], L.D()[i]);
         L.x()[i] = nx;
         L.D()[i] = 0;
         set_species(L, i, nx);
     }
-    if (g.leader()) L.X()[p.x_one] = 1.f;
+    L.X()[p.x_one] = 1.f;
     return false;
 }
 
@@ -875,9 +850,8 @@ TL_D bool wide_leap(const Grp& g, const SimParams& p, const Lay& L, float tauf, 
 // bits.  FP32 decides every channel whose running sum is further from the
 // target than the products' rounding (2^-23 a0, margin 4e-7 a0); the FP64
 // target decides the others.
-template <int W, class Lay>
-TL_D int thin_select(const GThin<W>& g, const SimParams& p, const Lay& L, float part, uint32_t w_hi,
-                     uint32_t w_lo) {
+template <class Lay>
+TL_D int thin_select(const SimParams& p, const Lay& L, float part, uint32_t w_hi, uint32_t w_lo) {
     const float t = ((float)(w_hi >> 6) * 1.4901161193847656e-08f) * part;  // 2^-26
     const float m = 4e-7f * part, above = t + m, below = t - m;
     float acc = 0.f;
@@ -1182,7 +1156,7 @@ TL_D void direct_steps(const Grp& g, const SimParams& p, const Lay& L, int set, 
         float a0;  // total for the waiting time
         if constexpr (kThin) {
             a0 = pa;
-            j = thin_select(g, p, L, pa, w_hi, w_lo);
+            j = thin_select(p, L, pa, w_hi, w_lo);
         } else if constexpr (Grp::kWidth == 0) {
             const double total = g.sumd((double)pa);
             a0 = (float)total;
@@ -1214,7 +1188,7 @@ TL_D void direct_steps(const Grp& g, const SimParams& p, const Lay& L, int set, 
                 c0 = (int)L.cp()[j];
                 n = (int)L.cp()[j + 1] - c0;
             }
-            constexpr int kBy = Grp::kWidth == 1 || Grp::kWidth == 2 ? Grp::kWidth : 4;
+            constexpr int kBy = Grp::kWidth == 1 || Grp::kWidth == 2 ? Grp::kWidth : 4;  // lanes
             if (g.rank() < kBy)
 #pragma unroll 1
                 for (int e = 4 * c0 + g.rank(); e < 4 * (c0 + n); e += kBy) {
@@ -1249,7 +1223,7 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
     // Scores read a critical channel's propensity, and teams form their sums
     // from a[].  Warps and CTAs gain (500 realizations of the 64 x 1024 network
     // 27.7 -> 27.15 ms, 250 species of the colloid 3.39 -> 3.34 ms), 16 lanes do
-    // not (81.9 -> 82.3 ms: two realizations share the warp that selects).
+    // not (80.5 -> 83.4 ms: two realizations share the warp that selects).
     constexpr bool kZero = !SENS && !WIDE && (Grp::kWidth == 32 || Grp::kWidth == 0);
     fast_props<kZero>(g, p, L, rate, pa, pac);
     float a0f;
@@ -1319,9 +1293,9 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
             bad = wide_leap<Grp, Lay, SENS>(g, p, L, tauf, jc, st.step, r, (uint32_t)set, over);
         } else {
             if constexpr (kThin) {
-                thin_fire<Grp::kWidth, Lay, SENS>(g, p, L, tauf, jc, st.step, r, (uint32_t)set);
+                thin_fire<Lay, SENS>(p, L, tauf, jc, st.step, r, (uint32_t)set);
                 g.sync();
-                bad = thin_commit(g, p, L, over);
+                bad = thin_commit(p, L, over);
             } else {
                 fast_fire<Grp, Lay, SENS>(g, p, L, tauf, jc, st.step, r, (uint32_t)set);
                 g.sync();
