@@ -442,12 +442,37 @@ static void thin_plan(int size, long long total, int nsm, int& thin, int& lanes)
 
 // Four-warp teams for a warp-group ensemble of up to eight realizations an SM:
 // enough channels for 128 threads, and a chain of steps that sets the time.
-// Measured on GB300, toy network (64 x 1024) to t = 0.002, ms, one warp a
+// Measured on GB300, toy network (128 x 256) to t = 0.002, ms, one warp a
 // realization -> a team: 10.9 -> 6.1 at 152 realizations, 10.9 -> 8.5 at 1216;
 // above eight realizations an SM the warps still run in one wave and a team no
 // longer does.
 static bool team_pays(const tl_model* m, long long total, int nsm) {
     return m->h.M >= 128 && total <= 8LL * nsm;
+}
+
+// Threads per CTA of a warp or sub-warp ensemble that runs in one wave.  The SM
+// with the most warps ends last, and CTAs of eight warps share out unevenly:
+// 500 of them put 32 warps on 44 of 152 SMs and 24 on the others.  Of 8 to 4
+// warps a CTA (an SM has four schedulers, and each CTA stages the tables) the
+// largest with the fewest warps on the fullest SM.  Measured on GB300, kernel
+// ms, 256 threads -> this rule: toy network (128 x 256) to t = 0.002, 1500
+// realizations 15.97 -> 14.88 (192), 2600 20.06 -> 17.77 (192), 3300 the same
+// (256), 4000 25.51 -> 23.31 (224); 12 x 20 network in direct-method steps, 4000
+// 1.270 -> 1.165; 45 x 83 network 13.91 -> 12.75.  Two or three warps a CTA
+// saved another warp an SM and were 1-3 % slower; with several waves the sizes
+// differ by +-2 % either way, and 256 stays.
+static int even_block(long long total, int groups_per_warp, int nsm, int most_warps) {
+    const long long warps = (total + groups_per_warp - 1) / groups_per_warp;
+    int best = most_warps;
+    long long most = 0;
+    for (int w = most_warps; w >= 4; --w) {
+        const long long ctas = (warps + w - 1) / w, full = (ctas + nsm - 1) / nsm * w;
+        if (w == most_warps || full < most) {
+            best = w;
+            most = full;
+        }
+    }
+    return 32 * best;
 }
 
 static tl_status make_plan(const tl_model* m, int variant, int block_req, int mode, bool sens, bool compat_stoich,
@@ -583,6 +608,13 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
     }
     const long long need = (total + groups_per_block - 1) / groups_per_block;
     pl.grid = (int)std::min<long long>((long long)nsm * bps, std::max<long long>(need, 1));
+    if (pl.kind >= 2 && pl.kind <= 32 && !pl.team && block_req <= 0 && need <= (long long)nsm * bps) {
+        const int block = even_block(total, 32 / pl.kind, nsm, pl.block / 32);
+        Plan q;
+        if (block < pl.block && make_plan(m, variant, block, mode, sens, compat_stoich, no_stage, total, q) == TL_OK &&
+            q.block == block && q.mode == pl.mode && (q.stage > 0) == staged && (long long)q.grid * (block / q.kind) >= total)
+            pl = q;
+    }
     return TL_OK;
 }
 

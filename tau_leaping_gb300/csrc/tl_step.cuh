@@ -1221,7 +1221,7 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
     const float* rate = p.frates + (size_t)set * p.M;  // halved for 2S
     float pa, pac;
     // Scores read a critical channel's propensity, and teams form their sums
-    // from a[].  Warps and CTAs gain (500 realizations of the 64 x 1024 network
+    // from a[].  Warps and CTAs gain (4000 realizations of the toy network
     // 27.7 -> 27.15 ms, 250 species of the colloid 3.39 -> 3.34 ms), 16 lanes do
     // not (80.5 -> 83.4 ms: two realizations share the warp that selects).
     constexpr bool kZero = !SENS && !WIDE && (Grp::kWidth == 32 || Grp::kWidth == 0);

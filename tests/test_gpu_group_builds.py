@@ -125,6 +125,18 @@ def test_thread_groups_of_every_ensemble_size(n):
     assert_same(m, general, variant=_ffi.VARIANT_THREAD, n=n, t_final=0.02)
 
 
+@pytest.mark.parametrize("kind", ["lanes16", "warp"])
+@pytest.mark.parametrize("n", [31, 1217, 2600, 4001, 4864, 4865])
+def test_ensembles_of_one_wave_on_even_ctas(kind, n):
+    """Smaller CTAs where they share an ensemble out more evenly: the same
+    realizations as on CTAs of 256 threads."""
+    m, _ = network(12, 20, 5)
+    kw = dict(t_final=0.01, n=n, seed=3, keep_samples=True, variant=KINDS[kind], max_steps=100, allow_truncation=True)
+    a, b = m.simulate(**kw), m.simulate(block_threads=256, **kw)
+    assert np.array_equal(a.samples, b.samples)
+    assert 32 <= a.block_threads <= 256 and a.leaps + a.ssa_steps == b.leaps + b.ssa_steps > 0
+
+
 @pytest.mark.parametrize("kind", ["thread", "lanes8", "warp", "cta"])
 def test_wide_leaps_are_bit_identical(kind):
     """More than 10^8 firings in a leap: sums past int32 in between."""
