@@ -316,7 +316,8 @@ def run_ours(args, wl, rank, world, local_rank):
     hbm_alg = cbytes + R * (1 + 1) * len(tracked) * w
     pk = peaks()
     ops = ops_per_step(m.n_species, m.n_channels, m.nnz_net)
-    rec, rec_src = ncu_record(f"k_fused_{args.workload}") if args.variant == 0 and not args.t_final and \
+    kernel = "k_tiny" if args.workload == "dimer" else "k_fast"  # models of up to 16 channels: k_tiny
+    rec, rec_src = ncu_record(f"{kernel}_{args.workload}") if args.variant == 0 and not args.t_final and \
         not args.realizations else (None, "ncu record covers the default launch only")
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -338,7 +339,7 @@ def run_ours(args, wl, rank, world, local_rank):
             "issue_slots_busy": rec["issue_slots_busy_pct"] / 100.0 if rec else None,
             "l2_traffic": rec.get("lts_bytes_per_launch") if rec else None,
             "ncu_source": rec_src, "ncu_case": rec.get("case") if rec else None,
-            "peak_src": pk["src"], "kernel": "k_fused", "kernel_ms": k_ms,
+            "peak_src": pk["src"], "kernel": kernel, "kernel_ms": k_ms,
             "alg_bytes_per_step": alg_bytes_per_step(m), "steps_per_launch": steps_per_launch,
             "ops_per_step": ops, "ops_per_s": ops * steps_per_launch / (k_ms / 1e3),
             "hbm_required_gbs": hbm_alg / (k_ms / 1e3) / 1e9,

@@ -273,9 +273,9 @@ tl_status tl_simulate(tl_model *m, const tl_run_cfg *cfg, tl_result *res);
  * Several (model, configuration) pairs in ONE persistent launch.  Each item
  * is simulated exactly as tl_simulate would (same streams, same outputs in
  * its result; grad non-NULL adds tl_sensitivity's gradients).  Small models
- * (<= 16 species and channels) run 32 realizations per warp, one per lane;
- * larger ones one realization per warp; every warp takes work from one
- * counter, so rate sets with uneven step counts or t_final balance out.
+ * (<= 16 species and channels) run several realizations per warp, one on each
+ * lane or group of lanes; larger ones one realization per warp (or per four
+ * warps, in small ensembles); every warp takes work from one counter, so rate sets with uneven step counts or t_final balance out.
  * Models must share the device and the population width; variant and
  * stream fields of the items' cfg are ignored (stream is the argument).
  */

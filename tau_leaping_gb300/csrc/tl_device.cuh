@@ -1,10 +1,10 @@
 // tl_device.cuh - device building blocks of the tau-leaping engine.
 //
-// Everything a realization does in one step lives here, written once and
-// instantiated for three cooperation widths (the "group" owning one
-// realization): one thread (G1), one warp (GWarp) or one CTA (GCta).  The
-// fused persistent kernel loops do_step() until a realization reaches
-// t_final; the plain form calls it once per launch.
+// Philox, the samplers, the groups (one thread, lanes of a warp, a warp or a
+// CTA for one realization) and the direct form of a step, do_step(), written
+// once for every group: the general build loops it until a realization reaches
+// t_final, the plain form calls it once per launch.  The builds without
+// compatibility switches run the steps of tl_step.cuh and tl_tiny.cuh.
 //
 // Reference semantics followed (CSSL-UWM/tau_leaping):
 //   propensity / criticality  tau_leaping/functions.h:100-123, model.cu:180-209
@@ -791,7 +791,7 @@ struct SimParams {
     int score_global;     // scores accumulate in global memory
     int state_global;     // global-slot builds: the state too
     int q_rounds;         // turns of a queue group before its queue is drained
-    int lanes;            // thin groups: lanes of a warp that take realizations
+    int lanes;            // thread groups: lanes of a warp that take realizations
     int row_warp;       // CTA groups: one warp per species row (long rows)
     unsigned char* gslots;  // CTA groups whose slot exceeds shared memory:
                             // one slot per CTA in global memory (else null)

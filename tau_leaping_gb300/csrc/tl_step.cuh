@@ -22,7 +22,7 @@
 //  * Long Poisson draws go through a queue (fast_fire), which lies over X[]:
 //    a leap does not read X between its step bound and its commit.
 //  * Direct-method steps draw their channel on exact integers (lane groups) or
-//    on FP32 with a margin (thin groups); the FP64 form decides the cases
+//    on FP32 with a margin (one thread); the FP64 form decides the cases
 //    neither can (ssa_select).
 // Measured on GB300 against do_step() with in-place draws (4000 to 60 000
 // realizations, ms): toy network 109.7 -> 63.3 on 16 lanes and 47.3 -> 29.8 on
@@ -240,7 +240,7 @@ TL_D float signed_prop(const SimParams& p, const Lay& L, const float* rate, int 
     return __uint_as_float(__float_as_uint(v) | cr);
 }
 
-// Propensities into a[] and the lane's partial sums; thin groups form the sums
+// Propensities into a[] and the lane's partial sums; one thread forms the sums
 // over all channels in order.  Critical channels are stored negative, or with
 // ZERO as 0, which spares every net entry of the step bound a max: what reads
 // their propensities forms them again (select_critical, direct steps).
@@ -846,7 +846,7 @@ TL_D bool wide_leap(const Grp& g, const SimParams& p, const Lay& L, float tauf, 
 // ---------------------------------------------------------------------------
 // Direct-method steps: the channel with probability a_j / a0 and a0 in FP32.
 // ---------------------------------------------------------------------------
-// Thin groups: one running sum in channel order, target u * a0 with u of 52
+// One thread: one running sum in channel order, target u * a0 with u of 52
 // bits.  FP32 decides every channel whose running sum is further from the
 // target than the products' rounding (2^-23 a0, margin 4e-7 a0); the FP64
 // target decides the others.
