@@ -1218,9 +1218,22 @@ static tl_status run(tl_model* m, const tl_run_cfg* cfg, tl_result* res, tl_grad
     return job_finish(J, ms, launches, ms_since(t0));
 }
 
+// The batch kernel's CTAs per SM: two (128 registers, no spills) while they
+// hold every unit at once, three (80 registers) beyond, where more warps hide
+// more of a step's latency.  Measured on GB300, ms at 2 -> 3 -> 4, gradients of
+// dimer sets (16) and toy network sets (4), realizations a set: dimer 1024
+// 1.63 -> 1.73 -> 1.83 (one wave), 4096 5.71 -> 4.71 -> 4.20, 16384 17.7 -> 15.8
+// -> 15.0; toy 700 20.4 -> 17.6 -> 18.8, 1500 32.9 -> 30.7 -> 31.5; both, 4096
+// and 700, 22.4 -> 19.6 -> 23.0; 64 x 4096 and 16 x 1024 to t = 10 and 0.1,
+// 1501 -> 1247 -> 1371.
+static int batch_minb(long long units, int warps, int nsm) {
+    return units > 2LL * warps * nsm ? TL_BATCH_MANY_MINB : TL_BATCH_MINB;
+}
+
 // One launch over several (model, configuration) items.  Items of small
-// models run as lane units (32 realizations per warp, one per lane), the
-// others as warp units (one realization per warp); a warp takes units from
+// models run as lane units (several realizations per warp, on one or 4 to 16
+// lanes each), the others as warp units (one realization per warp, or per team
+// of four warps where they all fit at once); a warp takes units from
 // one global counter, so uneven step counts and uneven t_final balance out.
 static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     const auto t0 = std::chrono::steady_clock::now();
@@ -1403,10 +1416,11 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     bp.params_bytes = (int)spb;
     bp.wctr = reinterpret_cast<unsigned long long*>(B + o_wctr);
     round_keys(jobs[0].p.k0, jobs[0].p.k1, bp.rk);
+    const int minb = batch_minb(units, warps, sm_count());
     const size_t smem = team ? team_smem : stage + (size_t)warps * (wslot + spb);
     int bps = team_bps;
-    cudaError_t le = team ? cudaSuccess : pop == 64 ? batch_occupancy<long long>(bmode, staged, thin, 32 * warps, smem, &bps)
-                               : batch_occupancy<int>(bmode, staged, thin, 32 * warps, smem, &bps);
+    cudaError_t le = team ? cudaSuccess : pop == 64 ? batch_occupancy<long long>(bmode, staged, minb, thin, 32 * warps, smem, &bps)
+                               : batch_occupancy<int>(bmode, staged, minb, thin, 32 * warps, smem, &bps);
     if (le != cudaSuccess) return cuda_fail(le, "batch occupancy");
     const int grid = (int)std::min<long long>((long long)sm_count() * std::max(bps, 1),
                                               team ? (units + 1) / 2 : (units + warps - 1) / warps);
@@ -1418,8 +1432,8 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     if (le == cudaSuccess)
         le = team ? (pop == 64 ? launch_batch_team<long long>(bp, bmode, thin, grid, smem, st, nullptr)
                                : launch_batch_team<int>(bp, bmode, thin, grid, smem, st, nullptr))
-             : pop == 64 ? launch_batch<long long>(bp, bmode, thin, 32 * warps, grid, smem, st)
-                       : launch_batch<int>(bp, bmode, thin, 32 * warps, grid, smem, st);
+             : pop == 64 ? launch_batch<long long>(bp, bmode, minb, thin, 32 * warps, grid, smem, st)
+                       : launch_batch<int>(bp, bmode, minb, thin, 32 * warps, grid, smem, st);
     if (le == cudaSuccess) le = cudaEventRecord(e1, st);
     if (le != cudaSuccess) return cuda_fail(le, "batch launch");
     for (auto& J : jobs) {

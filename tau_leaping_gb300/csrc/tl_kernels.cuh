@@ -1,13 +1,20 @@
 // tl_kernels.cuh - kernels of the engine (instantiated per population type
 // in tl_kernels_i32.cu / tl_kernels_i64.cu).
 //
-//  k_fused   persistent, work-stealing: each group (thread / warp / CTA)
-//            takes realizations from a global counter and runs do_step()
-//            until t_final.  The model constants are staged once per CTA
-//            into shared memory with a TMA bulk copy.
+//  k_fast    persistent, work-stealing: each group (thread / lanes / warp /
+//            four-warp team / CTA) takes realizations from a global counter
+//            and runs fast_step() (tl_step.cuh) until t_final.  The model
+//            tables are staged once per CTA into shared memory with a TMA bulk
+//            copy.
+//  k_tiny    the same for models of up to 16 channels and species, whose state
+//            lies in the registers of a few lanes (tl_tiny.cuh).
+//  k_fused   the general build: do_step(), which reads the compatibility
+//            switches at run time.
+//  k_batch, k_batch_team  many models and configurations in one launch.
 //  k_plain_* the unfused baseline: FP32 time, one realization per thread,
 //            state in global memory, one launch per step.
-//  k_stats   deterministic two-pass mean / sample-stddev per grid column.
+//  k_stats   deterministic two-pass mean / sample-stddev per grid column;
+//            k_stats_wide where there are many columns.
 //  k_grad    likelihood-ratio covariance per (set, species, channel).
 //  k_eval / k_replay / k_philox / k_poisson  parity entry points.
 #pragma once
@@ -329,9 +336,10 @@ __global__ void __launch_bounds__(256, TL_THREAD_MINB) k_tiny(const __grid_const
 // ---------------------------------------------------------------------------
 // FAST: the fast build, or with SENS the scores build, of every item;
 // otherwise the general one.  STAGED: every item's tables in shared memory.
-// W: lanes of a small item's realization (1: thread groups).
-template <class Pop, bool FAST, bool SENS, bool STAGED, int W>
-__global__ void __launch_bounds__(256, TL_BATCH_MINB) k_batch(BatchParams bp) {
+// W: lanes of a small item's realization (1: thread groups).  MINB: CTAs per SM
+// (batch_minb).
+template <class Pop, bool FAST, bool SENS, bool STAGED, int W, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_batch(BatchParams bp) {
     unsigned char* const smem = tl_smem;
     __shared__ __align__(8) unsigned long long mbar;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;

@@ -12,8 +12,8 @@ struct SimParams;
 
 // kind: 1 = thread, 32 = warp, 0 = CTA, 2/4/8/16 = lanes per realization,
 // kKindCtaGlobal = CTA with its propensities (or whole slot) in global memory;
-// in the fast and scores builds thread groups are thin groups of one lane or,
-// for small models, 4, 8 or 16 lanes (tl_tiny.cuh).
+// in the fast and scores builds a thread group is one lane (GThin) or, for
+// small models, 4, 8 or 16 lanes (tl_tiny.cuh).
 constexpr int kKindCtaGlobal = 64;
 constexpr int kKindTeam = 132;  // four warps for one realization of a warp group
 constexpr int kKindThin1 = 101, kKindTiny4 = 104, kKindTiny8 = 108, kKindTiny16 = 116;
@@ -47,11 +47,12 @@ constexpr int kModeFast = 0, kModeScores = 1, kModeGeneral = 2;
 #ifndef TL_GENERAL_MINB
 #define TL_GENERAL_MINB 5
 #endif
-// The batch kernel (thread and warp units, scores on) at 2 CTAs per SM
-// (128 registers): 1 gives 160 registers and one CTA per SM (-37 %), 4 and
-// 5 spill (-24 %, -22 %).
+// The batch kernel's CTAs per SM: batch_minb() chooses.
 #ifndef TL_BATCH_MINB
 #define TL_BATCH_MINB 2
+#endif
+#ifndef TL_BATCH_MANY_MINB
+#define TL_BATCH_MANY_MINB 3
 #endif
 // staged: the tables are staged in shared memory.
 template <class Pop>
@@ -73,16 +74,17 @@ struct FusedCall {
 template <class Pop>
 cudaError_t call_general_sub(const FusedCall& c);
 template <class Pop>
-cudaError_t call_fast(const FusedCall& c);  // thin and warp groups
+cudaError_t call_fast(const FusedCall& c);  // thread and warp groups
 template <class Pop>
 cudaError_t call_fast_cta(const FusedCall& c);
 template <class Pop>
 cudaError_t call_fast_sub(const FusedCall& c);
 struct BatchParams;
 template <class Pop>
-cudaError_t launch_batch(const BatchParams& bp, int mode, int thin, int block, int grid, size_t smem, cudaStream_t st);
+cudaError_t launch_batch(const BatchParams& bp, int mode, int minb, int thin, int block, int grid, size_t smem,
+                         cudaStream_t st);
 template <class Pop>
-cudaError_t batch_occupancy(int mode, bool staged, int thin, int block, size_t smem, int* blocks_per_sm);
+cudaError_t batch_occupancy(int mode, bool staged, int minb, int thin, int block, size_t smem, int* blocks_per_sm);
 // the same with four-warp teams in place of the warp units (staged tables only)
 template <class Pop>
 cudaError_t launch_batch_team(const BatchParams& bp, int mode, int thin, int grid, size_t smem, cudaStream_t st,

@@ -159,6 +159,19 @@ def test_global_propensities_and_batches_are_bit_identical():
         assert np.array_equal(x["samples"], y["samples"]) and x["leaps"] == y["leaps"]
 
 
+@pytest.mark.parametrize("n_small,n_big", [(300, 2431), (20000, 40), (9, 2600)])
+def test_batches_of_more_units_than_two_ctas_hold(n_small, n_big):
+    """The batch kernel's register budget follows the number of units; every
+    item equals its own call."""
+    big, _ = network(33, 60, 8)
+    small, _ = network(6, 11, 5)
+    kw = dict(t_final=0.002, seed=9, keep_samples=True, tracked=[0, 1, 2])
+    out = simulate_batch([dict(kw, model=small, n=n_small), dict(kw, model=big, n=n_big)])
+    for r, m, n, v in ((out[0], small, n_small, _ffi.VARIANT_THREAD), (out[1], big, n_big, _ffi.VARIANT_WARP)):
+        one = m.simulate(n=n, variant=v, **kw)
+        assert np.array_equal(r["samples"], one.samples) and r["leaps"] == one.leaps
+
+
 @pytest.mark.parametrize("n,K,intervals,sets", [(64, 64, 1, 1), (1001, 33, 2, 3), (257, 130, 1, 2)])
 def test_statistics_of_many_columns(n, K, intervals, sets):
     """Means and deviations of 64 columns and more: exact integer sums, so
