@@ -83,9 +83,11 @@ static bool fill_rates(const HostModel& h, const double* c, float* plain, float*
 //  col   per channel, chunks of four net entries: byte offset of the species
 //        in an int array << 12 | stoichiometry & 0xfff, 0 stoichiometry = none
 //  cp    first chunk of each channel, where a channel needs more than one
+//        (col and cp hold whole blocks of four channels, as a[] does: the
+//        firing pass may mark a channel of the padding, which has no entries)
 //  sp    per species the index in X of its |x - 1|, 0 if it has none
 //  tiny  a TinyTable, for models of up to 16 channels and species
-static void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned char>& out) {
+void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned char>& out) {
     const int N = h.N, M = h.M;
     std::vector<int> x2((size_t)N, 0);
     d.n_2s = 0;
@@ -114,9 +116,10 @@ static void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned ch
     for (int j = 0; j < M; ++j) max_col = std::max(max_col, h.net_cp[(size_t)j + 1] - h.net_cp[(size_t)j]);
     if (ent_chunks >= (1u << 20) || max_chunks >= (1 << 12)) return;
     for (int j = 0; j < M; ++j)
-        col_chunks += max_col <= 4 ? 1 : (size_t)(h.net_cp[(size_t)j + 1] - h.net_cp[(size_t)j] + 3) / 4;
+        col_chunks += (size_t)(h.net_cp[(size_t)j + 1] - h.net_cp[(size_t)j] + 3) / 4;
     d.n_rows = 0;
     for (int i = 0; i < N; ++i) d.n_rows += h.gkind[(size_t)i] != 0;
+    if (max_col <= 4) col_chunks = (size_t)pad;
     size_t off = 0;
     const auto sect = [&](size_t bytes) {
         const size_t o = off;
@@ -127,7 +130,7 @@ static void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned ch
     d.t_row = sect((size_t)d.n_rows * 8);
     d.t_ent = sect(ent_chunks * 16);
     d.t_col = sect(col_chunks * 16);
-    d.t_cp = max_col > 4 ? sect((size_t)(M + 1) * 4) : -1;
+    d.t_cp = max_col > 4 ? sect((size_t)(pad + 1) * 4) : -1;
     d.t_sp = sect((size_t)Np * 2);
     const bool tiny = N <= 16 && M <= 16;
     d.t_tiny = tiny ? sect(sizeof(TinyTable)) : 0;
@@ -176,7 +179,7 @@ static void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned ch
                                             ((uint32_t)unpack_v(h.net_rv[(size_t)q]) & 0xfffu);
         c4 += cp ? (size_t)(q1 - q0 + 3) / 4 : 1;
     }
-    if (cp) cp[M] = (uint32_t)c4;
+    if (cp) std::fill(cp + M, cp + pad + 1, (uint32_t)c4);
     unsigned short* sp = reinterpret_cast<unsigned short*>(out.data() + d.t_sp);
     for (int i = 0; i < N; ++i) sp[i] = (unsigned short)x2[(size_t)i];
     if (tiny) {

@@ -82,6 +82,9 @@ struct DevModel {
     int nnz_net = 0, nnz_raw = 0;
 };
 
+// Tables of the fast and scores builds and where they lie (d.t_*, d.fast_ok).
+void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned char>& out);
+
 }  // namespace tl
 
 struct tl_model {

@@ -507,7 +507,9 @@ __device__ __noinline__ void undo_leap(const Grp g, const SimParams& p, const La
 //    kind on all lanes and a channel's firing is spread over the lanes with
 //    its draw.  A PTRS lane moves on to its next draw after an accepted
 //    attempt instead of waiting for the warp's last one.
-// a[] is padded to whole blocks of four; the padding holds 0.
+// a[], k[] and the columns are padded to whole blocks of four channels: the
+// padding holds 0 and has no entries.  Its mean of 0 lies within the margin where
+// the word is below 5e-6 of its range, so it can be marked; it is dropped there.
 constexpr float kFireMargin = 5e-6f;
 constexpr int kMaxRounds = 7;  // marked channels of a queue group fit ten bits
 
@@ -641,6 +643,7 @@ TL_D void fast_fire(const Grp& g, const SimParams& p, const Lay& L, float tauf, 
             const int j = channel(q[i]);
             int k = 1;
             if (i < n_inv) {
+                if (j >= p.M) continue;
                 const float mu = fmaxf(a[j], 0.f) * tauf;
                 U4 w = group_words(L.rk, (uint32_t)j >> 2, step, r, set);
                 uint32_t word = word_of(w, j & 3);
