@@ -484,6 +484,7 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
     const int smax = max_smem_optin() - 2048;
     const bool autov = variant == TL_VARIANT_AUTO;
     const int nsm = sm_count();
+    pl = Plan{};  // nothing of a plan that pl held before (measured mode plans twice)
     if (autov) variant = heuristic_variant(m, sb, total, mode, nsm);
     pl.variant = variant;
     int groups_per_block = 1;
