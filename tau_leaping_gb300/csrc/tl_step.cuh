@@ -1110,8 +1110,9 @@ TL_D void direct_steps_lanes(const GWarp& g, const SimParams& p, const Lay& L, i
         st.step++;
         st.ssa++;
         if (++q == p.ssa_block || (p.max_steps > 0 && (long long)(st.step - st.rej) >= p.max_steps)) break;
-        // propensities
-        const float f = popf(x);
+        // propensities: products of |x|, as everywhere (a channel that lists a
+        // species twice can take it below zero)
+        const float f = fabsf(popf(x));
         const float f0 = g.bcast(f, src0), fs = g.bcast(f, src1), f2 = g.bcast(popf((Pop)(x - 1)), src0);
         const float f1 = single ? 1.f : twice ? fabsf(f2) : fs;
         pa = rate * (none ? 1.f : f0) * f1;

@@ -3,6 +3,8 @@ results are those of the same group kind launched directly."""
 import numpy as np
 import pytest
 
+from tests.test_gpu_group_builds import KINDS
+
 from tau_leaping_gb300 import Model, _ffi
 
 pytestmark = pytest.mark.gpu
@@ -30,3 +32,23 @@ def test_measured_mode_is_no_slower_than_the_planned_launch():
     planned = min(m.simulate(**kw).kernel_ms for _ in range(5))
     measured = min(m.simulate(flags=_ffi.FLAG_AUTOTUNE_MEASURE, **kw).kernel_ms for _ in range(5))
     assert measured <= 1.05 * planned, (measured, planned)
+
+
+@pytest.mark.parametrize("kind", ["thread", "lanes8", "warp", "cta"])
+@pytest.mark.parametrize("bits", [32, 64])
+def test_direct_steps_below_zero_match_the_general_build(kind, bits):
+    """A channel that lists a species twice as a reactant S + S takes two of
+    it while one is left; the propensities of the steps that follow are
+    products of |x| in every build."""
+    cols = [[(0, -1), (0, -1), (1, 1)], [(1, -1), (0, 1)], [(0, -1), (2, 1)], [(2, -2), (0, 3)], [(3, -1), (0, 1)]]
+    cols += [[(i, -1), ((i + 1) % 20, 1)] for i in range(4, 20)]
+    cp = np.cumsum([0] + [len(c) for c in cols])
+    x0 = [5, 4, 3, 2] + [2] * 16
+    m = Model.from_arrays(x0, [0.5, 0.2, 0.3, 0.1, 0.2] + [0.1] * 16, cp, [i for c in cols for i, _ in c],
+                          [v for c in cols for _, v in c], pop_bits=bits)
+    kw = dict(t_final=50.0, n=200, seed=3, intervals=3, keep_samples=True, max_steps=150, allow_truncation=True,
+              ssa_factor=10**9, n_critical=1, variant=KINDS[kind])
+    a, b = m.simulate(**kw), m.simulate(flags=_ffi.FLAG_COMPAT_G, **kw)
+    assert (b.samples < 0).any()
+    assert np.array_equal(a.samples, b.samples)
+    assert (a.leaps, a.ssa_steps, a.truncated) == (b.leaps, b.ssa_steps, b.truncated)
