@@ -748,9 +748,10 @@ TL_D bool fast_check(const Grp& g, const SimParams& p, const Lay& L, bool& over)
     const bool bad = g.any(sign < 0);
     over = false;
     if (sizeof(Pop) == 4 && bad) {
-        bool of = false;  // a sum that wrapped: |D| < 2^31
+        bool of = false;  // a sum that wrapped: |D| < 2^31, and not from below zero
 #pragma unroll 1
-        for (int i = g.rank(); i < p.N; i += g.size()) of |= L.D()[i] > 0 && add_pop(L.x()[i], L.D()[i]) < 0;
+        for (int i = g.rank(); i < p.N; i += g.size())
+            of |= L.x()[i] >= 0 && L.D()[i] > 0 && add_pop(L.x()[i], L.D()[i]) < 0;
         over = g.any(of);
     }
     return bad;
@@ -780,10 +781,11 @@ TL_D bool thin_commit(const SimParams& p, const Lay& L, bool& over) {
     bool bad = false;
     over = false;
     for (int i = 0; i < p.N; ++i) {
+        const Pop x = L.x()[i];
         const int d = L.D()[i];
-        const bool b = add_pop(L.x()[i], d) < 0;
+        const bool b = add_pop(x, d) < 0;
         bad |= b;
-        over |= sizeof(Pop) == 4 && b && d > 0;
+        over |= sizeof(Pop) == 4 && b && d > 0 && x >= 0;
     }
     if (bad) return true;
     for (int i = 0; i < p.N; ++i) {

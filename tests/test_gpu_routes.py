@@ -52,3 +52,19 @@ def test_direct_steps_below_zero_match_the_general_build(kind, bits):
     assert (b.samples < 0).any()
     assert np.array_equal(a.samples, b.samples)
     assert (a.leaps, a.ssa_steps, a.truncated) == (b.leaps, b.ssa_steps, b.truncated)
+
+
+@pytest.mark.parametrize("kind", ["thread", "lanes8", "warp", "cta"])
+def test_a_leap_from_below_zero_is_rejected_not_an_overflow(kind):
+    """Direct-method steps take S below zero (S + S from one species), then
+    births of A make the steps leaps: a leap that adds to S without lifting it to
+    zero is rejected until its halvings run out, in every build."""
+    cols = [[(0, -1), (0, -1)], [(0, 1)], [(1, 5)], [(1, -1)]] + [[(2 + i, -1), (2 + (i + 1) % 18, 1)] for i in range(18)]
+    cp = np.cumsum([0] + [len(c) for c in cols])
+    m = Model.from_arrays([1, 0] + [3] * 18, [20.0, 300.0, 1000.0, 1.0] + [0.01] * 18, cp, [i for c in cols for i, _ in c],
+                          [v for c in cols for _, v in c], pop_bits=32)
+    kw = dict(t_final=5.0, n=2000, seed=3, max_steps=150, allow_truncation=True, ssa_factor=1, variant=KINDS[kind])
+    for flags in (0, _ffi.FLAG_COMPAT_CRIT):
+        with pytest.raises(_ffi.TLError) as e:
+            m.simulate(flags=flags, **kw)
+        assert e.value.status == 12, (flags, str(e.value))
