@@ -740,7 +740,8 @@ static tl_status job_prepare(Job& J) {
         if (ds != TL_OK) return ds;
         halvable = m->d.halvable;
     }
-    if (!halvable) J.mode = kModeGeneral;
+    // the packed criticalities are signs of x - n_c and x - 2 n_c, in int32
+    if (!halvable || cfg->n_critical >= (1 << 30)) J.mode = kModeGeneral;
     if (cfg->n_rate_sets > 0 && cfg->t_final_sets)
         for (int s = 0; s < J.S; ++s) {
             J.htf[(size_t)s] = cfg->t_final_sets[s];

@@ -3,7 +3,7 @@ results are those of the same group kind launched directly."""
 import numpy as np
 import pytest
 
-from tests.test_gpu_group_builds import KINDS
+from tests.test_gpu_group_builds import KINDS, assert_same, network
 
 from tau_leaping_gb300 import Model, _ffi
 
@@ -68,3 +68,13 @@ def test_a_leap_from_below_zero_is_rejected_not_an_overflow(kind):
         with pytest.raises(_ffi.TLError) as e:
             m.simulate(flags=flags, **kw)
         assert e.value.status == 12, (flags, str(e.value))
+
+
+@pytest.mark.parametrize("kind", ["thread", "lanes8", "warp", "cta"])
+@pytest.mark.parametrize("n_critical", [2**30 - 1, 2**30, 2**30 + 2**29, 2**31 - 1])
+def test_thresholds_near_the_end_of_int32(kind, n_critical):
+    """Twice the threshold leaves int32 from 2^30 on."""
+    for bits in (32, 64):
+        m, general = network(12, 16, 5, bits, two_s=True)
+        r = assert_same(m, general, variant=KINDS[kind], n_critical=n_critical)
+        assert r is not None
