@@ -1,0 +1,24 @@
+// tl_shared.h - what kernels, launch code and host tests compute alike.
+#pragma once
+
+#include <cstdint>
+
+#ifdef __CUDACC__
+#define TL_SHARED __host__ __device__ __forceinline__
+#else
+#define TL_SHARED inline
+#endif
+
+namespace tl {
+
+// The Philox step counter wraps at 2^32; epochs counts that, so that caps and
+// counts of steps hold past it.  The counter's words repeat from there on.
+TL_SHARED void next_step(uint32_t& step, uint32_t& epochs) {
+    if (++step == 0u) ++epochs;
+}
+// Accepted steps: attempts and direct-method steps less the rejected attempts.
+TL_SHARED long long accepted(uint32_t epochs, uint32_t step, uint32_t rej) {
+    return (long long)((unsigned long long)epochs << 32 | step) - (long long)rej;
+}
+
+}  // namespace tl

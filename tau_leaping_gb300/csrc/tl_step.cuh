@@ -34,6 +34,7 @@
 #include <type_traits>
 
 #include "tl_device.cuh"
+#include "tl_shared.h"
 
 namespace tl {
 
@@ -989,13 +990,14 @@ TL_D int ssa_select(const Grp& g, const SimParams& p, const Lay& L, float part, 
 // block of direct-method steps.
 // ---------------------------------------------------------------------------
 // Every leap attempt and every direct-method step advances the Philox step
-// counter once: accepted steps = step - rej, leaps = accepted - ssa.
+// counter once: accepted() = step - rej in 64 bits, leaps = accepted - ssa.
 struct FastState {
     double t;
     double t_next;  // grid time kpt; done may be set before the last point: the state holds
     int kpt;        // next grid point to record
     uint32_t step;
     uint32_t rej, ssa;
+    uint32_t epochs;   // wraps of step
     uint32_t ex_from;  // the lanes hold the critical waiting times (unit rate) of the steps from here
     float ex;
     bool wide;     // the next step is a wide leap
@@ -1109,9 +1111,9 @@ TL_D void direct_steps_lanes(const GWarp& g, const SimParams& p, const Lay& L, i
             x = add_pop(x, d);
         }
         st.t = t_new;
-        st.step++;
+        next_step(st.step, st.epochs);
         st.ssa++;
-        if (++q == p.ssa_block || (p.max_steps > 0 && (long long)(st.step - st.rej) >= p.max_steps)) break;
+        if (++q == p.ssa_block || (p.max_steps > 0 && accepted(st.epochs, st.step, st.rej) >= p.max_steps)) break;
         // propensities: products of |x|, as everywhere (a channel that lists a
         // species twice can take it below zero)
         const float f = fabsf(popf(x));
@@ -1208,9 +1210,9 @@ TL_D void direct_steps(const Grp& g, const SimParams& p, const Lay& L, int set, 
         }
         g.sync();
         st.t = t_new;
-        st.step++;
+        next_step(st.step, st.epochs);
         st.ssa++;
-        if (++q == p.ssa_block || (p.max_steps > 0 && (long long)(st.step - st.rej) >= p.max_steps)) return;
+        if (++q == p.ssa_block || (p.max_steps > 0 && accepted(st.epochs, st.step, st.rej) >= p.max_steps)) return;
         float pac;
         fast_props<false>(g, p, L, rate, pa, pac);
         if (!g.any(pa > 0.f)) {
@@ -1317,7 +1319,7 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
         }
         if (!bad) break;
         // reject: halve tau1, fresh counters, same state and propensities
-        st.step++;
+        next_step(st.step, st.epochs);
         st.rej++;
         tau1 *= 0.5f;
         if (attempt + 1 > p.max_halv) {
@@ -1331,7 +1333,7 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
         add_scores(g, p, L, set, r, true, [&](int, float a, int k) { return (float)k - fabsf(a) * tau_used; });
     }
     g.sync();
-    st.step++;
+    next_step(st.step, st.epochs);
     if (clamp) {
         st.t = st.t_next;
         record_next(g, p, L, set, r, st);
@@ -1371,7 +1373,7 @@ TL_D void fast_realization(const Grp& g, const SimParams& p, const Lay& L, long 
     fast_refresh(g, p, L);
     fast_record(g, p, L, set, r, 0);
     g.sync();
-    FastState st{0.0, grid_time<double>(p, set, 1), 1, 0u, 0u, 0u, 0u - 32u, 0.f, false, false};  // ex: not drawn yet
+    FastState st{0.0, grid_time<double>(p, set, 1), 1, 0u, 0u, 0u, 0u, 0u - 32u, 0.f, false, false};  // ex: not drawn yet
     bool trunc = false;
     while (!st.done) {
         fast_step<Grp, Lay, SENS, false>(g, p, L, set, r, st);
@@ -1380,7 +1382,7 @@ TL_D void fast_realization(const Grp& g, const SimParams& p, const Lay& L, long 
             wide_step<Grp, Lay, SENS>(g, p, L, set, r, &tmp);
             st = tmp;
         }
-        if (!st.done && p.max_steps > 0 && (long long)(st.step - st.rej) >= p.max_steps) {
+        if (!st.done && p.max_steps > 0 && accepted(st.epochs, st.step, st.rej) >= p.max_steps) {
             st.done = true;
             trunc = true;
         }
@@ -1394,7 +1396,7 @@ TL_D void fast_realization(const Grp& g, const SimParams& p, const Lay& L, long 
         for (int j = g.rank(); j < p.M; j += g.size()) to[j] = L.score(0)[j];
     }
     if (g.leader()) {
-        const uint32_t leaps = st.step - st.rej - st.ssa;
+        const long long leaps = accepted(st.epochs, st.step, st.rej) - (long long)st.ssa;
         if (leaps) atomicAdd(p.ctr + 1, (unsigned long long)leaps);
         if (st.ssa) atomicAdd(p.ctr + 2, (unsigned long long)st.ssa);
         if (st.rej) atomicAdd(p.ctr + 3, (unsigned long long)st.rej);
