@@ -478,8 +478,61 @@ static int even_block(long long total, int groups_per_warp, int nsm, int most_wa
     return 32 * best;
 }
 
+// What a plan depends on besides the model and the launch: the leap condition's
+// eps and the time between two grid points.
+struct LeapScale {
+    double eps = 0.03, dt = 1.0;
+};
+
+// Whether most draws of a leap have means of 10 and more (PTRS), by the first
+// leap from x0: the mean of channel j is a_j times the CGP bound or dt.
+static bool mostly_long_draws(const HostModel& h, const LeapScale& ls) {
+    const int M = h.M, N = h.N;
+    std::vector<double> a((size_t)M);
+    const auto pop = [&](int i) { return (double)h.x0[(size_t)i]; };
+    for (int j = 0; j < M; ++j) {
+        const int o = h.order[(size_t)j], s0 = h.s0[(size_t)j], s1 = h.s1[(size_t)j];
+        a[(size_t)j] = h.rate[(size_t)j] * (o == 0 ? 1.0 : o == 1 ? pop(s0) : o == 2 ? pop(s0) * pop(s1) : pop(s0) * (pop(s0) - 1.0) * 0.5);
+    }
+    double tau = ls.dt;
+    for (int i = 0; i < N; ++i) {
+        if (!h.gkind[(size_t)i]) continue;
+        double mu = 0.0, s2 = 0.0;
+        for (int q = h.net_rp[(size_t)i]; q < h.net_rp[(size_t)i + 1]; ++q) {
+            const double v = unpack_v(h.net_vc[(size_t)q]), t = v * a[(size_t)unpack_idx(h.net_vc[(size_t)q])];
+            mu += t;
+            s2 += v * t;
+        }
+        const double num = std::max(ls.eps * pop(i) / (h.gkind[(size_t)i] == 1 ? 1.0 : 2.0), 1.0);
+        if (mu != 0.0) tau = std::min(tau, num / std::fabs(mu));
+        if (s2 > 0.0) tau = std::min(tau, num * num / s2);
+    }
+    int many = 0;
+    for (int j = 0; j < M; ++j) many += a[(size_t)j] * tau >= 10.0;
+    return 4 * many >= 3 * M;
+}
+
+// Lane groups of 2 to 16 lanes that the general build runs faster.  The fast
+// build's queue of long draws is one per group, and the groups of a warp drain
+// theirs one after another: what 32 and 16 lanes gain, 2 to 8 lose where nearly
+// every draw is long or one drain does not hold a leap.  Measured on GB300, ms,
+// fast -> general build:
+//   8 lanes, cyclic chains, 50 000 realizations: 32 species 0.507 -> 0.333 (int64
+//     0.558 -> 0.358), 17 species 0.415 -> 0.306, 64 species 0.96 -> 0.79; networks
+//     of 20 to 256 channels, up to 45 % long draws, 1.3 to 1.9 times faster on the fast one
+//   16 lanes: chains of 96 to 256 species 1.1 to 1.3 times faster on the fast
+//     build, 1024 species 17.4 -> 12.7 (30 000 realizations)
+//   4 lanes, 4000 realizations: 64 x 128 network 4.77 against 8.83, 96 x 192 5.37 -> 3.00,
+//     128 x 256 31.8 -> 16.9
+//   2 lanes: dimer decay 0.80 -> 0.55, 12 x 20 1.05 -> 0.89, 30 x 60 18.6 -> 8.0, 128 x 256 124 -> 38
+//     (only 8 x 12 and smaller direct-method models gain on the fast build)
+static bool general_is_faster(const HostModel& h, int kind, const LeapScale& ls) {
+    if (kind == 2 || (kind == 4 && h.M > 128)) return true;
+    return (kind <= 8 || h.M > 512) && mostly_long_draws(h, ls);
+}
+
 static tl_status make_plan(const tl_model* m, int variant, int block_req, int mode, bool sens, bool compat_stoich,
-                           bool no_stage, long long total, Plan& pl, bool force_gslot = false) {
+                           bool no_stage, long long total, const LeapScale& ls, Plan& pl, bool force_gslot = false) {
     const size_t sb = slot_bytes(m, mode != kModeFast);
     const int smax = max_smem_optin() - 2048;
     const bool autov = variant == TL_VARIANT_AUTO;
@@ -541,7 +594,9 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
     // the packed tables hold the model (CTA groups: wide forms too)?
     const bool packed = m->d.fast_ok && (pl.kind == 0 || (!m->d.chan8 && !m->d.ent_wide));
     // the sub-warp and global-slot kinds have no scores build
-    if (!packed || (mode == kModeScores && (pl.gslot || (pl.kind > 1 && pl.kind < 32)))) mode = kModeGeneral;
+    const bool sub = pl.kind > 1 && pl.kind < 32;
+    if (!packed || (mode == kModeScores && (pl.gslot || sub))) mode = kModeGeneral;
+    if (mode == kModeFast && sub && general_is_faster(m->h, pl.kind, ls)) mode = kModeGeneral;
     if (!fit(mode) && !pl.gslot) {
         // the general build's slot is smaller for wide models
         if (mode == kModeGeneral || !fit(kModeGeneral)) {
@@ -615,7 +670,7 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
     if (pl.kind >= 2 && pl.kind <= 32 && !pl.team && block_req <= 0 && need <= (long long)nsm * bps) {
         const int block = even_block(total, 32 / pl.kind, nsm, pl.block / 32);
         Plan q;
-        if (block < pl.block && make_plan(m, variant, block, mode, sens, compat_stoich, no_stage, total, q) == TL_OK &&
+        if (block < pl.block && make_plan(m, variant, block, mode, sens, compat_stoich, no_stage, total, ls, q) == TL_OK &&
             q.block == block && q.mode == pl.mode && (q.stage > 0) == staged && (long long)q.grid * (block / q.kind) >= total)
             pl = q;
     }
@@ -660,6 +715,7 @@ struct Job {
     unsigned char* base = nullptr;
     std::vector<unsigned char> hin;  // what goes to the device
     size_t o_in = 0;
+    LeapScale scale;
     std::vector<double> htf;
     std::vector<double> hgrid;  // [S][P] grid times
     Plan pl;
@@ -750,6 +806,7 @@ static tl_status job_prepare(Job& J) {
                 return TL_ERR_INVALID_ARGUMENT;
             }
         }
+    J.scale = LeapScale{cfg->eps, J.htf[0] / (double)cfg->n_intervals};
     // grid t_k = T*k/n_int (FP64, the last point T itself)
     J.hgrid.resize((size_t)J.S * J.P);
     for (int s = 0; s < J.S; ++s)
@@ -1071,7 +1128,7 @@ static tl_status autotune_measure(Job& J, cudaStream_t st) {
         for (const Cand& c : cands) {
             Plan pl;
             if (c.variant == TL_VARIANT_AUTO) pl = J.pl;
-            else if (make_plan(m, c.variant, c.block, J.mode, J.sens, J.compat_stoich, c.nostage, trial, pl) != TL_OK) continue;
+            else if (make_plan(m, c.variant, c.block, J.mode, J.sens, J.compat_stoich, c.nostage, trial, J.scale, pl) != TL_OK) continue;
             if (c.variant == TL_VARIANT_THREAD && c.block != pl.block) continue;
             // global slots exist for the launch the heuristic planned
             if (pl.gslot && (!planned_gslot || pl.grid > planned_grid)) continue;
@@ -1106,12 +1163,13 @@ static tl_status autotune_measure(Job& J, cudaStream_t st) {
         m->tuned_nostage = win.nostage ? 1 : 0;
     }
     tl_status ps = make_plan(m, m->tuned_variant, m->tuned_block, J.mode, J.sens, J.compat_stoich, m->tuned_nostage != 0,
-                             J.total, J.pl, m->tuned_variant == TL_VARIANT_AUTO && force_gslot);
+                             J.total, J.scale, J.pl, m->tuned_variant == TL_VARIANT_AUTO && force_gslot);
     if (ps != TL_OK) return ps;
     if (J.pl.gslot && (!planned_gslot || J.pl.grid > planned_grid)) {
         // a cached global-slot plan that needs more slots than were laid out:
         // keep the planned launch
-        ps = make_plan(m, TL_VARIANT_AUTO, 0, J.mode, J.sens, J.compat_stoich, planned_nostage, J.total, J.pl, force_gslot);
+        ps = make_plan(m, TL_VARIANT_AUTO, 0, J.mode, J.sens, J.compat_stoich, planned_nostage, J.total, J.scale,
+                       J.pl, force_gslot);
         if (ps != TL_OK) return ps;
     }
     bind_plan(m, J.pl, J.p);
@@ -1133,7 +1191,7 @@ static tl_status run(tl_model* m, const tl_run_cfg* cfg, tl_result* res, tl_grad
     const bool no_stage = (cfg->flags & TL_FLAG_NO_STAGE) != 0;
     J.measure = !J.plain && cfg->variant == TL_VARIANT_AUTO && (cfg->flags & TL_FLAG_AUTOTUNE_MEASURE);
     if (!J.plain) {
-        ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.sens, J.compat_stoich, no_stage, J.total, J.pl,
+        ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.sens, J.compat_stoich, no_stage, J.total, J.scale, J.pl,
                        (cfg->flags & TL_FLAG_GLOBAL_SLOTS) != 0);
         if (ps != TL_OK) return ps;
     } else {
@@ -1956,14 +2014,14 @@ extern "C" tl_status tl_simulate_static(tl_model* m, const tl_run_cfg* cfg, tl_r
     TLC(cudaSetDevice(m->d.device));
     cudaStream_t st = (cudaStream_t)cfg->stream;
     ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.sens, J.compat_stoich,
-                   (cfg->flags & TL_FLAG_NO_STAGE) != 0, J.total, J.pl, (cfg->flags & TL_FLAG_GLOBAL_SLOTS) != 0);
+                   (cfg->flags & TL_FLAG_NO_STAGE) != 0, J.total, J.scale, J.pl, (cfg->flags & TL_FLAG_GLOBAL_SLOTS) != 0);
     if (ps != TL_OK) return ps;
     Carver c;
     job_layout(J, c);
     if (c.off > (size_t)TL_STATIC_SCRATCH_BYTES && J.pl.state_global) {
         // the general build's global slots are smaller
         ps = make_plan(m, cfg->variant, cfg->block_threads, kModeGeneral, J.sens, J.compat_stoich,
-                       (cfg->flags & TL_FLAG_NO_STAGE) != 0, J.total, J.pl, (cfg->flags & TL_FLAG_GLOBAL_SLOTS) != 0);
+                       (cfg->flags & TL_FLAG_NO_STAGE) != 0, J.total, J.scale, J.pl, (cfg->flags & TL_FLAG_GLOBAL_SLOTS) != 0);
         if (ps != TL_OK) return ps;
         c = Carver{};
         job_layout(J, c);

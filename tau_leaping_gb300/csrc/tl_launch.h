@@ -27,7 +27,8 @@ struct TinyTable {
 };
 // mode: the kernel build a run needs.  Fast: no likelihood-ratio scores and
 // no reference-compatibility switches; Scores: with scores; General: both.
-// The sub-warp and global-slot kinds come in Fast and General only.
+// The sub-warp and global-slot kinds come in Fast and General only, two lanes in
+// General only.
 constexpr int kModeFast = 0, kModeScores = 1, kModeGeneral = 2;
 // Thread, sub-warp and warp groups launch at most 256 threads per CTA and
 // ask the compiler for a number of resident CTAs per SM, which sets the

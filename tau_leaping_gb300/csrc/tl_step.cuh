@@ -1196,7 +1196,7 @@ TL_D void direct_steps(const Grp& g, const SimParams& p, const Lay& L, int set, 
                 c0 = (int)L.cp()[j];
                 n = (int)L.cp()[j + 1] - c0;
             }
-            constexpr int kBy = Grp::kWidth == 1 || Grp::kWidth == 2 ? Grp::kWidth : 4;  // lanes
+            constexpr int kBy = Grp::kWidth == 1 ? 1 : 4;  // lanes
             if (g.rank() < kBy)
 #pragma unroll 1
                 for (int e = 4 * c0 + g.rank(); e < 4 * (c0 + n); e += kBy) {

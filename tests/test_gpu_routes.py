@@ -78,3 +78,18 @@ def test_thresholds_near_the_end_of_int32(kind, n_critical):
         m, general = network(12, 16, 5, bits, two_s=True)
         r = assert_same(m, general, variant=KINDS[kind], n_critical=n_critical)
         assert r is not None
+
+
+@pytest.mark.parametrize("variant,family,kw,t,n", [
+    (_ffi.VARIANT_AUTO, "chain", dict(n_species=32), 0.5, 50000), (_ffi.VARIANT_AUTO, "chain", dict(n_species=64, pop_bits=64), 0.5, 50000),
+    (_ffi.VARIANT_LANES2, "dimer", {}, 1.0, 4000), (_ffi.VARIANT_LANES4, "toy", {}, 0.001, 4000),
+    (_ffi.VARIANT_LANES4, "chain", dict(n_species=128), 0.3, 4000), (_ffi.VARIANT_LANES16, "chain", dict(n_species=1024), 0.3, 30000)])
+def test_narrow_groups_are_no_slower_than_the_general_build(variant, family, kw, t, n):
+    """Narrow groups take the build that runs faster; on the fast one these runs
+    took 1.2 to 3 times the general build's time."""
+    m = Model.generate(family, **kw)
+    run = dict(seed=3, tracked=[0], max_steps=200, allow_truncation=True, variant=variant, keep_samples=n <= 4000)
+    a = [m.simulate(t, n, **run) for _ in range(5)]
+    b = [m.simulate(t, n, flags=_ffi.FLAG_COMPAT_CRIT if family != "dimer" else _ffi.FLAG_COMPAT_G, **run) for _ in range(5)]
+    assert min(r.kernel_ms for r in a) <= 1.1 * min(r.kernel_ms for r in b)
+    assert np.allclose(a[0].mean, b[0].mean, rtol=0.02)
