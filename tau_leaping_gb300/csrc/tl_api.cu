@@ -58,8 +58,11 @@ struct Carver {
     }
 };
 
+// Whether halving a rate is exact: not near FP32's ends.
+static bool halves_exactly(float c) { return c == 0.f || (c >= 7.8886e-31f && c <= 1.1529e18f); }
+
 // One set's rates in FP32, as given and halved for 2S channels (the fast
-// builds).  False where halving might not be exact: near FP32's ends.
+// builds).  False where halving might not be exact.
 static bool fill_rates(const HostModel& h, const double* c, float* plain, float* halved) {
     bool exact = true;
     for (int j = 0; j < h.M; ++j) {
@@ -67,7 +70,7 @@ static bool fill_rates(const HostModel& h, const double* c, float* plain, float*
         const bool twice = h.order[(size_t)j] == 3;
         if (plain) plain[j] = cf;
         if (halved) halved[j] = twice ? 0.5f * cf : cf;
-        if (twice && cf != 0.f && !(cf >= 7.8886e-31f && cf <= 1.1529e18f)) exact = false;
+        if (twice && !halves_exactly(cf)) exact = false;
     }
     return exact;
 }
@@ -695,6 +698,10 @@ struct RunBuffers {
     float* a_all = nullptr;
 };
 
+// The rates of a call on the device: the model's own resident ones, or the
+// call's sets as given, halved for 2S channels (fast builds), or both.
+enum class RateForm { Model, Plain, Halved, Both };
+
 // One (model, configuration) pair of a call: validation, scratch layout,
 // device parameters, reduction and result.
 struct Job {
@@ -707,13 +714,15 @@ struct Job {
     bool sens = false, keep = false, plain = false, compat_stoich = false;
     int mode = kModeFast;  // the kernel build: scores and / or compatibility switches
     size_t w = 4;
-    std::vector<float> hrates;  // the call's rate sets; empty: the model's own
-    int rates_first = 0, rates_sets = 0;  // the sets of hrates that go to the device
+    // what goes to the device, the call's rate sets first, in the forms that the
+    // build reads (job_rates)
+    std::unique_ptr<unsigned char[]> hin;
+    size_t in_bytes = 0;
+    RateForm rate_form = RateForm::Model;
     bool measure = false;
     bool wide_stats = false, fixed_scratch = false;  // (the static entry's scratch holds no sums)
     size_t o_acc = 0;
     unsigned char* base = nullptr;
-    std::vector<unsigned char> hin;  // what goes to the device
     size_t o_in = 0;
     LeapScale scale;
     std::vector<double> htf;
@@ -727,6 +736,70 @@ struct Job {
     std::vector<unsigned char> hout;
     unsigned long long hc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 };
+
+// Bytes of the call's rate sets in J.hin.
+static size_t rate_bytes(const Job& J) {
+    const size_t copies = J.rate_form == RateForm::Model ? 0 : J.rate_form == RateForm::Both ? 2 : 1;
+    return al16(copies * (size_t)J.S * (size_t)J.m->h.M * 4);
+}
+// Bytes of the rest: end times, grid, tracked species, zeroed counters.
+static size_t rest_bytes(const Job& J) {
+    return al16((size_t)J.S * 8) + al16((size_t)J.S * J.P * 8) + al16((size_t)std::max(J.K, 1) * 4) + 64;
+}
+
+// n rates to FP32 times `by`, in vectors.  Returns a top bit where one may be
+// negative or not finite: every such double has its sign bit or, the lowest exponent bit added, gets it.
+static uint64_t convert_rates(const double* __restrict from, const float* __restrict by, float* __restrict to, size_t n) {
+    uint64_t any = 0;
+    for (size_t j = 0; j < n; ++j) {
+        uint64_t b;
+        memcpy(&b, from + j, 8);
+        any |= b | (b + 0x0010000000000000ull);
+        to[j] = (float)from[j] * by[j];
+    }
+    return any;
+}
+
+// The call's rate sets into J.hin in one form, checked on the way: one pass reads
+// the doubles and writes what is sent.  exact: halving is (see fill_rates).  Host time
+// of a call on GB300: 0.8 ns a rate (60 000 sets of 256 rates: 12 ms); 2.4 ns with
+// both forms made apart, zeroed and copied, 1.0 ns with one form zeroed and copied.
+static tl_status job_rates(Job& J, RateForm form, bool& exact) {
+    const HostModel& h = J.m->h;
+    const size_t M = (size_t)h.M, S = (size_t)J.S;
+    J.rate_form = form;
+    J.in_bytes = rate_bytes(J) + rest_bytes(J);
+    J.hin.reset(new unsigned char[J.in_bytes]);
+    std::vector<float> by(M, 1.f);
+    std::vector<int> twice;
+    for (size_t j = 0; j < M && form != RateForm::Plain; ++j)
+        if (h.order[j] == 3) {
+            by[j] = 0.5f;
+            twice.push_back((int)j);
+        }
+    float* const first = reinterpret_cast<float*>(J.hin.get());
+    float* const halved = form == RateForm::Both ? first + S * M : first;
+    uint64_t any = 0;
+    exact = true;
+    for (size_t s = 0; s < S; ++s) {
+        const double* const c = J.cfg->rate_sets + s * M;
+        float* const to = halved + s * M;
+        any |= convert_rates(c, by.data(), to, M);
+        for (const int j : twice) exact &= halves_exactly((float)c[j]);
+        if (form == RateForm::Both) {
+            float* const plain = first + s * M;
+            memcpy(plain, to, M * 4);
+            for (const int j : twice) plain[j] = (float)c[j];
+        }
+    }
+    if (any >> 63)  // a bad one, or -0.0
+        for (size_t q = 0; q < S * M; ++q)
+            if (!std::isfinite(J.cfg->rate_sets[q]) || J.cfg->rate_sets[q] < 0.0) {
+                set_last_error("rate constants must be finite and >= 0");
+                return TL_ERR_NUMERIC;
+            }
+    return TL_OK;
+}
 
 static tl_status job_prepare(Job& J) {
     tl_model* m = J.m;
@@ -781,20 +854,19 @@ static tl_status job_prepare(Job& J) {
     }
     J.htf.assign((size_t)J.S, cfg->t_final);
     bool halvable = true;
-    for (size_t q = 0; q < (size_t)cfg->n_rate_sets * (size_t)M; ++q)
-        if (!std::isfinite(cfg->rate_sets[q]) || cfg->rate_sets[q] < 0.0) {
-            set_last_error("rate constants must be finite and >= 0");
-            return TL_ERR_NUMERIC;
-        }
     if (cfg->n_rate_sets > 0) {
-        J.hrates.resize((size_t)2 * J.S * M);  // all sets as given, then halved for 2S channels
-        float* to = J.hrates.data();
-        for (int s = 0; s < J.S; ++s)
-            halvable &= fill_rates(h, cfg->rate_sets + (size_t)s * M, to + (size_t)s * M, to + (size_t)(J.S + s) * M);
+        // scored and measured runs may read both forms
+        const RateForm form = J.plain || J.mode == kModeGeneral        ? RateForm::Plain
+                              : J.mode == kModeScores || J.measure ? RateForm::Both
+                                                                       : RateForm::Halved;
+        const tl_status rs = job_rates(J, form, halvable);
+        if (rs != TL_OK) return rs;
     } else {
         const tl_status ds = ensure_device(m);  // the model's own rates are resident
         if (ds != TL_OK) return ds;
         halvable = m->d.halvable;
+        J.in_bytes = rest_bytes(J);
+        J.hin.reset(new unsigned char[J.in_bytes]);
     }
     // the packed criticalities are signs of x - n_c and x - 2 n_c, in int32
     if (!halvable || cfg->n_critical >= (1 << 30)) J.mode = kModeGeneral;
@@ -843,25 +915,25 @@ static void bind_plan(const tl_model* m, const Plan& pl, SimParams& p) {
 static void job_layout(Job& J, Carver& c) {
     const int M = J.m->h.M, N = J.m->h.N, K1 = std::max(J.K, 1);
     // what goes to the device in one copy: rate sets, end times, grid, tracked
-    // species and zeroed counters, which come back with the statistics.  The
-    // fast build reads only the halved rates, the general one the others.
-    J.rates_first = J.pl.mode == kModeFast && !J.plain && !J.measure ? J.S : 0;
-    J.rates_sets = J.hrates.empty() ? 0 : J.pl.mode == kModeScores || J.measure ? 2 * J.S : J.S;
+    // species and zeroed counters, which come back with the statistics.  Only
+    // a plan that fell back to the general build finds the wrong form here.
+    if (J.rate_form == RateForm::Halved && J.pl.mode == kModeGeneral) {
+        bool exact;
+        job_rates(J, RateForm::Plain, exact);
+    }
     size_t o = 0;
     const auto put = [&](size_t& at, size_t bytes) {
         at = o;
         o += al16(bytes);
     };
-    put(J.o_rates, (size_t)J.rates_sets * M * 4);
+    put(J.o_rates, rate_bytes(J));
     put(J.o_tf, (size_t)J.S * 8);
     put(J.o_grid, (size_t)J.S * J.P * 8);
     put(J.o_tr, (size_t)K1 * 4);
     put(J.o_ctr, 8 * 8);
-    const size_t in = o;
     put(J.o_mean, (size_t)J.S * J.P * K1 * 8);
     put(J.o_sd, (size_t)J.S * J.P * K1 * 8);
     const size_t at = c.take(o);
-    J.hin.resize(in);
     for (size_t* q : {&J.o_rates, &J.o_tf, &J.o_grid, &J.o_tr, &J.o_ctr, &J.o_mean, &J.o_sd}) *q += at;
     J.o_in = at;
     J.o_samp = c.take((size_t)J.total * J.P * K1 * J.w);
@@ -905,17 +977,19 @@ static tl_status job_bind(Job& J, unsigned char* B, cudaStream_t st) {
         rb.a_all = reinterpret_cast<float*>(B + J.o_aall);
     }
     const auto fill = [&](size_t at, const void* from, size_t bytes) {
-        if (bytes) memcpy(J.hin.data() + (at - J.o_in), from, bytes);
+        if (bytes) memcpy(J.hin.get() + (at - J.o_in), from, bytes);
     };
-    std::fill(J.hin.begin(), J.hin.end(), (unsigned char)0);
     const size_t M = (size_t)m->h.M;
-    fill(J.o_rates, J.hrates.data() + (size_t)J.rates_first * M * (J.rates_sets ? 1 : 0), (size_t)J.rates_sets * M * 4);
+    memset(J.hin.get() + (J.o_tf - J.o_in), 0, J.in_bytes - (J.o_tf - J.o_in));
     fill(J.o_tf, J.htf.data(), J.htf.size() * 8);
     fill(J.o_grid, J.hgrid.data(), J.hgrid.size() * 8);
     fill(J.o_tr, cfg->tracked, (size_t)J.K * 4);
-    TLC(cudaMemcpyAsync(B + J.o_in, J.hin.data(), J.hin.size(), cudaMemcpyHostToDevice, st));
-    const float* const plain = J.rates_sets ? rb.rates : m->d.rate;
-    const float* const halved = !J.rates_sets ? m->d.rate + M : J.rates_sets == J.S ? rb.rates : rb.rates + (size_t)J.S * M;
+    TLC(cudaMemcpyAsync(B + J.o_in, J.hin.get(), J.in_bytes, cudaMemcpyHostToDevice, st));
+    // (a run that reads one form finds it in both)
+    const float* const plain = J.rate_form == RateForm::Model ? m->d.rate : rb.rates;
+    const float* const halved = J.rate_form == RateForm::Model  ? m->d.rate + M
+                                : J.rate_form == RateForm::Both ? rb.rates + (size_t)J.S * M
+                                                                : rb.rates;
     SimParams& p = J.p;
     p = SimParams{};
     p.N = m->h.N;
@@ -1184,12 +1258,12 @@ static tl_status run(tl_model* m, const tl_run_cfg* cfg, tl_result* res, tl_grad
     J.cfg = cfg;
     J.res = res;
     J.grad = grad;
+    J.measure = cfg && cfg->variant == TL_VARIANT_AUTO && (cfg->flags & TL_FLAG_AUTOTUNE_MEASURE);
     tl_status ps = job_prepare(J);
     if (ps != TL_OK) return ps;
     TLC(cudaSetDevice(m->d.device));
     cudaStream_t st = (cudaStream_t)cfg->stream;
     const bool no_stage = (cfg->flags & TL_FLAG_NO_STAGE) != 0;
-    J.measure = !J.plain && cfg->variant == TL_VARIANT_AUTO && (cfg->flags & TL_FLAG_AUTOTUNE_MEASURE);
     if (!J.plain) {
         ps = make_plan(m, cfg->variant, cfg->block_threads, J.mode, J.sens, J.compat_stoich, no_stage, J.total, J.scale, J.pl,
                        (cfg->flags & TL_FLAG_GLOBAL_SLOTS) != 0);
