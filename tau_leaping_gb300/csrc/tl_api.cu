@@ -421,12 +421,46 @@ static int heuristic_variant(const tl_model* m, size_t sb, long long total, int 
     return TL_VARIANT_WARP;
 }
 
+// What a plan depends on besides the model and the launch: the leap condition's
+// eps and the time between two grid points.
+struct LeapScale {
+    double eps = 0.03, dt = 1.0;
+};
+
+// Whether most draws of a leap have means of 10 and more (PTRS), by the first
+// leap from x0: the mean of channel j is a_j times the CGP bound or dt.
+static bool mostly_long_draws(const HostModel& h, const LeapScale& ls) {
+    const int M = h.M, N = h.N;
+    std::vector<double> a((size_t)M);
+    const auto pop = [&](int i) { return (double)h.x0[(size_t)i]; };
+    for (int j = 0; j < M; ++j) {
+        const int o = h.order[(size_t)j], s0 = h.s0[(size_t)j], s1 = h.s1[(size_t)j];
+        a[(size_t)j] = h.rate[(size_t)j] * (o == 0 ? 1.0 : o == 1 ? pop(s0) : o == 2 ? pop(s0) * pop(s1) : pop(s0) * (pop(s0) - 1.0) * 0.5);
+    }
+    double tau = ls.dt;
+    for (int i = 0; i < N; ++i) {
+        if (!h.gkind[(size_t)i]) continue;
+        double mu = 0.0, s2 = 0.0;
+        for (int q = h.net_rp[(size_t)i]; q < h.net_rp[(size_t)i + 1]; ++q) {
+            const double v = unpack_v(h.net_vc[(size_t)q]), t = v * a[(size_t)unpack_idx(h.net_vc[(size_t)q])];
+            mu += t;
+            s2 += v * t;
+        }
+        const double num = std::max(ls.eps * pop(i) / (h.gkind[(size_t)i] == 1 ? 1.0 : 2.0), 1.0);
+        if (mu != 0.0) tau = std::min(tau, num / std::fabs(mu));
+        if (s2 > 0.0) tau = std::min(tau, num * num / s2);
+    }
+    int many = 0;
+    for (int j = 0; j < M; ++j) many += a[(size_t)j] * tau >= 10.0;
+    return 4 * many >= 3 * M;
+}
+
 // Thread-group plans of a model of `size` channels or species at most: lanes
 // per realization (W; 1: thread groups on shared memory, else tl_tiny.cuh), and
 // lanes of each warp that take realizations.  One realization's chain of
 // dependent steps sets the time of small and mid-sized ensembles, so W lanes
-// share its draws until the ensemble is some 56 warps per SM, more than twice
-// what is resident; past that the lanes do more as W realizations.  And the
+// share its draws until the ensemble is `most` warps per SM; past that the
+// lanes do more as W realizations.  And the
 // realizations of a warp lengthen one another's chains (they sit in different
 // steps, branches and draws), so small ensembles leave lanes idle.  Measured on
 // GB300 (ms; the last row: shared memory, four lanes, before tl_tiny.cuh):
@@ -438,13 +472,32 @@ static int heuristic_variant(const tl_model* m, size_t sb, long long total, int 
 //   shared, 32 lanes     3.08   3.11   3.12    3.45   6.94   15.9
 // and a 12 x 16 network in direct-method steps, W = 16 against 1: 1.29 against
 // 5.38 at 32, 4.67 against 6.91 at 10000, 20.0 against 8.03 at 50000.
-static void thin_plan(int size, long long total, int nsm, int& thin, int& lanes) {
+static void thin_plan(int size, long long total, int nsm, long long most, int& thin, int& lanes) {
     thin = size <= 4 ? 4 : size <= 8 ? 8 : size <= 16 ? 16 : 1;
-    if (total * thin > 56LL * 32 * nsm) thin = 1;
+    if (total * thin > most * 32 * nsm) thin = 1;
     lanes = 32;
     if (thin > 1)
         while (lanes > thin && total * 2 * thin <= (thin == 4 ? 10LL : 3LL) * nsm * lanes) lanes /= 2;
 }
+
+// `most` for an ensemble of its own.  W = 8 and 16: some 56, more than twice the
+// 24 that are resident.  W = 4: little more than one wave of them, since
+// one lane needs only 4 times the steps of four.  Dimer decay, ms, W = 4 and 1
+// (and one thread of the build before them): to t = 5e-4, 30000 realizations 0.80
+// and 0.94 (1.00), 35000 1.07 and 0.95 (1.01), 60000 1.44 and 1.17 (1.17); t = 1,
+// 30000 1.85 and 2.44 (2.74), 40000 2.67 and 2.67 (3.02), 60000 3.38 and 3.00 (3.43);
+// t = 4, 40000 3.32 and 3.54 (4.24), 60000 4.21 and 3.99 (4.85).  Not where nearly
+// every draw is long, which four lanes share well: cyclic chain of 4 species,
+// 60000 realizations of 8 steps 0.098 and 0.122 (0.141).
+static long long thin_most_warps(const HostModel& h, const LeapScale& ls) {
+    return std::max(h.N, h.M) > 4 || mostly_long_draws(h, ls) ? 56 : 28;
+}
+
+// And for a batch, whose kernel has 16 warps resident.  Sets of the dimer decay
+// alone, ms, W = 4 and 1: 48000 realizations to t = 0.01 1.83 and 2.10, t = 1 2.98 and
+// 3.58; 65536 2.56 and 2.13, 4.17 and 3.58; with scores 2.70 and 2.71, 4.34 and 4.36;
+// beside 4 x 700 toy realizations 6.63 and 6.41, 8.22 and 8.87.
+static long long thin_most_warps_batch(bool small_only, bool scores) { return small_only && !scores ? 48 : 56; }
 
 // Four-warp teams for a warp-group ensemble of up to eight realizations an SM:
 // enough channels for 128 threads, and a chain of steps that sets the time.
@@ -481,40 +534,6 @@ static int even_block(long long total, int groups_per_warp, int nsm, int most_wa
     return 32 * best;
 }
 
-// What a plan depends on besides the model and the launch: the leap condition's
-// eps and the time between two grid points.
-struct LeapScale {
-    double eps = 0.03, dt = 1.0;
-};
-
-// Whether most draws of a leap have means of 10 and more (PTRS), by the first
-// leap from x0: the mean of channel j is a_j times the CGP bound or dt.
-static bool mostly_long_draws(const HostModel& h, const LeapScale& ls) {
-    const int M = h.M, N = h.N;
-    std::vector<double> a((size_t)M);
-    const auto pop = [&](int i) { return (double)h.x0[(size_t)i]; };
-    for (int j = 0; j < M; ++j) {
-        const int o = h.order[(size_t)j], s0 = h.s0[(size_t)j], s1 = h.s1[(size_t)j];
-        a[(size_t)j] = h.rate[(size_t)j] * (o == 0 ? 1.0 : o == 1 ? pop(s0) : o == 2 ? pop(s0) * pop(s1) : pop(s0) * (pop(s0) - 1.0) * 0.5);
-    }
-    double tau = ls.dt;
-    for (int i = 0; i < N; ++i) {
-        if (!h.gkind[(size_t)i]) continue;
-        double mu = 0.0, s2 = 0.0;
-        for (int q = h.net_rp[(size_t)i]; q < h.net_rp[(size_t)i + 1]; ++q) {
-            const double v = unpack_v(h.net_vc[(size_t)q]), t = v * a[(size_t)unpack_idx(h.net_vc[(size_t)q])];
-            mu += t;
-            s2 += v * t;
-        }
-        const double num = std::max(ls.eps * pop(i) / (h.gkind[(size_t)i] == 1 ? 1.0 : 2.0), 1.0);
-        if (mu != 0.0) tau = std::min(tau, num / std::fabs(mu));
-        if (s2 > 0.0) tau = std::min(tau, num * num / s2);
-    }
-    int many = 0;
-    for (int j = 0; j < M; ++j) many += a[(size_t)j] * tau >= 10.0;
-    return 4 * many >= 3 * M;
-}
-
 // Lane groups of 2 to 16 lanes that the general build runs faster.  The fast
 // build's queue of long draws is one per group, and the groups of a warp drain
 // theirs one after another: what 32 and 16 lanes gain, 2 to 8 lose where nearly
@@ -546,7 +565,7 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
     int groups_per_block = 1;
     if (variant == TL_VARIANT_THREAD) {
         pl.kind = 1;
-        if (mode != kModeGeneral) thin_plan(std::max(m->h.N, m->h.M), total, nsm, pl.thin, pl.lanes);
+        if (mode != kModeGeneral) thin_plan(std::max(m->h.N, m->h.M), total, nsm, thin_most_warps(m->h, ls), pl.thin, pl.lanes);
         int b = block_req;
         if (b <= 0) {
             // spread small ensembles over every SM
@@ -1368,7 +1387,12 @@ static tl_status run(tl_model* m, const tl_run_cfg* cfg, tl_result* res, tl_grad
 // -> 15.0; toy 700 20.4 -> 17.6 -> 18.8, 1500 32.9 -> 30.7 -> 31.5; both, 4096
 // and 700, 22.4 -> 19.6 -> 23.0; 64 x 4096 and 16 x 1024 to t = 10 and 0.1,
 // 1501 -> 1247 -> 1371.
-static int batch_minb(long long units, int warps, int nsm) {
+// Batches of small items on one lane each alone run best at four (64 registers)
+// where three do not hold them at once: dimer sets, ms at 2 -> 4, 16 x 8192 realizations to t = 0.01 4.15 -> 3.65, t = 1 6.94 ->
+// 6.04, with scores 5.47 -> 4.80 and 8.75 -> 7.46; 64 x 4096 to t = 1 11.1 -> 10.1 and
+// 14.0 -> 12.7.
+static int batch_minb(long long units, int warps, int nsm, bool thin_only) {
+    if (thin_only && units > 3LL * warps * nsm) return TL_BATCH_THIN_MINB;
     return units > 2LL * warps * nsm ? TL_BATCH_MANY_MINB : TL_BATCH_MINB;
 }
 
@@ -1412,6 +1436,7 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     size_t wslot = 0;
     int bmode = kModeFast;  // the build every item can run on
     long long lane_total = 0;
+    bool small_only = true;  // every item runs as lane units
     int lane_size = 1;  // channels or species of the largest thread-group item
     for (int i = 0; i < n; ++i) {
         Job& J = jobs[(size_t)i];
@@ -1419,6 +1444,7 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
         bmode = std::max(bmode, J.mode);
         if (!m->d.fast_ok || m->d.chan8 || m->d.ent_wide) bmode = kModeGeneral;
         lane[(size_t)i] = (m->h.M <= 16 && m->h.N <= 16) ? 1 : 0;
+        small_only &= lane[(size_t)i] != 0;
         if (lane[(size_t)i]) {
             lane_total += J.total;
             lane_size = std::max(lane_size, std::max(m->h.M, m->h.N));
@@ -1429,7 +1455,8 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     for (;;) {
         thin = 1;
         unit_lanes = 32;
-        if (bmode != kModeGeneral) thin_plan(lane_size <= 4 ? 4 : 16, lane_total, sm_count(), thin, unit_lanes);
+        if (bmode != kModeGeneral) thin_plan(lane_size <= 4 ? 4 : 16, lane_total, sm_count(),
+                                             thin_most_warps_batch(small_only, bmode == kModeScores), thin, unit_lanes);
         wslot = 0;
         for (int i = 0; i < n; ++i) {
             Job& J = jobs[(size_t)i];
@@ -1558,7 +1585,7 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
     bp.params_bytes = (int)spb;
     bp.wctr = reinterpret_cast<unsigned long long*>(B + o_wctr);
     round_keys(jobs[0].p.k0, jobs[0].p.k1, bp.rk);
-    const int minb = batch_minb(units, warps, sm_count());
+    const int minb = batch_minb(units, warps, sm_count(), small_only && thin == 1 && staged && bmode != kModeGeneral);
     const size_t smem = team ? team_smem : stage + (size_t)warps * (wslot + spb);
     int bps = team_bps;
     cudaError_t le = team ? cudaSuccess : pop == 64 ? batch_occupancy<long long>(bmode, staged, minb, thin, 32 * warps, smem, &bps)

@@ -55,6 +55,9 @@ constexpr int kModeFast = 0, kModeScores = 1, kModeGeneral = 2;
 #ifndef TL_BATCH_MANY_MINB
 #define TL_BATCH_MANY_MINB 3
 #endif
+#ifndef TL_BATCH_THIN_MINB
+#define TL_BATCH_THIN_MINB 4
+#endif
 // staged: the tables are staged in shared memory.
 template <class Pop>
 cudaError_t launch_fused(const SimParams& p, int kind, int mode, bool staged, int block, int grid, size_t smem,
