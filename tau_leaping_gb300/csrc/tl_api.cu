@@ -322,7 +322,7 @@ struct SlotLayout {
     bool score_global = false;
 };
 
-static SlotLayout slot_layout(const tl_model* m, bool sens, int mode, int kind, int block) {
+static SlotLayout slot_layout(const tl_model* m, bool sens, int mode, int kind, int block, int most_rounds = 7) {
     SlotLayout L;
     const int N = m->h.N, M = m->h.M;
     if (mode == kModeGeneral) {
@@ -334,7 +334,7 @@ static SlotLayout slot_layout(const tl_model* m, bool sens, int mode, int kind, 
     if (kind != 1) {
         const int lanes = kind ? kind : block;
         const int turns = (M + 4 * lanes - 1) / (4 * lanes);
-        L.q_rounds = std::min(turns, lanes > 256 ? 4 : 7);
+        L.q_rounds = std::min({turns, lanes > 256 ? 4 : 7, most_rounds});
         q_bytes = (size_t)L.q_rounds * lanes * 4 * 2 + 4 * (size_t)(kind ? 1 : block / 32);  // and a counter each
     }
     const size_t Np = ((size_t)N + 3) & ~(size_t)3;  // whole blocks of four species
@@ -610,6 +610,12 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
             pl.block -= 32;
             groups_per_block = pl.block / pl.kind;
         }
+        // a CTA's queue is drained more often where that makes its slot fit (ms,
+        // general build -> so: colloid of 312 species 0.423 -> 0.258, of 328 0.464 -> 0.333)
+        for (int r = pl.slot.q_rounds - 1; r > 0 && pl.kind == 0 && !pl.gslot && pl.slot.bytes > (size_t)smax; --r) {
+            const SlotLayout less = slot_layout(m, sens, mode_, pl.kind, pl.block, r);
+            if (less.bytes <= (size_t)smax) pl.slot = less;
+        }
         return (size_t)groups_per_block * pl.slot.bytes <= (size_t)smax;
     };
     pl.gslot = force_gslot && pl.kind == 0;
@@ -620,8 +626,12 @@ static tl_status make_plan(const tl_model* m, int variant, int block_req, int mo
     if (!packed || (mode == kModeScores && (pl.gslot || sub))) mode = kModeGeneral;
     if (mode == kModeFast && sub && general_is_faster(m->h, pl.kind, ls)) mode = kModeGeneral;
     if (!fit(mode) && !pl.gslot) {
-        // the general build's slot is smaller for wide models
-        if (mode == kModeGeneral || !fit(kModeGeneral)) {
+        // The general build's slot is smaller for wide models.  A CTA's propensities
+        // go to global memory instead where the state stays in shared memory,
+        // ms on GB300, general -> so: colloid of 332 species 0.472 -> 0.356 (152
+        // realizations), chain of 15000 species 0.469 -> 0.370, 6000 x 40000 network 19.0 -> 10.7
+        const bool big_only = mode == kModeFast && pl.kind == 0 && pl.slot.state <= (size_t)smax;
+        if (mode == kModeGeneral || big_only || !fit(kModeGeneral)) {
             if (pl.kind != 0) {
                 set_last_error("model too large for the shared-memory slot of this variant");
                 return TL_ERR_UNSUPPORTED;
@@ -2119,8 +2129,8 @@ extern "C" tl_status tl_simulate_static(tl_model* m, const tl_run_cfg* cfg, tl_r
     if (ps != TL_OK) return ps;
     Carver c;
     job_layout(J, c);
-    if (c.off > (size_t)TL_STATIC_SCRATCH_BYTES && J.pl.state_global) {
-        // the general build's global slots are smaller
+    if (c.off > (size_t)TL_STATIC_SCRATCH_BYTES && J.pl.gslot && J.pl.mode != kModeGeneral) {
+        // the general build's slots are smaller and may fit shared memory
         ps = make_plan(m, cfg->variant, cfg->block_threads, kModeGeneral, J.sens, J.compat_stoich,
                        (cfg->flags & TL_FLAG_NO_STAGE) != 0, J.total, J.scale, J.pl, (cfg->flags & TL_FLAG_GLOBAL_SLOTS) != 0);
         if (ps != TL_OK) return ps;

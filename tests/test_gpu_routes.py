@@ -175,3 +175,22 @@ def test_batches_of_small_items_on_one_lane_each(n_items, n):
         out = simulate_batch([dict(model=m, t_final=0.002, n=n, seed=9, tracked=[0, 1], rate_sets=rs, sensitivity=sens)])[0]
         one = m.simulate(0.002, n, seed=9, tracked=[0, 1], rate_sets=rs)
         assert np.array_equal(out["mean"], one.mean) and out["leaps"] == one.leaps
+
+
+@pytest.mark.parametrize("N", [312, 320, 328, 332])
+@pytest.mark.parametrize("bits", [32, 64])
+def test_wide_models_at_the_edge_of_shared_memory(N, bits):
+    """48 672 to 55 112 channels: a queue of fewer turns, then the propensities
+    in global memory; the same realizations as with all of it there, from the
+    static entry as well, which has no room for those slots.  At 0.6 to 0.75 of the
+    general build's time, which these models had fallen back to."""
+    m = Model.generate("colloid", n_species=N, pop_bits=bits)
+    kw = dict(t_final=0.002, n=200, seed=3, tracked=[0, 1, N - 1])
+    a = m.simulate(keep_samples=True, **kw)
+    b = m.simulate(keep_samples=True, flags=_ffi.FLAG_GLOBAL_SLOTS, variant=_ffi.VARIANT_CTA, **kw)
+    assert np.array_equal(a.samples, b.samples) and a.leaps + a.ssa_steps == b.leaps + b.ssa_steps > 0
+    s = m.simulate_static(**kw)
+    assert np.array_equal(s.mean, a.mean) and (s.leaps, s.ssa_steps) == (a.leaps, a.ssa_steps)
+    # the general build in the same launch: populations far from critical, so the same trajectories
+    t, u = (min(m.simulate(flags=f, **dict(kw, n=152, tracked=[0])).kernel_ms for _ in range(5)) for f in (0, _ffi.FLAG_COMPAT_CRIT))
+    assert t <= 0.9 * u, (t, u)
