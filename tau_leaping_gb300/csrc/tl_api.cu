@@ -90,19 +90,19 @@ static bool fill_rates(const HostModel& h, const double* c, float* plain, float*
 //        firing pass may mark a channel of the padding, which has no entries)
 //  sp    per species the index in X of its |x - 1|, 0 if it has none
 //  tiny  a TinyTable, for models of up to 16 channels and species
-void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned char>& out) {
+static void fast_layout(const HostModel& h, DevModel& d) {
     const int N = h.N, M = h.M;
-    std::vector<int> x2((size_t)N, 0);
+    d.x2.assign((size_t)N, 0);
     d.n_2s = 0;
     for (int j = 0; j < M; ++j)
-        if (h.order[(size_t)j] == 3 && !x2[(size_t)h.s0[(size_t)j]]) {
-            x2[(size_t)h.s0[(size_t)j]] = 1;
+        if (h.order[(size_t)j] == 3 && !d.x2[(size_t)h.s0[(size_t)j]]) {
+            d.x2[(size_t)h.s0[(size_t)j]] = 1;
             ++d.n_2s;
         }
     const int Np = (N + 3) & ~3;  // X pads the species to whole blocks of four
     int next = Np;
     for (int i = 0; i < N; ++i)
-        if (x2[(size_t)i]) x2[(size_t)i] = next++;
+        if (d.x2[(size_t)i]) d.x2[(size_t)i] = next++;
     const int one = Np + d.n_2s;
     const int pad = (M + 3) & ~3;  // the zero block behind a[]
     d.chan8 = (size_t)one * 4 > 0xffff;
@@ -139,6 +139,16 @@ void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned char>& ou
     d.t_tiny = tiny ? sect(sizeof(TinyTable)) : 0;
     if (off >= (1u << 31)) return;
     d.f_stage_bytes = (int)std::max<size_t>(off, 16);
+    d.fast_ok = true;
+}
+
+void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned char>& out) {
+    if (!d.fast_ok) fast_layout(h, d);
+    if (!d.fast_ok) return;
+    const int N = h.N, M = h.M;
+    const std::vector<int>& x2 = d.x2;
+    const int one = ((N + 3) & ~3) + d.n_2s, pad = (M + 3) & ~3;
+    const bool tiny = N <= 16 && M <= 16;
     out.assign((size_t)d.f_stage_bytes, 0);
     uint32_t* chan = reinterpret_cast<uint32_t*>(out.data() + d.t_chan);
     for (int j = 0; j < M; ++j) {
@@ -154,33 +164,41 @@ void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned char>& ou
     }
     uint32_t* row = reinterpret_cast<uint32_t*>(out.data() + d.t_row);
     uint32_t* ent = reinterpret_cast<uint32_t*>(out.data() + d.t_ent);
+    // a packed entry's low bits (v + 2) & 7 -> the stoichiometry's FP32 bits >> 20, and its 12 bits
+    uint32_t vf[8], vi[8];
+    for (int b = 0; b < 8; ++b) {
+        const float f = (float)unpack_v(b);
+        memcpy(&vf[b], &f, 4);
+        vf[b] >>= 20;
+        vi[b] = (uint32_t)unpack_v(b) & 0xfffu;
+    }
     size_t e = 0;
     int nr = 0;
     for (int ii = 0; ii < N; ++ii) {
         const int i = h.rowperm[(size_t)ii];
         if (!h.gkind[(size_t)i]) continue;
-        const int q0 = h.net_rp[(size_t)i], q1 = h.net_rp[(size_t)i + 1], n = (q1 - q0 + 3) / 4;
-        row[2 * nr] = (uint32_t)(e / 4) | (uint32_t)n << 20;
+        const int q0 = h.net_rp[(size_t)i], n = h.net_rp[(size_t)i + 1] - q0, chunks = (n + 3) / 4;
+        const int32_t* const vc = h.net_vc.data() + q0;
+        row[2 * nr] = (uint32_t)(e / 4) | (uint32_t)chunks << 20;
         row[2 * nr + 1] = (uint32_t)i | (uint32_t)h.gkind[(size_t)i] << 28;
         ++nr;
-        for (int q = q0; q < q0 + 4 * n; ++q) {
-            const int c = q < q1 ? unpack_idx(h.net_vc[(size_t)q]) : pad, v = q < q1 ? unpack_v(h.net_vc[(size_t)q]) : 0;
-            const float vf = (float)v;
-            uint32_t vb;
-            memcpy(&vb, &vf, 4);
-            ent[e++] = d.ent_wide ? (uint32_t)c << 3 | (uint32_t)((v + 2) & 7) : (uint32_t)c << 14 | vb >> 20;
-        }
+        uint32_t* const to = ent + e;
+        if (d.ent_wide)
+            for (int q = 0; q < n; ++q) to[q] = (uint32_t)vc[q];
+        else
+            for (int q = 0; q < n; ++q) to[q] = (uint32_t)(vc[q] >> 3) << 14 | vf[vc[q] & 7];
+        for (int q = n; q < 4 * chunks; ++q) to[q] = d.ent_wide ? (uint32_t)pad << 3 | 2u : (uint32_t)pad << 14;
+        e += 4 * (size_t)chunks;
     }
     uint32_t* col = reinterpret_cast<uint32_t*>(out.data() + d.t_col);
     uint32_t* cp = d.t_cp >= 0 ? reinterpret_cast<uint32_t*>(out.data() + d.t_cp) : nullptr;
     size_t c4 = 0;
+    const int32_t* const rv = h.net_rv.data();
     for (int j = 0; j < M; ++j) {
-        const int q0 = h.net_cp[(size_t)j], q1 = h.net_cp[(size_t)j + 1];
+        const int q0 = h.net_cp[(size_t)j], n = h.net_cp[(size_t)j + 1] - q0;
         if (cp) cp[j] = (uint32_t)c4;
-        for (int q = q0; q < q1; ++q)
-            col[4 * c4 + (size_t)(q - q0)] = (uint32_t)unpack_idx(h.net_rv[(size_t)q]) << 14 |
-                                            ((uint32_t)unpack_v(h.net_rv[(size_t)q]) & 0xfffu);
-        c4 += cp ? (size_t)(q1 - q0 + 3) / 4 : 1;
+        for (int q = 0; q < n; ++q) col[4 * c4 + (size_t)q] = (uint32_t)(rv[q0 + q] >> 3) << 14 | vi[rv[q0 + q] & 7];
+        c4 += cp ? (size_t)(n + 3) / 4 : 1;
     }
     if (cp) std::fill(cp + M, cp + pad + 1, (uint32_t)c4);
     unsigned short* sp = reinterpret_cast<unsigned short*>(out.data() + d.t_sp);
@@ -194,57 +212,81 @@ void fast_tables(const HostModel& h, DevModel& d, std::vector<unsigned char>& ou
         }
         for (int i = 0; i < N; ++i) tt->gkind[i] = (uint8_t)h.gkind[(size_t)i];
     }
-    d.fast_ok = true;
 }
 
-static tl_status upload(tl_model* m) {
-    HostModel& h = m->h;
-    DevModel& d = m->d;
-    const int N = h.N, M = h.M;
+// Tables of the general build and the parity entry points:
+// [chan][ref order][gkind][perm][net rp][net vc][net cp][net rv] | [raw rp][raw vc]
+static void general_layout(const HostModel& h, DevModel& d) {
+    const size_t N = (size_t)h.N, M = (size_t)h.M;
     d.nnz_net = (int)h.net_vc.size();
     d.nnz_raw = (int)h.raw_vc.size();
-    // blob: [chan][ref order][gkind][perm][net rp][net vc][net cp][net rv] | [raw rp][raw vc]
     size_t off = 0;
     auto sect = [&](size_t bytes) {
         const size_t o = off;
         off += al16(bytes);
         return (int)o;
     };
-    d.off_chan = sect((size_t)M * 8);
-    d.off_rord = sect((size_t)M);
-    d.off_gkind = sect((size_t)N);
-    d.off_perm = sect((size_t)N * 4);
-    d.off_rp = sect((size_t)(N + 1) * 4);
+    d.off_chan = sect(M * 8);
+    d.off_rord = sect(M);
+    d.off_gkind = sect(N);
+    d.off_perm = sect(N * 4);
+    d.off_rp = sect((N + 1) * 4);
     d.off_vc = sect((size_t)d.nnz_net * 4);
-    d.off_cp = sect((size_t)(M + 1) * 4);
+    d.off_cp = sect((M + 1) * 4);
     d.off_rv = sect((size_t)d.nnz_net * 4);
     d.stage_bytes = (int)off;
-    d.off_raw_rp = sect((size_t)(N + 1) * 4);
+    d.off_raw_rp = sect((N + 1) * 4);
     d.off_raw_vc = sect((size_t)d.nnz_raw * 4);
     d.blob_bytes = off;
-    std::vector<unsigned char> hb(off, 0);
+}
+
+static void general_tables(const HostModel& h, const DevModel& d, std::vector<unsigned char>& hb) {
+    const size_t N = (size_t)h.N, M = (size_t)h.M;
+    hb.assign(d.blob_bytes, 0);
     // channel record: {s0, s1 | order << 28} (species indices < 2^28)
     int2* chan = reinterpret_cast<int2*>(hb.data() + d.off_chan);
-    for (int j = 0; j < M; ++j)
-        chan[j] = make_int2(h.s0[(size_t)j], h.s1[(size_t)j] | ((int)h.order[(size_t)j] << 28));
-    memcpy(hb.data() + d.off_rord, h.ref_order.data(), (size_t)M);
-    memcpy(hb.data() + d.off_gkind, h.gkind.data(), (size_t)N);
-    memcpy(hb.data() + d.off_perm, h.rowperm.data(), (size_t)N * 4);
-    memcpy(hb.data() + d.off_rp, h.net_rp.data(), (size_t)(N + 1) * 4);
+    for (size_t j = 0; j < M; ++j) chan[j] = make_int2(h.s0[j], h.s1[j] | ((int)h.order[j] << 28));
+    memcpy(hb.data() + d.off_rord, h.ref_order.data(), M);
+    memcpy(hb.data() + d.off_gkind, h.gkind.data(), N);
+    memcpy(hb.data() + d.off_perm, h.rowperm.data(), N * 4);
+    memcpy(hb.data() + d.off_rp, h.net_rp.data(), (N + 1) * 4);
     if (d.nnz_net) memcpy(hb.data() + d.off_vc, h.net_vc.data(), (size_t)d.nnz_net * 4);
-    memcpy(hb.data() + d.off_cp, h.net_cp.data(), (size_t)(M + 1) * 4);
+    memcpy(hb.data() + d.off_cp, h.net_cp.data(), (M + 1) * 4);
     if (d.nnz_net) memcpy(hb.data() + d.off_rv, h.net_rv.data(), (size_t)d.nnz_net * 4);
-    memcpy(hb.data() + d.off_raw_rp, h.raw_rp.data(), (size_t)(N + 1) * 4);
+    memcpy(hb.data() + d.off_raw_rp, h.raw_rp.data(), (N + 1) * 4);
     if (d.nnz_raw) memcpy(hb.data() + d.off_raw_vc, h.raw_vc.data(), (size_t)d.nnz_raw * 4);
-    // both table sets in one allocation and one copy
-    std::vector<unsigned char> fb;
-    fast_tables(h, d, fb);
-    const size_t f_off = off;
-    hb.resize(off + fb.size());
-    if (!fb.empty()) memcpy(hb.data() + f_off, fb.data(), fb.size());
-    TLC(cudaMalloc(&d.blob, hb.size()));
-    d.fblob = d.blob + f_off;
-    TLC(cudaMemcpy(d.blob, hb.data(), hb.size(), cudaMemcpyHostToDevice));
+}
+
+// The tables that a launch reads, on the device: each set is built and sent when
+// the first such launch comes.  The memory of both is there from the first
+// call on (upload), so the static entry allocates nothing here either.  First
+// call of a model on GB300, ms, both sets at once -> so (and the general one
+// alone, before there were two): colloid of 400 species, simulate 1.82 -> 1.04
+// (0.88), on the general build 1.83 -> 0.90 (0.88), replay 2.09 -> 1.08 (0.97).
+static tl_status ensure_tables(tl_model* m, bool general, bool fast, cudaStream_t st) {
+    DevModel& d = m->d;
+    for (const bool f : {false, true}) {
+        bool& sent = f ? d.fast_sent : d.general_sent;
+        if (sent || !(f ? fast && d.fast_ok : general)) continue;
+        std::vector<unsigned char> hb;
+        if (f) fast_tables(m->h, d, hb);
+        else general_tables(m->h, d, hb);
+        TLC(cudaMemcpyAsync(f ? d.fblob : d.blob, hb.data(), hb.size(), cudaMemcpyHostToDevice, st));
+        TLC(cudaStreamSynchronize(st));  // hb ends here
+        sent = true;
+    }
+    return TL_OK;
+}
+
+// The device memory of a model, its populations and rates.
+static tl_status upload(tl_model* m) {
+    HostModel& h = m->h;
+    DevModel& d = m->d;
+    const int N = h.N, M = h.M;
+    general_layout(h, d);
+    fast_layout(h, d);
+    TLC(cudaMalloc(&d.blob, d.blob_bytes + (d.fast_ok ? (size_t)d.f_stage_bytes : 0)));
+    d.fblob = d.blob + d.blob_bytes;
     const size_t w = h.pop_bits == 64 ? 8 : 4;
     TLC(cudaMalloc(&d.x0, (size_t)N * w));
     if (w == 8) {
@@ -1013,6 +1055,9 @@ static tl_status job_bind(Job& J, unsigned char* B, cudaStream_t st) {
     fill(J.o_tf, J.htf.data(), J.htf.size() * 8);
     fill(J.o_grid, J.hgrid.data(), J.hgrid.size() * 8);
     fill(J.o_tr, cfg->tracked, (size_t)J.K * 4);
+    const bool general = J.plain || J.pl.mode == kModeGeneral;
+    const tl_status ts = ensure_tables(m, general || J.measure, !general || J.measure, st);
+    if (ts != TL_OK) return ts;
     TLC(cudaMemcpyAsync(B + J.o_in, J.hin.get(), J.in_bytes, cudaMemcpyHostToDevice, st));
     // (a run that reads one form finds it in both)
     const float* const plain = J.rate_form == RateForm::Model ? m->d.rate : rb.rates;
@@ -1895,6 +1940,7 @@ tl_status tl_eval_leap(tl_model* m, const int64_t* x, int32_t n, double eps, uin
     const int N = h.N, M = h.M;
     {
         tl_status ds = ensure_device(m);
+        if (ds == TL_OK) ds = ensure_tables(m, true, false, 0);
         if (ds != TL_OK) return ds;
     }
     TLC(cudaSetDevice(m->d.device));
@@ -1952,6 +1998,7 @@ tl_status tl_replay(tl_model* m, const int64_t* x0, const int32_t* k, int32_t n_
         }
     {
         tl_status ds = ensure_device(m);
+        if (ds == TL_OK) ds = ensure_tables(m, true, false, 0);
         if (ds != TL_OK) return ds;
     }
     TLC(cudaSetDevice(m->d.device));

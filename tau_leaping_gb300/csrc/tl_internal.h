@@ -63,7 +63,8 @@ void set_last_error(const std::string& s);
 // ---------------------------------------------------------------------------
 struct DevModel {
     int device = 0;
-    unsigned char* blob = nullptr;  // staged constants (net) followed by raw CSR
+    unsigned char* blob = nullptr;  // tables of the general build, then those of the fast builds
+    bool general_sent = false, fast_sent = false;  // which of them are there
     size_t blob_bytes = 0;
     int stage_bytes = 0;            // bytes of the net part (what a CTA stages)
     int off_chan = 0, off_rord = 0, off_gkind = 0, off_perm = 0, off_rp = 0, off_vc = 0, off_cp = 0, off_rv = 0;
@@ -74,6 +75,7 @@ struct DevModel {
     int t_chan = 0, t_row = 0, t_ent = 0, t_col = 0, t_cp = -1, t_sp = 0, t_tiny = 0;
     int n_rows = 0;                 // species that react: rows of the step bound
     int n_2s = 0;                   // species of 2S channels
+    std::vector<int> x2;            // per species the index in X of its |x - 1|, 0 if it has none
     bool chan8 = false, ent_wide = false;
     bool fast_ok = false;           // the model fits the packed fields
     void* x0 = nullptr;             // Pop[N]
