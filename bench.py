@@ -198,6 +198,13 @@ def ncu_record(kernel_tag: str):
     return rec, "ncu capture of this kernel build"
 
 
+def kernel_of(r, R: int) -> str:
+    """The persistent kernel of a default launch of R realizations, from the
+    plan that ran: thread groups are k_tiny on four lanes a realization and
+    more, k_fast on one."""
+    return "k_tiny" if r.variant == 1 and r.grid * r.block_threads >= 4 * R else "k_fast"
+
+
 def alg_bytes_per_step(m) -> int:
     """Algorithmic bytes one realization-step moves: the model stream (packed
     CSR, CSC, per-channel constants c/order/s0/s1, row pointers) plus the
@@ -316,7 +323,7 @@ def run_ours(args, wl, rank, world, local_rank):
     hbm_alg = cbytes + R * (1 + 1) * len(tracked) * w
     pk = peaks()
     ops = ops_per_step(m.n_species, m.n_channels, m.nnz_net)
-    kernel = "k_tiny" if args.workload == "dimer" else "k_fast"  # models of up to 16 channels: k_tiny
+    kernel = kernel_of(r0, R)
     rec, rec_src = ncu_record(f"{kernel}_{args.workload}") if args.variant == 0 and not args.t_final and \
         not args.realizations else (None, "ncu record covers the default launch only")
     line = {
