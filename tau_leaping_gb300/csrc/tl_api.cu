@@ -12,6 +12,7 @@
 #include "tl_device.cuh"
 #include "tl_internal.h"
 #include "tl_launch.h"
+#include "tl_shared.h"
 
 namespace tl {
 
@@ -364,7 +365,7 @@ struct SlotLayout {
     bool score_global = false;
 };
 
-static SlotLayout slot_layout(const tl_model* m, bool sens, int mode, int kind, int block, int most_rounds = 7) {
+static SlotLayout slot_layout(const tl_model* m, bool sens, int mode, int kind, int block, int most_rounds = kMaxRounds) {
     SlotLayout L;
     const int N = m->h.N, M = m->h.M;
     if (mode == kModeGeneral) {
@@ -376,7 +377,7 @@ static SlotLayout slot_layout(const tl_model* m, bool sens, int mode, int kind, 
     if (kind != 1) {
         const int lanes = kind ? kind : block;
         const int turns = (M + 4 * lanes - 1) / (4 * lanes);
-        L.q_rounds = std::min({turns, lanes > 256 ? 4 : 7, most_rounds});
+        L.q_rounds = std::min({turns, lanes > 256 ? 4 : kMaxRounds, most_rounds});
         q_bytes = (size_t)L.q_rounds * lanes * 4 * 2 + 4 * (size_t)(kind ? 1 : block / 32);  // and a counter each
     }
     const size_t Np = ((size_t)N + 3) & ~(size_t)3;  // whole blocks of four species
@@ -1127,7 +1128,7 @@ static tl_status job_reduce(Job& J, cudaStream_t st) {
     cudaError_t le;
     if (J.K > 0) {
         le = J.wide_stats
-                 ? launch_stats_wide(rb.samples, J.R, J.P * J.K, J.S, J.base + J.o_acc, rb.mean, rb.sd, st)
+                 ? launch_stats_wide(rb.samples, J.R, J.P * J.K, J.S, J.base + J.o_acc, rb.mean, rb.sd, sm_count(), st)
              : J.w == 8 ? launch_stats<long long>(rb.samples, J.R, J.P, J.K, J.S, rb.mean, rb.sd, st)
                       : launch_stats<int>(rb.samples, J.R, J.P, J.K, J.S, rb.mean, rb.sd, st);
         if (le != cudaSuccess) return cuda_fail(le, "statistics launch");

@@ -242,7 +242,6 @@ __global__ void __launch_bounds__(KIND == 0 ? 1024 : 256, KIND == 0 ? 1 : KIND =
 template <int KIND>
 struct FastGroupOf {
     using type = typename GroupOf<KIND>::type;
-    static constexpr int kPerWarp = KIND == 0 ? 0 : 32 / KIND;
     static TL_D type make(double* red) { return GroupOf<KIND>::make(red); }
     static TL_D int index(const SimParams&) { return GroupOf<KIND>::index(); }
     static TL_D bool idle(const SimParams&) { return false; }

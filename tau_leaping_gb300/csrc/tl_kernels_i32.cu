@@ -15,13 +15,13 @@ cudaError_t launch_plain_tally(const SimParams& p, cudaStream_t st) {
 }
 
 cudaError_t launch_stats_wide(const void* samp, long long R, int PK, int S, void* acc, double* mean, double* sd,
-                              cudaStream_t st) {
+                              int sms, cudaStream_t st) {
     const size_t cols = (size_t)S * PK;
     cudaError_t e = cudaMemsetAsync(acc, 0, cols * 24, st);
     if (e != cudaSuccess) return e;
     // about eight CTAs an SM over the rows, 32 rows a CTA at least
     const int tiles = (PK + 31) / 32;
-    const long long want = (152LL * 8 + (long long)tiles * S - 1) / ((long long)tiles * S);
+    const long long want = (8LL * sms + (long long)tiles * S - 1) / ((long long)tiles * S);
     const int split = (int)std::max<long long>(1, std::min<long long>(std::min<long long>(want, (R + 31) / 32), 65535));
     k_stats_wide<<<dim3((unsigned)tiles, (unsigned)split, (unsigned)S), 256, 0, st>>>(
         reinterpret_cast<const int*>(samp), R, PK, reinterpret_cast<unsigned long long*>(acc));

@@ -103,7 +103,7 @@ cudaError_t launch_stats(const void* samp, long long R, int P, int K, int S, dou
                          cudaStream_t st);
 // the same for many columns of 32-bit populations; acc: 24 bytes a column
 cudaError_t launch_stats_wide(const void* samp, long long R, int PK, int S, void* acc, double* mean, double* sd,
-                              cudaStream_t st);
+                              int sms, cudaStream_t st);
 template <class Pop>
 cudaError_t launch_grad(const void* samp, const float* scores, long long R, int P, int K, int M, int S,
                         double* grad, double* se, double* meanf, cudaStream_t st);

@@ -11,6 +11,11 @@
 
 namespace tl {
 
+// Turns of four channels a lane that a queue group may mark before its queue is
+// drained: four bits each in a lane's 32-bit masks, and a warp's marks counted in ten bits.
+constexpr int kMaxRounds = 7;
+static_assert(4 * kMaxRounds <= 32 && 4 * 32 * kMaxRounds < 1 << 10, "masks and counts of the firing pass");
+
 // The Philox step counter wraps at 2^32; epochs counts that, so that caps and
 // counts of steps hold past it.  The counter's words repeat from there on.
 TL_SHARED void next_step(uint32_t& step, uint32_t& epochs) {

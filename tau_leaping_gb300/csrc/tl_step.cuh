@@ -512,7 +512,6 @@ __device__ __noinline__ void undo_leap(const Grp g, const SimParams& p, const La
 // padding holds 0 and has no entries.  Its mean of 0 lies within the margin where
 // the word is below 5e-6 of its range, so it can be marked; it is dropped there.
 constexpr float kFireMargin = 5e-6f;
-constexpr int kMaxRounds = 7;  // marked channels of a queue group fit ten bits
 
 // One attempt of a queued draw of mean < 10 (poisson_first).  Attempt 0 is on
 // the shared word w: k <= 1 by the exact tests unless k >= 2 is settled, else
