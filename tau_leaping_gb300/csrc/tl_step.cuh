@@ -510,7 +510,8 @@ __device__ __noinline__ void undo_leap(const Grp g, const SimParams& p, const La
 //    attempt instead of waiting for the warp's last one.
 // a[], k[] and the columns are padded to whole blocks of four channels: the
 // padding holds 0 and has no entries.  Its mean of 0 lies within the margin where
-// the word is below 5e-6 of its range, so it can be marked; it is dropped there.
+// the word is below 5e-6 of its range, so it can be marked: its draw is 0 firings of no
+// entries.  (A test for it in the queue's loop cost the 45 x 83 network 1.5 %.)
 constexpr float kFireMargin = 5e-6f;
 
 // One attempt of a queued draw of mean < 10 (poisson_first).  Attempt 0 is on
@@ -643,7 +644,6 @@ TL_D void fast_fire(const Grp& g, const SimParams& p, const Lay& L, float tauf, 
             const int j = channel(q[i]);
             int k = 1;
             if (i < n_inv) {
-                if (j >= p.M) continue;
                 const float mu = fmaxf(a[j], 0.f) * tauf;
                 U4 w = group_words(L.rk, (uint32_t)j >> 2, step, r, set);
                 uint32_t word = word_of(w, j & 3);
