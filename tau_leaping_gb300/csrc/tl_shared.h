@@ -21,6 +21,8 @@ static_assert(4 * kMaxRounds <= 32 && 4 * 32 * kMaxRounds < 1 << 10, "masks and 
 TL_SHARED void next_step(uint32_t& step, uint32_t& epochs) {
     if (++step == 0u) ++epochs;
 }
+// The same after `steps` of them, where epochs is of before them.
+TL_SHARED uint32_t wrapped(uint32_t step, int steps) { return step < (uint32_t)steps ? 1u : 0u; }
 // Accepted steps: attempts and direct-method steps less the rejected attempts.
 TL_SHARED long long accepted(uint32_t epochs, uint32_t step, uint32_t rej) {
     return (long long)((unsigned long long)epochs << 32 | step) - (long long)rej;

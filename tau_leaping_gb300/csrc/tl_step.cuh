@@ -996,7 +996,7 @@ struct FastState {
     int kpt;        // next grid point to record
     uint32_t step;
     uint32_t rej, ssa;
-    uint32_t epochs;   // wraps of step
+    uint32_t epochs;   // wraps of step before this leap or block
     uint32_t ex_from;  // the lanes hold the critical waiting times (unit rate) of the steps from here
     float ex;
     bool wide;     // the next step is a wide leap
@@ -1110,9 +1110,10 @@ TL_D void direct_steps_lanes(const GWarp& g, const SimParams& p, const Lay& L, i
             x = add_pop(x, d);
         }
         st.t = t_new;
-        next_step(st.step, st.epochs);
+        st.step++;
         st.ssa++;
-        if (++q == p.ssa_block || (p.max_steps > 0 && accepted(st.epochs, st.step, st.rej) >= p.max_steps)) break;
+        ++q;
+        if (q == p.ssa_block || (p.max_steps > 0 && accepted(st.epochs + wrapped(st.step, q), st.step, st.rej) >= p.max_steps)) break;
         // propensities: products of |x|, as everywhere (a channel that lists a
         // species twice can take it below zero)
         const float f = fabsf(popf(x));
@@ -1209,9 +1210,10 @@ TL_D void direct_steps(const Grp& g, const SimParams& p, const Lay& L, int set, 
         }
         g.sync();
         st.t = t_new;
-        next_step(st.step, st.epochs);
+        st.step++;
         st.ssa++;
-        if (++q == p.ssa_block || (p.max_steps > 0 && accepted(st.epochs, st.step, st.rej) >= p.max_steps)) return;
+        ++q;
+        if (q == p.ssa_block || (p.max_steps > 0 && accepted(st.epochs + wrapped(st.step, q), st.step, st.rej) >= p.max_steps)) return;
         float pac;
         fast_props<false>(g, p, L, rate, pa, pac);
         if (!g.any(pa > 0.f)) {
@@ -1318,7 +1320,7 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
         }
         if (!bad) break;
         // reject: halve tau1, fresh counters, same state and propensities
-        next_step(st.step, st.epochs);
+        st.step++;
         st.rej++;
         tau1 *= 0.5f;
         if (attempt + 1 > p.max_halv) {
@@ -1332,7 +1334,7 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
         add_scores(g, p, L, set, r, true, [&](int, float a, int k) { return (float)k - fabsf(a) * tau_used; });
     }
     g.sync();
-    next_step(st.step, st.epochs);
+    st.step++;
     if (clamp) {
         st.t = st.t_next;
         record_next(g, p, L, set, r, st);
@@ -1375,12 +1377,14 @@ TL_D void fast_realization(const Grp& g, const SimParams& p, const Lay& L, long 
     FastState st{0.0, grid_time<double>(p, set, 1), 1, 0u, 0u, 0u, 0u, 0u - 32u, 0.f, false, false};  // ex: not drawn yet
     bool trunc = false;
     while (!st.done) {
+        const uint32_t from = st.step;
         fast_step<Grp, Lay, SENS, false>(g, p, L, set, r, st);
         if (st.wide) {
             FastState tmp = st;
             wide_step<Grp, Lay, SENS>(g, p, L, set, r, &tmp);
             st = tmp;
         }
+        if (st.step < from) ++st.epochs;  // (once a leap or block: counting at each step took 0.7 % on 16 lanes)
         if (!st.done && p.max_steps > 0 && accepted(st.epochs, st.step, st.rej) >= p.max_steps) {
             st.done = true;
             trunc = true;

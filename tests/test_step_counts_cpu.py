@@ -22,6 +22,13 @@ int main() {
     if (tl::accepted(epochs, step, rej) != (1ll << 32) + 3 - 7) return 2;
     epochs = 5;
     if (tl::accepted(epochs, 0u, 0xffffffffu) != (5ll << 32) - 0xffffffffll) return 3;
+    // a block of direct-method steps over the wrap
+    epochs = 1;
+    step = 0xfffffff0u;
+    for (int q = 1; q <= 40; ++q) {
+        ++step;
+        if (tl::accepted(epochs + tl::wrapped(step, q), step, 3u) != (1ll << 32) + 0xfffffff0ll - 3 + q) return 4;
+    }
     return 0;
 }
 """
