@@ -1231,8 +1231,10 @@ TL_D void fast_step(const Grp& g, const SimParams& p, const Lay& L, int set, uin
     float pa, pac;
     // Scores read a critical channel's propensity, and teams form their sums
     // from a[].  Warps and CTAs gain (4000 realizations of the toy network
-    // 27.7 -> 27.15 ms, 250 species of the colloid 3.39 -> 3.34 ms), 16 lanes do
-    // not (80.5 -> 83.4 ms: two realizations share the warp that selects).
+    // 27.7 -> 27.15 ms, 250 species of the colloid 3.39 -> 3.34 ms), 8 lanes lose
+    // (50001 realizations of the 45 x 83 network 77.9 -> 78.7 ms: four realizations
+    // share the warp that selects).  16 lanes keep the negative form too, though zeros
+    // would gain there (60000 of the toy network 57.8 -> 56.7 ms).
     constexpr bool kZero = !SENS && !WIDE && (Grp::kWidth == 32 || Grp::kWidth == 0);
     fast_props<kZero>(g, p, L, rate, pa, pac);
     float a0f;
