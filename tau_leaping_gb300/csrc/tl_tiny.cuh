@@ -132,7 +132,7 @@ TL_D void tiny_realization(const TinyGroup<W>& g, const SimParams& p, const uint
     tiny_record(g, p, L, set, r, 0);
     double t = 0.0, t_next = grid_time<double>(p, set, 1);
     int kpt = 1;
-    uint32_t step = 0, rej = 0, ssa = 0, epochs = 0, w_from = 0u - 32u;
+    uint32_t step = 0, rej = 0, ssa = 0, epochs = 0, last = 0, w_from = 0u - 32u;
     U4 w{0u, 0u, 0u, 0u};  // the lanes hold the scalar words of the steps from w_from
     float ex = 0.f;        // and their waiting times at unit rate
     int ssa_left = 0;
@@ -154,6 +154,8 @@ TL_D void tiny_realization(const TinyGroup<W>& g, const SimParams& p, const uint
         if (SENS && c > 0.f) score += term / c;
     };
     for (;;) {
+        epochs += wrapped_past(step, last);
+        last = step;
         if (p.max_steps > 0 && accepted(epochs, step, rej) >= p.max_steps) {
             trunc = true;
             break;
@@ -202,7 +204,7 @@ TL_D void tiny_realization(const TinyGroup<W>& g, const SimParams& p, const uint
             for (int q = 0; q < W; ++q) d = q == j ? L.v(q) : d;
             L.set(L.x + (Pop)d, p.nc);
             t = t_new;
-            next_step(step, epochs);
+            ++step;
             ++ssa;
             --ssa_left;
             continue;
@@ -245,7 +247,7 @@ TL_D void tiny_realization(const TinyGroup<W>& g, const SimParams& p, const uint
             }
             if (!g.any(nx < 0)) break;
             // reject: halve tau1, fresh counters, same state and propensities
-            next_step(step, epochs);
+            ++step;
             ++rej;
             tau1 *= 0.5f;
             if (attempt + 1 > p.max_halv) {
@@ -257,7 +259,7 @@ TL_D void tiny_realization(const TinyGroup<W>& g, const SimParams& p, const uint
         if (stop) break;
         add_score((float)k - fabsf(aj) * tauf);
         L.set((Pop)nx, p.nc);
-        next_step(step, epochs);
+        ++step;
         if (clamp) {
             t = t_next;
             record_next();
@@ -271,7 +273,7 @@ TL_D void tiny_realization(const TinyGroup<W>& g, const SimParams& p, const uint
     while (kpt <= p.n_int) tiny_record(g, p, L, set, r, kpt++);
     if (SENS && p.scores && channel) p.scores[realization_index(p, set, r) * p.M + g.lane] = score;
     if (g.lane == 0) {
-        const long long leaps = accepted(epochs, step, rej) - (long long)ssa;
+        const long long leaps = accepted(epochs + wrapped_past(step, last), step, rej) - (long long)ssa;
         if (leaps) atomicAdd(p.ctr + 1, (unsigned long long)leaps);
         if (ssa) atomicAdd(p.ctr + 2, (unsigned long long)ssa);
         if (rej) atomicAdd(p.ctr + 3, (unsigned long long)rej);

@@ -16,7 +16,8 @@ int main() {
     long long want = 0xfffffffdll - rej;
     for (int q = 0; q < 6; ++q) {
         if (tl::accepted(epochs, step, rej) != want + q) return 1;
-        tl::next_step(step, epochs);
+        const uint32_t from = step++;
+        epochs += tl::wrapped_past(step, from);
     }
     // right after a wrap, more rejections than the counter shows
     if (tl::accepted(epochs, step, rej) != (1ll << 32) + 3 - 7) return 2;
