@@ -471,7 +471,8 @@ struct LeapScale {
 };
 
 // Whether most draws of a leap have means of 10 and more (PTRS), by the first
-// leap from x0: the mean of channel j is a_j times the CGP bound or dt.
+// leap from x0 at the model's own rates: the mean of channel j is a_j times the CGP
+// bound or dt.
 static bool mostly_long_draws(const HostModel& h, const LeapScale& ls) {
     const int M = h.M, N = h.N;
     std::vector<double> a((size_t)M);
@@ -540,7 +541,9 @@ static long long thin_most_warps(const HostModel& h, const LeapScale& ls) {
 // alone, ms, W = 4 and 1: 48000 realizations to t = 0.01 1.83 and 2.10, t = 1 2.98 and
 // 3.58; 65536 2.56 and 2.13, 4.17 and 3.58; with scores 2.70 and 2.71, 4.34 and 4.36;
 // beside 4 x 700 toy realizations 6.63 and 6.41, 8.22 and 8.87.
-static long long thin_most_warps_batch(bool small_only, bool scores) { return small_only && !scores ? 48 : 56; }
+static long long thin_most_warps_batch(int size, bool small_only, bool scores) {
+    return size <= 4 && small_only && !scores ? 48 : 56;
+}
 
 // Four-warp teams for a warp-group ensemble of up to eight realizations an SM:
 // enough channels for 128 threads, and a chain of steps that sets the time.
@@ -1512,7 +1515,7 @@ static tl_status run_batch(tl_batch_item* items, int n, cudaStream_t st) {
         thin = 1;
         unit_lanes = 32;
         if (bmode != kModeGeneral) thin_plan(lane_size <= 4 ? 4 : 16, lane_total, sm_count(),
-                                             thin_most_warps_batch(small_only, bmode == kModeScores), thin, unit_lanes);
+                                             thin_most_warps_batch(lane_size, small_only, bmode == kModeScores), thin, unit_lanes);
         wslot = 0;
         for (int i = 0; i < n; ++i) {
             Job& J = jobs[(size_t)i];

@@ -28,10 +28,10 @@ def test_measured_mode_launches_the_plan_that_it_chose(n, bits):
 def test_measured_mode_is_no_slower_than_the_planned_launch():
     """Teams are planned, never asked for by a block: 152 toy realizations take
     9.8 ms on them and 10.7 ms on the fastest launch that a block asks for."""
-    m = Model.generate("toy")
     kw = dict(t_final=0.002, n=152, seed=3, tracked=[0])
-    planned = min(m.simulate(**kw).kernel_ms for _ in range(5))
-    measured = min(m.simulate(flags=_ffi.FLAG_AUTOTUNE_MEASURE, **kw).kernel_ms for _ in range(5))
+    models = [Model.generate("toy") for _ in range(3)]  # each handle measures for itself
+    planned = min(m.simulate(**kw).kernel_ms for m in models for _ in range(3))
+    measured = min(m.simulate(flags=_ffi.FLAG_AUTOTUNE_MEASURE, **kw).kernel_ms for m in models for _ in range(3))
     assert measured <= 1.05 * planned, (measured, planned)
 
 
